@@ -154,6 +154,15 @@ __device__ __forceinline__ uint64_t spread3(uint64_t v) {
     return v;
 }
 
+// spread3 of 10 bits in 32-bit arithmetic: the codes of up to 30 bits.
+__device__ __forceinline__ uint32_t spread3_10(uint32_t v) {
+    v = (v | (v << 16)) & 0x030000ffu;
+    v = (v | (v << 8)) & 0x0300f00fu;
+    v = (v | (v << 4)) & 0x030c30c3u;
+    v = (v | (v << 2)) & 0x09249249u;
+    return v;
+}
+
 // morton_encode's bit loop takes, for code bit b (b < depth), bit (b+off)/3
 // of the slice of axis (b+off+1) % 3.  With j = b + off, that is the
 // interleave I whose bit j is bit j/3 of axis (j+1) % 3 (y, z, x for
@@ -173,6 +182,14 @@ __device__ __forceinline__ uint32_t morton_code(const MortonParams& P, const flo
     }
     const int bits = (P.depth + 2) / 3;
     const uint32_t keep = (1u << bits) - 1u;
+    if (bits <= 10) {
+        // the 64-bit interleave is about half of k_morton_hist's instructions:
+        // without it the build of 17.7 M triangles takes 1.997 against 2.017 ms
+        // (1.24 M: no change, the kernel waits for its gathers there)
+        const uint32_t I = spread3_10(m[1] & keep) | (spread3_10(m[2] & keep) << 1) |
+                           (spread3_10(m[0] & keep) << 2);
+        return (I >> P.offset) & ((1u << P.depth) - 1u);
+    }
     const uint64_t I = spread3(m[1] & keep) | (spread3(m[2] & keep) << 1) |
                        (spread3(m[0] & keep) << 2);
     const uint64_t code = I >> P.offset;
