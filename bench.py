@@ -1040,7 +1040,7 @@ def run_gpu(args):
     # one also permutes), then the render (+ k_fb_copy when pooled)
     launches_per_frame = 6 + emit_levels + (2 if pooled else 1)
     build_roofline = {"kernels": "k_bounds + k_morton_hist + 4x k_onesweep + "
-                                 "k_emit_level0_permute + %dx k_emit_level" % (emit_levels - 1),
+                                 "k_emit_level0 + %dx k_emit_level" % (emit_levels - 1),
                       "bound": "hbm",
                       "achieved": build_gbs,
                       "peak": peak, "unit": "GB/s", "frac": build_gbs / peak,

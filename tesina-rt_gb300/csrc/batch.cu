@@ -32,14 +32,6 @@
 
 namespace cg = cooperative_groups;
 
-// The unpooled many-view kernel (the server's) with the two-phase
-// traversal (1) or the plain loop (0, measured faster there: 1047 against
-// 982 Mrays/s of served capacity); the pooled kernel always uses the
-// two-phase loop (4 % faster on the 64 soups).
-#ifndef RT_WW_SERVED
-#define RT_WW_SERVED 0
-#endif
-
 namespace rt {
 
 constexpr int kMaxBatchScenes = 1024;
@@ -94,7 +86,7 @@ __global__ void __launch_bounds__(SORT_THREADS, 4) k_batch_build(BatchBuildArgs 
 
     // ---- stage 0: initialise bounds, histograms, look-back, arrival flags ---
     for (uint32_t i = gtid; i < (uint32_t)nsc * 8; i += gthreads)
-        A.scenes[i >> 3].bounds[i & 7] = (i & 7) < 3 ? 0xffffffffu : 0u;
+        A.scenes[i >> 3].bounds[i & 7] = 0u;
     for (uint32_t i = gtid; i < (uint32_t)nsc * 1024; i += gthreads)
         A.scenes[i >> 10].hist[i & 1023] = 0;
     for (int sc = 0; sc < nsc; ++sc) {
@@ -139,15 +131,11 @@ __global__ void __launch_bounds__(SORT_THREADS, 4) k_batch_build(BatchBuildArgs 
                     a = fminf(a, s_red[k][tid]);
                     b = fmaxf(b, s_red[k][3 + tid]);
                 }
-                atomicMin(&A.scenes[s0].bounds[tid], f2o(a));
-                atomicMax(&A.scenes[s0].bounds[3 + tid], f2o(b));
+                bounds_add(A.scenes[s0].bounds, tid, a, b);
             }
             __syncthreads();
         } else if (ok) {   // a scene boundary inside the step: per-triangle atomics
-            for (int c = 0; c < 3; ++c) {
-                atomicMin(&A.scenes[s].bounds[c], f2o(lo[c]));
-                atomicMax(&A.scenes[s].bounds[3 + c], f2o(hi[c]));
-            }
+            for (int c = 0; c < 3; ++c) bounds_add(A.scenes[s].bounds, c, lo[c], hi[c]);
         }
     }
     grid.sync();
@@ -247,32 +235,35 @@ __global__ void __launch_bounds__(SORT_THREADS, 4) k_batch_build(BatchBuildArgs 
 // One level of the emit over every scene that still has blocks at it: the
 // one-scene emit's blocks (emit_level, the same items, buffers and leave
 // rule), with block j of the launch taken by the scene whose range of the
-// level's blocks holds j.  The C == EMIT_C0 instance is level 0.
-static_assert(EMIT_C0 != EMIT_C1, "k_batch_emit tells level 0 by its block size");
-template <int C>
-__global__ void __launch_bounds__(C, C == EMIT_C0 ? RT_EMIT_MINB0 : RT_EMIT_MINB1) k_batch_emit(
+// level's blocks holds j.  T: EMIT_C0 threads for level 0, else
+// EMIT_T_WIDE, the scenes' levels being wide together.
+static_assert(EMIT_C0 != EMIT_T_WIDE, "k_batch_emit tells level 0 by its block size");
+template <int T>
+__global__ void __launch_bounds__(T, T == EMIT_C0 ? RT_EMIT_MINB0 : 2) k_batch_emit(
     const BatchScene* __restrict__ scenes, int count, int level, const uint32_t* __restrict__ off,
     uint32_t* __restrict__ status) {
     extern __shared__ __align__(16) unsigned char emit_smem[];
-    auto& S = *reinterpret_cast<EmitSmem<C>*>(emit_smem);
+    constexpr bool LEVEL0 = T == EMIT_C0;
+    constexpr int C = LEVEL0 ? EMIT_C0 : EMIT_C1;
+    auto& S = *reinterpret_cast<EmitSmem<C, T>*>(emit_smem);
     const int s = find_segment(off, count, blockIdx.x);
     const BatchScene& B = scenes[s];
     const uint32_t job = blockIdx.x - off[s];
     const EmitBuffers E = emit_buffers(B.n, B.emit);
     uint32_t n_in = emit_blocks0(B.n);   // blocks of the level below
-    if constexpr (C == EMIT_C0) {
+    if constexpr (LEVEL0) {
         // level 0 permutes its triangles into sorted order and joins them
-        // with their AABBs in registers (as k_emit_level0_permute)
+        // with their AABBs in registers (as k_emit_level0)
         const PermuteIO P{B.vals_sorted, B.idx_in,  B.map_in,   B.orig_in, B.pos,
                           B.idx_out,     B.map_out, B.orig_out, B.tris};
-        emit_level<C, true>(S, job, B.n, B.keys_sorted, nullptr, nullptr, nullptr, 0, E.items[0],
-                            E.counts[0], B.nodes, B.min_leaf, emit_leave(0, n_in), B.hdr, status,
-                            P);
+        emit_level<C, T, EMIT_PERMUTE>(S, job, B.n, B.keys_sorted, nullptr, nullptr, 0, E.items[0],
+                                    E.counts[0], B.nodes, B.tris, B.min_leaf, emit_leave(0, n_in),
+                                    B.hdr, status, P);
     } else {
         for (int l = 2; l <= level; ++l) n_in = emit_next_level(n_in);
         const int src = (level - 1) & 1;
-        emit_level<C>(S, job, B.n, B.keys_sorted, nullptr, E.items[src], E.counts[src], n_in,
-                      E.items[src ^ 1], E.counts[src ^ 1], B.nodes, B.min_leaf,
+        emit_level<C, T>(S, job, B.n, B.keys_sorted, E.items[src], E.counts[src], n_in,
+                      E.items[src ^ 1], E.counts[src ^ 1], B.nodes, B.tris, B.min_leaf,
                       emit_leave(level, emit_next_level(n_in)), B.hdr, status);
     }
 }
@@ -309,7 +300,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch(BatchRenderArgs 
                 int x, y;
                 pixel_of(warp_tile_order(local, V.width, V.height), V.width, V.height, 32, x, y);
                 const BvhHeader H = *V.scene.hdr;
-                const PixelResult pr = render_pixel<RT_WW_SERVED, REFR>(
+                const PixelResult pr = render_pixel<REFR>(
                     V.scene, H, *V.lights, V.cam, x, y, V.width, V.height, V.max_bounces, A.status);
                 ++n_prim;
                 n_sec += pr.secondary;
@@ -432,7 +423,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
             const BatchView& V = A.views[v];
             const BvhHeader H = *V.scene.hdr;
             const TRay r = make_tray(o, d, mk3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z), tmin);
-            hit = closest_hit_ww(V.scene, H, r, tmax, A.status);
+            hit = closest_hit(V.scene, H, r, tmax, A.status);
             hit_ok = hit.id >= 0;
         }
         const unsigned hm = __ballot_sync(0xffffffffu, hit_ok);
@@ -499,7 +490,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
             const BatchView& V = A.views[Q.hv[lo]];
             const BvhHeader H = *V.scene.hdr;
             const f3 p = mk3(Q.hp[0][lo], Q.hp[1][lo], Q.hp[2][lo]);
-            if (occluded<true>(V.scene, H, V.lights->light[l], p, A.status))
+            if (occluded(V.scene, H, V.lights->light[l], p, A.status))
                 atomicOr(&Q.hmask[lo], 1u << l);
         }
         __syncwarp();
@@ -698,11 +689,11 @@ cudaError_t launch_batch_build(const BatchBuildArgs& a, int grid, cudaStream_t s
         std::lock_guard<std::mutex> lk(mu);
         if (dev >= 64 || !((done >> dev) & 1)) {
             e = cudaFuncSetAttribute(k_batch_emit<EMIT_C0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sizeof(EmitSmem<EMIT_C0>));
+                                     (int)sizeof(EmitSmem<EMIT_C0, EMIT_C0>));
             if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(k_batch_emit<EMIT_C1>,
+                e = cudaFuncSetAttribute(k_batch_emit<EMIT_T_WIDE>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)sizeof(EmitSmem<EMIT_C1>));
+                                         (int)sizeof(EmitSmem<EMIT_C1, EMIT_T_WIDE>));
             if (e != cudaSuccess) return e;
             if (dev < 64) done |= 1ull << dev;
         }
@@ -711,10 +702,10 @@ cudaError_t launch_batch_build(const BatchBuildArgs& a, int grid, cudaStream_t s
         if (a.emit_jobs[L] == 0) continue;
         const uint32_t* off = a.emit_off + (size_t)L * (a.count + 1);
         if (L == 0)
-            k_batch_emit<EMIT_C0><<<a.emit_jobs[L], EMIT_C0, sizeof(EmitSmem<EMIT_C0>), s>>>(
+            k_batch_emit<EMIT_C0><<<a.emit_jobs[L], EMIT_C0, sizeof(EmitSmem<EMIT_C0, EMIT_C0>), s>>>(
                 a.scenes, a.count, L, off, a.status);
         else
-            k_batch_emit<EMIT_C1><<<a.emit_jobs[L], EMIT_C1, sizeof(EmitSmem<EMIT_C1>), s>>>(
+            k_batch_emit<EMIT_T_WIDE><<<a.emit_jobs[L], EMIT_T_WIDE, sizeof(EmitSmem<EMIT_C1, EMIT_T_WIDE>), s>>>(
                 a.scenes, a.count, L, off, a.status);
     }
     if (a.stage_ns) k_batch_stamp<<<1, 1, 0, s>>>(a.stage_ns + 6);

@@ -101,8 +101,8 @@ std::vector<rt::BatchScene> scene_table(rt_batch* b) {
         B.map_out = s->d_map[s->cur ^ 1];
         B.orig_out = s->d_orig[s->cur ^ 1];
         B.keys_unsorted = s->d_keys_unsorted;
-        B.keys1 = s->d_keys1;
-        B.vals1 = s->d_vals1;
+        B.keys1 = rt::sort_keys1(s->d_tris);
+        B.vals1 = rt::sort_vals1(s->d_tris, s->N);
         B.keys_sorted = s->d_keys_sorted;
         B.vals_sorted = s->d_vals_sorted;
         B.tris = s->d_tris;

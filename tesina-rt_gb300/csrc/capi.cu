@@ -93,13 +93,9 @@ namespace {
 
 void free_build(rt_scene* s) {
     sfree(s, s->d_keys_unsorted);
-    sfree(s, s->d_vals0);
-    sfree(s, s->d_keys1);
-    sfree(s, s->d_vals1);
     sfree(s, s->d_keys_sorted);
     sfree(s, s->d_vals_sorted);
     sfree(s, s->d_tris);
-    sfree(s, s->d_leafbox);
     sfree(s, s->d_nodes);
     sfree(s, s->d_hdr);
     sfree(s, s->d_scratch);
@@ -230,11 +226,9 @@ int32_t scene_ensure_build(rt_scene* s) {
     if (s->buildN >= n && s->scratch_bytes >= need_scratch && s->d_hdr) return RT_OK;
     free_build(s);
     const size_t nn = n > 1 ? n - 1 : 1;
-    if (salloc_n(s, &s->d_keys_unsorted, n) || salloc_n(s, &s->d_vals0, n) ||
-        salloc_n(s, &s->d_keys1, n) || salloc_n(s, &s->d_vals1, n) ||
-        salloc_n(s, &s->d_keys_sorted, n) || salloc_n(s, &s->d_vals_sorted, n) ||
-        salloc_n(s, &s->d_tris, 3 * (size_t)n) || salloc_n(s, &s->d_leafbox, 2 * (size_t)n) ||
-        salloc_n(s, &s->d_nodes, 4 * nn) || salloc_n(s, &s->d_hdr, 1) || salloc(s, &s->d_scratch, need_scratch)) {
+    if (salloc_n(s, &s->d_keys_unsorted, n) || salloc_n(s, &s->d_keys_sorted, n) ||
+        salloc_n(s, &s->d_vals_sorted, n) || salloc_n(s, &s->d_tris, 3 * (size_t)n) ||
+        salloc_n(s, &s->d_nodes, 8 * nn) || salloc_n(s, &s->d_hdr, 1) || salloc(s, &s->d_scratch, need_scratch)) {
         cudaGetLastError();
         free_build(s);
         return fail(RT_ERR_OOM, "device allocation of LBVH buffers for %u triangles failed", n);
@@ -242,6 +236,12 @@ int32_t scene_ensure_build(rt_scene* s) {
     s->buildN = n;
     s->scratch_bytes = need_scratch;
     return RT_OK;
+}
+
+void scene_release_build(rt_scene* s) {
+    sfree(s, s->d_scratch);
+    sfree(s, s->d_keys_unsorted);
+    s->scratch_bytes = 0;
 }
 
 SceneView scene_view(const rt_scene* s) {
@@ -728,13 +728,11 @@ static rt::LbvhArgs lbvh_args(rt_ctx* c, rt_scene* s) {
     a.map_out = s->d_map[s->cur ^ 1];
     a.orig_out = s->d_orig[s->cur ^ 1];
     a.keys_unsorted = s->d_keys_unsorted;
-    a.vals0 = s->d_vals0;
-    a.keys1 = s->d_keys1;
-    a.vals1 = s->d_vals1;
+    a.keys1 = rt::sort_keys1(s->d_tris);
+    a.vals1 = rt::sort_vals1(s->d_tris, s->N);
     a.keys_sorted = s->d_keys_sorted;
     a.vals_sorted = s->d_vals_sorted;
     a.tris = s->d_tris;
-    a.leafbox = s->d_leafbox;
     a.nodes = s->d_nodes;
     a.hdr = s->d_hdr;
     a.scratch = s->d_scratch;
@@ -797,7 +795,9 @@ int32_t rt_bvh_build_sah(rt_ctx* c, rt_scene* s, rt_stream stream) {
         CU(cudaMemcpyAsync(s->d_nodes, t.nodes.data(), sizeof(float4) * t.nodes.size(),
                            cudaMemcpyHostToDevice, cs));
     CU(cudaMemcpyAsync(s->d_hdr, &t.hdr, sizeof(t.hdr), cudaMemcpyHostToDevice, cs));
-    CU(rt::lbvh_permute(a, s->d_vals_sorted, cs));
+    uint8_t* more = reinterpret_cast<uint8_t*>(s->d_scratch);
+    CU(cudaMemcpyAsync(more, t.more.data(), s->N, cudaMemcpyHostToDevice, cs));
+    CU(rt::lbvh_permute(a, s->d_vals_sorted, more, cs));
     CU(cudaEventRecord(s->ev1, cs));
     CU(cudaStreamSynchronize(cs));   // the host tree lives until its copies are done
     CU(scene_write_end(s, cs));
@@ -839,8 +839,15 @@ int32_t rt_bvh_export(rt_ctx* c, rt_scene* s, rt_canon_node* out, uint32_t cap, 
     rt::BvhHeader h;
     CU(cudaMemcpy(&h, s->d_hdr, sizeof(h), cudaMemcpyDeviceToHost));
     const size_t nn = s->N > 1 ? s->N - 1 : 0;
-    std::vector<float4> nodes(4 * nn + 4);
-    if (nn) CU(cudaMemcpy(nodes.data(), s->d_nodes, sizeof(float4) * 4 * nn, cudaMemcpyDeviceToHost));
+    std::vector<float4> nodes(8 * nn + 8);
+    if (nn) CU(cudaMemcpy(nodes.data(), s->d_nodes, sizeof(float4) * 8 * nn, cudaMemcpyDeviceToHost));
+    // the device's minima and maxima: -0 below +0, a NaN operand dropped
+    auto least = [](float a, float b) {
+        return a < b || b != b || (a == b && std::signbit(a)) ? a : b;
+    };
+    auto most = [](float a, float b) {
+        return a > b || b != b || (a == b && !std::signbit(a)) ? a : b;
+    };
     std::vector<rt_canon_node> res;
     res.reserve(2 * (size_t)s->N);
     struct Item {
@@ -873,10 +880,19 @@ int32_t rt_bvh_export(rt_ctx* c, rt_scene* s, rt_canon_node* out, uint32_t cap, 
         } else {
             if (it.ref < 0 || (size_t)it.ref >= nn)
                 return fail(RT_ERR, "rt_bvh_export: corrupt node reference %d", it.ref);
-            const float4* q = &nodes[4 * (size_t)it.ref];
-            const int* qi = reinterpret_cast<const int*>(&q[3]);
-            Item L{qi[0], qi[2], it.depth + 1, {q[0].x, q[0].y, q[0].z}, {q[0].w, q[1].x, q[1].y}, me};
-            Item R{qi[1], qi[3], it.depth + 1, {q[1].z, q[1].w, q[2].x}, {q[2].y, q[2].z, q[2].w}, me};
+            // a pair of slots: the child itself, a leaf, or the two halves of
+            // an interior child
+            rt::Slot q[4];
+            memcpy(q, &nodes[8 * (size_t)it.ref], sizeof q);
+            auto child = [&](const rt::Slot& x, const rt::Slot& y) {
+                if (rt::slot_pair_is_leaf(y))
+                    return Item{~x.code, x.aux, it.depth + 1, {x.lox, x.loy, x.loz},
+                                {x.hix, x.hiy, x.hiz}, me};
+                return Item{rt::slot_pair_node(x), 0, it.depth + 1,
+                            {least(x.lox, y.lox), least(x.loy, y.loy), least(x.loz, y.loz)},
+                            {most(x.hix, y.hix), most(x.hiy, y.hiy), most(x.hiz, y.hiz)}, me};
+            };
+            const Item L = child(q[0], q[1]), R = child(q[2], q[3]);
             todo.push_back(R);
             todo.push_back(L);
         }

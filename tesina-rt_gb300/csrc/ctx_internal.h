@@ -73,13 +73,9 @@ struct rt_scene {
     rt_lights lights;
     // build products
     uint32_t* d_keys_unsorted = nullptr;
-    uint32_t* d_vals0 = nullptr;
-    uint32_t* d_keys1 = nullptr;
-    uint32_t* d_vals1 = nullptr;
     uint32_t* d_keys_sorted = nullptr;
     uint32_t* d_vals_sorted = nullptr;
     float4* d_tris = nullptr;
-    float4* d_leafbox = nullptr;
     float4* d_nodes = nullptr;
     rt::BvhHeader* d_hdr = nullptr;
     uint32_t* d_scratch = nullptr;
@@ -113,6 +109,9 @@ namespace rt {
 int32_t set_error(int32_t code, const char* fmt, ...);
 // Allocates (or keeps) the build buffers for the scene's triangle count.
 int32_t scene_ensure_build(rt_scene* s);
+// Frees, in the order of the scene's pool stream, what only a build uses
+// (served scenes are built once; another build would allocate it again).
+void scene_release_build(rt_scene* s);
 // Device view of the scene's current (sorted) order.
 SceneView scene_view(const rt_scene* s);
 // The persistent-kernel work counter for launches on stream s (nullptr if it

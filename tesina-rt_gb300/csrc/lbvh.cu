@@ -10,11 +10,11 @@
 //                   ballot ranking and decoupled look-back with a
 //                   bounded spin (replaces the bitonic network of
 //                   bvh-builder-sort.cl and bvh-builder.cpp:361-454);
-//   k_emit_level0_permute
-//                   rearrange_indices / rearrange_map (:49-72) and the
+//   k_emit_level0   rearrange_indices / rearrange_map (:49-72) and the
 //                   triangle records used by traversal, fused with level 0 of
 //                   the emit, which joins the triangles with their AABBs
-//                   still in registers;
+//                   still in registers; a refit's instance makes the records
+//                   and AABBs from the moved vertices;
 //   k_emit_level    bottom-up build of the radix tree (Apetrei's
 //                   agglomerative formulation of Karras' tree), collapsed to
 //                   the reference's leaf rule (find_middle, :484-552), with
@@ -22,9 +22,7 @@
 //                   computed on the way up; a few launches whose warps join
 //                   runs of 32 items (level 0 over 512 triangles per block,
 //                   then over what 8 blocks left).
-//   k_permute       the permutation alone, storing leaf AABBs (the stage-wise
-//                   entry point); k_refit_leaves the leaf AABBs of the
-//                   existing order (refit).
+//   k_permute       the permutation alone (under a tree built on the host).
 // The per-element work lives in lbvh_dev.cuh, shared with the many-scene
 // persistent build of batch.cu.
 #include <cuda_runtime.h>
@@ -35,17 +33,6 @@
 #include "lbvh_dev.cuh"
 #include "rt_internal.cuh"
 
-// The full build's level-0 emit performs the permutation itself (1), or a
-// separate k_permute stores the leaf AABBs for it (0).
-#ifndef RT_EMIT_PERMUTE
-#define RT_EMIT_PERMUTE 1
-#endif
-// The first radix pass makes the values 0..n-1 itself (1) instead of reading
-// them from a buffer k_morton_hist fills (0).
-#ifndef RT_SORT_IOTA
-#define RT_SORT_IOTA 1
-#endif
-constexpr bool kIotaVals = RT_SORT_IOTA != 0;
 // Digit width of the build's radix passes: 8 (four passes for 30-bit keys)
 // or 10 (three).  The pair sort entry points always use 8.
 #ifndef RT_SORT_BITS
@@ -73,7 +60,7 @@ __device__ __forceinline__ void pdl_enter() {
 
 template <typename... KArgs, typename... Args>
 static cudaError_t launch_dep(void (*kern)(KArgs...), unsigned grid, unsigned block, size_t smem,
-                              cudaStream_t s, Args... args) {
+                              cudaStream_t s, bool dependent, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
@@ -83,14 +70,18 @@ static cudaError_t launch_dep(void (*kern)(KArgs...), unsigned grid, unsigned bl
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = dependent ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
 __global__ void __launch_bounds__(256) k_bounds(const float4* __restrict__ pos,
                                                 const uint32_t* __restrict__ idx, uint32_t n,
-                                                uint32_t* __restrict__ bounds) {
+                                                uint32_t* __restrict__ bounds,
+                                                uint4* __restrict__ clear, uint32_t clear_n) {
     pdl_enter();
+    // the later kernels' counters are cleared here, beside the gathers
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < clear_n; i += gridDim.x * blockDim.x)
+        clear[i] = make_uint4(0u, 0u, 0u, 0u);
     float lo[3] = {1e37f, 1e37f, 1e37f}, hi[3] = {-1e37f, -1e37f, -1e37f};
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         float tl[3], th[3];
@@ -123,8 +114,7 @@ __global__ void __launch_bounds__(256) k_bounds(const float4* __restrict__ pos,
             a = fminf(a, s[k][c]);
             b = fmaxf(b, s[k][3 + c]);
         }
-        atomicMin(&bounds[c], f2o(a));
-        atomicMax(&bounds[3 + c], f2o(b));
+        bounds_add(bounds, c, a, b);
     }
 }
 
@@ -132,7 +122,6 @@ __global__ void __launch_bounds__(256) k_morton_hist(const float4* __restrict__ 
                                                      const uint32_t* __restrict__ idx, uint32_t n,
                                                      const uint32_t* __restrict__ bounds, int depth,
                                                      int passes, uint32_t* __restrict__ keys,
-                                                     uint32_t* __restrict__ vals,
                                                      uint32_t* __restrict__ hist) {
     pdl_enter();
     __shared__ uint32_t sh[kMaxBuildPasses][kBuildRadix];
@@ -144,7 +133,6 @@ __global__ void __launch_bounds__(256) k_morton_hist(const float4* __restrict__ 
         tri_aabb(pos, idx, i, lo, hi);
         const uint32_t code = morton_code(P, lo, hi);
         keys[i] = code;
-        if (vals) vals[i] = i;
         for (int p = 0; p < passes; ++p)
             atomicAdd(&sh[p][(code >> (kBuildBits * p)) & (uint32_t)(kBuildRadix - 1)], 1u);
     }
@@ -215,61 +203,45 @@ __global__ void __launch_bounds__(SORT_THREADS, 1) k_onesweep_wait_probe(
                                                status);
 }
 
+// The permutation of a tree built on the host, whose leaf marks (1: the next
+// triangle is in the same leaf) come from there too.
 __global__ void __launch_bounds__(256) k_permute(uint32_t n, PermuteIO P,
-                                                  float4* __restrict__ leafbox) {
-    pdl_enter();
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        permute_one(i, P, leafbox);
-}
-
-// Per-triangle AABBs of the current vertex positions in the existing sorted
-// order (refit_lbvh, bvh-builder.cpp:743-790) plus fresh triangle records.
-__global__ void __launch_bounds__(256) k_refit_leaves(uint32_t n, const uint32_t* __restrict__ idx,
-                                                      const float4* __restrict__ pos,
-                                                      float4* __restrict__ tris,
-                                                      float4* __restrict__ leafbox) {
+                                                  const uint8_t* __restrict__ more) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t a = __ldg(&idx[3 * (size_t)i]), b = __ldg(&idx[3 * (size_t)i + 1]),
-                       c = __ldg(&idx[3 * (size_t)i + 2]);
-        const float4 p0 = __ldg(&pos[a]), p1 = __ldg(&pos[b]), p2 = __ldg(&pos[c]);
-        tris[3 * (size_t)i] = make_float4(p0.x, p0.y, p0.z, 0.f);
-        tris[3 * (size_t)i + 1] = make_float4(p1.x - p0.x, p1.y - p0.y, p1.z - p0.z, 0.f);
-        tris[3 * (size_t)i + 2] = make_float4(p2.x - p0.x, p2.y - p0.y, p2.z - p0.z, 0.f);
-        float lo[3], hi[3];
-        tri_aabb(pos, idx, i, lo, hi);
-        leafbox[2 * (size_t)i] = make_float4(lo[0], lo[1], lo[2], 0.f);
-        leafbox[2 * (size_t)i + 1] = make_float4(hi[0], hi[1], hi[2], 0.f);
+        float4 lo, hi;
+        permute_tri(i, P, lo, hi);
+        if (more[i]) P.tris[3 * (size_t)i].w = 1.0f;
     }
 }
 
-// One level of the emit (emit_level), one block per run of items; blocks
-// are kept to a register budget that lets RT_EMIT_MINB0 (level 0) or
-// RT_EMIT_MINB1 (above) of them share an SM.
-template <int C>
-__global__ void __launch_bounds__(C, C == EMIT_C0 ? RT_EMIT_MINB0 : RT_EMIT_MINB1) k_emit_level(
-    uint32_t n, const uint32_t* __restrict__ skeys, const float4* __restrict__ leafbox,
-    const EmitItem* __restrict__ in, const uint32_t* __restrict__ in_count, uint32_t n_in,
-    EmitItem* __restrict__ out, uint32_t* __restrict__ out_count, float4* __restrict__ nodes,
+// One level of the emit above level 0 (emit_level), one block of T threads per
+// EMIT_GROUP blocks of the level below.
+template <int T>
+__global__ void __launch_bounds__(T, T == EMIT_T_WIDE ? 2 : 1) k_emit_level(
+    uint32_t n, const uint32_t* __restrict__ skeys, const EmitItem* __restrict__ in,
+    const uint32_t* __restrict__ in_count, uint32_t n_in, EmitItem* __restrict__ out,
+    uint32_t* __restrict__ out_count, float4* __restrict__ nodes, float4* __restrict__ tris,
     int min_leaf, uint32_t leave, BvhHeader* __restrict__ hdr, uint32_t* __restrict__ status) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char emit_smem[];
-    auto& S = *reinterpret_cast<EmitSmem<C>*>(emit_smem);
-    emit_level<C>(S, blockIdx.x, n, skeys, leafbox, in, in_count, n_in, out, out_count, nodes,
-                  min_leaf, leave, hdr, status);
+    auto& S = *reinterpret_cast<EmitSmem<EMIT_C1, T>*>(emit_smem);
+    emit_level<EMIT_C1, T>(S, blockIdx.x, n, skeys, in, in_count, n_in, out, out_count, nodes, tris,
+                        min_leaf, leave, hdr, status);
 }
 
-// Level 0 of a full build: each block first permutes its own triangles
-// (index buffer, material map, upload ids, triangle records) and joins them
-// with their boxes still in registers, so no leaf AABB goes through memory.
-__global__ void __launch_bounds__(EMIT_C0, RT_EMIT_MINB0) k_emit_level0_permute(
+// Level 0: each block first makes its own triangles' records (permuting
+// index buffer, material map and upload ids in a build) and joins them with
+// their boxes still in registers, so no leaf AABB goes through memory.
+template <EmitSource SRC>
+__global__ void __launch_bounds__(EMIT_C0, RT_EMIT_MINB0) k_emit_level0(
     uint32_t n, const uint32_t* __restrict__ skeys, PermuteIO P, EmitItem* __restrict__ out,
     uint32_t* __restrict__ out_count, float4* __restrict__ nodes, int min_leaf, uint32_t leave,
     BvhHeader* __restrict__ hdr, uint32_t* __restrict__ status) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char emit_smem[];
-    auto& S = *reinterpret_cast<EmitSmem<EMIT_C0>*>(emit_smem);
-    emit_level<EMIT_C0, true>(S, blockIdx.x, n, skeys, nullptr, nullptr, nullptr, 0, out,
-                              out_count, nodes, min_leaf, leave, hdr, status, P);
+    auto& S = *reinterpret_cast<EmitSmem<EMIT_C0, EMIT_C0>*>(emit_smem);
+    emit_level<EMIT_C0, EMIT_C0, SRC>(S, blockIdx.x, n, skeys, nullptr, nullptr, 0, out, out_count, nodes,
+                             P.tris, min_leaf, leave, hdr, status, P);
 }
 
 static size_t sort_scratch_bytes(uint32_t n, int passes) {
@@ -282,9 +254,9 @@ static size_t emit_scratch_bytes(uint32_t n) { return emit_buffers_bytes(n); }
 
 // The emit's levels: level 0 over triangles, then levels over the items left
 // by EMIT_GROUP blocks each until a single block reaches the root.  Item
-// buffers alternate: A holds level 0, 2, ... and B level 1, 3, ....  With
-// `perm`, level 0 also performs the permutation (k_emit_level0_permute);
-// without, it reads the leaf AABBs a previous launch stored.
+// buffers alternate: A holds level 0, 2, ... and B level 1, 3, ....  Level 0
+// performs the permutation `perm` (SRC = EMIT_PERMUTE) or the refit of the
+// triangles in their order.
 // The shared-memory opt-ins of the kernels with dynamic shared memory (a
 // property of the kernel on each device), once per device.
 static cudaError_t setup_kernels() {
@@ -299,9 +271,10 @@ static cudaError_t setup_kernels() {
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     };
-    opt_in((const void*)k_emit_level<EMIT_C0>, sizeof(EmitSmem<EMIT_C0>));
-    opt_in((const void*)k_emit_level0_permute, sizeof(EmitSmem<EMIT_C0>));
-    opt_in((const void*)k_emit_level<EMIT_C1>, sizeof(EmitSmem<EMIT_C1>));
+    opt_in((const void*)k_emit_level0<EMIT_PERMUTE>, sizeof(EmitSmem<EMIT_C0, EMIT_C0>));
+    opt_in((const void*)k_emit_level0<EMIT_REFIT>, sizeof(EmitSmem<EMIT_C0, EMIT_C0>));
+    opt_in((const void*)k_emit_level<EMIT_T_WIDE>, sizeof(EmitSmem<EMIT_C1, EMIT_T_WIDE>));
+    opt_in((const void*)k_emit_level<EMIT_T_NARROW>, sizeof(EmitSmem<EMIT_C1, EMIT_T_NARROW>));
     opt_in((const void*)k_onesweep<8, kOneWaveMinB>, onesweep_smem<8>());
     opt_in((const void*)k_onesweep<8, RT_SORT_MINB>, onesweep_smem<8>());
     opt_in((const void*)k_onesweep<kBuildBits, kOneWaveMinB>, onesweep_smem<kBuildBits>());
@@ -311,30 +284,31 @@ static cudaError_t setup_kernels() {
     return cudaSuccess;
 }
 
-static cudaError_t launch_emit(const LbvhArgs& a, uint8_t* emit_scratch, cudaStream_t s,
-                               const PermuteIO* perm = nullptr) {
+template <EmitSource SRC>
+static cudaError_t launch_emit(const LbvhArgs& a, uint8_t* emit_scratch, const PermuteIO& perm,
+                               cudaStream_t s) {
     const uint32_t n = a.n;
     if (cudaError_t e0 = setup_kernels()) return e0;
     const uint32_t nb0 = emit_blocks0(n);
     const EmitBuffers B = emit_buffers(n, emit_scratch);
-    cudaError_t e =
-        perm ? launch_dep(k_emit_level0_permute, nb0, EMIT_C0, sizeof(EmitSmem<EMIT_C0>), s, n,
-                          (const uint32_t*)a.keys_sorted, *perm, B.items[0], B.counts[0], a.nodes,
-                          a.min_leaf, emit_leave(0, nb0), a.hdr, a.status)
-             : launch_dep(k_emit_level<EMIT_C0>, nb0, EMIT_C0, sizeof(EmitSmem<EMIT_C0>), s, n,
-                          (const uint32_t*)a.keys_sorted, (const float4*)a.leafbox,
-                          (const EmitItem*)nullptr, (const uint32_t*)nullptr, 0u, B.items[0],
-                          B.counts[0], a.nodes, a.min_leaf, emit_leave(0, nb0), a.hdr, a.status);
+    // a refit starts here, after whatever moved the vertices: an ordinary launch
+    cudaError_t e = launch_dep(k_emit_level0<SRC>, nb0, EMIT_C0, sizeof(EmitSmem<EMIT_C0, EMIT_C0>),
+                               s, SRC == EMIT_PERMUTE, n, (const uint32_t*)a.keys_sorted, perm,
+                               B.items[0], B.counts[0], a.nodes, a.min_leaf, emit_leave(0, nb0),
+                               a.hdr, a.status);
     if (e) return e;
     uint32_t n_in = nb0;
     int src = 0;
     while (n_in > 1) {
         const uint32_t g = emit_next_level(n_in);
-        e = launch_dep(k_emit_level<EMIT_C1>, g, EMIT_C1, sizeof(EmitSmem<EMIT_C1>), s, n,
-                       (const uint32_t*)a.keys_sorted, (const float4*)a.leafbox,
-                       (const EmitItem*)B.items[src], (const uint32_t*)B.counts[src], n_in,
-                       B.items[src ^ 1], B.counts[src ^ 1], a.nodes, a.min_leaf, emit_leave(1, g),
-                       a.hdr, a.status);
+        const bool wide = g > (uint32_t)a.num_sms;
+        e = launch_dep(wide ? k_emit_level<EMIT_T_WIDE> : k_emit_level<EMIT_T_NARROW>, g,
+                       wide ? EMIT_T_WIDE : EMIT_T_NARROW,
+                       wide ? sizeof(EmitSmem<EMIT_C1, EMIT_T_WIDE>)
+                            : sizeof(EmitSmem<EMIT_C1, EMIT_T_NARROW>),
+                       s, true, n, (const uint32_t*)a.keys_sorted, (const EmitItem*)B.items[src],
+                       (const uint32_t*)B.counts[src], n_in, B.items[src ^ 1], B.counts[src ^ 1],
+                       a.nodes, a.tris, a.min_leaf, emit_leave(1, g), a.hdr, a.status);
         if (e) return e;
         n_in = g;
         src ^= 1;
@@ -371,25 +345,25 @@ cudaError_t lbvh_build(const LbvhArgs& a, cudaStream_t s) {
     uint32_t* lookback = tile_ctr + 4;
     cudaError_t e = setup_kernels();
     if (e) return e;
-    e = cudaMemsetAsync(a.scratch, 0, sort_scratch_bytes(n, passes), s);
+    e = cudaMemsetAsync(bounds, 0, 8 * sizeof(uint32_t), s);
     if (e) return e;
-    // bounds init: lo = ordered(+big) via 0xFF.. (max), hi = 0 (min)
-    e = cudaMemsetAsync(bounds, 0xff, 3 * sizeof(uint32_t), s);
-    if (e) return e;
+    static_assert((kMaxBuildPasses * kBuildRadix + 4) % 4 == 0 && kBuildRadix % 4 == 0, "whole uint4");
+    const size_t clear = (kMaxBuildPasses * kBuildRadix + 4 + (size_t)passes * tiles * kBuildRadix) / 4;
     const int sms = a.num_sms;
-    k_bounds<<<grid_for(n, 256, sms * 8), 256, 0, s>>>(a.pos, a.idx_in, n, bounds);
-    e = launch_dep(k_morton_hist, grid_for(n, 256, sms * 8), 256, 0, s, a.pos, a.idx_in, n,
-                   bounds, a.depth, passes, a.keys_unsorted, kIotaVals ? nullptr : a.vals0, hist);
+    k_bounds<<<grid_for(n, 256, sms * 8), 256, 0, s>>>(a.pos, a.idx_in, n, bounds,
+                                                       reinterpret_cast<uint4*>(hist), (uint32_t)clear);
+    e = launch_dep(k_morton_hist, grid_for(n, 256, sms * 8), 256, 0, s, true, a.pos, a.idx_in, n,
+                   bounds, a.depth, passes, a.keys_unsorted, hist);
     if (e) return e;
     const uint32_t* kin = a.keys_unsorted;
-    const uint32_t* vin = kIotaVals ? nullptr : a.vals0;
+    const uint32_t* vin = nullptr;   // the first pass makes the values 0..n-1 itself
     uint32_t* kbuf[2] = {a.keys1, a.keys_sorted};
     uint32_t* vbuf[2] = {a.vals1, a.vals_sorted};
     for (int p = 0; p < passes; ++p) {
         // the last pass always lands in keys_sorted / vals_sorted
         const int dst = ((passes - 1 - p) & 1) ? 0 : 1;
         e = launch_dep(onesweep_kernel<kBuildBits>(tiles, sms), (unsigned)tiles, SORT_THREADS,
-                       onesweep_smem<kBuildBits>(), s, kin, vin, kbuf[dst], vbuf[dst], n,
+                       onesweep_smem<kBuildBits>(), s, true, kin, vin, kbuf[dst], vbuf[dst], n,
                        kBuildBits * p, (const uint32_t*)(hist + kBuildRadix * p),
                        lookback + (size_t)p * tiles * kBuildRadix, tile_ctr + p, a.status);
         if (e) return e;
@@ -398,13 +372,8 @@ cudaError_t lbvh_build(const LbvhArgs& a, cudaStream_t s) {
     }
     const PermuteIO P{a.vals_sorted, a.idx_in,  a.map_in,   a.orig_in, a.pos,
                       a.idx_out,     a.map_out, a.orig_out, a.tris};
-#if RT_EMIT_PERMUTE
-    return launch_emit(a, reinterpret_cast<uint8_t*>(a.scratch) + lbvh_emit_offset(n), s, &P);
-#else
-    e = launch_dep(k_permute, grid_for(n, 256, sms * 16), 256, 0, s, n, P, a.leafbox);
-    if (e) return e;
-    return launch_emit(a, reinterpret_cast<uint8_t*>(a.scratch) + lbvh_emit_offset(n), s);
-#endif
+    return launch_emit<EMIT_PERMUTE>(a, reinterpret_cast<uint8_t*>(a.scratch) + lbvh_emit_offset(n),
+                                     P, s);
 }
 
 size_t radix_scratch_words(uint32_t n, int passes) {
@@ -463,20 +432,21 @@ cudaError_t radix_sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t*
     return cudaGetLastError();
 }
 
-cudaError_t lbvh_permute(const LbvhArgs& a, const uint32_t* order, cudaStream_t s) {
+cudaError_t lbvh_permute(const LbvhArgs& a, const uint32_t* order, const uint8_t* more,
+                         cudaStream_t s) {
     const PermuteIO P{order,     a.idx_in,  a.map_in,   a.orig_in, a.pos,
                       a.idx_out, a.map_out, a.orig_out, a.tris};
-    k_permute<<<grid_for(a.n, 256, a.num_sms * 16), 256, 0, s>>>(a.n, P, a.leafbox);
+    k_permute<<<grid_for(a.n, 256, a.num_sms * 16), 256, 0, s>>>(a.n, P, more);
     return cudaGetLastError();
 }
 
 cudaError_t lbvh_refit(const LbvhArgs& a, cudaStream_t s) {
-    const uint32_t n = a.n;
-    k_refit_leaves<<<grid_for(n, 256, a.num_sms * 16), 256, 0, s>>>(n, a.idx_out, a.pos, a.tris,
-                                                                    a.leafbox);
     // the emit is deterministic in the sorted keys, so rerunning it on the
     // same keys reproduces the same topology with the new boxes
-    return launch_emit(a, reinterpret_cast<uint8_t*>(a.scratch) + lbvh_emit_offset(n), s);
+    const PermuteIO P{nullptr,   nullptr, nullptr, nullptr, a.pos,
+                      a.idx_out, nullptr, nullptr, a.tris};
+    return launch_emit<EMIT_REFIT>(a, reinterpret_cast<uint8_t*>(a.scratch) + lbvh_emit_offset(a.n),
+                                   P, s);
 }
 
 }  // namespace rt

@@ -22,15 +22,13 @@ struct LbvhArgs {
     uint32_t* orig_out;
     // sort buffers
     uint32_t* keys_unsorted;  // Morton key per triangle (order before the build)
-    uint32_t* vals0;          // 0..n-1
-    uint32_t* keys1;
-    uint32_t* vals1;
+    uint32_t* keys1;          // the passes' other buffers (in the space of `tris`,
+    uint32_t* vals1;          // which the emit fills after the sort)
     uint32_t* keys_sorted;
     uint32_t* vals_sorted;    // sorted slot -> triangle (order before the build)
     // outputs
     float4* tris;             // 3 float4 per sorted triangle
-    float4* leafbox;          // 2 float4 per sorted triangle
-    float4* nodes;            // 4 float4 per radix-tree node (n - 1)
+    float4* nodes;            // 8 float4 per radix-tree node (n - 1)
     BvhHeader* hdr;
     uint32_t* scratch;        // lbvh_scratch_bytes(n, passes)
     uint32_t* status;         // device status word (RT_DEV_* bits)
@@ -45,10 +43,16 @@ cudaError_t launch_mangle(float4* pos, float4* nrm, uint32_t V, float arg, float
                           cudaStream_t s);
 cudaError_t lbvh_build(const LbvhArgs& a, cudaStream_t s);
 cudaError_t lbvh_refit(const LbvhArgs& a, cudaStream_t s);
-// The triangle data (indices, materials, ids, triangle records, leaf boxes)
-// of a.*_in rearranged into a.*_out by `order` (slot -> triangle), as the
-// LBVH build does with its sorted permutation.
-cudaError_t lbvh_permute(const LbvhArgs& a, const uint32_t* order, cudaStream_t s);
+// The triangle data (indices, materials, ids, triangle records) of a.*_in
+// rearranged into a.*_out by `order` (slot -> triangle), as the LBVH build
+// does with its sorted permutation; `more` holds the records' leaf marks.
+cudaError_t lbvh_permute(const LbvhArgs& a, const uint32_t* order, const uint8_t* more,
+                         cudaStream_t s);
+// keys1 / vals1 of an n-triangle scene in its triangle records' space.
+inline uint32_t* sort_keys1(float4* tris) { return reinterpret_cast<uint32_t*>(tris); }
+inline uint32_t* sort_vals1(float4* tris, uint32_t n) {
+    return reinterpret_cast<uint32_t*>(tris) + (((size_t)n + 3) & ~(size_t)3);
+}
 
 // Stable LSD radix sort of (key, value) pairs on the low key_bits bits with
 // caller-provided scratch (radix_scratch_words words) and temporaries of n

@@ -61,6 +61,23 @@ __device__ __forceinline__ void st_relaxed(uint32_t* p, uint32_t v) {
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// Plain loads of what an earlier kernel of a build wrote.  The build's kernels
+// start while their predecessor still runs, so its results are not read-only
+// for the kernel's lifetime, as the non-coherent loads that __ldg and const
+// __restrict__ give require: such a load may be moved above the wait for the
+// predecessor.  A volatile asm stays behind it.
+__device__ __forceinline__ uint32_t ld_dep(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint4 ld_dep(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
 // A shared-memory mbarrier and the 1-D bulk copy (the TMA engine without a
 // tensor map) that completes on it.
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
@@ -121,6 +138,13 @@ __device__ __forceinline__ void tri_aabb(const float4* __restrict__ pos,
     lo[2] = fminf(fminf(p0.z, p1.z), p2.z);
 }
 
+// Scene bounds as six words that start at zero: the complements of the lower
+// corner's ordered integers and the upper corner's, both maxima.
+__device__ __forceinline__ void bounds_add(uint32_t* bounds, int c, float lo, float hi) {
+    atomicMax(&bounds[c], ~f2o(lo));
+    atomicMax(&bounds[3 + c], f2o(hi));
+}
+
 // Per-scene constants of morton_encode (bvh-builder.cl:181-252).
 struct MortonParams {
     float glo[3], inv[3];
@@ -132,8 +156,8 @@ __device__ __forceinline__ MortonParams morton_params(const uint32_t* bounds, in
     MortonParams m;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        m.glo[c] = o2f(bounds[c]);
-        const float ghi = o2f(bounds[3 + c]);
+        m.glo[c] = o2f(~ld_dep(&bounds[c]));
+        const float ghi = o2f(ld_dep(&bounds[3 + c]));
         m.inv[c] = 1.0f / (ghi - m.glo[c]);
     }
     m.scale = (float)(1u << ((depth + 2) / 3));
@@ -451,7 +475,7 @@ __device__ __forceinline__ void onesweep_tile(SortSmemT<ITEMS, BITS>& S, uint32_
 #pragma unroll
     for (int q = 0; q < DPT; ++q) {
         h[q] = hsum;
-        hsum += __ldg(&hist[dgt0 + q]);
+        hsum += ld_dep(&hist[dgt0 + q]);
     }
     const uint32_t gbase = block_excl_scan_256(hsum, S.scan);
 #pragma unroll
@@ -490,15 +514,10 @@ struct PermuteIO {
     float4* tris;
 };
 
-__device__ __forceinline__ void permute_tri(uint32_t i, const PermuteIO& P, float4& lo, float4& hi) {
-    const uint32_t o = __ldg(&P.vals[i]);
-    const uint32_t a = __ldg(&P.idx_old[3 * (size_t)o]), b = __ldg(&P.idx_old[3 * (size_t)o + 1]),
-                   c = __ldg(&P.idx_old[3 * (size_t)o + 2]);
-    P.idx_new[3 * (size_t)i] = a;
-    P.idx_new[3 * (size_t)i + 1] = b;
-    P.idx_new[3 * (size_t)i + 2] = c;
-    P.map_new[i] = __ldg(&P.map_old[o]);
-    P.orig_new[i] = __ldg(&P.orig_old[o]);
+// Triangle record (its `more` mark clear) and AABB of sorted triangle i with
+// vertices a, b, c.
+__device__ __forceinline__ void tri_record(uint32_t i, const PermuteIO& P, uint32_t a, uint32_t b,
+                                           uint32_t c, float4& lo, float4& hi) {
     const float4 p0 = __ldg(&P.pos[a]), p1 = __ldg(&P.pos[b]), p2 = __ldg(&P.pos[c]);
     P.tris[3 * (size_t)i] = make_float4(p0.x, p0.y, p0.z, 0.f);
     P.tris[3 * (size_t)i + 1] = make_float4(p1.x - p0.x, p1.y - p0.y, p1.z - p0.z, 0.f);
@@ -512,20 +531,31 @@ __device__ __forceinline__ void permute_tri(uint32_t i, const PermuteIO& P, floa
     lo.w = hi.w = 0.f;
 }
 
-// permute_tri with the leaf AABB stored for a later emit (the many-scene
-// build and any caller of k_permute).
-__device__ __forceinline__ void permute_one(uint32_t i, const PermuteIO& P,
-                                            float4* __restrict__ leafbox) {
-    float4 lo, hi;
-    permute_tri(i, P, lo, hi);
-    leafbox[2 * (size_t)i] = lo;
-    leafbox[2 * (size_t)i + 1] = hi;
+__device__ __forceinline__ void permute_tri(uint32_t i, const PermuteIO& P, float4& lo, float4& hi) {
+    const uint32_t o = ld_dep(&P.vals[i]);
+    const uint32_t a = __ldg(&P.idx_old[3 * (size_t)o]), b = __ldg(&P.idx_old[3 * (size_t)o + 1]),
+                   c = __ldg(&P.idx_old[3 * (size_t)o + 2]);
+    P.idx_new[3 * (size_t)i] = a;
+    P.idx_new[3 * (size_t)i + 1] = b;
+    P.idx_new[3 * (size_t)i + 2] = c;
+    P.map_new[i] = __ldg(&P.map_old[o]);
+    P.orig_new[i] = __ldg(&P.orig_old[o]);
+    tri_record(i, P, a, b, c, lo, hi);
+}
+
+// Refit's counterpart of permute_tri: the triangle keeps its place, its
+// record and AABB are made from the current vertex positions
+// (refit_lbvh, bvh-builder.cpp:743-790).
+__device__ __forceinline__ void refit_tri(uint32_t i, const PermuteIO& P, float4& lo, float4& hi) {
+    const uint32_t* idx = P.idx_new;
+    tri_record(i, P, __ldg(&idx[3 * (size_t)i]), __ldg(&idx[3 * (size_t)i + 1]),
+               __ldg(&idx[3 * (size_t)i + 2]), lo, hi);
 }
 
 // delta(i): highest differing bit between sorted keys i and i+1, with the
 // index appended so that equal keys still order (Karras' augmentation).
 __device__ __forceinline__ uint64_t delta(const uint32_t* __restrict__ k, uint32_t i) {
-    const uint32_t x = __ldg(&k[i]) ^ __ldg(&k[i + 1]);
+    const uint32_t x = ld_dep(&k[i]) ^ ld_dep(&k[i + 1]);
     return ((uint64_t)x << 32) | (uint64_t)(i ^ (i + 1));
 }
 
@@ -576,9 +606,6 @@ constexpr int EMIT_GROUP = RT_EMIT_GROUP;   // blocks of one level gathered by a
 #ifndef RT_EMIT_MINB0
 #define RT_EMIT_MINB0 3
 #endif
-#ifndef RT_EMIT_MINB1
-#define RT_EMIT_MINB1 1
-#endif
 #ifndef RT_EMIT_LEAVE0
 #define RT_EMIT_LEAVE0 128u   // runs a level-0 block may leave unjoined
 #endif
@@ -587,6 +614,13 @@ constexpr int EMIT_GROUP = RT_EMIT_GROUP;   // blocks of one level gathered by a
 #endif
 constexpr int EMIT_C0 = RT_EMIT_C0;                // triangles per level-0 block
 constexpr int EMIT_C1 = EMIT_GROUP * EMIT_FMAX;    // items per block above level 0
+// Threads per block above level 0 (its warps take the items' chunks in
+// rounds): 256 in a level of more blocks than SMs, where two blocks per SM
+// hide each other's barriers, 512 in the last, narrow levels, which last as
+// long as one block does.  Against one thread per item (1024, one block per
+// SM) and three barriers per gather: level 1 of 17.7 M triangles 341 -> 239
+// us, of 1.24 M 30.7 -> 24.2 us, the last level 11.5 -> 9.4 us.
+constexpr int EMIT_T_WIDE = 256, EMIT_T_NARROW = 512;
 
 // Blocks of level 0 of an n-triangle scene, and of the level above nb blocks.
 __host__ __device__ __forceinline__ uint32_t emit_blocks0(uint32_t n) {
@@ -731,28 +765,37 @@ __device__ __forceinline__ float2 axis_range(const WarpScratch& W, uint32_t a, u
 // those two.  All of it comes from bit planes of the boundary levels, with
 // no rounds; the children's boxes come from sparse tables of the item boxes.
 // fminf / fmaxf order -0 below +0 and skip NaN whatever the operand order,
-// so any grouping of a range gives the bits of the bottom-up merge.
+// so any grouping of a range gives the bits of the bottom-up merge.  TRIS: the
+// items are consecutive triangles, lane l's it.l = it.l of lane 0 + l.
+template <bool TRIS>
 __device__ __forceinline__ bool warp_join(WarpItem& it, uint32_t cnt, uint64_t edge, uint32_t n,
                                           int min_leaf, float4* __restrict__ nodes,
-                                          WarpScratch& W, BvhHeader* __restrict__ hdr) {
+                                          float4* __restrict__ tris, WarpScratch& W,
+                                          BvhHeader* __restrict__ hdr) {
     const uint32_t lane = threadIdx.x & 31u;
     const unsigned FULL = 0xffffffffu;
     if (cnt == 0u) return false;
     const bool item = lane < cnt;
     __syncwarp();   // the lanes have read their items out of this space
     if (item) {
-        W.il[lane] = it.l;
-        W.ir[lane] = it.r;
         W.ikl[lane] = it.kl;
-        W.ikr[lane] = it.kr;
-        W.iref[lane] = it.ref;
-        W.icnt[lane] = it.cnt;
+        if (!TRIS) {
+            W.il[lane] = it.l;
+            W.ir[lane] = it.r;
+            W.ikr[lane] = it.kr;
+            W.iref[lane] = it.ref;
+            W.icnt[lane] = it.cnt;
+        }
     }
+    const uint32_t first = TRIS ? it.l - lane : 0u;   // TRIS: item a is triangle first + a
+    auto left_end = [&](uint32_t a) { return TRIS ? first + a : W.il[a]; };
+    auto right_end = [&](uint32_t a) { return TRIS ? first + a : W.ir[a]; };
+    auto right_key = [&](uint32_t a) { return TRIS ? W.ikl[a] : W.ikr[a]; };
     // --- topology, from the levels of the boundaries
     // the node split at boundary j = lane (1 <= j < cnt), when it lies
     // inside: left child items A..j-1 (split at lsplit's right end), right
     // child j..B (split at rsplit's)
-    bool local = false, out = false;
+    bool local = false, out = false, up_left = false;   // up_left: a left child
     uint32_t A = lane, B = lane, lsplit = 0u, rsplit = 0u;
     {
         const uint32_t lev = item ? delta_level(it.db) : 0u;
@@ -781,7 +824,8 @@ __device__ __forceinline__ bool warp_join(WarpItem& it, uint32_t cnt, uint64_t e
         if (item) {
             const uint32_t la = level_at(A, P);
             const uint32_t lb = B + 1u < cnt ? level_at(B + 1u, P) : edge_lev;
-            const uint32_t p = lb < la ? B + 1u : A;   // the parent's split
+            up_left = lb < la;
+            const uint32_t p = up_left ? B + 1u : A;   // the parent's split
             out = p == 0u || p >= cnt || !((LM >> p) & 1u);
         }
     }
@@ -817,25 +861,50 @@ __device__ __forceinline__ bool warp_join(WarpItem& it, uint32_t cnt, uint64_t e
     // right end of item `split`) or as the item itself
     auto ref_of = [&](uint32_t a, uint32_t b, uint32_t split, int32_t& ref, int32_t& c) {
         if (a == b) {
-            ref = W.iref[a];
-            c = W.icnt[a];
+            ref = TRIS ? (int32_t)(first + a) : W.iref[a];
+            c = TRIS ? 1 : W.icnt[a];
             return;
         }
-        const uint32_t L = W.il[a], count = W.ir[b] - L + 1u;
-        const bool interior = count >= (uint32_t)min_leaf + 3u && W.ikl[a] != W.ikr[b];
-        ref = interior ? (int32_t)W.ir[split] : (int32_t)L;
+        const uint32_t L = left_end(a), count = right_end(b) - L + 1u;
+        const bool interior = count >= (uint32_t)min_leaf + 3u && W.ikl[a] != right_key(b);
+        ref = interior ? (int32_t)right_end(split) : (int32_t)L;
         c = interior ? 0 : (int32_t)count;
     };
     if (local) {
-        int32_t lref, lcnt, rref, rcnt;
-        ref_of(A, lane - 1u, lsplit, lref, lcnt);
-        ref_of(lane, B, rsplit, rref, rcnt);
-        float4* np = nodes + 4 * (size_t)W.ir[lane - 1u];
-        np[0] = make_float4(llo[0], llo[1], llo[2], lhi[0]);
-        np[1] = make_float4(lhi[1], lhi[2], rlo[0], rlo[1]);
-        np[2] = make_float4(rlo[2], rhi[0], rhi[1], rhi[2]);
-        np[3] = make_float4(__int_as_float(lref), __int_as_float(rref), __int_as_float(lcnt),
-                            __int_as_float(rcnt));
+        const uint32_t gl = left_end(A), gr = right_end(B), self = right_end(lane - 1u);
+        if (gr - gl + 1u >= (uint32_t)min_leaf + 3u && W.ikl[A] != right_key(B)) {
+            // an interior node: its children fill its half of its parent's
+            // record, which lies beside its range; a child that is a leaf
+            // fills a half of the node's own record (an interior child fills
+            // that half itself)
+            const bool root = gl == 0u && gr == n - 1u;
+            const uint32_t up = up_left ? gr : gl - 1u, up_slot = up_left ? 0u : 2u;
+            auto put = [&](uint32_t side, uint32_t a, uint32_t b, uint32_t split, const float* lo,
+                           const float* hi) {
+                int32_t ref, c;
+                ref_of(a, b, split, ref, c);
+                const float4 s0 = make_float4(lo[0], lo[1], hi[0], hi[1]);
+                const float4 s1 = make_float4(lo[2], hi[2], __int_as_float(c > 0 ? ~ref : ref),
+                                              __int_as_float(c > 0 ? c : (int32_t)self));
+                if (!root) {
+                    float4* q = nodes + 8 * (size_t)up + 2 * (up_slot + side);
+                    q[0] = s0;
+                    q[1] = s1;
+                }
+                if (c > 0) {
+                    float4* q = nodes + 8 * (size_t)self + 4 * side;
+                    const float inf = __int_as_float(0x7f800000);
+                    q[0] = s0;
+                    q[1] = s1;
+                    q[2] = make_float4(inf, inf, inf, inf);
+                    q[3] = make_float4(inf, inf, s1.z, __int_as_float(EMPTY_SLOT));
+                }
+            };
+            put(0u, A, lane - 1u, lsplit, llo, lhi);
+            put(1u, lane, B, rsplit, rlo, rhi);
+        } else {
+            tris[3 * (size_t)self].w = 1.0f;   // a boundary inside a leaf
+        }
     }
     float4 q0, q1, q2;
     if (out) {
@@ -847,7 +916,7 @@ __device__ __forceinline__ bool warp_join(WarpItem& it, uint32_t cnt, uint64_t e
         const float hx = local ? fmaxf(lhi[0], rhi[0]) : lhi[0],
                     hy = local ? fmaxf(lhi[1], rhi[1]) : lhi[1],
                     hz = local ? fmaxf(lhi[2], rhi[2]) : lhi[2];
-        const uint32_t gl = W.il[A], gr = W.ir[B];
+        const uint32_t gl = left_end(A), gr = right_end(B);
         if (gl == 0u && gr == n - 1u) {   // the root
             hdr->root_ref = eref;
             hdr->root_cnt = ecnt;
@@ -857,7 +926,7 @@ __device__ __forceinline__ bool warp_join(WarpItem& it, uint32_t cnt, uint64_t e
             out = false;
         }
         q0 = make_float4(__uint_as_float(gl), __uint_as_float(gr), __uint_as_float(W.ikl[A]),
-                         __uint_as_float(W.ikr[B]));
+                         __uint_as_float(right_key(B)));
         q1 = make_float4(lx, ly, lz, hx);
         q2 = make_float4(hy, hz, __int_as_float(eref), __int_as_float(ecnt));
     }
@@ -889,92 +958,95 @@ __device__ __forceinline__ bool warp_join(WarpItem& it, uint32_t cnt, uint64_t e
     return mine;
 }
 
-// Shared state of one emit block: the items left over by its warps, in order.
-template <int C>
+// Shared state of an emit block of T threads over up to C items: the items,
+// in order, and the warps' scratch.  With a thread per item the scratch of
+// warp w takes the place of list[32w .. 32w+31].
+template <int C, int T>
 struct EmitSmem {
-    union {
-        EmitItem list[C];
-        WarpScratch scratch[C / 32];   // warp w's: list[32w .. 32w+31]
-    };
-    uint32_t wcount[C / 32], woff[C / 32 + 1];
+    EmitItem list[C];
+    WarpScratch scratch[T / 32];
+    uint32_t wcount[T / 32];
+    uint32_t goff[EMIT_GROUP + 1];
     uint64_t edge;   // boundary after the block's last item
 };
-
-// Gathers, in order, the runs still held by the warps' lanes into S.list and
-// returns their number.  Call with all C threads; `keep` marks held runs.
 template <int C>
-__device__ __forceinline__ uint32_t gather_runs(EmitSmem<C>& S, const WarpItem& it, bool keep) {
+struct EmitSmem<C, C> {
+    union {
+        EmitItem list[C];
+        WarpScratch scratch[C / 32];
+    };
+    uint32_t wcount[C / 32];
+    uint64_t edge;
+};
+
+// Appends, in order, the runs still held by the warps' lanes to the `base`
+// runs of S.list and returns their number.  Call with all T threads; `keep`
+// marks held runs.
+template <int C, int T>
+__device__ __forceinline__ uint32_t gather_runs(EmitSmem<C, T>& S, const WarpItem& it, bool keep,
+                                                uint32_t base = 0u) {
     const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
     const unsigned bal = __ballot_sync(0xffffffffu, keep);
     if (lane == 0) S.wcount[w] = __popc(bal);
     __syncthreads();   // also: every warp has read its chunk of S.list
-    if (w == 0) {
-        const uint32_t v = lane < (uint32_t)(C / 32) ? S.wcount[lane] : 0u;
-        uint32_t x = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t u = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= (uint32_t)o) x += u;
-        }
-        if (lane < (uint32_t)(C / 32)) S.woff[lane] = x - v;
-        if (lane == 31) S.woff[C / 32] = x;
-    }
-    __syncthreads();
-    if (keep) reg_to_item(it, S.list[S.woff[w] + __popc(bal & ((1u << lane) - 1u))]);
-    const uint32_t m = S.woff[C / 32];
+    // each warp sums the counts itself: no second barrier behind a scan
+    const uint32_t v = lane < (uint32_t)(T / 32) ? S.wcount[lane] : 0u;
+    const uint32_t before = __reduce_add_sync(0xffffffffu, lane < w ? v : 0u);
+    const uint32_t m = __reduce_add_sync(0xffffffffu, v);
+    if (keep) reg_to_item(it, S.list[base + before + __popc(bal & ((1u << lane) - 1u))]);
     __syncthreads();
     return m;
 }
 
-// One level of the emit for block `blk` (C threads = C / 32 warps).  Level 0
-// (in == null): the items are triangles blk*C .. blk*C+C-1; otherwise the
+// One level of the emit for block `blk` of T threads (T = C at level 0).  Level
+// 0 (SRC not EMIT_ITEMS): the items are triangles blk*C .. blk*C+C-1; otherwise the
 // items left by blocks blk*EMIT_GROUP .. of the previous level (in_count[k]
 // items at in[k * EMIT_FMAX]).  Leaves the block's own items at
 // out[blk * EMIT_FMAX] and their number in out_count[blk].  The block stops
 // joining once `leave` runs or fewer are left (leave <= EMIT_FMAX; 32: join
 // down to one warp's runs, as the root's level must).
 //
-// With PERMUTE, level 0 performs the permutation of its own triangles
-// (permute_tri with `perm`) and keeps their boxes in registers; `leafbox` is
-// then unused.
-template <int C, bool PERMUTE = false>
-__device__ __forceinline__ void emit_level(EmitSmem<C>& S, uint32_t blk, uint32_t n,
+// Level 0 makes its triangles' records itself and keeps their boxes in
+// registers: it performs the permutation of a build (SRC = EMIT_PERMUTE,
+// permute_tri with `perm`) or a refit (EMIT_REFIT, refit_tri).
+enum EmitSource { EMIT_ITEMS, EMIT_PERMUTE, EMIT_REFIT };
+template <int C, int T, EmitSource SRC = EMIT_ITEMS>
+__device__ __forceinline__ void emit_level(EmitSmem<C, T>& S, uint32_t blk, uint32_t n,
                                            const uint32_t* __restrict__ skeys,
-                                           const float4* __restrict__ leafbox,
                                            const EmitItem* __restrict__ in,
                                            const uint32_t* __restrict__ in_count,
                                            uint32_t n_in, EmitItem* __restrict__ out,
                                            uint32_t* __restrict__ out_count,
-                                           float4* __restrict__ nodes, int min_leaf,
+                                           float4* __restrict__ nodes,
+                                           float4* __restrict__ tris, int min_leaf,
                                            uint32_t leave, BvhHeader* __restrict__ hdr,
                                            uint32_t* __restrict__ status,
                                            const PermuteIO& perm = PermuteIO{}) {
-    static_assert(C % 32 == 0 && C >= EMIT_FMAX, "block size");
+    static_assert(C % T == 0 && T % 32 == 0 && T >= EMIT_FMAX, "block size");
+    static_assert(SRC == EMIT_ITEMS || T == C, "a thread per triangle");
     const uint32_t t = threadIdx.x, lane = t & 31u, w = t >> 5;
     WarpItem it;
     bool keep;
     uint32_t m;
-    if (!in) {
+    if constexpr (SRC != EMIT_ITEMS) {
         // level 0: warp w joins triangles b0 + 32w ..
         const uint32_t b0 = blk * (uint32_t)C, i = b0 + t;
         const uint32_t w0 = b0 + 32u * w;
         const uint32_t cnt = w0 < n ? min(32u, n - w0) : 0u;
         const bool have = i < n;
-        const uint32_t k = have ? __ldg(&skeys[i]) : 0u;
+        const uint32_t k = have ? ld_dep(&skeys[i]) : 0u;
         uint32_t kprev = __shfl_up_sync(0xffffffffu, k, 1);
-        if (lane == 0 && have && i > 0) kprev = __ldg(&skeys[i - 1]);
+        if (lane == 0 && have && i > 0) kprev = ld_dep(&skeys[i - 1]);
         it.l = it.r = i;
         it.kl = it.kr = k;
         it.db = (!have || i == 0) ? ~0ull
                                   : (((uint64_t)(kprev ^ k) << 32) | (uint64_t)((i - 1) ^ i));
         float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
         if (have) {
-            if constexpr (PERMUTE) {
+            if constexpr (SRC == EMIT_PERMUTE)
                 permute_tri(i, perm, lo, hi);
-            } else {
-                lo = leafbox[2 * (size_t)i];
-                hi = leafbox[2 * (size_t)i + 1];
-            }
+            else
+                refit_tri(i, perm, lo, hi);
         }
         it.lox = lo.x; it.loy = lo.y; it.loz = lo.z;
         it.hix = hi.x; it.hiy = hi.y; it.hiz = hi.z;
@@ -993,29 +1065,33 @@ __device__ __forceinline__ void emit_level(EmitSmem<C>& S, uint32_t blk, uint32_
             return;
         }
         if (t == 0) S.edge = delta_or_max(skeys, (int64_t)min(b0 + (uint32_t)C, n) - 1, n);
-        keep = warp_join(it, cnt, edge, n, min_leaf, nodes, S.scratch[w], hdr);
-        m = gather_runs<C>(S, it, keep);
+        keep = warp_join<true>(it, cnt, edge, n, min_leaf, nodes, tris, S.scratch[w], hdr);
+        m = gather_runs(S, it, keep);
     } else {
         // the items left by EMIT_GROUP blocks of the previous level, in order
         if (w == 0) {
             const uint32_t k = blk * EMIT_GROUP + lane;
             const uint32_t v = (lane < (uint32_t)EMIT_GROUP && k < n_in)
-                                   ? min(__ldg(&in_count[k]), (uint32_t)EMIT_FMAX) : 0u;
+                                   ? min(ld_dep(&in_count[k]), (uint32_t)EMIT_FMAX) : 0u;
             uint32_t x = v;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const uint32_t u = __shfl_up_sync(0xffffffffu, x, o);
                 if (lane >= (uint32_t)o) x += u;
             }
-            if (lane < (uint32_t)EMIT_GROUP) S.woff[lane] = x - v;
-            if (lane == 31) S.woff[EMIT_GROUP] = x;
+            if (lane < (uint32_t)EMIT_GROUP) S.goff[lane] = x - v;
+            if (lane == 31) S.goff[EMIT_GROUP] = x;
         }
         __syncthreads();
-        m = S.woff[EMIT_GROUP];
-        for (uint32_t e = t; e < m; e += C) {
+        m = S.goff[EMIT_GROUP];
+        for (uint32_t e = t; e < m; e += T) {
             int g = 0;
-            while (g + 1 < EMIT_GROUP && S.woff[g + 1] <= e) ++g;
-            S.list[e] = in[(size_t)(blk * EMIT_GROUP + g) * EMIT_FMAX + (e - S.woff[g])];
+            while (g + 1 < EMIT_GROUP && S.goff[g + 1] <= e) ++g;
+            const uint4* src = reinterpret_cast<const uint4*>(
+                in + (size_t)(blk * EMIT_GROUP + g) * EMIT_FMAX + (e - S.goff[g]));
+            uint4* dst = reinterpret_cast<uint4*>(&S.list[e]);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) dst[q] = ld_dep(src + q);
         }
         __syncthreads();   // the last item may have been copied by another thread
         if (t == 0 && m) S.edge = delta_or_max(skeys, (int64_t)S.list[m - 1].r, n);
@@ -1035,7 +1111,7 @@ __device__ __forceinline__ void emit_level(EmitSmem<C>& S, uint32_t blk, uint32_
             // few enough to be items of the next level as they are: the
             // next level joins them (a block's passes get longer and emptier
             // as its runs thin out)
-            for (uint32_t e = t; e < m; e += (uint32_t)C) out[(size_t)blk * EMIT_FMAX + e] = S.list[e];
+            for (uint32_t e = t; e < m; e += (uint32_t)T) out[(size_t)blk * EMIT_FMAX + e] = S.list[e];
             if (t == 0 && out_count) out_count[blk] = m;
             return;
         }
@@ -1043,7 +1119,7 @@ __device__ __forceinline__ void emit_level(EmitSmem<C>& S, uint32_t blk, uint32_
             if (w == 0) {
                 const uint32_t cnt = m;
                 if (lane < cnt) item_to_reg(S.list[lane], it);
-                keep = warp_join(it, cnt, S.edge, n, min_leaf, nodes, S.scratch[0], hdr);
+                keep = warp_join<false>(it, cnt, S.edge, n, min_leaf, nodes, tris, S.scratch[0], hdr);
                 const unsigned bal = __ballot_sync(0xffffffffu, keep);
                 if (keep) reg_to_item(it, out[(size_t)blk * EMIT_FMAX + __popc(bal & ((1u << lane) - 1u))]);
                 if (lane == 0 && out_count) out_count[blk] = __popc(bal);
@@ -1055,23 +1131,30 @@ __device__ __forceinline__ void emit_level(EmitSmem<C>& S, uint32_t blk, uint32_
             // every run left has its parent outside the block: all of them,
             // in order, are items of the next level
             const uint32_t nf = min(m, (uint32_t)EMIT_FMAX);
-            for (uint32_t e = t; e < nf; e += (uint32_t)C) out[(size_t)blk * EMIT_FMAX + e] = S.list[e];
+            for (uint32_t e = t; e < nf; e += (uint32_t)T) out[(size_t)blk * EMIT_FMAX + e] = S.list[e];
             if (t == 0) {
                 if (m > (uint32_t)EMIT_FMAX) atomicOr(status, RT_DEV_OVERFLOW);
                 if (out_count) out_count[blk] = nf;
             }
             return;
         }
-        // chunk w is [0, off) for w == 0, else [off + 32(w-1), off + 32w)
+        // chunk c is [0, off) for c == 0, else [off + 32(c-1), off + 32c); the
+        // block's warps take T / 32 chunks per round, and what a round leaves
+        // goes to the front of the list, over chunks that are done
         const uint32_t off = ((pass & 1u) && m + 16u <= (uint32_t)C) ? 16u : 32u;
-        const uint32_t c0 = w == 0 ? 0u : off + 32u * (w - 1u);
-        const uint32_t c1 = min(m, off + 32u * w);
-        const uint32_t cnt = c0 < m ? c1 - c0 : 0u;
-        if (lane < cnt) item_to_reg(S.list[c0 + lane], it);
-        const uint64_t edge = c1 < m ? S.list[c1].db : S.edge;
-        __syncthreads();   // the chunks are read: the list space becomes the warps' scratch
-        keep = warp_join(it, cnt, edge, n, min_leaf, nodes, S.scratch[w], hdr);
-        const uint32_t m_new = gather_runs<C>(S, it, keep);
+        uint32_t m_new = 0u;
+        for (uint32_t r0 = 0u; r0 == 0u || off + 32u * (r0 - 1u) < m; r0 += (uint32_t)(T / 32)) {
+            const uint32_t c = r0 + w;
+            const uint32_t c0 = c == 0 ? 0u : off + 32u * (c - 1u);
+            const uint32_t c1 = min(m, off + 32u * c);
+            const uint32_t cnt = c0 < m ? c1 - c0 : 0u;
+            if (lane < cnt) item_to_reg(S.list[c0 + lane], it);
+            const uint64_t edge = c1 < m ? S.list[c1].db : S.edge;
+            if (C == T) __syncthreads();   // the chunks are read: their space is the warps' scratch
+            keep = warp_join<false>(it, cnt, edge, n, min_leaf, nodes, tris, S.scratch[w], hdr);
+            m_new += gather_runs(S, it, keep, m_new);
+            if (C == T) break;
+        }
         stalls = m_new == m ? stalls + 1u : 0u;
         m = m_new;
     }

@@ -14,14 +14,20 @@ namespace rt {
 // --------------------------------------------------------------------------
 // BVH layout in HBM
 // --------------------------------------------------------------------------
-// Interior nodes are stored as child pairs (64 B = 4 x float4), indexed by
-// the split position of the Karras radix tree they come from:
-//   n0 = (c0.lo.x, c0.lo.y, c0.lo.z, c0.hi.x)
-//   n1 = (c0.hi.y, c0.hi.z, c1.lo.x, c1.lo.y)
-//   n2 = (c1.lo.z, c1.hi.x, c1.hi.y, c1.hi.z)
-//   n3 = (ref0, ref1, cnt0, cnt1) as int: cnt == 0 -> ref is an interior node
-//        index; cnt > 0 -> leaf over sorted triangles [ref, ref + cnt).
-// c0 is the left child (lower Morton range), c1 the right child.
+// Every interior node of the binary tree has a record of its four
+// grandchildren (128 B = 8 x float4), indexed by the split position of the
+// radix tree node (the last triangle of its left part): slots 0 and 1 are the
+// children of its left child, 2 and 3 those of its right child, 32 B each:
+//   lo.x lo.y hi.x hi.y lo.z hi.z code aux
+//   inner grandchild:  code = its record,            aux = the child's record
+//   leaf grandchild:   code = ~(first triangle),     aux = its triangle count
+// A child that is a leaf itself takes the first slot of its pair; the second
+// is then empty: a box at +infinity (no ray with a finite slab hits it), the
+// leaf's code again and aux = -1.  A traversal enters two binary levels by
+// reading one record: it waits for memory half as often as one that reads a
+// 64 B pair of children per level, for the same bytes per two levels.  The
+// corners are laid out so that one 256-bit load gives the register pairs of
+// the two-lane slab arithmetic (trace_dev.cuh).
 struct BvhHeader {
     int32_t root_ref;       // interior node index, or first triangle of a root leaf
     int32_t root_cnt;       // 0: interior root; > 0: the whole tree is one leaf
@@ -31,8 +37,25 @@ struct BvhHeader {
     float4 root_hi;
 };
 
+// Slot of a node record.
+struct Slot {
+    float lox, loy, hix, hiy, loz, hiz;
+    int32_t code, aux;
+};
+constexpr int32_t EMPTY_SLOT = -1;   // aux of the slot beside a leaf child
+
+// Whether the child whose second slot is b is a leaf, and else the child's
+// record from its first slot a: a's aux, or, a being a leaf, the triangle
+// where the child splits, a's last.
+__host__ __device__ __forceinline__ bool slot_pair_is_leaf(const Slot& b) { return b.aux == EMPTY_SLOT; }
+__host__ __device__ __forceinline__ int32_t slot_pair_node(const Slot& a) {
+    return a.code >= 0 ? a.aux : ~a.code + a.aux - 1;
+}
+
 // Triangle records in sorted order, 48 B: v0, e1 = v1 - v0, e2 = v2 - v0
-// (the same float subtractions as leaf_hit, trace-bvh.cl:297-298).
+// (the same float subtractions as leaf_hit, trace-bvh.cl:297-298).  v0.w is
+// 1 where the next triangle belongs to the same leaf, else 0: a leaf is found
+// from its first triangle alone.
 struct TriRec {
     float4 v0, e1, e2;
 };
@@ -42,7 +65,7 @@ struct TriRec {
 constexpr int kMaxRenderVariants = 32;
 
 struct SceneView {
-    const float4* __restrict__ nodes;
+    const float4* __restrict__ nodes;     // 8 float4 per record
     const float4* __restrict__ tris;      // 3 float4 per triangle
     const uint32_t* __restrict__ idx;     // sorted index buffer (3 per tri)
     const float4* __restrict__ nrm;       // vertex normals
@@ -147,12 +170,33 @@ __device__ __forceinline__ bool slab_shadow(const TRay& r, float tmax, float lox
     return tmin <= tmax;
 }
 
-// Möller–Trumbore of leaf_hit (trace-bvh.cl:275-328).
+// Slot k of record p, by one 256-bit load.
+__device__ __forceinline__ Slot load_slot(const float4* __restrict__ nodes, int32_t p, int k) {
+    Slot s;
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(s.lox), "=f"(s.loy), "=f"(s.hix), "=f"(s.hiy), "=f"(s.loz), "=f"(s.hiz),
+          "=r"(s.code), "=r"(s.aux)
+        : "l"(nodes + 8 * (size_t)p + 2 * k));
+    return s;
+}
+
+__device__ __forceinline__ void swap_if(bool c, int32_t& a, int32_t& b, float& ta, float& tb) {
+    const int32_t x = c ? b : a, y = c ? a : b;
+    const float u = c ? tb : ta, v = c ? ta : tb;
+    a = x;
+    b = y;
+    ta = u;
+    tb = v;
+}
+
+// Möller–Trumbore of leaf_hit (trace-bvh.cl:275-328); `more`: the triangle
+// after this one is in the same leaf.
 __device__ __forceinline__ bool mt(const float4* __restrict__ tris, uint32_t i, f3 o, f3 d, float& t,
-                                   float& u, float& v) {
+                                   float& u, float& v, bool& more) {
     const float4 a = __ldg(&tris[3 * (size_t)i + 0]);
     const float4 b = __ldg(&tris[3 * (size_t)i + 1]);
     const float4 c = __ldg(&tris[3 * (size_t)i + 2]);
+    more = a.w != 0.0f;
     f3 v0 = ld3(a), e1 = ld3(b), e2 = ld3(c);
     f3 h = cross(d, e2);
     float aa = dot(e1, h);

@@ -205,11 +205,15 @@ struct Builder {
     }
 };
 
+// Lays the tree out as the device's records (rt_internal.cuh): a node's
+// record is that of its split position, the last slot of its left child.
 struct Flat {
     const std::vector<TNode>& top;
     const std::vector<std::vector<TNode>>& sub;
     std::vector<float4>& nodes;
+    std::vector<uint8_t>& more;
     uint32_t max_interior_depth = 0;
+    uint32_t interior = 0;
 
     const TNode& at(int tree, int32_t k) const { return tree < 0 ? top[k] : sub[tree][k]; }
 
@@ -221,36 +225,50 @@ struct Flat {
         }
     }
 
-    // A child reference: a leaf's (first triangle, count) or an interior
-    // node's index (count 0), assigned in pre-order.
-    void ref_of(int tree, int32_t k, int32_t& ref, int32_t& cnt, Box& box) {
+    const TNode& child(int& tree, int32_t k) const {
         resolve(tree, k);
-        const TNode& n = at(tree, k);
-        box = n.box;
-        if (n.leaf) {
-            ref = (int32_t)n.start;
-            cnt = (int32_t)(n.end - n.start);
-            return;
-        }
-        ref = (int32_t)(nodes.size() / 4);
-        cnt = 0;
-        emit(tree, k);
+        return at(tree, k);
+    }
+    int32_t record(int tree, const TNode& n) const { return (int32_t)child(tree, n.l).end - 1; }
+
+    void store(int32_t rec, int slot, const Slot& s) {
+        std::memcpy(&nodes[8 * (size_t)rec + 2 * slot], &s, sizeof s);
     }
 
-    void emit(int tree, int32_t k) {
-        const TNode& n = at(tree, k);
+    // Fills the record of interior node n and those below it, and the leaf marks.
+    void emit(int tree, const TNode& n) {
         if (n.depth > max_interior_depth) max_interior_depth = n.depth;
-        const size_t me = nodes.size();
-        nodes.resize(me + 4);
-        int32_t rl, cl, rr, cr;
-        Box bl, br;
-        ref_of(tree, n.l, rl, cl, bl);
-        ref_of(tree, n.r, rr, cr, br);
-        nodes[me] = make_float4(bl.lo[0], bl.lo[1], bl.lo[2], bl.hi[0]);
-        nodes[me + 1] = make_float4(bl.hi[1], bl.hi[2], br.lo[0], br.lo[1]);
-        nodes[me + 2] = make_float4(br.lo[2], br.hi[0], br.hi[1], br.hi[2]);
-        int32_t q[4] = {rl, rr, cl, cr};
-        std::memcpy(&nodes[me + 3], q, sizeof q);
+        ++interior;
+        const int32_t self = record(tree, n);
+        for (int side = 0; side < 2; ++side) {
+            int ct = tree;
+            const TNode& c = child(ct, side ? n.r : n.l);
+            if (c.leaf) {
+                const float inf = std::numeric_limits<float>::infinity();
+                store(self, 2 * side, leaf(c));
+                store(self, 2 * side + 1,
+                      Slot{inf, inf, inf, inf, inf, inf, ~(int32_t)c.start, EMPTY_SLOT});
+                continue;
+            }
+            for (int k = 0; k < 2; ++k) {
+                int gt = ct;
+                const TNode& g = child(gt, k ? c.r : c.l);
+                Slot s = leaf(g);
+                if (!g.leaf) {
+                    s.code = record(gt, g);
+                    s.aux = record(ct, c);
+                }
+                store(self, 2 * side + k, s);
+            }
+            emit(ct, c);
+        }
+    }
+
+    Slot leaf(const TNode& c) {
+        if (c.leaf)
+            for (uint32_t i = c.start; i + 1 < c.end; ++i) more[i] = 1;
+        return Slot{c.box.lo[0], c.box.lo[1], c.box.hi[0], c.box.hi[1], c.box.lo[2], c.box.hi[2],
+                    ~(int32_t)c.start, (int32_t)(c.end - c.start)};
     }
 };
 
@@ -296,10 +314,9 @@ int sah_build(const float4* pos, uint32_t V, const uint32_t* idx, uint32_t N, in
         for (auto& th : pool) th.join();
     }
     if (too_deep) return -2;
-    // device layout: interior nodes in pre-order, leaves inline in their parents
-    out->nodes.clear();
-    out->nodes.reserve(4 * (size_t)(N > 1 ? N - 1 : 1));
-    Flat F{top, sub, out->nodes};
+    out->nodes.assign(8 * (size_t)(N > 1 ? N - 1 : 1), make_float4(0.f, 0.f, 0.f, 0.f));
+    out->more.assign(N, 0);
+    Flat F{top, sub, out->nodes, out->more};
     int tree = -1;
     int32_t root = 0;
     F.resolve(tree, root);
@@ -312,12 +329,12 @@ int sah_build(const float4* pos, uint32_t V, const uint32_t* idx, uint32_t N, in
         out->hdr.root_ref = (int32_t)R.start;
         out->hdr.root_cnt = (int32_t)(R.end - R.start);
     } else {
-        out->hdr.root_ref = 0;
+        out->hdr.root_ref = F.record(tree, R);
         out->hdr.root_cnt = 0;
-        F.emit(tree, root);
+        F.emit(tree, R);
     }
     out->max_interior_depth = F.max_interior_depth;
-    out->interior_nodes = (uint32_t)(out->nodes.size() / 4);
+    out->interior_nodes = F.interior;
     return 0;
 }
 

@@ -11,7 +11,8 @@ namespace rt {
 
 struct SahTree {
     std::vector<uint32_t> order;   // slot -> triangle (order before the build)
-    std::vector<float4> nodes;     // device node layout: 4 float4 per interior node
+    std::vector<float4> nodes;     // device records: 8 float4 per split position (N - 1)
+    std::vector<uint8_t> more;     // slot -> 1 where the next one is in the same leaf
     BvhHeader hdr;
     uint32_t interior_nodes = 0;
     uint32_t max_interior_depth = 0;

@@ -186,10 +186,9 @@ namespace {
 
 uint64_t scene_bytes(const rt_scene_desc* d) {
     const uint64_t V = d->vertex_count, N = d->triangle_count, M = d->material_count;
-    return 32 * V + 40 * N + 32 * M                     // geometry, both orders
-           + N * (24 + 48 + 32 + 64)                     // sort, triangles, leaves, nodes
-           + rt::lbvh_scratch_bytes((uint32_t)N, 4)      // radix and emit scratch
-           + 4096;
+    return 32 * V + 40 * N + 32 * M       // geometry, both orders
+           + N * (8 + 48 + 128)            // sorted keys and order, triangles, nodes
+           + 4096;                         // (a build's scratch goes back to the pool)
 }
 
 // Scene memory: a device pool that keeps what is freed for later uploads.
@@ -281,6 +280,7 @@ int32_t create_scene(rt_server* S, const rt_scene_desc* d, cudaStream_t stream, 
         rt_scene_destroy(S->ctx, sc);
         return r;
     }
+    rt::scene_release_build(sc);
     if (cudaMallocFromPoolAsync(reinterpret_cast<void**>(&out->d_lights), sizeof(rt_lights),
                                 S->pool, stream) ||
         cudaMemcpyAsync(out->d_lights, &d->lights, sizeof(rt_lights), cudaMemcpyHostToDevice,

@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render(RenderArgs a) {
         if (gid < pixels) {
             int x, y;
             pixel_of(warp_tile_order(gid, a.width, a.height), a.width, a.height, 32, x, y);
-            const PixelResult pr = render_pixel<false, REFR>(S, H, sL, a.cam, x, y, a.width,
+            const PixelResult pr = render_pixel<REFR>(S, H, sL, a.cam, x, y, a.width,
                                                              a.height, a.max_bounces, a.status);
             const uint32_t acc_r = pr.r, acc_g = pr.g, acc_b = pr.b;
             ++n_prim;

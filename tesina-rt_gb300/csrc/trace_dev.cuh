@@ -10,13 +10,24 @@
 //                 (src/kernel/secondary-ray-generator.cl:258-270)
 //   primary_dir   generate_primary_rays (src/kernel/primary-ray-generator.cl:27-103)
 //
-// Traversal order is the reference's: depth first, near child first where
-// near = left iff dot(dir, right.lo - left.lo) > 0 (trace-bvh.cl:391-409).
-// Both child boxes are tested when their parent is visited; the far child is
-// pushed with its entry distance A, and popped only if A <= the current tMax.
-// Because tMax only shrinks, this accepts exactly the nodes the reference
-// accepts when it tests the far child's box at pop time, so leaves are
-// visited in the same order and equal-t ties resolve the same way.
+// Traversal.  The reference walks a binary tree depth first, near child first
+// where near = left iff dot(dir, right.lo - left.lo) > 0
+// (trace-bvh.cl:391-409), tests a node's box when it reaches it and lets a
+// later hit of equal t win.  The kernels walk two of its levels per step over
+// four-wide records (rt_internal.cuh) and visit the same leaves in the same
+// order.  A child's box lies inside its parent's, and the slab test is
+// monotone in the box (IEEE subtraction and multiplication by one factor,
+// minima and maxima), so a box that passes has ancestors that all passed, at
+// this tMax or an earlier, larger one: which leaves the reference reaches is
+// decided by the leaves' own boxes at their turn.  Inner boxes in between may
+// be skipped; the order of the four grandchildren comes from the three sign
+// tests of the two levels, on lower corners that the minima give exactly.  A
+// pushed entry keeps its entry distance A and is dropped if A > tMax when
+// popped (tMax only shrinks, the far distances do not change).  Monotonicity
+// needs slabs without 0 * inf: a ray with an infinite inverse component, an
+// infinite or NaN origin, no usable axis or an infinite tMax (within which an
+// empty slot's box at infinity lies) is "careful": it takes the two binary
+// levels one at a time in the same loop.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -25,27 +36,18 @@
 
 namespace rt {
 
-constexpr int STACK = 32;
-
 struct Hit {
     int32_t id;
     float t, u, v;
 };
 
-__device__ __forceinline__ void load_node(const float4* __restrict__ nodes, int32_t p, float4& n0,
-                                          float4& n1, float4& n2, int4& n3) {
-    const float4* q = nodes + 4 * (size_t)p;
-    n0 = __ldg(q);
-    n1 = __ldg(q + 1);
-    n2 = __ldg(q + 2);
-    n3 = __ldg(reinterpret_cast<const int4*>(q + 3));
-}
-
+// Leaf of a scene whose root is a leaf: `cnt` triangles.
 __device__ __forceinline__ void leaf_closest(const SceneView& S, const TRay& r, int32_t start,
                                              int32_t cnt, Hit& best) {
     for (int32_t i = start; i < start + cnt; ++i) {
         float t, u, v;
-        if (!mt(S.tris, (uint32_t)i, r.o, r.d, t, u, v)) continue;
+        bool more;
+        if (!mt(S.tris, (uint32_t)i, r.o, r.d, t, u, v, more)) continue;
         if (t <= best.t && t >= r.tmin) best = Hit{i, t, u, v};
     }
 }
@@ -54,158 +56,99 @@ __device__ __forceinline__ bool leaf_any(const SceneView& S, const TRay& r, int3
                                          int32_t cnt, float tmax) {
     for (int32_t i = start; i < start + cnt; ++i) {
         float t, u, v;
-        if (!mt(S.tris, (uint32_t)i, r.o, r.d, t, u, v)) continue;
+        bool more;
+        if (!mt(S.tris, (uint32_t)i, r.o, r.d, t, u, v, more)) continue;
         if (t < tmax && t > r.tmin) return true;
     }
     return false;
 }
 
-// Traversal stack of the two-phase loop: node references with their leaf
-// counts and (DIST) the entry distances the closest-hit search prunes by.
-template <bool DIST>
-struct TravStack {
-    int32_t ref[STACK], cnt[STACK];
-    float a[DIST ? STACK : 1];
-    int sp = 0;
-    __device__ __forceinline__ bool push(int32_t r, int32_t c, float d) {
-        if (sp >= STACK) return false;
-        ref[sp] = r;
-        cnt[sp] = c;
-        if (DIST) a[sp] = d;
-        ++sp;
-        return true;
-    }
-    // The next entry (DIST: the next whose entry distance is within tmax)
-    // into cur / cur_cnt; cur = -1 when none is left.
-    __device__ __forceinline__ void pop(float tmax, int32_t& cur, int32_t& cur_cnt) {
-        cur = -1;
-        while (sp > 0) {
-            --sp;
-            if (!DIST || a[sp] <= tmax) {
-                cur = ref[sp];
-                cur_cnt = cnt[sp];
-                return;
-            }
-        }
-    }
+// Leaf of an inner node: from its first triangle to the first record whose
+// `more` mark is clear.
+__device__ __forceinline__ void leaf_closest(const SceneView& S, const TRay& r, int32_t i,
+                                             Hit& best) {
+    bool more;
+    do {
+        float t, u, v;
+        if (mt(S.tris, (uint32_t)i, r.o, r.d, t, u, v, more) && t <= best.t && t >= r.tmin)
+            best = Hit{i, t, u, v};
+        ++i;
+    } while (more);
+}
+
+__device__ __forceinline__ bool leaf_any(const SceneView& S, const TRay& r, int32_t i, float tmax) {
+    bool more;
+    do {
+        float t, u, v;
+        if (mt(S.tris, (uint32_t)i, r.o, r.d, t, u, v, more) && t < tmax && t > r.tmin) return true;
+        ++i;
+    } while (more);
+    return false;
+}
+
+// A ray's slab constants as register pairs for the two-lane f32 adds and
+// multiplies (exact in each lane: lo + (-o) is lo - o).
+struct SlabRay {
+    float2 no_xy, no_zz, iv_xy, iv_zz;
+    float tmin;
 };
-
-// Traversal in two phases per round (Aila & Laine's "while-while" loop with
-// speculative traversal): a lane walks inner nodes, setting aside the first
-// leaf it reaches and walking on, until every lane of the warp holds a leaf;
-// then the lanes intersect their leaves.  Leaves are still intersected in
-// the depth-first order above.  Nodes walked past a set-aside leaf are
-// accepted against the tMax before that leaf; any of them the exact order
-// would have dropped starts beyond the final tMax, so none of its triangles
-// is accepted (t >= entry > tMax): the same hit, equal-t ties included.
-static __device__ Hit closest_hit_ww(const SceneView& S, const BvhHeader& H, const TRay& r,
-                                     float tmax, uint32_t* status) {
-    Hit best{-1, tmax, 0.f, 0.f};
-    float A;
-    if (!slab(r, best.t, H.root_lo.x, H.root_lo.y, H.root_lo.z, H.root_hi.x, H.root_hi.y,
-              H.root_hi.z, A))
-        return best;
-    if (H.root_cnt > 0) {
-        leaf_closest(S, r, H.root_ref, H.root_cnt, best);
-        return best;
-    }
-    TravStack<true> st;
-    // the next node (inner: cnt 0, leaf: cnt > 0, none: ref < 0) and the
-    // leaf set aside
-    int32_t cur = H.root_ref, cur_cnt = 0, lf = -1, lf_cnt = 0;
-    auto pop = [&]() { st.pop(best.t, cur, cur_cnt); };
-    for (;;) {
-        while (cur >= 0 && cur_cnt == 0) {
-            float4 n0, n1, n2;
-            int4 n3;
-            load_node(S.nodes, cur, n0, n1, n2, n3);
-            // c0 = left: lo (n0.x, n0.y, n0.z) hi (n0.w, n1.x, n1.y)
-            // c1 = right: lo (n1.z, n1.w, n2.x) hi (n2.y, n2.z, n2.w)
-            const f3 dl = mk3(n1.z - n0.x, n1.w - n0.y, n2.x - n0.z);
-            const bool left_first = dot(r.d, dl) > 0.0f;
-            float a0, a1;
-            const bool h0 = slab(r, best.t, n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, a0);
-            const bool h1 = slab(r, best.t, n1.z, n1.w, n2.x, n2.y, n2.z, n2.w, a1);
-            const bool hf = left_first ? h0 : h1, hs = left_first ? h1 : h0;
-            if (hs && !st.push(left_first ? n3.y : n3.x, left_first ? n3.w : n3.z,
-                               left_first ? a1 : a0))
-                atomicOr(status, RT_DEV_OVERFLOW);
-            if (hf) {
-                cur = left_first ? n3.x : n3.y;
-                cur_cnt = left_first ? n3.z : n3.w;
-            } else {
-                pop();
-            }
-            if (cur >= 0 && cur_cnt > 0 && lf < 0) {   // set the leaf aside, walk on
-                lf = cur;
-                lf_cnt = cur_cnt;
-                pop();
-            }
-            if (__all_sync(__activemask(), lf >= 0)) break;
-        }
-        while (lf >= 0) {
-            leaf_closest(S, r, lf, lf_cnt, best);
-            lf = -1;
-            if (cur >= 0 && cur_cnt > 0) {
-                lf = cur;
-                lf_cnt = cur_cnt;
-                pop();
-            }
-        }
-        if (cur < 0) return best;
-    }
+__device__ __forceinline__ SlabRay slab_ray(const TRay& r) {
+    return SlabRay{make_float2(-r.o.x, -r.o.y), make_float2(-r.o.z, -r.o.z),
+                   make_float2(r.inv.x, r.inv.y), make_float2(r.inv.z, r.inv.z), r.tmin};
+}
+__device__ __forceinline__ float2 add_mul2(float2 a, float2 b, float2 c) {
+    float2 r;
+    asm("{\n\t.reg .b64 a, b, c;\n\t"
+        "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+        "add.rn.f32x2 a, a, b;\n\tmul.rn.f32x2 a, a, c;\n\tmov.b64 {%0, %1}, a;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return r;
 }
 
-// Any hit ends the search, whatever the order: the same two-phase loop.
-static __device__ bool any_hit_ww(const SceneView& S, const BvhHeader& H, const TRay& r, float tmax,
-                                  uint32_t* status) {
-    if (!slab_shadow(r, tmax, H.root_lo.x, H.root_lo.y, H.root_lo.z, H.root_hi.x, H.root_hi.y,
-                     H.root_hi.z))
-        return false;
-    if (H.root_cnt > 0) return leaf_any(S, r, H.root_ref, H.root_cnt, tmax);
-    TravStack<false> st;
-    int32_t cur = H.root_ref, cur_cnt = 0, lf = -1, lf_cnt = 0;
-    auto pop = [&]() { st.pop(0.f, cur, cur_cnt); };
-    for (;;) {
-        while (cur >= 0 && cur_cnt == 0) {
-            float4 n0, n1, n2;
-            int4 n3;
-            load_node(S.nodes, cur, n0, n1, n2, n3);
-            const f3 dl = mk3(n1.z - n0.x, n1.w - n0.y, n2.x - n0.z);
-            const bool left_first = dot(r.d, dl) > 0.0f;
-            const bool h0 = slab_shadow(r, tmax, n0.x, n0.y, n0.z, n0.w, n1.x, n1.y);
-            const bool h1 = slab_shadow(r, tmax, n1.z, n1.w, n2.x, n2.y, n2.z, n2.w);
-            const bool hf = left_first ? h0 : h1, hs = left_first ? h1 : h0;
-            if (hs && !st.push(left_first ? n3.y : n3.x, left_first ? n3.w : n3.z, 0.f))
-                atomicOr(status, RT_DEV_OVERFLOW);
-            if (hf) {
-                cur = left_first ? n3.x : n3.y;
-                cur_cnt = left_first ? n3.z : n3.w;
-            } else {
-                pop();
-            }
-            if (cur >= 0 && cur_cnt > 0 && lf < 0) {
-                lf = cur;
-                lf_cnt = cur_cnt;
-                pop();
-            }
-            if (__all_sync(__activemask(), lf >= 0)) break;
-        }
-        while (lf >= 0) {
-            if (leaf_any(S, r, lf, lf_cnt, tmax)) return true;
-            lf = -1;
-            if (cur >= 0 && cur_cnt > 0) {
-                lf = cur;
-                lf_cnt = cur_cnt;
-                pop();
-            }
-        }
-        if (cur < 0) return false;
-    }
+// The slab test of a slot (`slab`; also slab_shadow's result wherever no slab
+// is NaN by 0 * inf: the two differ in their NaN rules only).
+__device__ __forceinline__ bool slab_slot(const SlabRay& r, float tmax, const Slot& s, float& A) {
+    const float2 l = add_mul2(make_float2(s.lox, s.loy), r.no_xy, r.iv_xy);
+    const float2 h = add_mul2(make_float2(s.hix, s.hiy), r.no_xy, r.iv_xy);
+    const float2 z = add_mul2(make_float2(s.loz, s.hiz), r.no_zz, r.iv_zz);
+    A = fmaxf(max3f(r.tmin, fminf(l.x, h.x), fminf(l.y, h.y)), fminf(z.x, z.y));
+    const float B = fminf(min3f(tmax, fmaxf(l.x, h.x), fmaxf(l.y, h.y)), fmaxf(z.x, z.y));
+    return A <= B;
 }
 
+// Rays whose slab tests need not be monotone (see the top of the file).
+__device__ __forceinline__ bool careful_ray(const TRay& r) {
+    const float INF = __int_as_float(0x7f800000);
+    const bool inf = fabsf(r.inv.x) == INF || fabsf(r.inv.y) == INF || fabsf(r.inv.z) == INF;
+    const bool axis = r.inv.x == r.inv.x || r.inv.y == r.inv.y || r.inv.z == r.inv.z;
+    return inf || !axis || !(fabsf(r.o.x) < INF && fabsf(r.o.y) < INF && fabsf(r.o.z) < INF);
+}
+
+// The two binary children of a record in place of its four grandchildren:
+// slot 0 and 2 become the left and right child, 1 and 3 are to be ignored.
+__device__ __forceinline__ void binary_step(Slot& a, const Slot& b) {
+    if (slot_pair_is_leaf(b)) return;   // the child is a leaf, in slot a alone
+    const int32_t self = slot_pair_node(a);
+    a.lox = fminf(a.lox, b.lox); a.loy = fminf(a.loy, b.loy); a.loz = fminf(a.loz, b.loz);
+    a.hix = fmaxf(a.hix, b.hix); a.hiy = fmaxf(a.hiy, b.hiy); a.hiz = fmaxf(a.hiz, b.hiz);
+    a.code = self;
+}
+
+// Stack entries: a path of 32 binary levels (the deepest tree: 32 key bits)
+// is 16 steps, each of which leaves at most three entries behind.
+constexpr int STACK = 48;
+constexpr int32_t NO_NODE = (int32_t)0x80000000;   // below every leaf code
+
+// What bounds it: each step waits for one record (L1 / L2 latency) and the
+// lanes of a warp take different numbers of steps.  Two binary levels per
+// step against one (64 B pair records, four 128-bit loads): mid-scale frame
+// from host buffers 5.05 -> 3.10 ms, 3840 x 2160 of 17.7 M triangles 18.4-20.2
+// -> 10.3 ms, the mid-scale field under glass 25.5 -> 13.0 ms, 64 soups built
+// and rendered 17.8 -> 10.1 ms.  Leaves, met directly or popped, are tested in
+// one place, so that the lanes that have one test it together.
 static __device__ Hit closest_hit(const SceneView& S, const BvhHeader& H, const TRay& r, float tmax,
-                           uint32_t* status) {
+                                  uint32_t* status) {
     Hit best{-1, tmax, 0.f, 0.f};
     float A;
     if (!slab(r, best.t, H.root_lo.x, H.root_lo.y, H.root_lo.z, H.root_hi.x, H.root_hi.y,
@@ -215,111 +158,119 @@ static __device__ Hit closest_hit(const SceneView& S, const BvhHeader& H, const 
         leaf_closest(S, r, H.root_ref, H.root_cnt, best);
         return best;
     }
-    int32_t st_ref[STACK], st_cnt[STACK];
-    float st_a[STACK];
+    int2 st[STACK];   // code, entry distance
     int sp = 0;
+    const SlabRay w = slab_ray(r);
+    const bool careful = careful_ray(r) || !(tmax < __int_as_float(0x7f800000));
+    const float MISS = __int_as_float(0x7fc00000);   // NaN: an entry distance never is
     int32_t cur = H.root_ref;
     for (;;) {
-        float4 n0, n1, n2;
-        int4 n3;
-        load_node(S.nodes, cur, n0, n1, n2, n3);
-        // c0 = left: lo (n0.x, n0.y, n0.z) hi (n0.w, n1.x, n1.y)
-        // c1 = right: lo (n1.z, n1.w, n2.x) hi (n2.y, n2.z, n2.w)
-        const f3 dl = mk3(n1.z - n0.x, n1.w - n0.y, n2.x - n0.z);
-        const bool left_first = dot(r.d, dl) > 0.0f;
-        float a0, a1;
-        const bool h0 = slab(r, best.t, n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, a0);
-        const bool h1 = slab(r, best.t, n1.z, n1.w, n2.x, n2.y, n2.z, n2.w, a1);
-        const bool hf = left_first ? h0 : h1, hs = left_first ? h1 : h0;
-        const int32_t rf = left_first ? n3.x : n3.y, rs = left_first ? n3.y : n3.x;
-        const int32_t cf = left_first ? n3.z : n3.w, cs = left_first ? n3.w : n3.z;
-        const float as = left_first ? a1 : a0;
-        if (hs) {
-            if (sp < STACK) {
-                st_ref[sp] = rs;
-                st_cnt[sp] = cs;
-                st_a[sp] = as;
-                ++sp;
-            } else {
-                atomicOr(status, RT_DEV_OVERFLOW);
-            }
+        Slot s0 = load_slot(S.nodes, cur, 0), s1 = load_slot(S.nodes, cur, 1),
+             s2 = load_slot(S.nodes, cur, 2), s3 = load_slot(S.nodes, cur, 3);
+        // the reference's three near-first tests (an empty slot's corner is +inf)
+        const bool l_first =
+            dot(r.d, mk3(fminf(s2.lox, s3.lox) - fminf(s0.lox, s1.lox),
+                         fminf(s2.loy, s3.loy) - fminf(s0.loy, s1.loy),
+                         fminf(s2.loz, s3.loz) - fminf(s0.loz, s1.loz))) > 0.0f;
+        const bool ll_first = dot(r.d, mk3(s1.lox - s0.lox, s1.loy - s0.loy, s1.loz - s0.loz)) > 0.0f;
+        const bool rl_first = dot(r.d, mk3(s3.lox - s2.lox, s3.loy - s2.loy, s3.loz - s2.loz)) > 0.0f;
+        if (careful) {
+            binary_step(s0, s1);
+            binary_step(s2, s3);
         }
-        bool descend = false;
-        if (hf) {
-            if (cf > 0)
-                leaf_closest(S, r, rf, cf, best);
-            else {
-                cur = rf;
-                descend = true;
-            }
+        float a0, a1, a2, a3;
+        if (!slab_slot(w, best.t, s0, a0)) a0 = MISS;
+        if (!slab_slot(w, best.t, s1, a1) || careful) a1 = MISS;
+        if (!slab_slot(w, best.t, s2, a2)) a2 = MISS;
+        if (!slab_slot(w, best.t, s3, a3) || careful) a3 = MISS;
+        int32_t c0 = s0.code, c1 = s1.code, c2 = s2.code, c3 = s3.code;
+        // careful: slot 0 before slot 1 whatever the (meaningless) inner test says
+        swap_if(!ll_first, c0, c1, a0, a1);
+        swap_if(!rl_first, c2, c3, a2, a3);
+        swap_if(!l_first, c0, c2, a0, a2);
+        swap_if(!l_first, c1, c3, a1, a3);
+        // far to near: the nearest hit goes on, the others are pushed
+        int32_t next = NO_NODE;
+        float na = 0.f;
+        if (sp > STACK - 3) {
+            atomicOr(status, RT_DEV_OVERFLOW);
+        } else {
+            auto take = [&](int32_t c, float a) {
+                if (a == a) {
+                    if (next != NO_NODE) st[sp++] = make_int2(next, __float_as_int(na));
+                    next = c;
+                    na = a;
+                }
+            };
+            take(c3, a3);
+            take(c2, a2);
+            take(c1, a1);
+            take(c0, a0);
         }
-        if (descend) continue;
-        // pop
-        bool found = false;
-        while (sp > 0) {
-            --sp;
-            if (!(st_a[sp] <= best.t)) continue;
-            if (st_cnt[sp] > 0) {
-                leaf_closest(S, r, st_ref[sp], st_cnt[sp], best);
-                continue;
+        auto pop = [&]() {
+            next = NO_NODE;
+            while (sp > 0) {
+                const int2 e = st[--sp];
+                if (__int_as_float(e.y) <= best.t) {
+                    next = e.x;
+                    break;
+                }
             }
-            cur = st_ref[sp];
-            found = true;
-            break;
+        };
+        if (next == NO_NODE) pop();
+        while (next < 0) {   // leaves, met directly or popped, in one place
+            if (next == NO_NODE) return best;
+            leaf_closest(S, r, ~next, best);
+            pop();
         }
-        if (!found) return best;
+        cur = next;
     }
 }
 
+// Whether anything blocks the ray.  tMax does not shrink, so the order of
+// the visits does not matter.
 static __device__ bool any_hit(const SceneView& S, const BvhHeader& H, const TRay& r, float tmax,
-                        uint32_t* status) {
+                               uint32_t* status) {
     if (!slab_shadow(r, tmax, H.root_lo.x, H.root_lo.y, H.root_lo.z, H.root_hi.x, H.root_hi.y,
                      H.root_hi.z))
         return false;
     if (H.root_cnt > 0) return leaf_any(S, r, H.root_ref, H.root_cnt, tmax);
-    int32_t st_ref[STACK], st_cnt[STACK];
+    int32_t st[STACK];
     int sp = 0;
+    const SlabRay w = slab_ray(r);
+    const bool careful = careful_ray(r);
     int32_t cur = H.root_ref;
     for (;;) {
-        float4 n0, n1, n2;
-        int4 n3;
-        load_node(S.nodes, cur, n0, n1, n2, n3);
-        const f3 dl = mk3(n1.z - n0.x, n1.w - n0.y, n2.x - n0.z);
-        const bool left_first = dot(r.d, dl) > 0.0f;
-        const bool h0 = slab_shadow(r, tmax, n0.x, n0.y, n0.z, n0.w, n1.x, n1.y);
-        const bool h1 = slab_shadow(r, tmax, n1.z, n1.w, n2.x, n2.y, n2.z, n2.w);
-        const bool hf = left_first ? h0 : h1, hs = left_first ? h1 : h0;
-        const int32_t rf = left_first ? n3.x : n3.y, rs = left_first ? n3.y : n3.x;
-        const int32_t cf = left_first ? n3.z : n3.w, cs = left_first ? n3.w : n3.z;
-        if (hs) {
-            if (sp < STACK) {
-                st_ref[sp] = rs;
-                st_cnt[sp] = cs;
-                ++sp;
-            } else {
-                atomicOr(status, RT_DEV_OVERFLOW);
+        int32_t next = NO_NODE;
+        auto take = [&](bool hit, int32_t c) {
+            if (hit) {
+                if (next != NO_NODE) st[sp++] = next;
+                next = c;
+            }
+        };
+        if (sp > STACK - 3) {
+            atomicOr(status, RT_DEV_OVERFLOW);
+        } else if (careful) {   // the shadow kernel's own NaN rules
+#pragma unroll 1
+            for (int k = 0; k < 4; k += 2) {
+                Slot a = load_slot(S.nodes, cur, k);
+                binary_step(a, load_slot(S.nodes, cur, k + 1));
+                take(slab_shadow(r, tmax, a.lox, a.loy, a.loz, a.hix, a.hiy, a.hiz), a.code);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const Slot s = load_slot(S.nodes, cur, k);
+                float A;
+                take(slab_slot(w, tmax, s, A), s.code);
             }
         }
-        if (hf) {
-            if (cf > 0) {
-                if (leaf_any(S, r, rf, cf, tmax)) return true;
-            } else {
-                cur = rf;
-                continue;
-            }
+        if (next == NO_NODE && sp > 0) next = st[--sp];
+        while (next < 0) {
+            if (next == NO_NODE || leaf_any(S, r, ~next, tmax)) return next != NO_NODE;
+            next = sp > 0 ? st[--sp] : NO_NODE;
         }
-        bool found = false;
-        while (sp > 0) {
-            --sp;
-            if (st_cnt[sp] > 0) {
-                if (leaf_any(S, r, st_ref[sp], st_cnt[sp], tmax)) return true;
-                continue;
-            }
-            cur = st_ref[sp];
-            found = true;
-            break;
-        }
-        if (!found) return false;
+        cur = next;
     }
 }
 
@@ -351,8 +302,6 @@ __device__ __forceinline__ HitInfo complete_hit(const SceneView& S, f3 o, f3 d, 
 
 // Shadow ray of shadow_trace_single for one light (shadow-trace-bvh.cl:
 // 375-418); point lights as spot lights without a cone.
-// WW: the two-phase traversal (any_hit_ww) instead of any_hit.
-template <bool WW = false>
 __device__ __forceinline__ bool occluded(const SceneView& S, const BvhHeader& H, const rt_light& L,
                                          f3 hp, uint32_t* status) {
     f3 dir;
@@ -368,7 +317,7 @@ __device__ __forceinline__ bool occluded(const SceneView& S, const BvhHeader& H,
     }
     const f3 inv = mk3(1.0f / dir.x, 1.0f / dir.y, 1.0f / dir.z);
     const TRay r = make_tray(hp, dir, inv, 0.01f);
-    return WW ? any_hit_ww(S, H, r, 1e37f, status) : any_hit(S, H, r, 1e37f, status);
+    return any_hit(S, H, r, 1e37f, status);
 }
 
 // Light direction (from the light toward the hit) and colour at a hit, as
@@ -602,8 +551,8 @@ constexpr int REFR_STACK = 16;   // pending rays per lane: one per level of the 
 // contribution * reflectiveness * (1 - R), R = Schlick's factor, 1 without
 // refraction), each traced, shadowed and shaded as the reference's wavefront
 // does.  The sums are integers, so the depth-first order of this tree walk
-// gives the wavefront's image.  WW: the two-phase traversal.
-template <bool WW = false, bool REFR = false>
+// gives the wavefront's image.
+template <bool REFR = false>
 __device__ __forceinline__ PixelResult render_pixel(const SceneView& S, const BvhHeader& H,
                                                     const rt_lights& L, const rt_camera& cam,
                                                     int x, int y, int w, int h, int max_bounces,
@@ -618,7 +567,7 @@ __device__ __forceinline__ PixelResult render_pixel(const SceneView& S, const Bv
         bool next = false;
         const f3 inv = mk3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
         const TRay r = make_tray(o, d, inv, tmin);
-        const Hit hit = WW ? closest_hit_ww(S, H, r, tmax, status) : closest_hit(S, H, r, tmax, status);
+        const Hit hit = closest_hit(S, H, r, tmax, status);
         if (hit.id >= 0) {
             ++res.hits;
             const HitInfo hi = complete_hit(S, o, d, hit);
@@ -626,7 +575,7 @@ __device__ __forceinline__ PixelResult render_pixel(const SceneView& S, const Bv
             uint32_t mask = 0;
             for (int l = 0; l < L.count; ++l)
                 if (!light_vanishes(L.light[l], mat, hi.hp, hi.n, d) &&
-                    occluded<WW>(S, H, L.light[l], hi.hp, status))
+                    occluded(S, H, L.light[l], hi.hp, status))
                     mask |= 1u << l;
             res.shadow += (uint32_t)L.count;
             const uint3 c = shade_hit(L, mat, hi.hp, hi.n, d, contribution, mask);
