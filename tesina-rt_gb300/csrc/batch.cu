@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
             const BatchView& V = A.views[v];
             const BvhHeader H = *V.scene.hdr;
             const TRay r = make_tray(o, d, mk3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z), tmin);
-            hit = closest_hit(V.scene, H, r, tmax, A.status);
+            hit = closest_hit<false, false>(V.scene, H, r, tmax, A.status);
             hit_ok = hit.id >= 0;
         }
         const unsigned hm = __ballot_sync(0xffffffffu, hit_ok);

@@ -227,7 +227,7 @@ int32_t scene_ensure_build(rt_scene* s) {
     free_build(s);
     const size_t nn = n > 1 ? n - 1 : 1;
     if (salloc_n(s, &s->d_keys_unsorted, n) || salloc_n(s, &s->d_keys_sorted, n) ||
-        salloc_n(s, &s->d_vals_sorted, n) || salloc_n(s, &s->d_tris, 3 * (size_t)n) ||
+        salloc_n(s, &s->d_vals_sorted, n) || salloc_n(s, &s->d_tris, 3 * ((size_t)n + 1)) ||
         salloc_n(s, &s->d_nodes, 8 * nn) || salloc_n(s, &s->d_hdr, 1) || salloc(s, &s->d_scratch, need_scratch)) {
         cudaGetLastError();
         free_build(s);

@@ -129,7 +129,7 @@ __device__ __forceinline__ Hit root_closest(const InstanceRoot& R, f3 o, f3 d, f
     const f3 to = mat_apply(R.trinv, o, 1.0f);
     const TRay tr = make_tray(to, td, mk3(1.0f / td.x, 1.0f / td.y, 1.0f / td.z), tmin);
     const BvhHeader H = *R.scene.hdr;
-    Hit h = closest_hit(R.scene, H, tr, tmax, status);
+    Hit h = closest_hit<true, false>(R.scene, H, tr, tmax, status);
     if (h.id >= 0) {
         const f3 hp = mat_apply(R.tr, add(to, muls(td, h.t)), 1.0f);
         const f3 dv = sub(hp, o);
@@ -218,7 +218,7 @@ __device__ __forceinline__ bool occluded_multi(const InstanceArgs& A, const rt_l
         const f3 to = mat_apply(R.trinv, hp, 1.0f);
         const TRay tr = make_tray(to, td, mk3(1.0f / td.x, 1.0f / td.y, 1.0f / td.z), 0.01f);
         const BvhHeader H = *R.scene.hdr;
-        if (any_hit(R.scene, H, tr, 1e37f, A.status)) return true;
+        if (any_hit<true, false>(R.scene, H, tr, 1e37f, A.status)) return true;
     }
     return false;
 }
@@ -267,8 +267,10 @@ struct InstPool {
 };
 }  // namespace
 
+// 5 blocks per SM, 102 registers: at 6 the four-wide traversal spills (16 roots
+// at 1920 x 1080: 2.16 -> 2.11 ms; 4 blocks 2.24).
 #ifndef RT_INST_MINB
-#define RT_INST_MINB 6
+#define RT_INST_MINB 5
 #endif
 template <int MAXB>
 __global__ void __launch_bounds__(128, MAXB == 6 ? 5 : RT_INST_MINB) k_render_instances(InstanceArgs A) {

@@ -55,7 +55,7 @@ __host__ __device__ __forceinline__ int32_t slot_pair_node(const Slot& a) {
 // Triangle records in sorted order, 48 B: v0, e1 = v1 - v0, e2 = v2 - v0
 // (the same float subtractions as leaf_hit, trace-bvh.cl:297-298).  v0.w is
 // 1 where the next triangle belongs to the same leaf, else 0: a leaf is found
-// from its first triangle alone.
+// from its first triangle alone.  One record past the last is allocated.
 struct TriRec {
     float4 v0, e1, e2;
 };
@@ -189,15 +189,14 @@ __device__ __forceinline__ void swap_if(bool c, int32_t& a, int32_t& b, float& t
     tb = v;
 }
 
-// Möller–Trumbore of leaf_hit (trace-bvh.cl:275-328); `more`: the triangle
-// after this one is in the same leaf.
-__device__ __forceinline__ bool mt(const float4* __restrict__ tris, uint32_t i, f3 o, f3 d, float& t,
-                                   float& u, float& v, bool& more) {
-    const float4 a = __ldg(&tris[3 * (size_t)i + 0]);
-    const float4 b = __ldg(&tris[3 * (size_t)i + 1]);
-    const float4 c = __ldg(&tris[3 * (size_t)i + 2]);
-    more = a.w != 0.0f;
-    f3 v0 = ld3(a), e1 = ld3(b), e2 = ld3(c);
+__device__ __forceinline__ TriRec load_tri(const float4* __restrict__ tris, int32_t i) {
+    const float4* q = tris + 3 * (size_t)i;
+    return TriRec{__ldg(q), __ldg(q + 1), __ldg(q + 2)};
+}
+
+// Möller–Trumbore of leaf_hit (trace-bvh.cl:275-328).
+__device__ __forceinline__ bool mt(const TriRec& T, f3 o, f3 d, float& t, float& u, float& v) {
+    f3 v0 = ld3(T.v0), e1 = ld3(T.e1), e2 = ld3(T.e2);
     f3 h = cross(d, e2);
     float aa = dot(e1, h);
     if (aa > -1e-26f && aa < 1e-26f) return false;

@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_pool(RenderArgs a) {
         Hit hit{-1, 0.f, 0.f, 0.f};
         if (have) {
             const TRay r = make_tray(o, d, mk3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z), tmin);
-            hit = closest_hit(S, H, r, tmax, a.status);
+            hit = closest_hit<false, false>(S, H, r, tmax, a.status);
             hit_ok = hit.id >= 0;
         }
         const unsigned hm = __ballot_sync(0xffffffffu, hit_ok);
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_pool_refr(RenderArgs a
         Hit hit{-1, 0.f, 0.f, 0.f};
         if (have) {
             const TRay r = make_tray(o, d, mk3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z), tmin);
-            hit = closest_hit(S, H, r, tmax, a.status);
+            hit = closest_hit<false, true>(S, H, r, tmax, a.status);
             hit_ok = hit.id >= 0;
         }
         const unsigned hm = __ballot_sync(0xffffffffu, hit_ok);
@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_pool_refr(RenderArgs a
                                        mk3(Q.hd[0][k], Q.hd[1][k], Q.hd[2][k]));
             },
             [&](int k, int l) {
-                if (occluded(S, H, sL.light[l], mk3(Q.hp[0][k], Q.hp[1][k], Q.hp[2][k]), a.status))
+                if (occluded<false, true>(S, H, sL.light[l], mk3(Q.hp[0][k], Q.hp[1][k], Q.hp[2][k]), a.status))
                     atomicOr(&Q.hmask[k], 1u << l);
             });
         __syncwarp();
@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(128) k_trace(SceneView S, const rt_sample* __r
     const rt_ray& ray = smp[i].ray;
     const f3 o = f3_of(ray.ori), d = f3_of(ray.dir);
     const TRay r = make_tray(o, d, f3_of(ray.inv_dir), ray.tmin);
-    const Hit h = closest_hit(S, sH, r, ray.tmax, status);
+    const Hit h = closest_hit<true, true>(S, sH, r, ray.tmax, status);
     if (h.id < 0) {
         hits[i].hit = 0;
         return;
@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(128) k_shadow(SceneView S, rt_lights Ls, int n
     const f3 hp = f3_of(hits[i].hit_point);
     uint32_t mask = 0;
     for (int l = 0; l < Ls.count; ++l)
-        if (occluded(S, sH, Ls.light[l], hp, status)) mask |= 1u << l;
+        if (occluded<true, true>(S, sH, Ls.light[l], hp, status)) mask |= 1u << l;
     hits[i].shadow_hit = (uint8_t)mask;
 }
 

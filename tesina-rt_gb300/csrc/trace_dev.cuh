@@ -46,8 +46,7 @@ __device__ __forceinline__ void leaf_closest(const SceneView& S, const TRay& r, 
                                              int32_t cnt, Hit& best) {
     for (int32_t i = start; i < start + cnt; ++i) {
         float t, u, v;
-        bool more;
-        if (!mt(S.tris, (uint32_t)i, r.o, r.d, t, u, v, more)) continue;
+        if (!mt(load_tri(S.tris, i), r.o, r.d, t, u, v)) continue;
         if (t <= best.t && t >= r.tmin) best = Hit{i, t, u, v};
     }
 }
@@ -56,34 +55,52 @@ __device__ __forceinline__ bool leaf_any(const SceneView& S, const TRay& r, int3
                                          int32_t cnt, float tmax) {
     for (int32_t i = start; i < start + cnt; ++i) {
         float t, u, v;
-        bool more;
-        if (!mt(S.tris, (uint32_t)i, r.o, r.d, t, u, v, more)) continue;
+        if (!mt(load_tri(S.tris, i), r.o, r.d, t, u, v)) continue;
         if (t < tmax && t > r.tmin) return true;
     }
     return false;
 }
 
 // Leaf of an inner node: from its first triangle to the first record whose
-// `more` mark is clear.
+// `more` mark is clear.  PAIR: two records are read at a time, so that most
+// leaves (at most three triangles with the usual minimum) wait for memory
+// once; the second may lie one past the scene's last record, which is
+// allocated.  Worth its registers where the kernel has them to spare: the
+// stage kernels (1000 x 701 of 10k triangles, whole pipeline 712 -> 672 us) and
+// the glass pool (12.1 -> 11.9 ms); the instanced render loses 8 % to spills.
+template <bool PAIR>
 __device__ __forceinline__ void leaf_closest(const SceneView& S, const TRay& r, int32_t i,
                                              Hit& best) {
-    bool more;
-    do {
+    for (;;) {
+        const TriRec A = load_tri(S.tris, i);
+        TriRec B;
+        if (PAIR) B = load_tri(S.tris, i + 1);
         float t, u, v;
-        if (mt(S.tris, (uint32_t)i, r.o, r.d, t, u, v, more) && t <= best.t && t >= r.tmin)
-            best = Hit{i, t, u, v};
+        if (mt(A, r.o, r.d, t, u, v) && t <= best.t && t >= r.tmin) best = Hit{i, t, u, v};
+        if (A.v0.w == 0.0f) return;
         ++i;
-    } while (more);
+        if (!PAIR) continue;
+        if (mt(B, r.o, r.d, t, u, v) && t <= best.t && t >= r.tmin) best = Hit{i, t, u, v};
+        if (B.v0.w == 0.0f) return;
+        ++i;
+    }
 }
 
+template <bool PAIR>
 __device__ __forceinline__ bool leaf_any(const SceneView& S, const TRay& r, int32_t i, float tmax) {
-    bool more;
-    do {
+    for (;;) {
+        const TriRec A = load_tri(S.tris, i);
+        TriRec B;
+        if (PAIR) B = load_tri(S.tris, i + 1);
         float t, u, v;
-        if (mt(S.tris, (uint32_t)i, r.o, r.d, t, u, v, more) && t < tmax && t > r.tmin) return true;
+        if (mt(A, r.o, r.d, t, u, v) && t < tmax && t > r.tmin) return true;
+        if (A.v0.w == 0.0f) return false;
         ++i;
-    } while (more);
-    return false;
+        if (!PAIR) continue;
+        if (mt(B, r.o, r.d, t, u, v) && t < tmax && t > r.tmin) return true;
+        if (B.v0.w == 0.0f) return false;
+        ++i;
+    }
 }
 
 // A ray's slab constants as register pairs for the two-lane f32 adds and
@@ -145,8 +162,34 @@ constexpr int32_t NO_NODE = (int32_t)0x80000000;   // below every leaf code
 // step against one (64 B pair records, four 128-bit loads): mid-scale frame
 // from host buffers 5.05 -> 3.10 ms, 3840 x 2160 of 17.7 M triangles 18.4-20.2
 // -> 10.3 ms, the mid-scale field under glass 25.5 -> 13.0 ms, 64 soups built
-// and rendered 17.8 -> 10.1 ms.  Leaves, met directly or popped, are tested in
-// one place, so that the lanes that have one test it together.
+// and rendered 17.8 -> 10.1 ms.
+//
+// Leaves, met directly or popped, are tested in one place, by the lanes that
+// have one together: a lane that reaches a leaf waits until the lanes with a
+// leaf are a third of those still searching (leaf_turn).  At once, a leaf step
+// had 5.2-6.8 lanes where a node step had 17-18; against that rule: 4K of 17.7
+// M triangles 12.7 -> 11.8 ms, glass 13.3 -> 12.1, 64 soups 10.1 -> 9.3, stage
+// pipeline 870 -> 712 us, thumbnail 71 -> 74 us (a fixed 4 to 16 lanes gains
+// less; setting a leaf aside and walking on loses 2-5 %).  STAY: lanes whose
+// search has ended stay for the votes, which keeps the warp together; faster
+// in the stage kernels (784 -> 712 us), the instanced render and the
+// one-path-per-lane kernels (served burst 5.5 -> 4.8 ms), slower in the pooled
+// ones.
+template <bool STAY>
+__device__ __forceinline__ bool leaf_turn(unsigned group, int32_t next, bool& ended) {
+    if (STAY) {
+        const unsigned lm = __ballot_sync(group, next < 0 && next != NO_NODE);
+        const unsigned nm = __ballot_sync(group, next >= 0);
+        ended = (lm | nm) == 0u;
+        return 2 * __popc(lm) >= __popc(nm) && next < 0 && next != NO_NODE;
+    }
+    ended = next == NO_NODE;
+    if (ended) return false;
+    const unsigned am = __activemask(), lm = __ballot_sync(am, next < 0);
+    return 3 * __popc(lm) >= __popc(am) && next < 0;
+}
+
+template <bool STAY, bool PAIR>
 static __device__ Hit closest_hit(const SceneView& S, const BvhHeader& H, const TRay& r, float tmax,
                                   uint32_t* status) {
     Hit best{-1, tmax, 0.f, 0.f};
@@ -163,8 +206,19 @@ static __device__ Hit closest_hit(const SceneView& S, const BvhHeader& H, const 
     const SlabRay w = slab_ray(r);
     const bool careful = careful_ray(r) || !(tmax < __int_as_float(0x7f800000));
     const float MISS = __int_as_float(0x7fc00000);   // NaN: an entry distance never is
-    int32_t cur = H.root_ref;
-    for (;;) {
+    const unsigned group = STAY ? __activemask() : 0u;
+    int32_t next = H.root_ref;
+    auto pop = [&]() {
+        next = NO_NODE;
+        while (sp > 0) {
+            const int2 e = st[--sp];
+            if (__int_as_float(e.y) <= best.t) {
+                next = e.x;
+                break;
+            }
+        }
+    };
+    auto node = [&](int32_t cur) {
         Slot s0 = load_slot(S.nodes, cur, 0), s1 = load_slot(S.nodes, cur, 1),
              s2 = load_slot(S.nodes, cur, 2), s3 = load_slot(S.nodes, cur, 3);
         // the reference's three near-first tests (an empty slot's corner is +inf)
@@ -190,7 +244,7 @@ static __device__ Hit closest_hit(const SceneView& S, const BvhHeader& H, const 
         swap_if(!l_first, c0, c2, a0, a2);
         swap_if(!l_first, c1, c3, a1, a3);
         // far to near: the nearest hit goes on, the others are pushed
-        int32_t next = NO_NODE;
+        next = NO_NODE;
         float na = 0.f;
         if (sp > STACK - 3) {
             atomicOr(status, RT_DEV_OVERFLOW);
@@ -207,28 +261,23 @@ static __device__ Hit closest_hit(const SceneView& S, const BvhHeader& H, const 
             take(c1, a1);
             take(c0, a0);
         }
-        auto pop = [&]() {
-            next = NO_NODE;
-            while (sp > 0) {
-                const int2 e = st[--sp];
-                if (__int_as_float(e.y) <= best.t) {
-                    next = e.x;
-                    break;
-                }
-            }
-        };
         if (next == NO_NODE) pop();
-        while (next < 0) {   // leaves, met directly or popped, in one place
-            if (next == NO_NODE) return best;
-            leaf_closest(S, r, ~next, best);
+    };
+    for (;;) {
+        if (next >= 0) node(next);
+        bool ended;
+        const bool leaf = leaf_turn<STAY>(group, next, ended);
+        if (ended) return best;
+        if (leaf) {
+            leaf_closest<PAIR>(S, r, ~next, best);
             pop();
         }
-        cur = next;
     }
 }
 
 // Whether anything blocks the ray.  tMax does not shrink, so the order of
 // the visits does not matter.
+template <bool STAY, bool PAIR>
 static __device__ bool any_hit(const SceneView& S, const BvhHeader& H, const TRay& r, float tmax,
                                uint32_t* status) {
     if (!slab_shadow(r, tmax, H.root_lo.x, H.root_lo.y, H.root_lo.z, H.root_hi.x, H.root_hi.y,
@@ -239,9 +288,11 @@ static __device__ bool any_hit(const SceneView& S, const BvhHeader& H, const TRa
     int sp = 0;
     const SlabRay w = slab_ray(r);
     const bool careful = careful_ray(r);
-    int32_t cur = H.root_ref;
-    for (;;) {
-        int32_t next = NO_NODE;
+    const unsigned group = STAY ? __activemask() : 0u;
+    int32_t next = H.root_ref;
+    bool found = false;
+    auto node = [&](int32_t cur) {
+        next = NO_NODE;
         auto take = [&](bool hit, int32_t c) {
             if (hit) {
                 if (next != NO_NODE) st[sp++] = next;
@@ -266,11 +317,16 @@ static __device__ bool any_hit(const SceneView& S, const BvhHeader& H, const TRa
             }
         }
         if (next == NO_NODE && sp > 0) next = st[--sp];
-        while (next < 0) {
-            if (next == NO_NODE || leaf_any(S, r, ~next, tmax)) return next != NO_NODE;
-            next = sp > 0 ? st[--sp] : NO_NODE;
+    };
+    for (;;) {
+        if (next >= 0) node(next);
+        bool ended;
+        const bool leaf = leaf_turn<STAY>(group, next, ended);
+        if (ended) return found;
+        if (leaf) {
+            found = leaf_any<PAIR>(S, r, ~next, tmax);
+            next = !found && sp > 0 ? st[--sp] : NO_NODE;
         }
-        cur = next;
     }
 }
 
@@ -302,6 +358,7 @@ __device__ __forceinline__ HitInfo complete_hit(const SceneView& S, f3 o, f3 d, 
 
 // Shadow ray of shadow_trace_single for one light (shadow-trace-bvh.cl:
 // 375-418); point lights as spot lights without a cone.
+template <bool STAY = false, bool PAIR = false>
 __device__ __forceinline__ bool occluded(const SceneView& S, const BvhHeader& H, const rt_light& L,
                                          f3 hp, uint32_t* status) {
     f3 dir;
@@ -317,7 +374,7 @@ __device__ __forceinline__ bool occluded(const SceneView& S, const BvhHeader& H,
     }
     const f3 inv = mk3(1.0f / dir.x, 1.0f / dir.y, 1.0f / dir.z);
     const TRay r = make_tray(hp, dir, inv, 0.01f);
-    return any_hit(S, H, r, 1e37f, status);
+    return any_hit<STAY, PAIR>(S, H, r, 1e37f, status);
 }
 
 // Light direction (from the light toward the hit) and colour at a hit, as
@@ -567,7 +624,7 @@ __device__ __forceinline__ PixelResult render_pixel(const SceneView& S, const Bv
         bool next = false;
         const f3 inv = mk3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
         const TRay r = make_tray(o, d, inv, tmin);
-        const Hit hit = closest_hit(S, H, r, tmax, status);
+        const Hit hit = closest_hit<true, false>(S, H, r, tmax, status);
         if (hit.id >= 0) {
             ++res.hits;
             const HitInfo hi = complete_hit(S, o, d, hit);
@@ -575,7 +632,7 @@ __device__ __forceinline__ PixelResult render_pixel(const SceneView& S, const Bv
             uint32_t mask = 0;
             for (int l = 0; l < L.count; ++l)
                 if (!light_vanishes(L.light[l], mat, hi.hp, hi.n, d) &&
-                    occluded(S, H, L.light[l], hi.hp, status))
+                    occluded<true, false>(S, H, L.light[l], hi.hp, status))
                     mask |= 1u << l;
             res.shadow += (uint32_t)L.count;
             const uint3 c = shade_hit(L, mat, hi.hp, hi.n, d, contribution, mask);
