@@ -113,6 +113,17 @@ __device__ __forceinline__ SlabRay slab_ray(const TRay& r) {
     return SlabRay{make_float2(-r.o.x, -r.o.y), make_float2(-r.o.z, -r.o.z),
                    make_float2(r.inv.x, r.inv.y), make_float2(r.inv.z, r.inv.z), r.tmin};
 }
+// dot(d, b - a) > 0 for the lower corners a and b of two boxes, in dot()'s
+// order (b - a as the two-lane b + a * -1, which rounds the same).
+__device__ __forceinline__ bool near_first(f3 d, float ax, float ay, float az, float bx, float by,
+                                           float bz) {
+    float px, py;
+    asm("{\n\t.reg .b64 a, b, c, m;\n\t"
+        "mov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\tmov.b64 m, {%8, %8};\n\t"
+        "fma.rn.f32x2 a, a, m, b;\n\tmul.rn.f32x2 a, a, c;\n\tmov.b64 {%0, %1}, a;\n\t}"
+        : "=f"(px), "=f"(py) : "f"(ax), "f"(ay), "f"(bx), "f"(by), "f"(d.x), "f"(d.y), "f"(-1.0f));
+    return (px + py) + d.z * (bz - az) > 0.0f;
+}
 __device__ __forceinline__ float2 add_mul2(float2 a, float2 b, float2 c) {
     float2 r;
     asm("{\n\t.reg .b64 a, b, c;\n\t"
@@ -123,14 +134,15 @@ __device__ __forceinline__ float2 add_mul2(float2 a, float2 b, float2 c) {
     return r;
 }
 
-// The slab test of a slot (`slab`; also slab_shadow's result wherever no slab
+// The slab test of a slot, with the entry and exit distances (`slab`; also slab_shadow's result wherever no slab
 // is NaN by 0 * inf: the two differ in their NaN rules only).
-__device__ __forceinline__ bool slab_slot(const SlabRay& r, float tmax, const Slot& s, float& A) {
+__device__ __forceinline__ bool slab_slot(const SlabRay& r, float tmax, const Slot& s, float& A,
+                                          float& B) {
     const float2 l = add_mul2(make_float2(s.lox, s.loy), r.no_xy, r.iv_xy);
     const float2 h = add_mul2(make_float2(s.hix, s.hiy), r.no_xy, r.iv_xy);
     const float2 z = add_mul2(make_float2(s.loz, s.hiz), r.no_zz, r.iv_zz);
     A = fmaxf(max3f(r.tmin, fminf(l.x, h.x), fminf(l.y, h.y)), fminf(z.x, z.y));
-    const float B = fminf(min3f(tmax, fmaxf(l.x, h.x), fmaxf(l.y, h.y)), fmaxf(z.x, z.y));
+    B = fminf(min3f(tmax, fmaxf(l.x, h.x), fmaxf(l.y, h.y)), fmaxf(z.x, z.y));
     return A <= B;
 }
 
@@ -223,43 +235,35 @@ static __device__ Hit closest_hit(const SceneView& S, const BvhHeader& H, const 
              s2 = load_slot(S.nodes, cur, 2), s3 = load_slot(S.nodes, cur, 3);
         // the reference's three near-first tests (an empty slot's corner is +inf)
         const bool l_first =
-            dot(r.d, mk3(fminf(s2.lox, s3.lox) - fminf(s0.lox, s1.lox),
-                         fminf(s2.loy, s3.loy) - fminf(s0.loy, s1.loy),
-                         fminf(s2.loz, s3.loz) - fminf(s0.loz, s1.loz))) > 0.0f;
-        const bool ll_first = dot(r.d, mk3(s1.lox - s0.lox, s1.loy - s0.loy, s1.loz - s0.loz)) > 0.0f;
-        const bool rl_first = dot(r.d, mk3(s3.lox - s2.lox, s3.loy - s2.loy, s3.loz - s2.loz)) > 0.0f;
+            near_first(r.d, fminf(s0.lox, s1.lox), fminf(s0.loy, s1.loy), fminf(s0.loz, s1.loz),
+                       fminf(s2.lox, s3.lox), fminf(s2.loy, s3.loy), fminf(s2.loz, s3.loz));
+        const bool ll_first = near_first(r.d, s0.lox, s0.loy, s0.loz, s1.lox, s1.loy, s1.loz);
+        const bool rl_first = near_first(r.d, s2.lox, s2.loy, s2.loz, s3.lox, s3.loy, s3.loz);
         if (careful) {
             binary_step(s0, s1);
             binary_step(s2, s3);
         }
-        float a0, a1, a2, a3;
-        if (!slab_slot(w, best.t, s0, a0)) a0 = MISS;
-        if (!slab_slot(w, best.t, s1, a1) || careful) a1 = MISS;
-        if (!slab_slot(w, best.t, s2, a2)) a2 = MISS;
-        if (!slab_slot(w, best.t, s3, a3) || careful) a3 = MISS;
+        float a0, a1, a2, a3, far;
+        if (!slab_slot(w, best.t, s0, a0, far)) a0 = MISS;
+        if (!slab_slot(w, best.t, s1, a1, far) || careful) a1 = MISS;
+        if (!slab_slot(w, best.t, s2, a2, far)) a2 = MISS;
+        if (!slab_slot(w, best.t, s3, a3, far) || careful) a3 = MISS;
         int32_t c0 = s0.code, c1 = s1.code, c2 = s2.code, c3 = s3.code;
         // careful: slot 0 before slot 1 whatever the (meaningless) inner test says
         swap_if(!ll_first, c0, c1, a0, a1);
         swap_if(!rl_first, c2, c3, a2, a3);
         swap_if(!l_first, c0, c2, a0, a2);
         swap_if(!l_first, c1, c3, a1, a3);
-        // far to near: the nearest hit goes on, the others are pushed
-        next = NO_NODE;
-        float na = 0.f;
+        // the nearest hit goes on, the others are pushed, far to near
         if (sp > STACK - 3) {
             atomicOr(status, RT_DEV_OVERFLOW);
+            next = NO_NODE;
         } else {
-            auto take = [&](int32_t c, float a) {
-                if (a == a) {
-                    if (next != NO_NODE) st[sp++] = make_int2(next, __float_as_int(na));
-                    next = c;
-                    na = a;
-                }
-            };
-            take(c3, a3);
-            take(c2, a2);
-            take(c1, a1);
-            take(c0, a0);
+            const bool h0 = a0 == a0, h1 = a1 == a1, h2 = a2 == a2, h3 = a3 == a3;
+            if (h3 && (h0 || h1 || h2)) st[sp++] = make_int2(c3, __float_as_int(a3));
+            if (h2 && (h0 || h1)) st[sp++] = make_int2(c2, __float_as_int(a2));
+            if (h1 && h0) st[sp++] = make_int2(c1, __float_as_int(a1));
+            next = h0 ? c0 : h1 ? c1 : h2 ? c2 : h3 ? c3 : NO_NODE;
         }
         if (next == NO_NODE) pop();
     };
@@ -276,7 +280,10 @@ static __device__ Hit closest_hit(const SceneView& S, const BvhHeader& H, const 
 }
 
 // Whether anything blocks the ray.  tMax does not shrink, so the order of
-// the visits does not matter.
+// the visits does not matter to the answer; of the children that the ray meets
+// it enters the one it crosses for longest, the likeliest to hold a blocker.
+// Against the last child first: 64 soups 9.29 -> 8.97 ms, glass 11.9 -> 11.7,
+// 4K of 17.7 M triangles 11.75 -> 11.60 (the nearest child first: 13.9).
 template <bool STAY, bool PAIR>
 static __device__ bool any_hit(const SceneView& S, const BvhHeader& H, const TRay& r, float tmax,
                                uint32_t* status) {
@@ -309,12 +316,27 @@ static __device__ bool any_hit(const SceneView& S, const BvhHeader& H, const TRa
                 take(slab_shadow(r, tmax, a.lox, a.loy, a.loz, a.hix, a.hiy, a.hiz), a.code);
             }
         } else {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const Slot s = load_slot(S.nodes, cur, k);
-                float A;
-                take(slab_slot(w, tmax, s, A), s.code);
-            }
+            const Slot s0 = load_slot(S.nodes, cur, 0), s1 = load_slot(S.nodes, cur, 1),
+                       s2 = load_slot(S.nodes, cur, 2), s3 = load_slot(S.nodes, cur, 3);
+            float longest = 0.f;
+            auto visit = [&](const Slot& s) {
+                float A, B;
+                if (!slab_slot(w, tmax, s, A, B)) return;
+                const float len = B - A;
+                if (next == NO_NODE) {
+                    next = s.code;
+                    longest = len;
+                    return;
+                }
+                const bool first = len > longest;
+                st[sp++] = first ? next : s.code;
+                next = first ? s.code : next;
+                longest = first ? len : longest;
+            };
+            visit(s0);
+            visit(s1);
+            visit(s2);
+            visit(s3);
         }
         if (next == NO_NODE && sp > 0) next = st[--sp];
     };
