@@ -33,15 +33,11 @@
 #include "lbvh_dev.cuh"
 #include "rt_internal.cuh"
 
-// Digit width of the build's radix passes: 8 (four passes for 30-bit keys)
-// or 10 (three).  The pair sort entry points always use 8.
-#ifndef RT_SORT_BITS
-#define RT_SORT_BITS 8
-#endif
-constexpr int kBuildBits = RT_SORT_BITS;
+// Radix passes of 8-bit digits (10-bit ones were slower: a tile's fixed work
+// grows with the digit count).
+constexpr int kBuildBits = 8;
 constexpr int kBuildRadix = 1 << kBuildBits;
-constexpr int kMaxBuildPasses = (32 + kBuildBits - 1) / kBuildBits;
-static_assert(kBuildBits == 8 || kBuildBits == 10, "build digit width");
+constexpr int kMaxBuildPasses = 4;
 
 namespace rt {
 
@@ -161,33 +157,29 @@ __global__ void __launch_bounds__(256) k_radix_hist(const uint32_t* __restrict__
     }
 }
 
-// One radix pass of BITS-bit digits; dynamic shared memory of
-// sizeof(SortSmemT<SORT_ITEMS, BITS>).  MINB tiles resident per SM bound the
-// registers: a pass whose tiles all fit in one wave at 2 per SM runs the
-// MINB = 2 instance (126 registers, 7 % faster per mid-scale build), a longer
-// one RT_SORT_MINB (3, 80 registers: the third tile hides latency).
-template <int BITS, int MINB>
+// One radix pass of 8-bit digits; dynamic shared memory of sizeof(SortSmem).
+// MINB tiles resident per SM bound the registers: a pass whose tiles all fit in
+// one wave at 2 per SM runs the MINB = 2 instance (7 % faster per mid-scale
+// build), a longer one RT_SORT_MINB (3, 80 registers: the third tile hides
+// latency).
+template <int MINB>
 __global__ void __launch_bounds__(SORT_THREADS, MINB) k_onesweep(
     const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint32_t* __restrict__ kout,
     uint32_t* __restrict__ vout, uint32_t n, int shift, const uint32_t* __restrict__ hist,
     uint32_t* __restrict__ lookback, uint32_t* __restrict__ tile_ctr, uint32_t* __restrict__ status) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char sort_smem[];
-    auto& S = *reinterpret_cast<SortSmemT<SORT_ITEMS, BITS>*>(sort_smem);
+    auto& S = *reinterpret_cast<SortSmem*>(sort_smem);
     if (threadIdx.x == 0) S.tile = atomicAdd(tile_ctr, 1u);   // tiles in launch order
     __syncthreads();
-    onesweep_tile<SORT_ITEMS, LB_SPIN_LIMIT, BITS>(S, S.tile, kin, vin, kout, vout, n, shift, hist,
-                                                   lookback, status);
+    onesweep_tile<>(S, S.tile, kin, vin, kout, vout, n, shift, hist, lookback, status);
 }
-template <int BITS>
-constexpr size_t onesweep_smem() { return sizeof(SortSmemT<SORT_ITEMS, BITS>); }
 
 constexpr int kOneWaveMinB = 2;
 // The instance for a pass of `tiles` tiles on `sms` SMs.
-template <int BITS>
 static auto onesweep_kernel(size_t tiles, int sms) {
-    return tiles <= (size_t)kOneWaveMinB * (size_t)sms ? k_onesweep<BITS, kOneWaveMinB>
-                                                       : k_onesweep<BITS, RT_SORT_MINB>;
+    return tiles <= (size_t)kOneWaveMinB * (size_t)sms ? k_onesweep<kOneWaveMinB>
+                                                       : k_onesweep<RT_SORT_MINB>;
 }
 
 // Self-test of the look-back timeout: one block sorts tile 1 of a pass
@@ -275,10 +267,8 @@ static cudaError_t setup_kernels() {
     opt_in((const void*)k_emit_level0<EMIT_REFIT>, sizeof(EmitSmem<EMIT_C0, EMIT_C0>));
     opt_in((const void*)k_emit_level<EMIT_T_WIDE>, sizeof(EmitSmem<EMIT_C1, EMIT_T_WIDE>));
     opt_in((const void*)k_emit_level<EMIT_T_NARROW>, sizeof(EmitSmem<EMIT_C1, EMIT_T_NARROW>));
-    opt_in((const void*)k_onesweep<8, kOneWaveMinB>, onesweep_smem<8>());
-    opt_in((const void*)k_onesweep<8, RT_SORT_MINB>, onesweep_smem<8>());
-    opt_in((const void*)k_onesweep<kBuildBits, kOneWaveMinB>, onesweep_smem<kBuildBits>());
-    opt_in((const void*)k_onesweep<kBuildBits, RT_SORT_MINB>, onesweep_smem<kBuildBits>());
+    opt_in((const void*)k_onesweep<kOneWaveMinB>, sizeof(SortSmem));
+    opt_in((const void*)k_onesweep<RT_SORT_MINB>, sizeof(SortSmem));
     if (e != cudaSuccess) return e;
     if (dev < 64) done |= 1ull << dev;
     return cudaSuccess;
@@ -362,8 +352,8 @@ cudaError_t lbvh_build(const LbvhArgs& a, cudaStream_t s) {
     for (int p = 0; p < passes; ++p) {
         // the last pass always lands in keys_sorted / vals_sorted
         const int dst = ((passes - 1 - p) & 1) ? 0 : 1;
-        e = launch_dep(onesweep_kernel<kBuildBits>(tiles, sms), (unsigned)tiles, SORT_THREADS,
-                       onesweep_smem<kBuildBits>(), s, true, kin, vin, kbuf[dst], vbuf[dst], n,
+        e = launch_dep(onesweep_kernel(tiles, sms), (unsigned)tiles, SORT_THREADS,
+                       sizeof(SortSmem), s, true, kin, vin, kbuf[dst], vbuf[dst], n,
                        kBuildBits * p, (const uint32_t*)(hist + kBuildRadix * p),
                        lookback + (size_t)p * tiles * kBuildRadix, tile_ctr + p, a.status);
         if (e) return e;
@@ -423,7 +413,7 @@ cudaError_t radix_sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t*
         const bool to_out = ((passes - 1 - p) & 1) == 0;
         uint32_t* ko = to_out ? kout : ktmp;
         uint32_t* vo = to_out ? vout : vtmp;
-        onesweep_kernel<8>(tiles, num_sms)<<<(unsigned)tiles, SORT_THREADS, onesweep_smem<8>(), s>>>(
+        onesweep_kernel(tiles, num_sms)<<<(unsigned)tiles, SORT_THREADS, sizeof(SortSmem), s>>>(
             ki, vi, ko, vo, n, 8 * p, hist + 256 * p, lookback + (size_t)p * tiles * 256,
             tile_ctr + p, status);
         ki = ko;

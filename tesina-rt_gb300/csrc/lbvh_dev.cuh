@@ -13,9 +13,6 @@
 
 namespace rt {
 
-#ifndef RT_SORT_VEC_LOADS
-#define RT_SORT_VEC_LOADS 1   // whole tiles staged in shared memory: 0 no, 1 by 128-bit loads, 2 by bulk copy
-#endif
 #ifndef RT_SORT_MINB
 #define RT_SORT_MINB 3   // radix tiles resident per SM (register budget)
 #endif
@@ -76,51 +73,6 @@ __device__ __forceinline__ uint4 ld_dep(const uint4* p) {
     asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
-}
-
-// A shared-memory mbarrier and the 1-D bulk copy (the TMA engine without a
-// tensor map) that completes on it.
-__device__ __forceinline__ uint32_t smem_addr(const void* p) {
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_inval(uint64_t* bar) {
-    asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)),
-                 "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(smem_addr(bar)), "r"(parity) : "memory");
-    return ok != 0;
-}
-// global -> shared, `bytes` a multiple of 16, both addresses 16-byte aligned
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-        ::"r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(smem_addr(bar)) : "memory");
-}
-__device__ __forceinline__ void fence_proxy_async_smem() {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-constexpr uint32_t BULK_WAIT_LIMIT = 1u << 22;   // polls of a bulk copy's mbarrier
-// atomicAdd with acquire-release ordering at GPU scope: the caller's earlier
-// writes are visible to whoever reads the counter's new value, and the
-// caller sees everything released by earlier adders.
-__device__ __forceinline__ uint32_t atomic_add_acq_rel(uint32_t* p, uint32_t v) {
-    uint32_t old;
-    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v)
-                 : "memory");
-    return old;
 }
 
 // build_primitive_bbox (bvh-builder.cl:100-130) of one triangle.
@@ -220,7 +172,8 @@ __device__ __forceinline__ uint32_t morton_code(const MortonParams& P, const flo
     return P.depth >= 32 ? (uint32_t)code : (uint32_t)code & ((1u << P.depth) - 1u);
 }
 
-// Exclusive scan of one value per thread over a 256-thread block.
+// Exclusive scan of one value per thread over a 256-thread block; one barrier
+// (each warp sums the earlier warps' totals itself).
 __device__ __forceinline__ uint32_t block_excl_scan_256(uint32_t v, uint32_t* s_warp) {
     const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
     uint32_t x = v;
@@ -231,19 +184,8 @@ __device__ __forceinline__ uint32_t block_excl_scan_256(uint32_t v, uint32_t* s_
     }
     if (l == 31) s_warp[w] = x;
     __syncthreads();
-    if (w == 0) {
-        uint32_t t = l < SORT_WARPS ? s_warp[l] : 0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t y = __shfl_up_sync(0xffffffffu, t, o);
-            if (l >= o) t += y;
-        }
-        if (l < SORT_WARPS) s_warp[l] = t;
-    }
-    __syncthreads();
-    const uint32_t warp_base = w ? s_warp[w - 1] : 0;
-    __syncthreads();
-    return warp_base + x - v;
+    const uint32_t before = __reduce_add_sync(0xffffffffu, l < w ? s_warp[l] : 0u);
+    return before + x - v;
 }
 
 // Phase marks of a radix tile (k = 0..6), for timing harnesses; none by default.
@@ -251,80 +193,62 @@ __device__ __forceinline__ uint32_t block_excl_scan_256(uint32_t v, uint32_t* s_
 #define RT_SORT_MARK(k)
 #endif
 
-template <int ITEMS, int BITS = 8>
+template <int ITEMS>
 struct __align__(16) SortSmemT {
-    static constexpr int RADIX = 1 << BITS;
     uint32_t keys[SORT_THREADS * ITEMS];
     uint32_t vals[SORT_THREADS * ITEMS];
-    uint32_t whist[SORT_WARPS][RADIX];
-    uint32_t goff[RADIX];
-    uint32_t lstart[RADIX];
-    uint64_t bar;   // the bulk tile load's mbarrier
-    uint32_t scan[SORT_WARPS];
+    uint32_t whist[SORT_WARPS][256];
+    uint32_t goff[256];
+    uint32_t scan[2][SORT_WARPS];
     uint32_t tile;
 };
 using SortSmem = SortSmemT<SORT_ITEMS>;
 
-// One tile of a stable LSD radix pass (BITS-bit digit at `shift`; each
-// thread owns 2^BITS / SORT_THREADS consecutive digits): warp-striped loads,
-// ballot ranking in index order, decoupled look-back over the earlier tiles
-// of the same sequence, shared-memory staging and a coalesced scatter.  Must
-// be called by all SORT_THREADS threads of a block; a tile holds
-// SORT_THREADS * ITEMS keys.  A null `vin` stands for the values 0, 1, 2, ...
-// (the first pass of a build).  A look-back that polls an unpublished word
+// One tile of a stable LSD radix pass (8-bit digit at `shift`, one digit per
+// thread): warp-striped keys, ballot ranking in index order, the tile in digit
+// order in shared memory, decoupled look-back over the earlier tiles of the
+// same sequence, and a coalesced scatter.  Must be called by all SORT_THREADS
+// threads of a block; a tile holds SORT_THREADS * ITEMS keys (WHOLE: all of
+// them; the last tile of a sequence may hold fewer).  A null `vin` stands for
+// the values 0, 1, 2, ... (the first pass of a build).  `hist` holds the pass's
+// 256 digit counts, `lookback` 256 words per tile: tile 0 publishes the global
+// offset of each digit with its count, so the later tiles' prefixes are
+// scatter offsets as they are.  A look-back that polls an unpublished word
 // more than SPIN_LIMIT times gives up: it sets RT_DEV_TIMEOUT in *status and
-// goes on with the counts it has, so every block ends; the tile's writes
-// then stay inside [0, n), since a partial prefix only lowers the scatter
-// offsets, which start at the digit's global offset.  `hist` holds the
-// pass's 2^BITS digit counts, `lookback` 2^BITS words per tile.
-template <int ITEMS = SORT_ITEMS, uint32_t SPIN_LIMIT = LB_SPIN_LIMIT, int BITS = 8>
-__device__ __forceinline__ void onesweep_tile(SortSmemT<ITEMS, BITS>& S, uint32_t tile,
-                                              const uint32_t* __restrict__ kin,
-                                              const uint32_t* __restrict__ vin,
-                                              uint32_t* __restrict__ kout,
-                                              uint32_t* __restrict__ vout, uint32_t n, int shift,
-                                              const uint32_t* __restrict__ hist,
-                                              uint32_t* __restrict__ lookback,
-                                              uint32_t* __restrict__ status) {
-    constexpr int RADIX = 1 << BITS;
-    constexpr int DPT = RADIX / SORT_THREADS;   // digits per thread
-    constexpr uint32_t DMASK = (uint32_t)RADIX - 1u;
-    static_assert(DPT >= 1 && RADIX % SORT_THREADS == 0, "digits per thread");
+// goes on with the counts it has, so every block ends; its writes stay inside
+// [0, n): a partial prefix only lowers the offsets, a key's place in its tile is
+// added, and what would lie at or beyond n is dropped.
+//
+// What bounds it: the chain of one tile, about 14 us of load and ranking
+// (6.0-6.6), staging (1.3-1.7), look-back (3.4-4.0: 8 to 11 round trips) and
+// scatter (1.3), which the look-back ties to the tiles before it.  Without bound
+// checks in whole tiles, a scan of the digit counts in every tile and two of
+// three barriers per scan, and with the first look-back words requested before
+// the staging: build of 1.24 M triangles 213 -> 210 us, 10k-triangle frame 381 ->
+// 376; at 17.7 M pairs (9.5 waves of tiles) no change.
+template <int ITEMS, uint32_t SPIN_LIMIT, bool WHOLE>
+__device__ __forceinline__ void onesweep_tile_body(SortSmemT<ITEMS>& S, uint32_t tile,
+                                                   const uint32_t* __restrict__ kin,
+                                                   const uint32_t* __restrict__ vin,
+                                                   uint32_t* __restrict__ kout,
+                                                   uint32_t* __restrict__ vout, uint32_t n,
+                                                   int shift, const uint32_t* __restrict__ hist,
+                                                   uint32_t* __restrict__ lookback,
+                                                   uint32_t* __restrict__ status) {
+    constexpr uint32_t TILE = SORT_THREADS * ITEMS;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     RT_SORT_MARK(0);
-    for (int i = tid; i < SORT_WARPS * RADIX; i += SORT_THREADS) (&S.whist[0][0])[i] = 0;
-    __syncthreads();
-    const size_t base = (size_t)tile * (SORT_THREADS * ITEMS);
+    const uint32_t base = tile * TILE;                 // n < 2^30
+    const uint32_t valid = WHOLE ? TILE : n - base;    // keys of this tile
+    const uint32_t mine = (uint32_t)warp * (ITEMS * 32) + lane;   // this thread's first key
     const uint32_t lanemask_lt = (1u << lane) - 1u;
-
     uint32_t k[ITEMS], v[ITEMS], rank[ITEMS];
-#if RT_SORT_VEC_LOADS
+    static_assert(ITEMS % 4 == 0, "whole 128-bit words per thread");
     // a whole, 16-byte aligned tile: 128-bit loads into shared memory, then
     // the warp-striped layout the ranking needs from there
-    const bool vec = base + (size_t)(SORT_THREADS * ITEMS) <= n &&
-                     ((reinterpret_cast<uintptr_t>(kin) | reinterpret_cast<uintptr_t>(vin)) & 15u) == 0;
-    static_assert(ITEMS % 4 == 0, "whole 128-bit words per thread");
+    const bool vec =
+        WHOLE && ((reinterpret_cast<uintptr_t>(kin) | reinterpret_cast<uintptr_t>(vin)) & 15u) == 0;
     if (vec) {
-#if RT_SORT_VEC_LOADS == 2
-        // one bulk copy per array, completing on the tile's mbarrier
-        constexpr uint32_t TB = SORT_THREADS * ITEMS * 4;
-        if (tid == 0) {
-            mbar_init(&S.bar);
-            fence_proxy_async_smem();   // earlier generic accesses of the buffers come first
-            mbar_arrive_expect_tx(&S.bar, vin ? 2 * TB : TB);
-            bulk_load(S.keys, kin + base, TB, &S.bar);
-            if (vin) bulk_load(S.vals, vin + base, TB, &S.bar);
-        }
-        __syncthreads();   // the barrier is initialised before anyone polls it
-        uint32_t polls = 0;
-        while (!mbar_try_wait(&S.bar, 0) && ++polls < BULK_WAIT_LIMIT) {
-        }
-        if (polls >= BULK_WAIT_LIMIT) {
-            atomicOr(status, RT_DEV_TIMEOUT);
-            while (!mbar_try_wait(&S.bar, 0) && ++polls < 2 * BULK_WAIT_LIMIT) {
-            }
-        }
-#else
         const uint4* k4 = reinterpret_cast<const uint4*>(kin + base);
         const uint4* v4 = reinterpret_cast<const uint4*>(vin + base);
 #pragma unroll
@@ -333,33 +257,27 @@ __device__ __forceinline__ void onesweep_tile(SortSmemT<ITEMS, BITS>& S, uint32_
             reinterpret_cast<uint4*>(S.keys)[e] = __ldcs(&k4[e]);
             if (vin) reinterpret_cast<uint4*>(S.vals)[e] = __ldcs(&v4[e]);
         }
-        __syncthreads();
-#endif
+    }
+    for (int i = tid; i < SORT_WARPS * 64; i += SORT_THREADS)
+        reinterpret_cast<uint4*>(&S.whist[0][0])[i] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    if (vec) {
 #pragma unroll
-        for (int j = 0; j < ITEMS; ++j) {
-            const int e = warp * (ITEMS * 32) + j * 32 + lane;
-            k[j] = S.keys[e];
-            v[j] = vin ? S.vals[e] : (uint32_t)(base + e);
-        }
-    } else
-#endif
+        for (int j = 0; j < ITEMS; ++j) k[j] = S.keys[mine + j * 32];
+    } else {
 #pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-        const size_t g = base + (size_t)warp * (ITEMS * 32) + j * 32 + lane;
-        const bool ok = g < n;
-        k[j] = ok ? __ldcs(&kin[g]) : 0xffffffffu;
-        v[j] = ok ? (vin ? __ldcs(&vin[g]) : (uint32_t)g) : 0u;
+        for (int j = 0; j < ITEMS; ++j)
+            k[j] = WHOLE || mine + j * 32 < valid ? __ldcs(&kin[base + mine + j * 32]) : 0xffffffffu;
     }
 #pragma unroll
     for (int j = 0; j < ITEMS; ++j) {
-        const size_t g = base + (size_t)warp * (ITEMS * 32) + j * 32 + lane;
-        const bool ok = g < n;
-        const uint32_t d = (k[j] >> shift) & DMASK;
+        const bool ok = WHOLE || mine + j * 32 < valid;
+        const uint32_t d = (k[j] >> shift) & 255u;
         // lanes holding the same digit: one ballot per digit bit (a fixed
         // cost, where a match instruction grows with the distinct digits)
-        uint32_t peers = __ballot_sync(0xffffffffu, ok);
+        uint32_t peers = WHOLE ? 0xffffffffu : __ballot_sync(0xffffffffu, ok);
 #pragma unroll
-        for (int b = 0; b < BITS; ++b) {
+        for (int b = 0; b < 8; ++b) {
             const uint32_t bit = __ballot_sync(0xffffffffu, (d >> b) & 1u);
             peers &= ((d >> b) & 1u) ? bit : ~bit;
         }
@@ -367,95 +285,78 @@ __device__ __forceinline__ void onesweep_tile(SortSmemT<ITEMS, BITS>& S, uint32_
         if (ok) prev = S.whist[warp][d];
         __syncwarp();
         if (ok) {
-            rank[j] = prev + __popc(peers & lanemask_lt);
-            const int leader = __ffs(peers) - 1;
-            if (lane == leader) S.whist[warp][d] = prev + __popc(peers);
+            const uint32_t below = __popc(peers & lanemask_lt);
+            rank[j] = prev + below;
+            if (below == 0u) S.whist[warp][d] = prev + __popc(peers);
         }
         __syncwarp();
+    }
+    // the values, which the ranking does not need (its registers)
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+        const uint32_t e = mine + j * 32;
+        v[j] = !vin ? base + e : vec ? S.vals[e] : WHOLE || e < valid ? __ldcs(&vin[base + e]) : 0u;
     }
     __syncthreads();
 
     RT_SORT_MARK(1);
-    // this thread's digits: tid * DPT .. tid * DPT + DPT - 1
-    const uint32_t dgt0 = (uint32_t)tid * DPT;
-    uint32_t cnt[DPT], lstart[DPT];
-    uint32_t tsum = 0;
+    // thread tid's digit: counts of the warps, summed in warp order
+    uint32_t cnt = 0;
 #pragma unroll
-    for (int q = 0; q < DPT; ++q) {
-        uint32_t c = 0;
-#pragma unroll
-        for (int w = 0; w < SORT_WARPS; ++w) {
-            const uint32_t x = S.whist[w][dgt0 + q];
-            S.whist[w][dgt0 + q] = c;
-            c += x;
-        }
-        cnt[q] = c;
-        lstart[q] = tsum;
-        tsum += c;
+    for (int w = 0; w < SORT_WARPS; ++w) cnt += S.whist[w][tid];
+    uint32_t excl = 0;
+    uint32_t* my = &lookback[(size_t)tile * 256 + tid];
+    if (tile == 0) {
+        excl = block_excl_scan_256(ld_dep(&hist[tid]), S.scan[1]);
+        st_relaxed(my, LB_PREFIX | (excl + cnt));
+    } else {
+        st_relaxed(my, LB_AGG | cnt);   // as early as the count is known
     }
-    uint32_t* my = &lookback[(size_t)tile * RADIX + dgt0];
+    const uint32_t lstart = block_excl_scan_256(cnt, S.scan[0]);
+    uint32_t c = lstart;
 #pragma unroll
-    for (int q = 0; q < DPT; ++q)   // as early as the counts are known
-        st_relaxed(my + q, (tile == 0 ? LB_PREFIX : LB_AGG) | cnt[q]);
-    const uint32_t lbase = block_excl_scan_256(tsum, S.scan);
-#pragma unroll
-    for (int q = 0; q < DPT; ++q) {
-        lstart[q] += lbase;
-        S.lstart[dgt0 + q] = lstart[q];
+    for (int w = 0; w < SORT_WARPS; ++w) {   // first place in the tile of each warp's keys
+        const uint32_t x = S.whist[w][tid];
+        S.whist[w][tid] = c;
+        c += x;
     }
     __syncthreads();
-    // the tile in digit order in shared memory (frees the registers of the
-    // keys for the look-back's window)
+    // the first look-back words are on their way while the tile is staged
+    uint32_t win[LB_WINDOW];
+    auto read_window = [&](int32_t p) {
+#pragma unroll
+        for (int t = 0; t < LB_WINDOW; ++t)   // tile 0 is always a prefix: p - t < 0 is never summed
+            win[t] = p - t >= 0 ? ld_relaxed(&lookback[(size_t)(p - t) * 256 + tid]) : LB_PREFIX;
+    };
+    int32_t p = (int32_t)tile - 1;
+    if (tile > 0) read_window(p);
 #pragma unroll
     for (int j = 0; j < ITEMS; ++j) {
-        const size_t g = base + (size_t)warp * (ITEMS * 32) + j * 32 + lane;
-        if (g < n) {
-            const uint32_t d = (k[j] >> shift) & DMASK;
-            const uint32_t p = S.lstart[d] + S.whist[warp][d] + rank[j];
-            S.keys[p] = k[j];
-            S.vals[p] = v[j];
+        if (WHOLE || mine + j * 32 < valid) {
+            const uint32_t at = S.whist[warp][(k[j] >> shift) & 255u] + rank[j];
+            S.keys[at] = k[j];
+            S.vals[at] = v[j];
         }
     }
     // Decoupled look-back.  Each word holds its whole message (flag and
     // count), so relaxed accesses suffice; the words of LB_WINDOW earlier
-    // tiles are read per round trip and summed nearest first, for each digit
-    // up to its first inclusive prefix, and for all of them up to the first
-    // tile that has not published a digit still open.
+    // tiles are read per round trip and summed nearest first, up to the first
+    // inclusive prefix or the first tile that has not published.
     RT_SORT_MARK(2);
-    uint32_t excl[DPT];
-#pragma unroll
-    for (int q = 0; q < DPT; ++q) excl[q] = 0;
     if (tile > 0) {
-        constexpr uint32_t ALL = (1u << DPT) - 1u;
-        uint32_t open = ALL;   // digits without an inclusive prefix yet
-        int64_t p = (int64_t)tile - 1;
         uint32_t spins = 0;
+        bool open = true;   // no inclusive prefix yet
         for (;;) {
-            uint32_t w[LB_WINDOW][DPT];
-#pragma unroll
-            for (int t = 0; t < LB_WINDOW; ++t)   // tile 0 is always a prefix: p - t < 0 is never summed
-#pragma unroll
-                for (int q = 0; q < DPT; ++q)
-                    w[t][q] = p - t >= 0 ? ld_relaxed(&lookback[(size_t)(p - t) * RADIX + dgt0 + q])
-                                         : LB_PREFIX;
             int used = 0;
             bool wait = false;
 #pragma unroll
             for (int t = 0; t < LB_WINDOW; ++t) {
                 if (open && !wait) {
-                    bool miss = false;
-#pragma unroll
-                    for (int q = 0; q < DPT; ++q)
-                        miss |= ((open >> q) & 1u) && (w[t][q] & ~LB_MASK) == 0u;
-                    if (miss) {
+                    if ((win[t] & ~LB_MASK) == 0u) {
                         wait = true;
                     } else {
-#pragma unroll
-                        for (int q = 0; q < DPT; ++q)
-                            if ((open >> q) & 1u) {
-                                excl[q] += w[t][q] & LB_MASK;
-                                if ((w[t][q] & ~LB_MASK) == LB_PREFIX) open &= ~(1u << q);
-                            }
+                        excl += win[t] & LB_MASK;
+                        open = (win[t] & ~LB_MASK) != LB_PREFIX;
                         ++used;
                     }
                 }
@@ -466,37 +367,42 @@ __device__ __forceinline__ void onesweep_tile(SortSmemT<ITEMS, BITS>& S, uint32_
                 atomicOr(status, RT_DEV_TIMEOUT);
                 break;
             }
+            read_window(p);
         }
-#pragma unroll
-        for (int q = 0; q < DPT; ++q) st_relaxed(my + q, LB_PREFIX | (excl[q] + cnt[q]));
+        st_relaxed(my, LB_PREFIX | (excl + cnt));
     }
     RT_SORT_MARK(3);
-    uint32_t h[DPT], hsum = 0;
-#pragma unroll
-    for (int q = 0; q < DPT; ++q) {
-        h[q] = hsum;
-        hsum += ld_dep(&hist[dgt0 + q]);
-    }
-    const uint32_t gbase = block_excl_scan_256(hsum, S.scan);
-#pragma unroll
-    for (int q = 0; q < DPT; ++q) S.goff[dgt0 + q] = gbase + h[q] + excl[q] - lstart[q];
+    S.goff[tid] = excl - lstart;
     __syncthreads();
     RT_SORT_MARK(4);
-    const uint32_t valid_n = (uint32_t)min((size_t)(SORT_THREADS * ITEMS), (size_t)n - base);
-    for (uint32_t i = tid; i < valid_n; i += SORT_THREADS) {
+#pragma unroll 4
+    for (uint32_t i = tid; i < valid; i += SORT_THREADS) {
         const uint32_t key = S.keys[i];
-        const uint32_t d = (key >> shift) & DMASK;
-        const uint32_t dst = S.goff[d] + i;
+        const uint32_t dst = S.goff[(key >> shift) & 255u] + i;
         if (dst < n) {   // always, unless a wait gave up (RT_DEV_TIMEOUT)
             kout[dst] = key;
             vout[dst] = S.vals[i];
         }
     }
-    __syncthreads();   // the shared buffers are reused by the next tile
-#if RT_SORT_VEC_LOADS == 2
-    if (vec && tid == 0) mbar_inval(&S.bar);
-#endif
     RT_SORT_MARK(5);
+}
+
+// A caller that takes several tiles with one S has a barrier between them.
+template <int ITEMS = SORT_ITEMS, uint32_t SPIN_LIMIT = LB_SPIN_LIMIT>
+__device__ __forceinline__ void onesweep_tile(SortSmemT<ITEMS>& S, uint32_t tile,
+                                              const uint32_t* __restrict__ kin,
+                                              const uint32_t* __restrict__ vin,
+                                              uint32_t* __restrict__ kout,
+                                              uint32_t* __restrict__ vout, uint32_t n, int shift,
+                                              const uint32_t* __restrict__ hist,
+                                              uint32_t* __restrict__ lookback,
+                                              uint32_t* __restrict__ status) {
+    if ((size_t)(tile + 1) * (SORT_THREADS * ITEMS) <= n)
+        onesweep_tile_body<ITEMS, SPIN_LIMIT, true>(S, tile, kin, vin, kout, vout, n, shift, hist,
+                                                    lookback, status);
+    else
+        onesweep_tile_body<ITEMS, SPIN_LIMIT, false>(S, tile, kin, vin, kout, vout, n, shift, hist,
+                                                     lookback, status);
 }
 
 // rearrange_indices / rearrange_map (bvh-builder.cl:49-72) of sorted slot i,
