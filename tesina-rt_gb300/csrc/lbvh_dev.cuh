@@ -771,14 +771,16 @@ __device__ __forceinline__ bool warp_join(WarpItem& it, uint32_t cnt, uint64_t e
         const float vlo = k == 0 ? it.lox : (k == 1 ? it.loy : it.loz);
         const float vhi = k == 0 ? it.hix : (k == 1 ? it.hiy : it.hiz);
         __syncwarp();   // the previous axis' queries are done
-        if (item) W.st[0][lane] = make_float2(vlo, vhi);
+        float2 u = make_float2(vlo, vhi);   // this lane's entry of the level below
+        if (item) W.st[0][lane] = u;
 #pragma unroll
         for (int t = 1; t < 5; ++t) {
             __syncwarp();
             const uint32_t h = 1u << (t - 1);
             if (lane + 2u * h <= cnt) {
-                const float2 u = W.st[t - 1][lane], v = W.st[t - 1][lane + h];
-                W.st[t][lane] = make_float2(fminf(u.x, v.x), fmaxf(u.y, v.y));
+                const float2 v = W.st[t - 1][lane + h];
+                u = make_float2(fminf(u.x, v.x), fmaxf(u.y, v.y));
+                W.st[t][lane] = u;
             }
         }
         __syncwarp();
