@@ -322,9 +322,9 @@ def measure_batched(ctx, lib, torch, reps=5):
             "batched_ms": statistics.median(t_b), "plain_mrays_s": mp, "batched_mrays_s": mb,
             "speedup": mb / mp, "identical_pixels": bool(same and rays_b == rays_plain),
             # build: the cooperative launch + one emit launch per level of the
-            # largest scene; render: the pooled kernel + the RGBA8 conversion
-            "launches_per_batch": 1 + max(emit_levels_of(it["scene"].n_tris) for it in items) + 2,
-            "launches_plain": sum(7 + emit_levels_of(it["scene"].n_tris) + 2 for it in items)}
+            # largest scene; render: the pooled kernel
+            "launches_per_batch": 1 + max(emit_levels_of(it["scene"].n_tris) for it in items) + 1,
+            "launches_plain": sum(7 + emit_levels_of(it["scene"].n_tris) for it in items)}
 
 
 def measure_stress(ctx, lib, torch, builds=5, cpu=True):
@@ -1037,8 +1037,8 @@ def run_gpu(args):
     # the emit's levels: 512 triangles per level-0 block, then 8 blocks per block
     emit_levels = emit_levels_of(n_tris)
     # k_bounds, k_morton_hist, 4 radix passes, the emit levels (the first
-    # one also permutes), then the render (+ k_fb_copy when pooled)
-    launches_per_frame = 6 + emit_levels + (2 if pooled else 1)
+    # one also permutes), then the render
+    launches_per_frame = 6 + emit_levels + 1
     build_roofline = {"kernels": "k_bounds + k_morton_hist + 4x k_onesweep + "
                                  "k_emit_level0 + %dx k_emit_level" % (emit_levels - 1),
                       "bound": "hbm",

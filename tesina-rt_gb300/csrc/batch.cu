@@ -64,6 +64,23 @@ __device__ __forceinline__ int find_segment(const uint32_t* off, int count, uint
     return lo;
 }
 
+// The same over offsets in global memory (read once per 32-pixel tile, from
+// L1: a copy of up to 4,097 of them in every block's shared memory took 16 KB
+// per block from the L1 that serves the traversal: with it and the smaller pool
+// below, 64 soups take 7.97 instead of 8.94 ms, the served burst 4.8 instead of
+// 5.1).
+__device__ __forceinline__ int find_segment_ldg(const uint32_t* off, int count, uint32_t g) {
+    int lo = 0, hi = count - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (__ldg(&off[mid]) <= g)
+            lo = mid;
+        else
+            hi = mid - 1;
+    }
+    return lo;
+}
+
 __global__ void __launch_bounds__(SORT_THREADS, 4) k_batch_build(BatchBuildArgs A) {
     cg::grid_group grid = cg::this_grid();
     __shared__ SortSmemT<kBatchItems> S;
@@ -277,10 +294,7 @@ __global__ void k_batch_stamp(unsigned long long* t) { *t = globaltimer(); }
 // refracting materials).
 template <int THREADS, int MINB, bool REFR = false>
 __global__ void __launch_bounds__(THREADS, MINB) k_render_batch(BatchRenderArgs A) {
-    __shared__ uint32_t s_poff[kMaxBatchViews + 1];
-    for (int i = threadIdx.x; i <= A.count; i += blockDim.x) s_poff[i] = A.pix_off[i];
-    __syncthreads();
-    const uint32_t total = s_poff[A.count];
+    const uint32_t total = __ldg(&A.pix_off[A.count]);
     const int lane = threadIdx.x & 31;
     uint32_t n_prim = 0, n_sec = 0, n_shadow = 0, n_hits = 0;
     for (;;) {
@@ -291,12 +305,12 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch(BatchRenderArgs 
         for (uint32_t base = base0; base < base0 + A.chunk && base < total; base += 32) {
             const uint32_t g = base + lane;
             // the view of the warp's first pixel; lanes past its end look their own up
-            const int v0 = find_segment(s_poff, A.count, base);
-            const bool same = g < s_poff[v0 + 1];
+            const int v0 = find_segment_ldg(A.pix_off, A.count, base);
+            const bool same = g < __ldg(&A.pix_off[v0 + 1]);
             if (g < total) {
-                const int v = same ? v0 : find_segment(s_poff, A.count, g);
+                const int v = same ? v0 : find_segment_ldg(A.pix_off, A.count, g);
                 const BatchView& V = A.views[v];
-                const int local = (int)(g - s_poff[v]);
+                const int local = (int)(g - __ldg(&A.pix_off[v]));
                 int x, y;
                 pixel_of(warp_tile_order(local, V.width, V.height), V.width, V.height, 32, x, y);
                 const BvhHeader H = *V.scene.hdr;
@@ -306,12 +320,8 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch(BatchRenderArgs 
                 n_sec += pr.secondary;
                 n_shadow += pr.shadow;
                 n_hits += pr.hits;
-                uchar4 px;
-                px.x = to_unorm8(pr.r, A.inv1e6);
-                px.y = to_unorm8(pr.g, A.inv1e6);
-                px.z = to_unorm8(pr.b, A.inv1e6);
-                px.w = 255;
-                reinterpret_cast<uchar4*>(A.rgba)[(size_t)V.rgba_offset + V.width * y + x] = px;
+                reinterpret_cast<uchar4*>(A.rgba)[(size_t)V.rgba_offset + V.width * y + x] =
+                    rgba8_of(make_uint3(pr.r, pr.g, pr.b), A.inv1e6);
             }
         }
     }
@@ -333,24 +343,30 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch(BatchRenderArgs 
 // k_render_batch_pool: the rays of k_render_batch scheduled as in
 // k_render_pool (trace.cu): warp tiles of primary rays, dense (hit, light)
 // shadow tasks, and a per-warp pool of reflection rays traced 32 at a time,
-// whichever views and pixels they belong to.  Fixed-point contributions are
-// summed into A.accum (3 per pixel of the launch's concatenated pixel space,
-// integer sums being independent of order) and k_batch_fb writes RGBA8 at
-// each view's offset afterwards.  Bit-identical to k_render_batch.
+// whichever views and pixels they belong to.  A pixel's fixed-point sum travels
+// with its ray and the lane that ends the path writes RGBA8, as in
+// k_render_pool.  Bit-identical to k_render_batch.
 // ---------------------------------------------------------------------------
 // MAXB > 0: scenes with refracting materials, as k_render_pool_refr
 // (trace.cu) follows them: a hit continues its reflected and refracted rays,
 // the pool is taken from the top and holds 32 (MAXB + 2) rays, enough for
-// views of up to MAXB bounces; a push past it raises RT_DEV_OVERFLOW.
+// views of up to MAXB bounces; a push past it raises RT_DEV_OVERFLOW.  Its pixels
+// have several rays on the way, so they are summed in A.accum (3 per pixel of
+// the launch's concatenated pixel space, integer sums being independent of
+// order) and k_batch_fb writes RGBA8 at each view's offset afterwards.
 namespace {
-template <int BPOOL>
+// As WarpPool (trace.cu): a hit of the current step takes its ray's place.
+// CARRY: the pixels' sums travel with the rays.
+template <int BPOOL, bool CARRY>
 struct WarpPoolB {
     float ro[3][BPOOL], rd[3][BPOOL], rc[BPOOL];
-    int rv[BPOOL], rai[BPOOL], rbounce[BPOOL];   // view, sum index, bounce
-    float hp[3][32], hn[3][32], hd[3][32], hc[32];
-    int hid[32], hv[32], hai[32], hbounce[32], hoff[33];
+    // view, place of the pixel (CARRY: in rgba, else in accum), bounce
+    int rv[BPOOL], rbounce[BPOOL];
+    uint32_t rai[BPOOL], racc[3][CARRY ? BPOOL : 1];
+    float hn[3][32];
+    int hid[32], hoff[33];
     unsigned hmask[32];
-    unsigned char hinv[32];
+    uint8_t hslot[32], hinv[32];
     uint8_t task[32 * RT_MAX_LIGHTS];   // shadow tasks that need a ray
     int pool_n;
 };
@@ -359,14 +375,14 @@ struct WarpPoolB {
 template <int THREADS, int MINB, int MAXB = 0>
 __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRenderArgs A) {
     constexpr int BPOOL = MAXB ? 32 * (MAXB + 2) : 64;
-    __shared__ uint32_t s_poff[kMaxBatchViews + 1];
-    __shared__ WarpPoolB<BPOOL> sQ[THREADS / 32];
-    for (int i = threadIdx.x; i <= A.count; i += blockDim.x) s_poff[i] = A.pix_off[i];
+    constexpr bool CARRY = MAXB == 0;
+    static_assert(BPOOL <= 256, "places of the pool in 8 bits");
+    __shared__ WarpPoolB<BPOOL, CARRY> sQ[THREADS / 32];
     const int lane = threadIdx.x & 31;
-    WarpPoolB<BPOOL>& Q = sQ[threadIdx.x >> 5];
+    WarpPoolB<BPOOL, CARRY>& Q = sQ[threadIdx.x >> 5];
     if (lane == 0) Q.pool_n = 0;
-    __syncthreads();
-    const uint32_t total = s_poff[A.count];
+    __syncwarp();
+    const uint32_t total = __ldg(&A.pix_off[A.count]);
     const unsigned lt = (1u << lane) - 1u;
     uint32_t n_prim = 0, n_sec = 0, n_shadow = 0, n_hits = 0;
     bool tiles = true;
@@ -374,24 +390,23 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
         const int pn = Q.pool_n;
         bool have = false;
         f3 o = mk3(0.f, 0.f, 0.f), d = o;
-        float c = 1.0f, tmin = 0.0f, tmax = 1e36f;
-        int v = 0, ai = 0, bounce = 0;
+        float tmin = 0.0f, tmax = 1e36f;
+        int v = 0;
+        bool primary = false;
+        uint32_t ai = 0;           // a primary ray's pixel
+        int first = pn;            // place of the step's first ray
         if (pn >= 32 || (!tiles && pn > 0)) {
             const int k = min(32, pn);
-            const int j = pn - k + lane;
+            first = pn - k;
             have = lane < k;
             if (have) {
+                const int j = first + lane;
                 o = mk3(Q.ro[0][j], Q.ro[1][j], Q.ro[2][j]);
                 d = mk3(Q.rd[0][j], Q.rd[1][j], Q.rd[2][j]);
-                c = Q.rc[j];
                 v = Q.rv[j];
-                ai = Q.rai[j];
-                bounce = Q.rbounce[j];
                 tmin = 0.0001f;
                 tmax = 1e37f;
             }
-            __syncwarp();
-            if (lane == 0) Q.pool_n = pn - k;
         } else if (tiles) {
             uint32_t base = 0;
             if (lane == 0) base = atomicAdd(A.work_counter, 32u);
@@ -401,15 +416,17 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
                 continue;
             }
             const uint32_t g = base + lane;
-            const int v0 = find_segment(s_poff, A.count, base);
+            const int v0 = find_segment_ldg(A.pix_off, A.count, base);
             have = g < total;
             if (have) {
-                v = g < s_poff[v0 + 1] ? v0 : find_segment(s_poff, A.count, g);
+                v = g < __ldg(&A.pix_off[v0 + 1]) ? v0 : find_segment_ldg(A.pix_off, A.count, g);
                 const BatchView& V = A.views[v];
+                const uint32_t view_px = __ldg(&A.pix_off[v]);
                 int x, y;
-                pixel_of(warp_tile_order((int)(g - s_poff[v]), V.width, V.height), V.width,
+                pixel_of(warp_tile_order((int)(g - view_px), V.width, V.height), V.width,
                          V.height, 32, x, y);
-                ai = (int)s_poff[v] + V.width * y + x;
+                ai = (CARRY ? V.rgba_offset : view_px) + (uint32_t)(V.width * y + x);
+                primary = true;
                 o = mk3(V.cam.pos[0], V.cam.pos[1], V.cam.pos[2]);
                 d = primary_dir(V.cam, x, y, V.width, V.height, 0.0f, 0.0f);
                 ++n_prim;
@@ -428,21 +445,30 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
         }
         const unsigned hm = __ballot_sync(0xffffffffu, hit_ok);
         const int nh = __popc(hm);
+        const int at = first + lane;
         int nl = 0;
         if (hit_ok) {
             const int k = __popc(hm & lt);
             const HitInfo hi = complete_hit(A.views[v].scene, o, d, hit);
-            Q.hp[0][k] = hi.hp.x; Q.hp[1][k] = hi.hp.y; Q.hp[2][k] = hi.hp.z;
+            Q.ro[0][at] = hi.hp.x; Q.ro[1][at] = hi.hp.y; Q.ro[2][at] = hi.hp.z;
             Q.hn[0][k] = hi.n.x; Q.hn[1][k] = hi.n.y; Q.hn[2][k] = hi.n.z;
-            Q.hd[0][k] = d.x; Q.hd[1][k] = d.y; Q.hd[2][k] = d.z;
-            Q.hc[k] = c;
             Q.hid[k] = hit.id;
-            Q.hv[k] = v;
-            Q.hai[k] = ai;
-            Q.hbounce[k] = bounce;
+            Q.hslot[k] = (uint8_t)at;
             Q.hinv[k] = hi.inverse_n;
             Q.hmask[k] = 0u;
+            if (primary) {
+                Q.rd[0][at] = d.x; Q.rd[1][at] = d.y; Q.rd[2][at] = d.z;
+                Q.rc[at] = 1.0f;
+                Q.rv[at] = v;
+                Q.rai[at] = ai;
+                Q.rbounce[at] = 0;
+                if (CARRY) Q.racc[0][at] = Q.racc[1][at] = Q.racc[2][at] = 0u;
+            }
             nl = A.views[v].lights->count;
+        } else if (CARRY && have) {   // the path ends in the void
+            const uint3 sum = primary ? make_uint3(0u, 0u, 0u)
+                                      : make_uint3(Q.racc[0][at], Q.racc[1][at], Q.racc[2][at]);
+            reinterpret_cast<uchar4*>(A.rgba)[primary ? ai : Q.rai[at]] = rgba8_of(sum, A.inv1e6);
         }
         // shadow tasks: hit k owns tasks hoff[k] .. hoff[k+1]-1 (one per light)
         int ex = nl;
@@ -473,12 +499,13 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
                         hi2 = mid - 1;
                 }
                 l = t - Q.hoff[lo];
-                const BatchView& V = A.views[Q.hv[lo]];
+                const int j = Q.hslot[lo];
+                const BatchView& V = A.views[Q.rv[j]];
                 nd = !light_vanishes(V.lights->light[l],
                                      V.scene.mats[__ldg(&V.scene.map[Q.hid[lo]])],
-                                     mk3(Q.hp[0][lo], Q.hp[1][lo], Q.hp[2][lo]),
+                                     mk3(Q.ro[0][j], Q.ro[1][j], Q.ro[2][j]),
                                      mk3(Q.hn[0][lo], Q.hn[1][lo], Q.hn[2][lo]),
-                                     mk3(Q.hd[0][lo], Q.hd[1][lo], Q.hd[2][lo]));
+                                     mk3(Q.rd[0][j], Q.rd[1][j], Q.rd[2][j]));
             }
             const unsigned bm = __ballot_sync(0xffffffffu, nd);
             if (nd) Q.task[nt + __popc(bm & lt)] = (uint8_t)(lo | (l << 5));
@@ -487,9 +514,10 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
         __syncwarp();
         for (int i = lane; i < nt; i += 32) {
             const int e = Q.task[i], lo = e & 31, l = e >> 5;
-            const BatchView& V = A.views[Q.hv[lo]];
+            const int j = Q.hslot[lo];
+            const BatchView& V = A.views[Q.rv[j]];
             const BvhHeader H = *V.scene.hdr;
-            const f3 p = mk3(Q.hp[0][lo], Q.hp[1][lo], Q.hp[2][lo]);
+            const f3 p = mk3(Q.ro[0][j], Q.ro[1][j], Q.ro[2][j]);
             if (occluded(V.scene, H, V.lights->light[l], p, A.status))
                 atomicOr(&Q.hmask[lo], 1u << l);
         }
@@ -497,25 +525,30 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
         bool push = false, push_t = false;
         f3 np = mk3(0.f, 0.f, 0.f), nd = np, td = np;
         float nc = 0.f, tc = 0.f;
-        int nv = 0, nai = 0, nbounce = 0;
+        int nv = 0, nbounce = 0;
+        uint32_t nai = 0;
+        uint3 sum = make_uint3(0u, 0u, 0u);
         if (lane < nh) {
-            const int k = lane;
-            const BatchView& V = A.views[Q.hv[k]];
-            const f3 p = mk3(Q.hp[0][k], Q.hp[1][k], Q.hp[2][k]);
+            const int k = lane, j = Q.hslot[k];
+            nv = Q.rv[j];
+            const BatchView& V = A.views[nv];
+            const f3 p = mk3(Q.ro[0][j], Q.ro[1][j], Q.ro[2][j]);
             const f3 n = mk3(Q.hn[0][k], Q.hn[1][k], Q.hn[2][k]);
-            const f3 dk = mk3(Q.hd[0][k], Q.hd[1][k], Q.hd[2][k]);
-            const float ck = Q.hc[k];
+            const f3 dk = mk3(Q.rd[0][j], Q.rd[1][j], Q.rd[2][j]);
+            const float ck = Q.rc[j];
             const rt_material mat = V.scene.mats[__ldg(&V.scene.map[Q.hid[k]])];
             const uint3 col = shade_hit(*V.lights, mat, p, n, dk, ck, Q.hmask[k]);
-            const int ak = Q.hai[k];
-            if (col.x | col.y | col.z) {   // a zero colour adds nothing
-                atomicAdd(&A.accum[3 * (size_t)ak], col.x);
-                atomicAdd(&A.accum[3 * (size_t)ak + 1], col.y);
-                atomicAdd(&A.accum[3 * (size_t)ak + 2], col.z);
+            nai = Q.rai[j];
+            if (CARRY) {
+                sum = make_uint3(Q.racc[0][j] + col.x, Q.racc[1][j] + col.y, Q.racc[2][j] + col.z);
+            } else if (col.x | col.y | col.z) {   // a zero colour adds nothing
+                atomicAdd(&A.accum[3 * (size_t)nai], col.x);
+                atomicAdd(&A.accum[3 * (size_t)nai + 1], col.y);
+                atomicAdd(&A.accum[3 * (size_t)nai + 2], col.z);
             }
             ++n_hits;
             n_shadow += (uint32_t)V.lights->count;
-            const int bk = Q.hbounce[k];
+            const int bk = Q.rbounce[j];
             if (bk < V.max_bounces) {
                 float R = 1.0f;
                 if (MAXB > 0 && mat.refractive_index > 0.0f &&
@@ -529,44 +562,33 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
                     push = true;
                 }
                 np = p;
-                nv = Q.hv[k];
-                nai = ak;
                 nbounce = bk + 1;
             }
+            if (CARRY && !push)
+                reinterpret_cast<uchar4*>(A.rgba)[nai] = rgba8_of(sum, A.inv1e6);
         }
         const unsigned pm = __ballot_sync(0xffffffffu, push);
         const unsigned pt = MAXB > 0 ? __ballot_sync(0xffffffffu, push_t) : 0u;
-        const int pbase = Q.pool_n;
-        if (push) {
-            const int j = pbase + __popc(pm & lt);
-            if (MAXB == 0 || j < BPOOL) {
-                Q.ro[0][j] = np.x; Q.ro[1][j] = np.y; Q.ro[2][j] = np.z;
-                Q.rd[0][j] = nd.x; Q.rd[1][j] = nd.y; Q.rd[2][j] = nd.z;
-                Q.rc[j] = nc;
-                Q.rv[j] = nv;
-                Q.rai[j] = nai;
-                Q.rbounce[j] = nbounce;
-                ++n_sec;
-            } else {
+        __syncwarp();   // every lane has read its hit's place
+        auto put = [&](int j, f3 dir, float contribution) {
+            if (MAXB > 0 && j >= BPOOL) {
                 atomicOr(A.status, RT_DEV_OVERFLOW);
+                return;
             }
-        }
-        if (MAXB > 0 && push_t) {
-            const int j = pbase + __popc(pm) + __popc(pt & lt);
-            if (j < BPOOL) {
-                Q.ro[0][j] = np.x; Q.ro[1][j] = np.y; Q.ro[2][j] = np.z;
-                Q.rd[0][j] = td.x; Q.rd[1][j] = td.y; Q.rd[2][j] = td.z;
-                Q.rc[j] = tc;
-                Q.rv[j] = nv;
-                Q.rai[j] = nai;
-                Q.rbounce[j] = nbounce;
-                ++n_sec;
-            } else {
-                atomicOr(A.status, RT_DEV_OVERFLOW);
+            Q.ro[0][j] = np.x; Q.ro[1][j] = np.y; Q.ro[2][j] = np.z;
+            Q.rd[0][j] = dir.x; Q.rd[1][j] = dir.y; Q.rd[2][j] = dir.z;
+            Q.rc[j] = contribution;
+            Q.rv[j] = nv;
+            Q.rai[j] = nai;
+            Q.rbounce[j] = nbounce;
+            if (CARRY) {
+                Q.racc[0][j] = sum.x; Q.racc[1][j] = sum.y; Q.racc[2][j] = sum.z;
             }
-        }
-        __syncwarp();
-        if (lane == 0) Q.pool_n = min(BPOOL, pbase + __popc(pm) + __popc(pt));
+            ++n_sec;
+        };
+        if (push) put(first + __popc(pm & lt), nd, nc);
+        if (MAXB > 0 && push_t) put(first + __popc(pm) + __popc(pt & lt), td, tc);
+        if (lane == 0) Q.pool_n = min(BPOOL, first + __popc(pm) + __popc(pt));
         __syncwarp();
     }
     if (A.stats) {
@@ -589,12 +611,9 @@ __global__ void k_batch_fb(BatchRenderArgs A) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= A.total) return;
     const int v = find_segment(A.pix_off, A.count, i);
-    uchar4 o;
-    o.x = to_unorm8(A.accum[3 * (size_t)i], A.inv1e6);
-    o.y = to_unorm8(A.accum[3 * (size_t)i + 1], A.inv1e6);
-    o.z = to_unorm8(A.accum[3 * (size_t)i + 2], A.inv1e6);
-    o.w = 255;
-    reinterpret_cast<uchar4*>(A.rgba)[(size_t)A.views[v].rgba_offset + (i - A.pix_off[v])] = o;
+    const uint32_t* q = A.accum + 3 * (size_t)i;
+    reinterpret_cast<uchar4*>(A.rgba)[(size_t)A.views[v].rgba_offset + (i - A.pix_off[v])] =
+        rgba8_of(make_uint3(q[0], q[1], q[2]), A.inv1e6);
 }
 
 struct BatchRenderVariant {
@@ -603,6 +622,7 @@ struct BatchRenderVariant {
     bool pooled;
     bool refract;      // follows refracted rays
     int max_bounces;   // deepest view it holds (0: any)
+    bool sums() const { return pooled && refract; }   // adds pixels up in BatchRenderArgs::accum
 };
 // Variant 0 serves the request loop (many short launches, where the unpooled
 // kernel measured faster); rt_batch takes the first pooled one (one large
@@ -631,6 +651,10 @@ bool batch_render_variant_pooled(int v) {
     return v >= 0 && v < batch_render_variant_count() && kBatchVariants[v].pooled;
 }
 
+bool batch_render_variant_sums(int v) {
+    return v >= 0 && v < batch_render_variant_count() && kBatchVariants[v].sums();
+}
+
 bool batch_render_variant_refracts(int v) {
     return v >= 0 && v < batch_render_variant_count() && kBatchVariants[v].refract;
 }
@@ -650,14 +674,14 @@ int batch_refract_variant(bool pooled, int max_bounces) {
 
 cudaError_t launch_batch_render(const BatchRenderArgs& a, int variant, int grid, cudaStream_t s) {
     if (variant < 0 || variant >= batch_render_variant_count()) return cudaErrorInvalidValue;
-    const bool pooled = kBatchVariants[variant].pooled;
-    if (pooled) {
+    const bool sums = kBatchVariants[variant].sums();
+    if (sums) {
         if (!a.accum) return cudaErrorInvalidValue;
         cudaError_t e = cudaMemsetAsync(a.accum, 0, 3 * sizeof(uint32_t) * (size_t)a.total, s);
         if (e != cudaSuccess) return e;
     }
     kBatchVariants[variant].fn<<<grid, kBatchVariants[variant].threads, 0, s>>>(a);
-    if (pooled && a.total) k_batch_fb<<<(a.total + 255) / 256, 256, 0, s>>>(a);
+    if (sums && a.total) k_batch_fb<<<(a.total + 255) / 256, 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -71,7 +71,7 @@ struct BatchRenderArgs {
     uint32_t* status;
     int chunk;
     float inv1e6;
-    uint32_t* accum;            // pooled variants: 3 sums per pixel of the launch
+    uint32_t* accum;            // batch_render_variant_sums: 3 sums per pixel of the launch
     uint32_t total;             // pixels of the launch (pix_off[count])
 };
 
@@ -82,8 +82,10 @@ int sort_tile_size();
 cudaError_t launch_batch_build(const BatchBuildArgs& a, int grid, cudaStream_t s);
 int batch_render_variant_count();
 int batch_render_variant_info(int v, int* threads, const void** fn);
-// True for variants that sum into BatchRenderArgs::accum before RGBA8.
+// True for the variants that pool rays per warp, and for those of them that
+// sum into BatchRenderArgs::accum before RGBA8.
 bool batch_render_variant_pooled(int v);
+bool batch_render_variant_sums(int v);
 // True for the variants that follow refracted rays (scenes with refracting
 // materials); batch_refract_variant gives the unpooled one (pooled = false)
 // or the pooled one with the smallest ray pool that holds views of

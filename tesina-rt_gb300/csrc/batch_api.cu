@@ -41,7 +41,7 @@ struct rt_batch {
     std::vector<size_t> scratch_at;         // word offset of each scene's scratch
     rt::BatchView* d_views = nullptr;
     uint32_t* d_pix_off = nullptr;
-    uint32_t* d_accum = nullptr;            // render sums, 3 per pixel (pooled render)
+    uint32_t* d_accum = nullptr;            // render sums, 3 per pixel (glass)
     rt_lights* d_lights = nullptr;          // one per distinct scene
     int build_grid = 0;
     int render_variant = 0, render_grid = 0, render_chunk = 32;
@@ -295,7 +295,6 @@ int32_t rt_batch_set(rt_ctx* c, rt_batch* b, const rt_batch_view* views, int32_t
         cudaMalloc(&b->d_ctr, 4 * 8) || cudaMalloc(&b->d_scratch, 4 * words) ||
         cudaMalloc(&b->d_views, sizeof(rt::BatchView) * count) ||
         cudaMalloc(&b->d_pix_off, 4 * (count + 1)) ||
-        cudaMalloc(&b->d_accum, 3 * sizeof(uint32_t) * std::max<size_t>(1, poff.back())) ||
         cudaMalloc(&b->d_lights, sizeof(rt_lights) * ns) ||
         cudaMalloc(&b->d_stage, sizeof(unsigned long long) * 8) ||
         cudaMalloc(&b->d_emit_off, 4 * std::max<size_t>(1, eoff.size()))) {
@@ -340,6 +339,12 @@ int32_t rt_batch_set(rt_ctx* c, rt_batch* b, const rt_batch_view* views, int32_t
                 b->render_variant = v;
                 break;
             }
+    }
+    if (rt::batch_render_variant_sums(b->render_variant) &&
+        cudaMalloc(&b->d_accum, 3 * sizeof(uint32_t) * std::max<size_t>(1, poff.back()))) {
+        cudaGetLastError();
+        free_tables(b);
+        return fail(RT_ERR_OOM, "rt_batch_set: device allocation failed");
     }
     rt::batch_render_variant_info(b->render_variant, &threads, &fn);
     int rbps = 0;

@@ -1047,7 +1047,7 @@ static cudaError_t launch_render_cfg(rt_ctx* c, rt::RenderArgs a, const rt_rende
     if (grid < 1) grid = 1;
     a.chunk = cfg.chunk;
     a.accum = nullptr;
-    if (rt::render_variant_pooled(cfg.variant)) {
+    if (rt::render_variant_sums(cfg.variant)) {
         a.accum = a.image_rgb ? a.image_rgb : rt::accum_buffer(c, cs, (size_t)pixels);
         if (!a.accum) return cudaErrorMemoryAllocation;
     }

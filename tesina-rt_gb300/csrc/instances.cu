@@ -42,7 +42,9 @@ struct InstanceArgs {
     rt_lights lights;
     rt_camera cam;
     int width, height, max_bounces;
-    uint32_t* accum;          // 3 fixed-point sums per pixel, zeroed before the launch
+    uint8_t* rgba;            // RGBA8 image
+    uint32_t* image_rgb;      // optional fixed-point image, 3 per pixel
+    uint32_t* accum;          // glass: 3 fixed-point sums per pixel, zeroed before the launch
     rt_render_stats* stats;
     uint32_t* work_counter;
     uint32_t* status;
@@ -248,24 +250,40 @@ __device__ __forceinline__ void multi_surface(const InstanceArgs& A, const Multi
 // list of (hit, light) tasks, and the continuing paths' reflection rays from
 // a pool in shared memory, 32 at a time whichever pixels they belong to.
 // Contributions are fixed-point sums per pixel (independent of order), so
-// the image is the one the per-pixel loop gives.
+// the image is the one the per-pixel loop gives; the sum travels with the
+// pixel's ray and the lane that ends the path writes the pixel.
 // MAXB > 0: meshes with refracting materials: a hit continues its reflected
 // and refracted rays (as k_render_pool_refr does), the pool is taken from the
 // top and holds 32 (MAXB + 2) rays, enough for frames of up to MAXB bounces;
-// a push past it raises RT_DEV_OVERFLOW instead of writing.
+// a push past it raises RT_DEV_OVERFLOW instead of writing.  The sums of its
+// pixels, which have several rays on the way, are added up in A.accum.
 namespace {
-template <int IPOOL>
+// As WarpPool (trace.cu): a hit of the current step takes its ray's place.
+// CARRY: the pixels' sums travel with the rays.
+template <int IPOOL, bool CARRY>
 struct InstPool {
     float ro[3][IPOOL], rd[3][IPOOL], rc[IPOOL];
     int rpix[IPOOL], rbounce[IPOOL];
-    float hp[3][32], hn[3][32], hd[3][32], hc[32];
-    int hid[32], hroot[32], hpix[32], hbounce[32];
+    uint32_t racc[3][CARRY ? IPOOL : 1];
+    float hn[3][32];
+    int hid[32], hroot[32];
     unsigned hmask[32];
-    unsigned char hinv[32];
+    uint8_t hslot[32], hinv[32];
     uint8_t task[32 * RT_MAX_LIGHTS];   // shadow tasks that need a ray
     int pool_n;
 };
 }  // namespace
+
+// The pixel's sum, as it is and as RGBA8.
+__device__ __forceinline__ void write_pixel(const InstanceArgs& A, int pix, uint3 sum) {
+    if (A.image_rgb) {
+        uint32_t* q = A.image_rgb + 3 * (size_t)pix;
+        q[0] = sum.x;
+        q[1] = sum.y;
+        q[2] = sum.z;
+    }
+    reinterpret_cast<uchar4*>(A.rgba)[pix] = rgba8_of(sum, A.inv1e6);
+}
 
 // 5 blocks per SM, 102 registers: at 6 the four-wide traversal spills (16 roots
 // at 1920 x 1080: 2.16 -> 2.11 ms; 4 blocks 2.24).
@@ -275,11 +293,13 @@ struct InstPool {
 template <int MAXB>
 __global__ void __launch_bounds__(128, MAXB == 6 ? 5 : RT_INST_MINB) k_render_instances(InstanceArgs A) {
     constexpr int IPOOL = MAXB ? 32 * (MAXB + 2) : 64;   // reflections only: < 32 left + 32 new
+    constexpr bool CARRY = MAXB == 0;
+    static_assert(IPOOL <= 256, "places of the pool in 8 bits");
     __shared__ InstanceArgs sA;
-    __shared__ InstPool<IPOOL> sQ[4];
+    __shared__ InstPool<IPOOL, CARRY> sQ[4];
     if (threadIdx.x == 0) sA = A;
     const int lane = threadIdx.x & 31;
-    InstPool<IPOOL>& Q = sQ[threadIdx.x >> 5];
+    InstPool<IPOOL, CARRY>& Q = sQ[threadIdx.x >> 5];
     if (lane == 0) Q.pool_n = 0;
     __syncthreads();
     const int pixels = sA.width * sA.height;
@@ -290,23 +310,20 @@ __global__ void __launch_bounds__(128, MAXB == 6 ? 5 : RT_INST_MINB) k_render_in
         const int pn = Q.pool_n;
         bool have = false;
         f3 o = mk3(0.f, 0.f, 0.f), d = o;
-        float c = 1.0f, tmin = 0.0f, tmax = 1e36f;
-        int pix = 0, bounce = 0;
+        float tmin = 0.0f, tmax = 1e36f;
+        int tile_pix = -1;      // a primary ray's pixel
+        int first = pn;         // place of the step's first ray
         if (pn >= 32 || (!tiles && pn > 0)) {
             const int k = min(32, pn);
-            const int j = pn - k + lane;
+            first = pn - k;
             have = lane < k;
             if (have) {
+                const int j = first + lane;
                 o = mk3(Q.ro[0][j], Q.ro[1][j], Q.ro[2][j]);
                 d = mk3(Q.rd[0][j], Q.rd[1][j], Q.rd[2][j]);
-                c = Q.rc[j];
-                pix = Q.rpix[j];
-                bounce = Q.rbounce[j];
                 tmin = 0.0001f;
                 tmax = 1e37f;
             }
-            __syncwarp();
-            if (lane == 0) Q.pool_n = pn - k;
         } else if (tiles) {
             int base = 0;
             if (lane == 0) base = (int)atomicAdd(sA.work_counter, 32u);
@@ -320,7 +337,7 @@ __global__ void __launch_bounds__(128, MAXB == 6 ? 5 : RT_INST_MINB) k_render_in
             if (have) {
                 int x, y;
                 pixel_of(warp_tile_order(gid, sA.width, sA.height), sA.width, sA.height, 32, x, y);
-                pix = sA.width * y + x;
+                tile_pix = sA.width * y + x;
                 o = mk3(sA.cam.pos[0], sA.cam.pos[1], sA.cam.pos[2]);
                 d = primary_dir(sA.cam, x, y, sA.width, sA.height, 0.0f, 0.0f);
                 ++n_prim;
@@ -333,35 +350,48 @@ __global__ void __launch_bounds__(128, MAXB == 6 ? 5 : RT_INST_MINB) k_render_in
         const bool hit_ok = mh.h.id >= 0;
         const unsigned hm = __ballot_sync(0xffffffffu, hit_ok);
         const int nh = __popc(hm);
+        const int at = first + lane;
         if (hit_ok) {
             const int k = __popc(hm & lt);
             f3 hp, n;
             bool inv;
             multi_surface(sA, mh, o, d, hp, n, inv);
             Q.hinv[k] = inv;
-            Q.hp[0][k] = hp.x; Q.hp[1][k] = hp.y; Q.hp[2][k] = hp.z;
+            Q.ro[0][at] = hp.x; Q.ro[1][at] = hp.y; Q.ro[2][at] = hp.z;
             Q.hn[0][k] = n.x; Q.hn[1][k] = n.y; Q.hn[2][k] = n.z;
-            Q.hd[0][k] = d.x; Q.hd[1][k] = d.y; Q.hd[2][k] = d.z;
-            Q.hc[k] = c;
             Q.hid[k] = mh.h.id;
             Q.hroot[k] = mh.root;
-            Q.hpix[k] = pix;
-            Q.hbounce[k] = bounce;
+            Q.hslot[k] = (uint8_t)at;
             Q.hmask[k] = 0u;
+            if (tile_pix >= 0) {
+                Q.rd[0][at] = d.x; Q.rd[1][at] = d.y; Q.rd[2][at] = d.z;
+                Q.rc[at] = 1.0f;
+                Q.rpix[at] = tile_pix;
+                Q.rbounce[at] = 0;
+                if (CARRY) Q.racc[0][at] = Q.racc[1][at] = Q.racc[2][at] = 0u;
+            }
+        } else if (CARRY && have) {   // the path ends in the void
+            if (tile_pix >= 0)
+                write_pixel(sA, tile_pix, make_uint3(0u, 0u, 0u));
+            else
+                write_pixel(sA, Q.rpix[at],
+                            make_uint3(Q.racc[0][at], Q.racc[1][at], Q.racc[2][at]));
         }
         __syncwarp();
         const int nl = sA.lights.count;
         shadow_tasks(   // light-major, as k_render_pool
             nh, nl, Q.task,
             [&](int k, int l) {
+                const int j = Q.hslot[k];
                 const SceneView& Sk = sA.roots[Q.hroot[k]].scene;
                 return !light_vanishes(sA.lights.light[l], Sk.mats[__ldg(&Sk.map[Q.hid[k]])],
-                                       mk3(Q.hp[0][k], Q.hp[1][k], Q.hp[2][k]),
+                                       mk3(Q.ro[0][j], Q.ro[1][j], Q.ro[2][j]),
                                        mk3(Q.hn[0][k], Q.hn[1][k], Q.hn[2][k]),
-                                       mk3(Q.hd[0][k], Q.hd[1][k], Q.hd[2][k]));
+                                       mk3(Q.rd[0][j], Q.rd[1][j], Q.rd[2][j]));
             },
             [&](int k, int l) {
-                if (occluded_multi(sA, sA.lights.light[l], mk3(Q.hp[0][k], Q.hp[1][k], Q.hp[2][k])))
+                const int j = Q.hslot[k];
+                if (occluded_multi(sA, sA.lights.light[l], mk3(Q.ro[0][j], Q.ro[1][j], Q.ro[2][j])))
                     atomicOr(&Q.hmask[k], 1u << l);
             });
         __syncwarp();
@@ -369,24 +399,27 @@ __global__ void __launch_bounds__(128, MAXB == 6 ? 5 : RT_INST_MINB) k_render_in
         f3 np = mk3(0.f, 0.f, 0.f), nd = np, td = np;
         float nc = 0.f, tc = 0.f;
         int npix = 0, nbounce = 0;
+        uint3 sum = make_uint3(0u, 0u, 0u);
         if (lane < nh) {
-            const int k = lane;
-            const f3 p = mk3(Q.hp[0][k], Q.hp[1][k], Q.hp[2][k]);
+            const int k = lane, j = Q.hslot[k];
+            const f3 p = mk3(Q.ro[0][j], Q.ro[1][j], Q.ro[2][j]);
             const f3 n = mk3(Q.hn[0][k], Q.hn[1][k], Q.hn[2][k]);
-            const f3 dk = mk3(Q.hd[0][k], Q.hd[1][k], Q.hd[2][k]);
-            const float ck = Q.hc[k];
+            const f3 dk = mk3(Q.rd[0][j], Q.rd[1][j], Q.rd[2][j]);
+            const float ck = Q.rc[j];
             const SceneView& S = sA.roots[Q.hroot[k]].scene;
             const rt_material mat = S.mats[__ldg(&S.map[Q.hid[k]])];
             const uint3 col = shade_hit(sA.lights, mat, p, n, dk, ck, Q.hmask[k]);
-            const int pk = Q.hpix[k];
-            if (col.x | col.y | col.z) {   // a zero colour adds nothing
-                atomicAdd(&sA.accum[3 * (size_t)pk], col.x);
-                atomicAdd(&sA.accum[3 * (size_t)pk + 1], col.y);
-                atomicAdd(&sA.accum[3 * (size_t)pk + 2], col.z);
+            npix = Q.rpix[j];
+            if (CARRY) {
+                sum = make_uint3(Q.racc[0][j] + col.x, Q.racc[1][j] + col.y, Q.racc[2][j] + col.z);
+            } else if (col.x | col.y | col.z) {   // a zero colour adds nothing
+                atomicAdd(&sA.accum[3 * (size_t)npix], col.x);
+                atomicAdd(&sA.accum[3 * (size_t)npix + 1], col.y);
+                atomicAdd(&sA.accum[3 * (size_t)npix + 2], col.z);
             }
             ++n_hits;
             n_shadow += (uint32_t)nl;
-            const int bk = Q.hbounce[k];
+            const int bk = Q.rbounce[j];
             if (bk < sA.max_bounces) {
                 float R = 1.0f;
                 if (MAXB > 0 && mat.refractive_index > 0.0f &&
@@ -400,41 +433,31 @@ __global__ void __launch_bounds__(128, MAXB == 6 ? 5 : RT_INST_MINB) k_render_in
                     push = true;
                 }
                 np = p;
-                npix = pk;
                 nbounce = bk + 1;
             }
+            if (CARRY && !push) write_pixel(sA, npix, sum);
         }
         const unsigned pm = __ballot_sync(0xffffffffu, push);
         const unsigned pt = MAXB > 0 ? __ballot_sync(0xffffffffu, push_t) : 0u;
-        const int pbase = Q.pool_n;
-        if (push) {
-            const int j = pbase + __popc(pm & lt);
-            if (MAXB == 0 || j < IPOOL) {
-                Q.ro[0][j] = np.x; Q.ro[1][j] = np.y; Q.ro[2][j] = np.z;
-                Q.rd[0][j] = nd.x; Q.rd[1][j] = nd.y; Q.rd[2][j] = nd.z;
-                Q.rc[j] = nc;
-                Q.rpix[j] = npix;
-                Q.rbounce[j] = nbounce;
-                ++n_sec;
-            } else {
+        __syncwarp();   // every lane has read its hit's place
+        auto put = [&](int j, f3 dir, float contribution) {
+            if (MAXB > 0 && j >= IPOOL) {
                 atomicOr(sA.status, RT_DEV_OVERFLOW);
+                return;
             }
-        }
-        if (MAXB > 0 && push_t) {
-            const int j = pbase + __popc(pm) + __popc(pt & lt);
-            if (j < IPOOL) {
-                Q.ro[0][j] = np.x; Q.ro[1][j] = np.y; Q.ro[2][j] = np.z;
-                Q.rd[0][j] = td.x; Q.rd[1][j] = td.y; Q.rd[2][j] = td.z;
-                Q.rc[j] = tc;
-                Q.rpix[j] = npix;
-                Q.rbounce[j] = nbounce;
-                ++n_sec;
-            } else {
-                atomicOr(sA.status, RT_DEV_OVERFLOW);
+            Q.ro[0][j] = np.x; Q.ro[1][j] = np.y; Q.ro[2][j] = np.z;
+            Q.rd[0][j] = dir.x; Q.rd[1][j] = dir.y; Q.rd[2][j] = dir.z;
+            Q.rc[j] = contribution;
+            Q.rpix[j] = npix;
+            Q.rbounce[j] = nbounce;
+            if (CARRY) {
+                Q.racc[0][j] = sum.x; Q.racc[1][j] = sum.y; Q.racc[2][j] = sum.z;
             }
-        }
-        __syncwarp();
-        if (lane == 0) Q.pool_n = min(IPOOL, pbase + __popc(pm) + __popc(pt));
+            ++n_sec;
+        };
+        if (push) put(first + __popc(pm & lt), nd, nc);
+        if (MAXB > 0 && push_t) put(first + __popc(pm) + __popc(pt & lt), td, tc);
+        if (lane == 0) Q.pool_n = min(IPOOL, first + __popc(pm) + __popc(pt));
         __syncwarp();
     }
     if (sA.stats) {
@@ -589,8 +612,13 @@ int32_t rt_instances_render(rt_ctx* c, rt_instances* I, const rt_camera* cam, in
     A.height = h;
     A.max_bounces = max_bounces;
     const size_t px = (size_t)w * h;
-    A.accum = img ? img : rt::accum_buffer(c, cs, px);
-    if (!A.accum) return fail(RT_ERR_OOM, "rt_instances_render: pixel sums");
+    A.rgba = rgba;
+    A.image_rgb = img;
+    A.accum = nullptr;
+    if (refracts) {
+        A.accum = img ? img : rt::accum_buffer(c, cs, px);
+        if (!A.accum) return fail(RT_ERR_OOM, "rt_instances_render: pixel sums");
+    }
     A.stats = stats;
     A.work_counter = work;
     A.status = c->d_status;
@@ -618,10 +646,10 @@ int32_t rt_instances_render(rt_ctx* c, rt_instances* I, const rt_camera* cam, in
     if (I->rendered && I->render_stream != cs) CU(cudaStreamWaitEvent(cs, I->ev_render, 0));
     rt::k_instance_boxes<<<(unsigned)((A.count + 127) / 128), 128, 0, cs>>>(I->d_roots, A.count,
                                                                             I->d_cull);
-    CU(cudaMemsetAsync(A.accum, 0, 3 * sizeof(uint32_t) * px, cs));
+    if (refracts) CU(cudaMemsetAsync(A.accum, 0, 3 * sizeof(uint32_t) * px, cs));
     kern<<<(unsigned)grid, 128, 0, cs>>>(A);
     CU(cudaGetLastError());
-    CU(rt::launch_fb_copy(A.accum, rgba, px, c->inv1e6, cs));
+    if (refracts) CU(rt::launch_fb_copy(A.accum, rgba, px, c->inv1e6, cs));
     for (rt_scene* s : I->scenes) CU(rt::scene_read_end(s, cs));
     CU(cudaEventRecord(I->ev_render, cs));
     I->render_stream = cs;

@@ -50,12 +50,8 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render(RenderArgs a) {
                 a.image_rgb[3 * (size_t)pix + 1] = acc_g;
                 a.image_rgb[3 * (size_t)pix + 2] = acc_b;
             }
-            uchar4 px;
-            px.x = to_unorm8(acc_r, a.inv1e6);
-            px.y = to_unorm8(acc_g, a.inv1e6);
-            px.z = to_unorm8(acc_b, a.inv1e6);
-            px.w = 255;
-            reinterpret_cast<uchar4*>(a.rgba)[pix] = px;
+            reinterpret_cast<uchar4*>(a.rgba)[pix] =
+                rgba8_of(make_uint3(acc_r, acc_g, acc_b), a.inv1e6);
         }
         }
     }
@@ -79,25 +75,45 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render(RenderArgs a) {
 // together (coherent); the hits' shadow rays are traced as a dense list of
 // (hit, light) tasks; each hit is shaded and, if the path continues, its
 // reflection ray goes into the warp's pool in shared memory, which is traced
-// 32 rays at a time whichever pixels they come from.  A pixel's fixed-point
-// contributions are added into its accumulator (integer sums do not depend
-// on order) and k_fb_copy turns the sums into RGBA8 afterwards.  Every ray is
+// 32 rays at a time whichever pixels they come from.  A pixel has one ray on
+// the way at a time, so its fixed-point sum travels with the ray, and the lane
+// that ends the path writes the pixel: no accumulation buffer to clear, add to
+// and convert afterwards (thumbnail 74 -> 66 us, 1920 x 1080 frames 0.5-1.5 %).
+// Every ray is
 // traversed and shaded exactly as in render_pixel, so the image is
 // bit-identical to k_render's.
 // ---------------------------------------------------------------------------
 namespace {
-constexpr int POOL = 64;   // reflection rays a warp can hold: < 32 left + 32 new
+constexpr int POOL = 64;   // rays a warp can hold: < 32 left + 32 of the current step
 
+// The rays of a warp.  The ones left wait in places 0 .. pool_n - 1; those of
+// the current step keep or take the places above, where a hit puts its point
+// over its ray's origin, until the step's own reflection rays are written over
+// them.  The L1 shares the SM's memory with this: a further 1.1 KB per warp (the
+// hits in arrays of their own) cost 1-3 % of a frame.
 struct WarpPool {
-    float ro[3][POOL], rd[3][POOL], rc[POOL];   // pooled rays: origin, direction, contribution
+    float ro[3][POOL], rd[3][POOL], rc[POOL];   // origin or hit point, direction, contribution
     int rpix[POOL], rbounce[POOL];
-    float hp[3][32], hn[3][32], hd[3][32], hc[32];   // hits of the current step
-    int hid[32], hpix[32], hbounce[32];
+    uint32_t racc[3][POOL];                     // the pixel's sum so far
+    float hn[3][32];                            // hits of the current step
+    int hid[32];
     unsigned hmask[32];
-    uint8_t task[32 * RT_MAX_LIGHTS];   // shadow tasks that need a ray
+    uint8_t hslot[32];                          // their places
+    uint8_t task[32 * RT_MAX_LIGHTS];           // shadow tasks that need a ray
     int pool_n;
 };
 }  // namespace
+
+// The pixel's sum, as it is and as RGBA8.
+__device__ __forceinline__ void write_pixel(const RenderArgs& a, int pix, uint3 sum) {
+    if (a.image_rgb) {
+        uint32_t* q = a.image_rgb + 3 * (size_t)pix;
+        q[0] = sum.x;
+        q[1] = sum.y;
+        q[2] = sum.z;
+    }
+    reinterpret_cast<uchar4*>(a.rgba)[pix] = rgba8_of(sum, a.inv1e6);
+}
 
 template <int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) k_render_pool(RenderArgs a) {
@@ -123,23 +139,20 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_pool(RenderArgs a) {
         //    of primary rays, else what is left in the pool
         bool have = false;
         f3 o = mk3(0.f, 0.f, 0.f), d = o;
-        float c = 1.0f, tmin = 0.0f, tmax = 1e36f;
-        int pix = 0, bounce = 0;
+        float tmin = 0.0f, tmax = 1e36f;
+        int tile_pix = -1;      // a primary ray's pixel
+        int first = pn;         // place of the step's first ray
         if (pn >= 32 || (!tiles && pn > 0)) {
             const int k = min(32, pn);
-            const int j = pn - k + lane;
+            first = pn - k;
             have = lane < k;
             if (have) {
+                const int j = first + lane;
                 o = mk3(Q.ro[0][j], Q.ro[1][j], Q.ro[2][j]);
                 d = mk3(Q.rd[0][j], Q.rd[1][j], Q.rd[2][j]);
-                c = Q.rc[j];
-                pix = Q.rpix[j];
-                bounce = Q.rbounce[j];
                 tmin = 0.0001f;
                 tmax = 1e37f;
             }
-            __syncwarp();
-            if (lane == 0) Q.pool_n = pn - k;
         } else if (tiles) {
             int base = 0;
             if (lane == 0) base = (int)atomicAdd(a.work_counter, 32u);
@@ -153,7 +166,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_pool(RenderArgs a) {
             if (have) {
                 int x, y;
                 pixel_of(warp_tile_order(gid, a.width, a.height), a.width, a.height, 32, x, y);
-                pix = a.width * y + x;
+                tile_pix = a.width * y + x;
                 o = mk3(a.cam.pos[0], a.cam.pos[1], a.cam.pos[2]);
                 d = primary_dir(a.cam, x, y, a.width, a.height, 0.0f, 0.0f);
                 ++n_prim;
@@ -171,17 +184,28 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_pool(RenderArgs a) {
         }
         const unsigned hm = __ballot_sync(0xffffffffu, hit_ok);
         const int nh = __popc(hm);
+        const int at = first + lane;
         if (hit_ok) {
             const int k = __popc(hm & lt);
             const HitInfo hi = complete_hit(S, o, d, hit);
-            Q.hp[0][k] = hi.hp.x; Q.hp[1][k] = hi.hp.y; Q.hp[2][k] = hi.hp.z;
+            Q.ro[0][at] = hi.hp.x; Q.ro[1][at] = hi.hp.y; Q.ro[2][at] = hi.hp.z;
             Q.hn[0][k] = hi.n.x; Q.hn[1][k] = hi.n.y; Q.hn[2][k] = hi.n.z;
-            Q.hd[0][k] = d.x; Q.hd[1][k] = d.y; Q.hd[2][k] = d.z;
-            Q.hc[k] = c;
             Q.hid[k] = hit.id;
-            Q.hpix[k] = pix;
-            Q.hbounce[k] = bounce;
+            Q.hslot[k] = (uint8_t)at;
             Q.hmask[k] = 0u;
+            if (tile_pix >= 0) {
+                Q.rd[0][at] = d.x; Q.rd[1][at] = d.y; Q.rd[2][at] = d.z;
+                Q.rc[at] = 1.0f;
+                Q.rpix[at] = tile_pix;
+                Q.rbounce[at] = 0;
+                Q.racc[0][at] = Q.racc[1][at] = Q.racc[2][at] = 0u;
+            }
+        } else if (have) {   // the path ends in the void
+            if (tile_pix >= 0)
+                write_pixel(a, tile_pix, make_uint3(0u, 0u, 0u));
+            else
+                write_pixel(a, Q.rpix[at],
+                            make_uint3(Q.racc[0][at], Q.racc[1][at], Q.racc[2][at]));
         }
         __syncwarp();
         // 3. shadow rays of every hit and light, 32 at a time
@@ -194,13 +218,15 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_pool(RenderArgs a) {
         shadow_tasks(
             nh, nl, Q.task,
             [&](int k, int l) {
+                const int j = Q.hslot[k];
                 return !light_vanishes(sL.light[l], S.mats[__ldg(&S.map[Q.hid[k]])],
-                                       mk3(Q.hp[0][k], Q.hp[1][k], Q.hp[2][k]),
+                                       mk3(Q.ro[0][j], Q.ro[1][j], Q.ro[2][j]),
                                        mk3(Q.hn[0][k], Q.hn[1][k], Q.hn[2][k]),
-                                       mk3(Q.hd[0][k], Q.hd[1][k], Q.hd[2][k]));
+                                       mk3(Q.rd[0][j], Q.rd[1][j], Q.rd[2][j]));
             },
             [&](int k, int l) {
-                if (occluded(S, H, sL.light[l], mk3(Q.hp[0][k], Q.hp[1][k], Q.hp[2][k]), a.status))
+                const int j = Q.hslot[k];
+                if (occluded(S, H, sL.light[l], mk3(Q.ro[0][j], Q.ro[1][j], Q.ro[2][j]), a.status))
                     atomicOr(&Q.hmask[k], 1u << l);
             });
         __syncwarp();
@@ -209,45 +235,43 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_pool(RenderArgs a) {
         f3 np = mk3(0.f, 0.f, 0.f), nd = np;
         float nc = 0.f;
         int npix = 0, nbounce = 0;
+        uint3 sum = make_uint3(0u, 0u, 0u);
         if (lane < nh) {
-            const int k = lane;
-            const f3 p = mk3(Q.hp[0][k], Q.hp[1][k], Q.hp[2][k]);
+            const int k = lane, j = Q.hslot[k];
+            const f3 p = mk3(Q.ro[0][j], Q.ro[1][j], Q.ro[2][j]);
             const f3 n = mk3(Q.hn[0][k], Q.hn[1][k], Q.hn[2][k]);
-            const f3 dk = mk3(Q.hd[0][k], Q.hd[1][k], Q.hd[2][k]);
-            const float ck = Q.hc[k];
+            const f3 dk = mk3(Q.rd[0][j], Q.rd[1][j], Q.rd[2][j]);
+            const float ck = Q.rc[j];
             const rt_material mat = S.mats[__ldg(&S.map[Q.hid[k]])];
             const uint3 col = shade_hit(sL, mat, p, n, dk, ck, Q.hmask[k]);
-            const int pk = Q.hpix[k];
-            if (col.x | col.y | col.z) {   // a zero colour adds nothing
-                atomicAdd(&a.accum[3 * (size_t)pk], col.x);
-                atomicAdd(&a.accum[3 * (size_t)pk + 1], col.y);
-                atomicAdd(&a.accum[3 * (size_t)pk + 2], col.z);
-            }
+            npix = Q.rpix[j];
+            sum = make_uint3(Q.racc[0][j] + col.x, Q.racc[1][j] + col.y, Q.racc[2][j] + col.z);
             ++n_hits;
             n_shadow += (uint32_t)nl;
-            const int bk = Q.hbounce[k];
+            const int bk = Q.rbounce[j];
             if (bk != a.max_bounces && mat.reflectiveness > 0.0f) {
                 reflect_ray(dk, n, nd);
                 np = p;
                 nc = ck * mat.reflectiveness * 1.0f;
-                npix = pk;
                 nbounce = bk + 1;
                 push = true;
                 ++n_sec;
+            } else {
+                write_pixel(a, npix, sum);
             }
         }
         const unsigned pm = __ballot_sync(0xffffffffu, push);
-        const int pbase = Q.pool_n;
+        __syncwarp();   // every lane has read its hit's place
         if (push) {
-            const int j = pbase + __popc(pm & lt);
+            const int j = first + __popc(pm & lt);
             Q.ro[0][j] = np.x; Q.ro[1][j] = np.y; Q.ro[2][j] = np.z;
             Q.rd[0][j] = nd.x; Q.rd[1][j] = nd.y; Q.rd[2][j] = nd.z;
             Q.rc[j] = nc;
             Q.rpix[j] = npix;
             Q.rbounce[j] = nbounce;
+            Q.racc[0][j] = sum.x; Q.racc[1][j] = sum.y; Q.racc[2][j] = sum.z;
         }
-        __syncwarp();
-        if (lane == 0) Q.pool_n = pbase + __popc(pm);
+        if (lane == 0) Q.pool_n = first + __popc(pm);
         __syncwarp();
     }
     if (a.stats) {
@@ -276,13 +300,13 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_pool(RenderArgs a) {
 // ---------------------------------------------------------------------------
 namespace {
 template <int RPOOL>
-struct RefrPool {
+struct RefrPool {   // as WarpPool
     float ro[3][RPOOL], rd[3][RPOOL], rc[RPOOL];
     int rpix[RPOOL], rbounce[RPOOL];
-    float hp[3][32], hn[3][32], hd[3][32], hc[32];
-    int hid[32], hpix[32], hbounce[32];
+    float hn[3][32];
+    int hid[32];
     unsigned hmask[32];
-    unsigned char hinv[32];
+    uint8_t hslot[32], hinv[32];
     uint8_t task[32 * RT_MAX_LIGHTS];   // shadow tasks that need a ray
     int pool_n;
 };
@@ -291,6 +315,7 @@ struct RefrPool {
 template <int THREADS, int MINB, int MAXB>
 __global__ void __launch_bounds__(THREADS, MINB) k_render_pool_refr(RenderArgs a) {
     constexpr int RPOOL = 32 * (MAXB + 2);
+    static_assert(RPOOL <= 256, "places of the pool in 8 bits");
     const SceneView S = a.scene;
     __shared__ BvhHeader sH;
     __shared__ rt_lights sL;
@@ -311,23 +336,20 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_pool_refr(RenderArgs a
         const int pn = Q.pool_n;
         bool have = false;
         f3 o = mk3(0.f, 0.f, 0.f), d = o;
-        float c = 1.0f, tmin = 0.0f, tmax = 1e36f;
-        int pix = 0, bounce = 0;
+        float tmin = 0.0f, tmax = 1e36f;
+        int tile_pix = -1;      // a primary ray's pixel
+        int first = pn;         // place of the step's first ray
         if (pn >= 32 || (!tiles && pn > 0)) {
             const int k = min(32, pn);
-            const int j = pn - k + lane;
+            first = pn - k;
             have = lane < k;
             if (have) {
+                const int j = first + lane;
                 o = mk3(Q.ro[0][j], Q.ro[1][j], Q.ro[2][j]);
                 d = mk3(Q.rd[0][j], Q.rd[1][j], Q.rd[2][j]);
-                c = Q.rc[j];
-                pix = Q.rpix[j];
-                bounce = Q.rbounce[j];
                 tmin = 0.0001f;
                 tmax = 1e37f;
             }
-            __syncwarp();
-            if (lane == 0) Q.pool_n = pn - k;
         } else if (tiles) {
             int base = 0;
             if (lane == 0) base = (int)atomicAdd(a.work_counter, 32u);
@@ -341,7 +363,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_pool_refr(RenderArgs a
             if (have) {
                 int x, y;
                 pixel_of(warp_tile_order(gid, a.width, a.height), a.width, a.height, 32, x, y);
-                pix = a.width * y + x;
+                tile_pix = a.width * y + x;
                 o = mk3(a.cam.pos[0], a.cam.pos[1], a.cam.pos[2]);
                 d = primary_dir(a.cam, x, y, a.width, a.height, 0.0f, 0.0f);
                 ++n_prim;
@@ -358,56 +380,62 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_pool_refr(RenderArgs a
         }
         const unsigned hm = __ballot_sync(0xffffffffu, hit_ok);
         const int nh = __popc(hm);
+        const int at = first + lane;
         if (hit_ok) {
             const int k = __popc(hm & lt);
             const HitInfo hi = complete_hit(S, o, d, hit);
-            Q.hp[0][k] = hi.hp.x; Q.hp[1][k] = hi.hp.y; Q.hp[2][k] = hi.hp.z;
+            Q.ro[0][at] = hi.hp.x; Q.ro[1][at] = hi.hp.y; Q.ro[2][at] = hi.hp.z;
             Q.hn[0][k] = hi.n.x; Q.hn[1][k] = hi.n.y; Q.hn[2][k] = hi.n.z;
-            Q.hd[0][k] = d.x; Q.hd[1][k] = d.y; Q.hd[2][k] = d.z;
-            Q.hc[k] = c;
             Q.hid[k] = hit.id;
-            Q.hpix[k] = pix;
-            Q.hbounce[k] = bounce;
             Q.hinv[k] = hi.inverse_n;
+            Q.hslot[k] = (uint8_t)at;
             Q.hmask[k] = 0u;
+            if (tile_pix >= 0) {
+                Q.rd[0][at] = d.x; Q.rd[1][at] = d.y; Q.rd[2][at] = d.z;
+                Q.rc[at] = 1.0f;
+                Q.rpix[at] = tile_pix;
+                Q.rbounce[at] = 0;
+            }
         }
         __syncwarp();
         const int nl = sL.count;
-        shadow_tasks(
+        shadow_tasks(   // light-major, as k_render_pool
             nh, nl, Q.task,
             [&](int k, int l) {
+                const int j = Q.hslot[k];
                 return !light_vanishes(sL.light[l], S.mats[__ldg(&S.map[Q.hid[k]])],
-                                       mk3(Q.hp[0][k], Q.hp[1][k], Q.hp[2][k]),
+                                       mk3(Q.ro[0][j], Q.ro[1][j], Q.ro[2][j]),
                                        mk3(Q.hn[0][k], Q.hn[1][k], Q.hn[2][k]),
-                                       mk3(Q.hd[0][k], Q.hd[1][k], Q.hd[2][k]));
+                                       mk3(Q.rd[0][j], Q.rd[1][j], Q.rd[2][j]));
             },
             [&](int k, int l) {
-                if (occluded<false, true>(S, H, sL.light[l], mk3(Q.hp[0][k], Q.hp[1][k], Q.hp[2][k]), a.status))
+                const int j = Q.hslot[k];
+                if (occluded<false, true>(S, H, sL.light[l],
+                                          mk3(Q.ro[0][j], Q.ro[1][j], Q.ro[2][j]), a.status))
                     atomicOr(&Q.hmask[k], 1u << l);
             });
         __syncwarp();
-        // shading; the continuing rays of each hit: reflected, refracted
-        bool push_r = false, push_t = false;
+        bool push = false, push_t = false;
         f3 np = mk3(0.f, 0.f, 0.f), nd = np, td = np;
         float nc = 0.f, tc = 0.f;
         int npix = 0, nbounce = 0;
         if (lane < nh) {
-            const int k = lane;
-            const f3 p = mk3(Q.hp[0][k], Q.hp[1][k], Q.hp[2][k]);
+            const int k = lane, j = Q.hslot[k];
+            const f3 p = mk3(Q.ro[0][j], Q.ro[1][j], Q.ro[2][j]);
             const f3 n = mk3(Q.hn[0][k], Q.hn[1][k], Q.hn[2][k]);
-            const f3 dk = mk3(Q.hd[0][k], Q.hd[1][k], Q.hd[2][k]);
-            const float ck = Q.hc[k];
+            const f3 dk = mk3(Q.rd[0][j], Q.rd[1][j], Q.rd[2][j]);
+            const float ck = Q.rc[j];
             const rt_material mat = S.mats[__ldg(&S.map[Q.hid[k]])];
             const uint3 col = shade_hit(sL, mat, p, n, dk, ck, Q.hmask[k]);
-            const int pk = Q.hpix[k];
+            npix = Q.rpix[j];
             if (col.x | col.y | col.z) {   // a zero colour adds nothing
-                atomicAdd(&a.accum[3 * (size_t)pk], col.x);
-                atomicAdd(&a.accum[3 * (size_t)pk + 1], col.y);
-                atomicAdd(&a.accum[3 * (size_t)pk + 2], col.z);
+                atomicAdd(&a.accum[3 * (size_t)npix], col.x);
+                atomicAdd(&a.accum[3 * (size_t)npix + 1], col.y);
+                atomicAdd(&a.accum[3 * (size_t)npix + 2], col.z);
             }
             ++n_hits;
             n_shadow += (uint32_t)nl;
-            const int bk = Q.hbounce[k];
+            const int bk = Q.rbounce[j];
             if (bk < a.max_bounces) {
                 float R = 1.0f;
                 if (mat.refractive_index > 0.0f &&
@@ -418,44 +446,30 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_pool_refr(RenderArgs a
                 if (mat.reflectiveness > 0.0f) {
                     reflect_ray(dk, n, nd);
                     nc = ck * mat.reflectiveness * R;
-                    push_r = true;
+                    push = true;
                 }
                 np = p;
-                npix = pk;
                 nbounce = bk + 1;
             }
         }
-        const unsigned pr = __ballot_sync(0xffffffffu, push_r);
+        const unsigned pm = __ballot_sync(0xffffffffu, push);
         const unsigned pt = __ballot_sync(0xffffffffu, push_t);
-        const int pbase = Q.pool_n;
-        if (push_r) {
-            const int j = pbase + __popc(pr & lt);
-            if (j < RPOOL) {
-                Q.ro[0][j] = np.x; Q.ro[1][j] = np.y; Q.ro[2][j] = np.z;
-                Q.rd[0][j] = nd.x; Q.rd[1][j] = nd.y; Q.rd[2][j] = nd.z;
-                Q.rc[j] = nc;
-                Q.rpix[j] = npix;
-                Q.rbounce[j] = nbounce;
-                ++n_sec;
-            } else {
+        __syncwarp();   // every lane has read its hit's place
+        auto put = [&](int j, f3 dir, float contribution) {
+            if (j >= RPOOL) {
                 atomicOr(a.status, RT_DEV_OVERFLOW);
+                return;
             }
-        }
-        if (push_t) {
-            const int j = pbase + __popc(pr) + __popc(pt & lt);
-            if (j < RPOOL) {
-                Q.ro[0][j] = np.x; Q.ro[1][j] = np.y; Q.ro[2][j] = np.z;
-                Q.rd[0][j] = td.x; Q.rd[1][j] = td.y; Q.rd[2][j] = td.z;
-                Q.rc[j] = tc;
-                Q.rpix[j] = npix;
-                Q.rbounce[j] = nbounce;
-                ++n_sec;
-            } else {
-                atomicOr(a.status, RT_DEV_OVERFLOW);
-            }
-        }
-        __syncwarp();
-        if (lane == 0) Q.pool_n = min(RPOOL, pbase + __popc(pr) + __popc(pt));
+            Q.ro[0][j] = np.x; Q.ro[1][j] = np.y; Q.ro[2][j] = np.z;
+            Q.rd[0][j] = dir.x; Q.rd[1][j] = dir.y; Q.rd[2][j] = dir.z;
+            Q.rc[j] = contribution;
+            Q.rpix[j] = npix;
+            Q.rbounce[j] = nbounce;
+            ++n_sec;
+        };
+        if (push) put(first + __popc(pm & lt), nd, nc);
+        if (push_t) put(first + __popc(pm) + __popc(pt & lt), td, tc);
+        if (lane == 0) Q.pool_n = min(RPOOL, first + __popc(pm) + __popc(pt));
         __syncwarp();
     }
     if (a.stats) {
@@ -710,12 +724,7 @@ __global__ void k_fb_copy(const uint32_t* __restrict__ img, uchar4* __restrict__
                           float inv1e6) {
     const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if (i >= px) return;
-    uchar4 o;
-    o.x = to_unorm8(img[3 * i], inv1e6);
-    o.y = to_unorm8(img[3 * i + 1], inv1e6);
-    o.z = to_unorm8(img[3 * i + 2], inv1e6);
-    o.w = 255;
-    rgba[i] = o;
+    rgba[i] = rgba8_of(make_uint3(img[3 * i], img[3 * i + 1], img[3 * i + 2]), inv1e6);
 }
 
 // ---------------------------------------------------------------------------
@@ -731,6 +740,9 @@ struct RenderVariant {
     bool pooled;
     bool refract;     // follows the refracted rays of refracting materials
     int max_bounces;  // deepest frame it holds (0: any)
+    // a pixel's sum is added up in RenderArgs::accum (several of its rays may
+    // be on the way at once)
+    bool sums() const { return pooled && refract; }
 };
 static const RenderVariant kVariants[] = {
     {64, 8, k_render<64, 8>, false},    {64, 12, k_render<64, 12>, false},
@@ -758,6 +770,8 @@ int render_variant_info(int v, int* threads, int* min_blocks, const void** fn) {
 
 bool render_variant_pooled(int v) { return v >= 0 && v < kNumVariants && kVariants[v].pooled; }
 
+bool render_variant_sums(int v) { return v >= 0 && v < kNumVariants && kVariants[v].sums(); }
+
 bool render_variant_refracts(int v) { return v >= 0 && v < kNumVariants && kVariants[v].refract; }
 
 bool render_variant_fits(int v, int max_bounces) {
@@ -781,13 +795,13 @@ int render_refract_variant(int max_bounces) {
 cudaError_t launch_render(const RenderArgs& a, int variant, int grid, cudaStream_t s) {
     if (variant < 0 || variant >= kNumVariants) return cudaErrorInvalidValue;
     const size_t px = (size_t)a.width * a.height;
-    if (kVariants[variant].pooled) {
+    if (kVariants[variant].sums()) {
         if (!a.accum) return cudaErrorInvalidValue;
         cudaError_t e = cudaMemsetAsync(a.accum, 0, 3 * sizeof(uint32_t) * px, s);
         if (e != cudaSuccess) return e;
     }
     kVariants[variant].fn<<<grid, kVariants[variant].threads, 0, s>>>(a);
-    if (kVariants[variant].pooled && px)
+    if (kVariants[variant].sums() && px)
         k_fb_copy<<<blocks(px, 256), 256, 0, s>>>(a.accum, reinterpret_cast<uchar4*>(a.rgba), px,
                                                   a.inv1e6);
     return cudaGetLastError();

@@ -20,14 +20,18 @@ struct RenderArgs {
     uint32_t* work_counter;       // zeroed before launch
     uint32_t* status;
     int chunk;                    // pixels per warp work fetch, multiple of 32
-    uint32_t* accum;              // pooled variants: fixed-point sums (3 per pixel)
+    uint32_t* accum;              // render_variant_sums: fixed-point sums (3 per pixel)
 };
 
 // Render kernel variants (block size, minimum blocks per SM) for the autotuner.
 int render_variant_count();
 int render_variant_info(int v, int* threads, int* min_blocks, const void** fn);
-// True for variants that accumulate into RenderArgs::accum (k_render_pool).
+// True for the variants that pool rays per warp (k_render_pool,
+// k_render_pool_refr), and for those of them that add a pixel's contributions
+// up in RenderArgs::accum (k_render_pool_refr: a pixel has several rays on the
+// way at once).
 bool render_variant_pooled(int v);
+bool render_variant_sums(int v);
 // True for the variants that follow refracted rays; the scenes with
 // refracting materials render with one of them.
 bool render_variant_refracts(int v);

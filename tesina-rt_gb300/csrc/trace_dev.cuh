@@ -604,6 +604,11 @@ __device__ __forceinline__ uint8_t to_unorm8(uint32_t v, float inv1e6) {
     return (uint8_t)__float2uint_rn(clamp01(f) * 255.0f);
 }
 
+__device__ __forceinline__ uchar4 rgba8_of(uint3 sum, float inv1e6) {
+    return make_uchar4(to_unorm8(sum.x, inv1e6), to_unorm8(sum.y, inv1e6),
+                       to_unorm8(sum.z, inv1e6), 255);
+}
+
 
 // Result of one pixel's Whitted path.
 struct PixelResult {
