@@ -361,14 +361,15 @@ template <int BPOOL, bool CARRY>
 struct WarpPoolB {
     float ro[3][BPOOL], rd[3][BPOOL], rc[BPOOL];
     // view, place of the pixel (CARRY: in rgba, else in accum), bounce
-    int rv[BPOOL], rbounce[BPOOL];
+    uint16_t rv[BPOOL];
+    uint8_t rbounce[BPOOL];
     uint32_t rai[BPOOL], racc[3][CARRY ? BPOOL : 1];
     float hn[3][32];
-    int hid[32], hoff[33];
+    int hid[32];
     unsigned hmask[32];
-    uint8_t hslot[32], hinv[32];
+    uint16_t hoff[32];
+    uint8_t hslot[CARRY ? 32 : 64];     // the hits' places; glass: then inverse_n
     uint8_t task[32 * RT_MAX_LIGHTS];   // shadow tasks that need a ray
-    int pool_n;
 };
 }  // namespace
 
@@ -377,17 +378,16 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
     constexpr int BPOOL = MAXB ? 32 * (MAXB + 2) : 64;
     constexpr bool CARRY = MAXB == 0;
     static_assert(BPOOL <= 256, "places of the pool in 8 bits");
+    static_assert(kMaxBatchViews <= 65536, "views in 16 bits");
     __shared__ WarpPoolB<BPOOL, CARRY> sQ[THREADS / 32];
     const int lane = threadIdx.x & 31;
     WarpPoolB<BPOOL, CARRY>& Q = sQ[threadIdx.x >> 5];
-    if (lane == 0) Q.pool_n = 0;
-    __syncwarp();
     const uint32_t total = __ldg(&A.pix_off[A.count]);
     const unsigned lt = (1u << lane) - 1u;
     uint32_t n_prim = 0, n_sec = 0, n_shadow = 0, n_hits = 0;
     bool tiles = true;
+    int pn = 0;   // rays waiting in the pool
     for (;;) {
-        const int pn = Q.pool_n;
         bool have = false;
         f3 o = mk3(0.f, 0.f, 0.f), d = o;
         float tmin = 0.0f, tmax = 1e36f;
@@ -454,12 +454,12 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
             Q.hn[0][k] = hi.n.x; Q.hn[1][k] = hi.n.y; Q.hn[2][k] = hi.n.z;
             Q.hid[k] = hit.id;
             Q.hslot[k] = (uint8_t)at;
-            Q.hinv[k] = hi.inverse_n;
+            if (!CARRY) Q.hslot[32 + k] = hi.inverse_n;
             Q.hmask[k] = 0u;
             if (primary) {
                 Q.rd[0][at] = d.x; Q.rd[1][at] = d.y; Q.rd[2][at] = d.z;
                 Q.rc[at] = 1.0f;
-                Q.rv[at] = v;
+                Q.rv[at] = (uint16_t)v;
                 Q.rai[at] = ai;
                 Q.rbounce[at] = 0;
                 if (CARRY) Q.racc[0][at] = Q.racc[1][at] = Q.racc[2][at] = 0u;
@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
                                       : make_uint3(Q.racc[0][at], Q.racc[1][at], Q.racc[2][at]);
             reinterpret_cast<uchar4*>(A.rgba)[primary ? ai : Q.rai[at]] = rgba8_of(sum, A.inv1e6);
         }
-        // shadow tasks: hit k owns tasks hoff[k] .. hoff[k+1]-1 (one per light)
+        // shadow tasks: hit k owns those from hoff[k] on, one per light
         int ex = nl;
 #pragma unroll
         for (int s = 1; s < 32; s <<= 1) {
@@ -478,8 +478,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
             if (lane >= s) ex += u;
         }
         const int ntask = __shfl_sync(0xffffffffu, ex, 31);
-        if (hit_ok) Q.hoff[__popc(hm & lt)] = ex - nl;
-        if (lane == 0) Q.hoff[nh] = ntask;
+        if (hit_ok) Q.hoff[__popc(hm & lt)] = (uint16_t)(ex - nl);
         __syncwarp();
         // the tasks whose light adds nothing are settled without a ray
         // (light_vanishes); the others are listed densely (hit | light << 5)
@@ -552,7 +551,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
             if (bk < V.max_bounces) {
                 float R = 1.0f;
                 if (MAXB > 0 && mat.refractive_index > 0.0f &&
-                    refract_ray(dk, n, Q.hinv[k] != 0, mat.refractive_index, R, td)) {
+                    refract_ray(dk, n, Q.hslot[32 + k] != 0, mat.refractive_index, R, td)) {
                     tc = ck * mat.reflectiveness * (1.0f - R);
                     push_t = true;
                 }
@@ -578,9 +577,9 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
             Q.ro[0][j] = np.x; Q.ro[1][j] = np.y; Q.ro[2][j] = np.z;
             Q.rd[0][j] = dir.x; Q.rd[1][j] = dir.y; Q.rd[2][j] = dir.z;
             Q.rc[j] = contribution;
-            Q.rv[j] = nv;
+            Q.rv[j] = (uint16_t)nv;
             Q.rai[j] = nai;
-            Q.rbounce[j] = nbounce;
+            Q.rbounce[j] = (uint8_t)nbounce;
             if (CARRY) {
                 Q.racc[0][j] = sum.x; Q.racc[1][j] = sum.y; Q.racc[2][j] = sum.z;
             }
@@ -588,7 +587,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
         };
         if (push) put(first + __popc(pm & lt), nd, nc);
         if (MAXB > 0 && push_t) put(first + __popc(pm) + __popc(pt & lt), td, tc);
-        if (lane == 0) Q.pool_n = min(BPOOL, first + __popc(pm) + __popc(pt));
+        pn = min(BPOOL, first + __popc(pm) + __popc(pt));
         __syncwarp();
     }
     if (A.stats) {

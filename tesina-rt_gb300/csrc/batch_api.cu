@@ -350,6 +350,8 @@ int32_t rt_batch_set(rt_ctx* c, rt_batch* b, const rt_batch_view* views, int32_t
     int rbps = 0;
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&rbps, fn, threads, 0));
     b->render_grid = std::max(1, rbps) * c->num_sms;
+    int hint = -1;
+    rt::set_carveout(c, fn, std::max(1, rbps), &hint);
     b->render_chunk = 32;
     return RT_OK;
 }

@@ -261,6 +261,29 @@ void scene_use_pool(rt_scene* s, cudaMemPool_t pool, cudaStream_t stream) {
     s->pool_stream = stream;
 }
 
+void set_carveout(const rt_ctx* c, const void* fn, int blocks_per_sm, int* current) {
+    cudaFuncAttributes fa;
+    if (c->smem_per_sm > 0 && cudaFuncGetAttributes(&fa, fn) == cudaSuccess) {
+        // the SM's shared-memory sizes; a block takes 1 KB for the system and
+        // whole units of 128 bytes
+        static const int kSizesKB[] = {0, 8, 16, 32, 64, 100, 132, 164, 196, 228};
+        const int64_t block = ((int64_t)fa.sharedSizeBytes + 1024 + 127) / 128 * 128;
+        const int64_t need = blocks_per_sm * block;
+        int pct = 100;
+        for (const int kb : kSizesKB)
+            if (need <= (int64_t)kb * 1024 && (int64_t)kb * 1024 <= c->smem_per_sm) {
+                // rounded down: the hint is met by the next size at or above it
+                pct = (int)((int64_t)kb * 1024 * 100 / c->smem_per_sm);
+                break;
+            }
+        if (pct != *current &&
+            cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, pct) ==
+                cudaSuccess)
+            *current = pct;
+    }
+    cudaGetLastError();
+}
+
 uint32_t* work_counter(rt_ctx* c, cudaStream_t s) {
     if (!s || s == c->stream) return c->d_work;
     std::lock_guard<std::mutex> lk(c->work_mu);
@@ -1023,22 +1046,8 @@ static cudaError_t launch_render_cfg(rt_ctx* c, rt::RenderArgs a, const rt_rende
     rt::render_variant_info(cfg.variant, &threads, &minb, &fn);
     int bps = cfg.blocks_per_sm > 0 ? cfg.blocks_per_sm : c->variant_occupancy[cfg.variant];
     if (bps > c->variant_occupancy[cfg.variant]) bps = c->variant_occupancy[cfg.variant];
-    // Shared memory for just the launched blocks per SM: the rest of the
-    // SM's 256 KB of L1 / shared memory caches nodes, triangles and the
-    // traversal stacks.  Process-wide per kernel: set when it changes.
-    if (c->smem_per_sm > 0) {
-        cudaFuncAttributes fa;
-        if (cudaFuncGetAttributes(&fa, fn) == cudaSuccess) {
-            const int64_t need = (int64_t)bps * ((int64_t)fa.sharedSizeBytes + 1024);
-            int pct = (int)((need * 100 + c->smem_per_sm - 1) / c->smem_per_sm);
-            if (pct > 100) pct = 100;
-            if (pct != c->variant_carveout[cfg.variant] &&
-                cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, pct) ==
-                    cudaSuccess)
-                c->variant_carveout[cfg.variant] = pct;
-        }
-        cudaGetLastError();
-    }
+    // process-wide per kernel: set when it changes
+    rt::set_carveout(c, fn, bps, &c->variant_carveout[cfg.variant]);
     const int64_t pixels = (int64_t)a.width * a.height;
     const int64_t warps_needed = (pixels + cfg.chunk - 1) / cfg.chunk;
     int64_t grid = (int64_t)c->num_sms * bps;

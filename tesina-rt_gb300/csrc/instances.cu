@@ -263,14 +263,14 @@ namespace {
 template <int IPOOL, bool CARRY>
 struct InstPool {
     float ro[3][IPOOL], rd[3][IPOOL], rc[IPOOL];
-    int rpix[IPOOL], rbounce[IPOOL];
+    int rpix[IPOOL];
+    uint8_t rbounce[IPOOL];
     uint32_t racc[3][CARRY ? IPOOL : 1];
     float hn[3][32];
     int hid[32], hroot[32];
     unsigned hmask[32];
     uint8_t hslot[32], hinv[32];
     uint8_t task[32 * RT_MAX_LIGHTS];   // shadow tasks that need a ray
-    int pool_n;
 };
 }  // namespace
 
@@ -300,14 +300,13 @@ __global__ void __launch_bounds__(128, MAXB == 6 ? 5 : RT_INST_MINB) k_render_in
     if (threadIdx.x == 0) sA = A;
     const int lane = threadIdx.x & 31;
     InstPool<IPOOL, CARRY>& Q = sQ[threadIdx.x >> 5];
-    if (lane == 0) Q.pool_n = 0;
     __syncthreads();
     const int pixels = sA.width * sA.height;
     const unsigned lt = (1u << lane) - 1u;
     uint64_t n_sec = 0, n_shadow = 0, n_hits = 0, n_prim = 0;
     bool tiles = true;
+    int pn = 0;   // rays waiting in the pool
     for (;;) {
-        const int pn = Q.pool_n;
         bool have = false;
         f3 o = mk3(0.f, 0.f, 0.f), d = o;
         float tmin = 0.0f, tmax = 1e36f;
@@ -449,7 +448,7 @@ __global__ void __launch_bounds__(128, MAXB == 6 ? 5 : RT_INST_MINB) k_render_in
             Q.rd[0][j] = dir.x; Q.rd[1][j] = dir.y; Q.rd[2][j] = dir.z;
             Q.rc[j] = contribution;
             Q.rpix[j] = npix;
-            Q.rbounce[j] = nbounce;
+            Q.rbounce[j] = (uint8_t)nbounce;
             if (CARRY) {
                 Q.racc[0][j] = sum.x; Q.racc[1][j] = sum.y; Q.racc[2][j] = sum.z;
             }
@@ -457,7 +456,7 @@ __global__ void __launch_bounds__(128, MAXB == 6 ? 5 : RT_INST_MINB) k_render_in
         };
         if (push) put(first + __popc(pm & lt), nd, nc);
         if (MAXB > 0 && push_t) put(first + __popc(pm) + __popc(pt & lt), td, tc);
-        if (lane == 0) Q.pool_n = min(IPOOL, first + __popc(pm) + __popc(pt));
+        pn = min(IPOOL, first + __popc(pm) + __popc(pt));
         __syncwarp();
     }
     if (sA.stats) {
@@ -628,6 +627,8 @@ int32_t rt_instances_render(rt_ctx* c, rt_instances* I, const rt_camera* cam, in
         int b = 0;
         CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern, 128, 0));
         occ = b > 0 ? b : 1;
+        int hint = -1;
+        rt::set_carveout(c, (const void*)kern, occ, &hint);
     }
     int64_t grid = (int64_t)c->num_sms * occ;
     const int64_t useful = ((int64_t)px + 127) / 128;   // one 32-pixel tile per warp

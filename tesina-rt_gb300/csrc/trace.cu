@@ -86,21 +86,21 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render(RenderArgs a) {
 namespace {
 constexpr int POOL = 64;   // rays a warp can hold: < 32 left + 32 of the current step
 
-// The rays of a warp.  The ones left wait in places 0 .. pool_n - 1; those of
+// The rays of a warp.  The ones left wait in the first places; those of
 // the current step keep or take the places above, where a hit puts its point
 // over its ray's origin, until the step's own reflection rays are written over
 // them.  The L1 shares the SM's memory with this: a further 1.1 KB per warp (the
 // hits in arrays of their own) cost 1-3 % of a frame.
 struct WarpPool {
     float ro[3][POOL], rd[3][POOL], rc[POOL];   // origin or hit point, direction, contribution
-    int rpix[POOL], rbounce[POOL];
+    int rpix[POOL];
+    uint8_t rbounce[POOL];                      // at most 64
     uint32_t racc[3][POOL];                     // the pixel's sum so far
     float hn[3][32];                            // hits of the current step
     int hid[32];
     unsigned hmask[32];
     uint8_t hslot[32];                          // their places
     uint8_t task[32 * RT_MAX_LIGHTS];           // shadow tasks that need a ray
-    int pool_n;
 };
 }  // namespace
 
@@ -126,15 +126,14 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_pool(RenderArgs a) {
         reinterpret_cast<uint32_t*>(&sL)[i] = reinterpret_cast<const uint32_t*>(&a.lights)[i];
     const int lane = threadIdx.x & 31;
     WarpPool& Q = sQ[threadIdx.x >> 5];
-    if (lane == 0) Q.pool_n = 0;
     __syncthreads();
     const BvhHeader& H = sH;
     const int pixels = a.width * a.height;
     const unsigned lt = (1u << lane) - 1u;
     uint64_t n_sec = 0, n_shadow = 0, n_hits = 0, n_prim = 0;
     bool tiles = true;
+    int pn = 0;   // rays waiting in the pool
     for (;;) {
-        const int pn = Q.pool_n;
         // 1. rays to trace: a full batch from the pool, else a new tile
         //    of primary rays, else what is left in the pool
         bool have = false;
@@ -268,10 +267,10 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_pool(RenderArgs a) {
             Q.rd[0][j] = nd.x; Q.rd[1][j] = nd.y; Q.rd[2][j] = nd.z;
             Q.rc[j] = nc;
             Q.rpix[j] = npix;
-            Q.rbounce[j] = nbounce;
+            Q.rbounce[j] = (uint8_t)nbounce;
             Q.racc[0][j] = sum.x; Q.racc[1][j] = sum.y; Q.racc[2][j] = sum.z;
         }
-        if (lane == 0) Q.pool_n = first + __popc(pm);
+        pn = first + __popc(pm);
         __syncwarp();
     }
     if (a.stats) {
@@ -302,13 +301,13 @@ namespace {
 template <int RPOOL>
 struct RefrPool {   // as WarpPool
     float ro[3][RPOOL], rd[3][RPOOL], rc[RPOOL];
-    int rpix[RPOOL], rbounce[RPOOL];
+    int rpix[RPOOL];
+    uint8_t rbounce[RPOOL];
     float hn[3][32];
     int hid[32];
     unsigned hmask[32];
     uint8_t hslot[32], hinv[32];
     uint8_t task[32 * RT_MAX_LIGHTS];   // shadow tasks that need a ray
-    int pool_n;
 };
 }  // namespace
 
@@ -325,15 +324,14 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_pool_refr(RenderArgs a
         reinterpret_cast<uint32_t*>(&sL)[i] = reinterpret_cast<const uint32_t*>(&a.lights)[i];
     const int lane = threadIdx.x & 31;
     RefrPool<RPOOL>& Q = sQ[threadIdx.x >> 5];
-    if (lane == 0) Q.pool_n = 0;
     __syncthreads();
     const BvhHeader& H = sH;
     const int pixels = a.width * a.height;
     const unsigned lt = (1u << lane) - 1u;
     uint64_t n_sec = 0, n_shadow = 0, n_hits = 0, n_prim = 0;
     bool tiles = true;
+    int pn = 0;   // rays waiting in the pool
     for (;;) {
-        const int pn = Q.pool_n;
         bool have = false;
         f3 o = mk3(0.f, 0.f, 0.f), d = o;
         float tmin = 0.0f, tmax = 1e36f;
@@ -464,12 +462,12 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_pool_refr(RenderArgs a
             Q.rd[0][j] = dir.x; Q.rd[1][j] = dir.y; Q.rd[2][j] = dir.z;
             Q.rc[j] = contribution;
             Q.rpix[j] = npix;
-            Q.rbounce[j] = nbounce;
+            Q.rbounce[j] = (uint8_t)nbounce;
             ++n_sec;
         };
         if (push) put(first + __popc(pm & lt), nd, nc);
         if (push_t) put(first + __popc(pm) + __popc(pt & lt), td, tc);
-        if (lane == 0) Q.pool_n = min(RPOOL, first + __popc(pm) + __popc(pt));
+        pn = min(RPOOL, first + __popc(pm) + __popc(pt));
         __syncwarp();
     }
     if (a.stats) {
