@@ -194,21 +194,21 @@ __device__ __forceinline__ TriRec load_tri(const float4* __restrict__ tris, int3
     return TriRec{__ldg(q), __ldg(q + 1), __ldg(q + 2)};
 }
 
-// Möller–Trumbore of leaf_hit (trace-bvh.cl:275-328).
+// Möller–Trumbore of leaf_hit (trace-bvh.cl:275-328).  Its rejections come
+// together at the end: the values computed past a rejection are not used, and
+// the few extra operations cost less than four branches that a warp rarely
+// takes together.
 __device__ __forceinline__ bool mt(const TriRec& T, f3 o, f3 d, float& t, float& u, float& v) {
     f3 v0 = ld3(T.v0), e1 = ld3(T.e1), e2 = ld3(T.e2);
     f3 h = cross(d, e2);
     float aa = dot(e1, h);
-    if (aa > -1e-26f && aa < 1e-26f) return false;
     float f = 1.0f / aa;
     f3 s = sub(o, v0);
     u = f * dot(s, h);
-    if (u < 0.0f || u > 1.0f) return false;
     f3 q = cross(s, e1);
     v = f * dot(d, q);
-    if (v < 0.0f || u + v > 1.0f) return false;
     t = f * dot(e2, q);
-    return true;
+    return !(aa > -1e-26f && aa < 1e-26f) & !(u < 0.0f) & !(u > 1.0f) & !(v < 0.0f) & !(u + v > 1.0f);
 }
 
 }  // namespace rt
