@@ -1049,6 +1049,18 @@ static cudaError_t launch_render_cfg(rt_ctx* c, rt::RenderArgs a, const rt_rende
     // process-wide per kernel: set when it changes
     rt::set_carveout(c, fn, bps, &c->variant_carveout[cfg.variant]);
     const int64_t pixels = (int64_t)a.width * a.height;
+    // Left to us: fewer warps for a small frame.  Its tiles are gone before
+    // warps at full residency have pooled enough rays to run dense, so up to
+    // about 160 tiles (of 32 pixels) per SM fewer warps with more tiles each are
+    // faster: with 8 and 5 blocks of 128 threads, 800 x 600 of 10k triangles
+    // (99 tiles per SM) 265 and 249 us, 384 x 384 (30) 226 and 216, 1920 x 1080
+    // (426) 405 and 427.  Refracting scenes branch and fill the pools sooner:
+    // fewer warps lose there (800 x 600: 3.53 -> 3.65 ms).
+    if (cfg.blocks_per_sm == 0 && rt::render_variant_pooled(cfg.variant) &&
+        !rt::render_variant_refracts(cfg.variant)) {
+        const int64_t tiles = pixels / 32 / c->num_sms, warps = 12 + tiles / 8;
+        bps = (int)std::min<int64_t>(bps, std::max<int64_t>(1, warps / (threads / 32)));
+    }
     const int64_t warps_needed = (pixels + cfg.chunk - 1) / cfg.chunk;
     int64_t grid = (int64_t)c->num_sms * bps;
     const int64_t max_useful = (warps_needed + threads / 32 - 1) / (threads / 32);
