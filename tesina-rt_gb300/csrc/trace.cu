@@ -487,37 +487,72 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_pool_refr(RenderArgs a
 // ---------------------------------------------------------------------------
 // stage-wise kernels on reference-layout buffers
 // ---------------------------------------------------------------------------
-__global__ void k_gen_primary(rt_camera cam, int w, int h, int q, const rt_pixel_sample* ps,
-                              size_t count, size_t offset, rt_sample* out) {
+// The stages' samples (80 B) and hits (64 B) are arrays of records that a lane
+// handles one of.  Read or written word by word, each access of a warp falls
+// into 32 sectors; the records of a warp go through shared memory instead, in
+// accesses of 32 neighbouring words.  Words, because the callers' arrays need
+// no more than a word's alignment.  A pitch of 20 words lets eight lanes' 16-byte
+// parts meet each bank once.  k_gen_primary, 1000 x 701: 60 -> 14 us; the whole
+// pipeline of 10k triangles 629 -> 610.
+constexpr int STAGE_PITCH = 20;
+
+// The first `cnt` (at most 32) records at g to the warp's stage.
+template <int WORDS>
+__device__ __forceinline__ void stage_in(float* sm, const void* g, int cnt) {
+    const float* q = static_cast<const float*>(g);
+    const int lane = threadIdx.x & 31;
+    float v[WORDS];
+#pragma unroll
+    for (int k = 0; k < WORDS; ++k)
+        if (32 * k + lane < cnt * WORDS) v[k] = q[32 * k + lane];
+#pragma unroll
+    for (int k = 0; k < WORDS; ++k) {
+        const int w = 32 * k + lane;
+        if (w < cnt * WORDS) sm[w / WORDS * STAGE_PITCH + w % WORDS] = v[k];
+    }
+    __syncwarp();
+}
+
+// The records of the lanes in `mask` from the warp's stage to g.
+template <int WORDS>
+__device__ __forceinline__ void stage_out(const float* sm, void* g, unsigned mask) {
+    float* q = static_cast<float*>(g);
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < WORDS; ++k) {
+        const int w = 32 * k + lane;
+        if (mask >> (w / WORDS) & 1) q[w] = sm[w / WORDS * STAGE_PITCH + w % WORDS];
+    }
+}
+
+__device__ __forceinline__ void put4(float* sm, float x, float y, float z, float w) {
+    *reinterpret_cast<float4*>(sm) = make_float4(x, y, z, w);
+}
+
+__global__ void __launch_bounds__(256) k_gen_primary(rt_camera cam, int w, int h, int q,
+                                                     const rt_pixel_sample* ps, size_t count,
+                                                     size_t offset, rt_sample* out) {
+    __shared__ __align__(16) float stage[256 * STAGE_PITCH];
     const size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (k >= count) return;
-    const int gid = (int)(offset + k);
-    const int pixels = w * h;
-    rt_pixel_sample p = {0.f, 0.f, 1.f};
-    if (ps) p = ps[gid / pixels];
-    int x, y;
-    pixel_of(gid, w, h, q, x, y);
-    const f3 d = primary_dir(cam, x, y, w, h, p.ox, p.oy);
-    rt_sample s;
-    s.ray.ori[0] = cam.pos[0];
-    s.ray.ori[1] = cam.pos[1];
-    s.ray.ori[2] = cam.pos[2];
-    s.ray.ori[3] = 0.f;
-    s.ray.dir[0] = d.x;
-    s.ray.dir[1] = d.y;
-    s.ray.dir[2] = d.z;
-    s.ray.dir[3] = 0.f;
-    s.ray.inv_dir[0] = 1.0f / d.x;
-    s.ray.inv_dir[1] = 1.0f / d.y;
-    s.ray.inv_dir[2] = 1.0f / d.z;
-    s.ray.inv_dir[3] = 0.f;
-    s.ray.tmin = 0.0f;
-    s.ray.tmax = 1e36f;
-    s.ray._pad[0] = s.ray._pad[1] = 0.f;
-    s.pixel = w * y + x;
-    s.contribution = p.contribution;
-    s._pad[0] = s._pad[1] = 0;
-    out[k] = s;
+    const unsigned mask = __ballot_sync(0xffffffffu, k < count);
+    float* sm = stage + threadIdx.x * STAGE_PITCH;
+    if (k < count) {
+        const int gid = (int)(offset + k);
+        const int pixels = w * h;
+        rt_pixel_sample p = {0.f, 0.f, 1.f};
+        if (ps) p = ps[gid / pixels];
+        int x, y;
+        pixel_of(gid, w, h, q, x, y);
+        const f3 d = primary_dir(cam, x, y, w, h, p.ox, p.oy);
+        put4(sm, cam.pos[0], cam.pos[1], cam.pos[2], 0.f);
+        put4(sm + 4, d.x, d.y, d.z, 0.f);
+        put4(sm + 8, 1.0f / d.x, 1.0f / d.y, 1.0f / d.z, 0.f);
+        put4(sm + 12, 0.0f, 1e36f, 0.f, 0.f);
+        put4(sm + 16, __int_as_float(w * y + x), p.contribution, 0.f, 0.f);
+    }
+    const int lane = threadIdx.x & 31;
+    if (mask) stage_out<20>(sm - lane * STAGE_PITCH, out + (k - lane), mask);
 }
 
 __device__ __forceinline__ f3 f3_of(const float* v) { return mk3(v[0], v[1], v[2]); }
@@ -526,65 +561,74 @@ __global__ void __launch_bounds__(128) k_trace(SceneView S, const rt_sample* __r
                                                int n, rt_hit* __restrict__ hits,
                                                uint32_t* status) {
     __shared__ BvhHeader sH;
+    __shared__ __align__(16) float stage[128 * STAGE_PITCH];
     if (threadIdx.x == 0) sH = *S.hdr;
     __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const rt_ray& ray = smp[i].ray;
-    const f3 o = f3_of(ray.ori), d = f3_of(ray.dir);
-    const TRay r = make_tray(o, d, f3_of(ray.inv_dir), ray.tmin);
-    const Hit h = closest_hit<true, true>(S, sH, r, ray.tmax, status);
-    if (h.id < 0) {
-        hits[i].hit = 0;
-        return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31, base = i - lane;
+    if (base >= n) return;
+    float* sm = stage + threadIdx.x * STAGE_PITCH;
+    float* warp = sm - lane * STAGE_PITCH;
+    stage_in<20>(warp, smp + base, min(32, n - base));
+    bool hit = false;
+    if (i < n) {
+        const rt_ray& ray = *reinterpret_cast<const rt_ray*>(sm);
+        const f3 o = f3_of(ray.ori), d = f3_of(ray.dir);
+        const TRay r = make_tray(o, d, f3_of(ray.inv_dir), ray.tmin);
+        const Hit h = closest_hit<true, true>(S, sH, r, ray.tmax, status);
+        hit = h.id >= 0;
+        if (hit) {
+            const HitInfo hi = complete_hit(S, o, d, h);
+            const uint32_t head = 1u | (uint32_t)hits[i].shadow_hit << 8 | (uint32_t)hi.inverse_n << 16;
+            put4(sm, __uint_as_float(head), h.t, __int_as_float(h.id), 0.f);
+            put4(sm + 4, 0.f, 0.f, 0.f, 0.f);
+            put4(sm + 8, hi.n.x, hi.n.y, hi.n.z, 0.f);
+            put4(sm + 12, hi.hp.x, hi.hp.y, hi.hp.z, 0.f);
+        } else {
+            hits[i].hit = 0;
+        }
     }
-    const HitInfo hi = complete_hit(S, o, d, h);
-    rt_hit out;
-    out.hit = 1;
-    out.shadow_hit = hits[i].shadow_hit;
-    out.inverse_n = hi.inverse_n;
-    out.reserved = 0;
-    out.t = h.t;
-    out.id = h.id;
-    out._pad0 = 0.f;
-    out.uv[0] = out.uv[1] = 0.f;
-    out._pad1[0] = out._pad1[1] = 0.f;
-    out.n[0] = hi.n.x;
-    out.n[1] = hi.n.y;
-    out.n[2] = hi.n.z;
-    out.n[3] = 0.f;
-    out.hit_point[0] = hi.hp.x;
-    out.hit_point[1] = hi.hp.y;
-    out.hit_point[2] = hi.hp.z;
-    out.hit_point[3] = 0.f;
-    hits[i] = out;
+    stage_out<16>(warp, hits + base, __ballot_sync(0xffffffffu, hit));
 }
 
 __global__ void __launch_bounds__(128) k_shadow(SceneView S, rt_lights Ls, int n,
                                                 rt_hit* __restrict__ hits, uint32_t* status) {
     __shared__ BvhHeader sH;
+    __shared__ __align__(16) float stage[128 * STAGE_PITCH];
     if (threadIdx.x == 0) sH = *S.hdr;
     __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31, base = i - lane;
+    if (base >= n) return;
+    float* sm = stage + threadIdx.x * STAGE_PITCH;
+    stage_in<16>(sm - lane * STAGE_PITCH, hits + base, min(32, n - base));
     if (i >= n) return;
-    if (!hits[i].hit) return;
-    const f3 hp = f3_of(hits[i].hit_point);
+    const rt_hit& h = *reinterpret_cast<const rt_hit*>(sm);
+    if (!h.hit) return;
+    const f3 hp = f3_of(h.hit_point);
     uint32_t mask = 0;
     for (int l = 0; l < Ls.count; ++l)
         if (occluded<true, true>(S, sH, Ls.light[l], hp, status)) mask |= 1u << l;
     hits[i].shadow_hit = (uint8_t)mask;
 }
 
-__global__ void k_shade(SceneView S, rt_lights Ls, const rt_sample* __restrict__ smp,
-                        const rt_hit* __restrict__ hits, int n, uint32_t* __restrict__ image) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const rt_hit& h = hits[i];
-    if (!h.hit) return;
+__global__ void __launch_bounds__(128) k_shade(SceneView S, rt_lights Ls,
+                                               const rt_sample* __restrict__ smp,
+                                               const rt_hit* __restrict__ hits, int n,
+                                               uint32_t* __restrict__ image) {
+    __shared__ __align__(16) float stage[2][128 * STAGE_PITCH];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31, base = i - lane;
+    if (base >= n) return;
+    const int at = threadIdx.x * STAGE_PITCH, warp = at - lane * STAGE_PITCH;
+    stage_in<16>(stage[0] + warp, hits + base, min(32, n - base));
+    const rt_hit& h = *reinterpret_cast<const rt_hit*>(stage[0] + at);
+    const bool hit = i < n && h.hit;
+    if (!__any_sync(0xffffffffu, hit)) return;
+    stage_in<20>(stage[1] + warp, smp + base, min(32, n - base));
+    if (!hit) return;
+    const rt_sample& sp = *reinterpret_cast<const rt_sample*>(stage[1] + at);
     const rt_material mat = S.mats[__ldg(&S.map[h.id])];
-    const uint3 c = shade_hit(Ls, mat, f3_of(h.hit_point), f3_of(h.n), f3_of(smp[i].ray.dir),
-                              smp[i].contribution, h.shadow_hit);
-    uint32_t* px = image + 3 * (size_t)smp[i].pixel;
+    const uint3 c = shade_hit(Ls, mat, f3_of(h.hit_point), f3_of(h.n), f3_of(sp.ray.dir),
+                              sp.contribution, h.shadow_hit);
+    uint32_t* px = image + 3 * (size_t)sp.pixel;
     atomicAdd(px, c.x);
     atomicAdd(px + 1, c.y);
     atomicAdd(px + 2, c.z);
@@ -627,28 +671,39 @@ __global__ void k_sec_count(SceneView S, const rt_sample* __restrict__ in,
     }
 }
 
-__global__ void k_sec_scan(uint32_t* __restrict__ block_counts, int nblocks, int max_out,
-                           int32_t* __restrict__ d_count) {
-    // single block, sequential chunks of 1024
-    __shared__ uint32_t s[1024];
-    __shared__ uint32_t carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int b0 = 0; b0 < nblocks; b0 += 1024) {
-        const int i = b0 + threadIdx.x;
-        const uint32_t v = i < nblocks ? block_counts[i] : 0;
-        s[threadIdx.x] = v;
-        __syncthreads();
-        for (int off = 1; off < 1024; off <<= 1) {
-            const uint32_t t = threadIdx.x >= (unsigned)off ? s[threadIdx.x - off] : 0;
-            __syncthreads();
-            s[threadIdx.x] += t;
-            __syncthreads();
+// Exclusive scan by one block, 4096 counts a turn (5,478 counts: 11 -> 5 us
+// against a scan in shared memory with two barriers per doubling).
+__global__ void __launch_bounds__(1024) k_sec_scan(uint32_t* __restrict__ block_counts, int nblocks,
+                                                   int max_out, int32_t* __restrict__ d_count) {
+    __shared__ uint32_t tot[2][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t carry = 0;
+    for (int b0 = 0, turn = 0; b0 < nblocks; b0 += 4096, turn ^= 1) {
+        const int i = b0 + 4 * threadIdx.x;
+        uint32_t v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = i + k < nblocks ? block_counts[i + k] : 0;
+        const uint32_t own = v[0] + v[1] + v[2] + v[3];
+        auto scan = [&](uint32_t x) {   // inclusive, over the warp
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const uint32_t t = __shfl_up_sync(0xffffffffu, x, off);
+                if (lane >= off) x += t;
+            }
+            return x;
+        };
+        const uint32_t in_warp = scan(own);
+        if (lane == 31) tot[turn][w] = in_warp;
+        __syncthreads();   // one barrier a turn: the next turn writes the other totals
+        const uint32_t warps = scan(tot[turn][lane]);
+        const uint32_t before = __shfl_sync(0xffffffffu, warps, (w + 31) & 31);
+        uint32_t at = carry + (w ? before : 0) + in_warp - own;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (i + k < nblocks) block_counts[i + k] = at;
+            at += v[k];
         }
-        if (i < nblocks) block_counts[i] = carry + s[threadIdx.x] - v;
-        __syncthreads();
-        if (threadIdx.x == 0) carry += s[1023];
-        __syncthreads();
+        carry += __shfl_sync(0xffffffffu, warps, 31);
     }
     if (threadIdx.x == 0) *d_count = (int32_t)min(carry, (uint32_t)max_out);
 }
