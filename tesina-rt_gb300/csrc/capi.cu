@@ -227,7 +227,7 @@ int32_t scene_ensure_build(rt_scene* s) {
     free_build(s);
     const size_t nn = n > 1 ? n - 1 : 1;
     if (salloc_n(s, &s->d_keys_unsorted, n) || salloc_n(s, &s->d_keys_sorted, n) ||
-        salloc_n(s, &s->d_vals_sorted, n) || salloc_n(s, &s->d_tris, 3 * ((size_t)n + 1)) ||
+        salloc_n(s, &s->d_vals_sorted, n) || salloc_n(s, &s->d_tris, 3 * ((size_t)n + 3)) ||
         salloc_n(s, &s->d_nodes, 8 * nn) || salloc_n(s, &s->d_hdr, 1) || salloc(s, &s->d_scratch, need_scratch)) {
         cudaGetLastError();
         free_build(s);
@@ -972,7 +972,7 @@ int32_t rt_trace(rt_ctx* c, rt_scene* s, const rt_sample* smp, int32_t n, rt_hit
     if (r) return r;
     cudaStream_t cs = st(c, stream);
     CU(scene_read_begin(s, cs));
-    CU(rt::launch_trace(view_of(s), smp, n, hits, c->d_status, cs));
+    CU(rt::launch_trace(view_of(s), smp, n, hits, c->d_status, c->num_sms, cs));
     CU(scene_read_end(s, cs));
     return RT_OK;
 }
@@ -986,7 +986,7 @@ int32_t rt_shadow_trace(rt_ctx* c, rt_scene* s, const rt_sample* smp, int32_t n,
     if (r) return r;
     cudaStream_t cs = st(c, stream);
     CU(scene_read_begin(s, cs));
-    CU(rt::launch_shadow(view_of(s), s->lights, n, hits, c->d_status, cs));
+    CU(rt::launch_shadow(view_of(s), s->lights, n, hits, c->d_status, c->num_sms, cs));
     CU(scene_read_end(s, cs));
     return RT_OK;
 }

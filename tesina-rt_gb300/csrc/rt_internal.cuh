@@ -55,7 +55,7 @@ __host__ __device__ __forceinline__ int32_t slot_pair_node(const Slot& a) {
 // Triangle records in sorted order, 48 B: v0, e1 = v1 - v0, e2 = v2 - v0
 // (the same float subtractions as leaf_hit, trace-bvh.cl:297-298).  v0.w is
 // 1 where the next triangle belongs to the same leaf, else 0: a leaf is found
-// from its first triangle alone.  One record past the last is allocated.
+// from its first triangle alone.  Three records past the last are allocated.
 struct TriRec {
     float4 v0, e1, e2;
 };

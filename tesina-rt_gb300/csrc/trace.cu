@@ -5,7 +5,7 @@
 
 #include "rt_internal.cuh"
 #include "trace.cuh"
-#include "trace_dev.cuh"
+#include "trace_quad.cuh"
 
 namespace rt {
 
@@ -497,32 +497,34 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_pool_refr(RenderArgs a
 constexpr int STAGE_PITCH = 20;
 
 // The first `cnt` (at most 32) records at g to the warp's stage.
-template <int WORDS>
+template <int WORDS, int RECORDS = 32>
 __device__ __forceinline__ void stage_in(float* sm, const void* g, int cnt) {
     const float* q = static_cast<const float*>(g);
     const int lane = threadIdx.x & 31;
-    float v[WORDS];
+    constexpr int TURNS = WORDS * RECORDS / 32;
+    float v[TURNS];
 #pragma unroll
-    for (int k = 0; k < WORDS; ++k)
+    for (int k = 0; k < TURNS; ++k)
         if (32 * k + lane < cnt * WORDS) v[k] = q[32 * k + lane];
 #pragma unroll
-    for (int k = 0; k < WORDS; ++k) {
+    for (int k = 0; k < TURNS; ++k) {
         const int w = 32 * k + lane;
         if (w < cnt * WORDS) sm[w / WORDS * STAGE_PITCH + w % WORDS] = v[k];
     }
     __syncwarp();
 }
 
-// The records of the lanes in `mask` from the warp's stage to g.
-template <int WORDS>
+// The records in `mask` (a bit for each, 32 / RECORDS bits apart) from the
+// warp's stage to g.
+template <int WORDS, int RECORDS = 32>
 __device__ __forceinline__ void stage_out(const float* sm, void* g, unsigned mask) {
     float* q = static_cast<float*>(g);
     const int lane = threadIdx.x & 31;
     __syncwarp();
 #pragma unroll
-    for (int k = 0; k < WORDS; ++k) {
+    for (int k = 0; k < WORDS * RECORDS / 32; ++k) {
         const int w = 32 * k + lane;
-        if (mask >> (w / WORDS) & 1) q[w] = sm[w / WORDS * STAGE_PITCH + w % WORDS];
+        if (mask >> (w / WORDS * (32 / RECORDS)) & 1) q[w] = sm[w / WORDS * STAGE_PITCH + w % WORDS];
     }
 }
 
@@ -557,25 +559,38 @@ __global__ void __launch_bounds__(256) k_gen_primary(rt_camera cam, int w, int h
 
 __device__ __forceinline__ f3 f3_of(const float* v) { return mk3(v[0], v[1], v[2]); }
 
+// A warp takes `per` rays: 32, or with QUAD up to eight, by four lanes each
+// (trace_quad.cuh).
+template <bool QUAD>
 __global__ void __launch_bounds__(128) k_trace(SceneView S, const rt_sample* __restrict__ smp,
                                                int n, rt_hit* __restrict__ hits,
-                                               uint32_t* status) {
+                                               uint32_t* status, int per) {
+    constexpr int RAYS = QUAD ? 8 : 32;   // places of a warp
     __shared__ BvhHeader sH;
-    __shared__ __align__(16) float stage[128 * STAGE_PITCH];
+    __shared__ __align__(16) float stage[4 * RAYS * STAGE_PITCH];
+    __shared__ QuadStack stacks[QUAD ? 4 * RAYS : 1];
     if (threadIdx.x == 0) sH = *S.hdr;
     __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31, base = i - lane;
+    const int lane = threadIdx.x & 31, ray_of = threadIdx.x / (32 / RAYS);   // in the block
+    const int base = blockIdx.x * 4 * per + threadIdx.x / 32 * per, i = base + ray_of % RAYS;
     if (base >= n) return;
-    float* sm = stage + threadIdx.x * STAGE_PITCH;
-    float* warp = sm - lane * STAGE_PITCH;
-    stage_in<20>(warp, smp + base, min(32, n - base));
+    n = min(n, base + per);
+    float* sm = stage + ray_of * STAGE_PITCH;
+    float* warp = sm - ray_of % RAYS * STAGE_PITCH;
+    stage_in<20, RAYS>(warp, smp + base, min(RAYS, n - base));
+    const rt_ray& ray = *reinterpret_cast<const rt_ray*>(sm);
+    const f3 o = f3_of(ray.ori), d = f3_of(ray.dir);
     bool hit = false;
-    if (i < n) {
-        const rt_ray& ray = *reinterpret_cast<const rt_ray*>(sm);
-        const f3 o = f3_of(ray.ori), d = f3_of(ray.dir);
+    if (QUAD || i < n) {
         const TRay r = make_tray(o, d, f3_of(ray.inv_dir), ray.tmin);
-        const Hit h = closest_hit<true, true>(S, sH, r, ray.tmax, status);
-        hit = h.id >= 0;
+        const float tmax = ray.tmax;
+        Hit h;
+        if (QUAD)
+            h = closest_hit_quad(S, sH, r, tmax, i < n, stacks[QUAD ? ray_of : 0].e, status);
+        else
+            h = closest_hit<true, true>(S, sH, r, tmax, status);
+        const bool mine = i < n && (!QUAD || lane % 4 == 0);   // one lane writes
+        hit = mine && h.id >= 0;
         if (hit) {
             const HitInfo hi = complete_hit(S, o, d, h);
             const uint32_t head = 1u | (uint32_t)hits[i].shadow_hit << 8 | (uint32_t)hi.inverse_n << 16;
@@ -583,28 +598,45 @@ __global__ void __launch_bounds__(128) k_trace(SceneView S, const rt_sample* __r
             put4(sm + 4, 0.f, 0.f, 0.f, 0.f);
             put4(sm + 8, hi.n.x, hi.n.y, hi.n.z, 0.f);
             put4(sm + 12, hi.hp.x, hi.hp.y, hi.hp.z, 0.f);
-        } else {
+        } else if (mine) {
             hits[i].hit = 0;
         }
     }
-    stage_out<16>(warp, hits + base, __ballot_sync(0xffffffffu, hit));
+    stage_out<16, RAYS>(warp, hits + base, __ballot_sync(0xffffffffu, hit));
 }
 
+template <bool QUAD>
 __global__ void __launch_bounds__(128) k_shadow(SceneView S, rt_lights Ls, int n,
-                                                rt_hit* __restrict__ hits, uint32_t* status) {
+                                                rt_hit* __restrict__ hits, uint32_t* status, int per) {
+    constexpr int RAYS = QUAD ? 8 : 32;   // places of a warp
     __shared__ BvhHeader sH;
-    __shared__ __align__(16) float stage[128 * STAGE_PITCH];
+    __shared__ __align__(16) float stage[4 * RAYS * STAGE_PITCH];
+    __shared__ QuadStack stacks[QUAD ? 4 * RAYS : 1];
     if (threadIdx.x == 0) sH = *S.hdr;
     __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31, base = i - lane;
+    const int lane = threadIdx.x & 31, ray_of = threadIdx.x / (32 / RAYS);   // in the block
+    const int base = blockIdx.x * 4 * per + threadIdx.x / 32 * per, i = base + ray_of % RAYS;
     if (base >= n) return;
-    float* sm = stage + threadIdx.x * STAGE_PITCH;
-    stage_in<16>(sm - lane * STAGE_PITCH, hits + base, min(32, n - base));
-    if (i >= n) return;
+    n = min(n, base + per);
+    const float* sm = stage + ray_of * STAGE_PITCH;
+    stage_in<16, RAYS>(stage + (ray_of - ray_of % RAYS) * STAGE_PITCH, hits + base, min(RAYS, n - base));
     const rt_hit& h = *reinterpret_cast<const rt_hit*>(sm);
-    if (!h.hit) return;
+    const bool hit = i < n && h.hit;
     const f3 hp = f3_of(h.hit_point);
     uint32_t mask = 0;
+    if (QUAD) {
+        for (int l = 0; l < Ls.count; ++l) {
+            f3 dir = mk3(0.f, 0.f, 0.f);
+            const bool live = hit && shadow_dir(Ls.light[l], hp, dir);
+            const f3 inv = mk3(1.0f / dir.x, 1.0f / dir.y, 1.0f / dir.z);
+            const TRay r = make_tray(hp, dir, inv, 0.01f);
+            if (any_hit_quad(S, sH, r, 1e37f, live, stacks[QUAD ? ray_of : 0].e, status) || !live)
+                mask |= 1u << l;
+        }
+        if (hit && lane % 4 == 0) hits[i].shadow_hit = (uint8_t)mask;
+        return;
+    }
+    if (!hit) return;
     for (int l = 0; l < Ls.count; ++l)
         if (occluded<true, true>(S, sH, Ls.light[l], hp, status)) mask |= 1u << l;
     hits[i].shadow_hit = (uint8_t)mask;
@@ -867,17 +899,35 @@ cudaError_t launch_gen_primary(const rt_camera& cam, int w, int h, int q, const 
     return cudaGetLastError();
 }
 
+// Launches with few rays take four lanes per ray (trace_quad.cuh).  Up to 768
+// rays per SM (primary rays of 10k / 200k triangles, trace and shadow: 65k rays
+// 140 -> 117 / 185 -> 153 us, 131k 150 -> 141 / 216 -> 192, 262k 181 -> 187 /
+// 262 -> 269); and of these, fewer than eight to a warp as long as that leaves
+// no more than 16 warps per SM (2k to 20k rays, whole pipeline 532 -> 520 us).
+static int quad_rays_per_warp(int n, int sms) {
+    if (n > 768 * sms) return 0;
+    int per = 8;
+    while (per > 1 && n <= 16 * sms * (per / 2)) per /= 2;
+    return per;
+}
+
 cudaError_t launch_trace(const SceneView& S, const rt_sample* smp, int n, rt_hit* hits,
-                         uint32_t* status, cudaStream_t s) {
+                         uint32_t* status, int sms, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    k_trace<<<blocks(n, 128), 128, 0, s>>>(S, smp, n, hits, status);
+    if (const int per = quad_rays_per_warp(n, sms))
+        k_trace<true><<<blocks(n, 4 * per), 128, 0, s>>>(S, smp, n, hits, status, per);
+    else
+        k_trace<false><<<blocks(n, 128), 128, 0, s>>>(S, smp, n, hits, status, 32);
     return cudaGetLastError();
 }
 
 cudaError_t launch_shadow(const SceneView& S, const rt_lights& L, int n, rt_hit* hits,
-                          uint32_t* status, cudaStream_t s) {
+                          uint32_t* status, int sms, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    k_shadow<<<blocks(n, 128), 128, 0, s>>>(S, L, n, hits, status);
+    if (const int per = quad_rays_per_warp(n, sms))
+        k_shadow<true><<<blocks(n, 4 * per), 128, 0, s>>>(S, L, n, hits, status, per);
+    else
+        k_shadow<false><<<blocks(n, 128), 128, 0, s>>>(S, L, n, hits, status, 32);
     return cudaGetLastError();
 }
 

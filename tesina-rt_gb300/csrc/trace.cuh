@@ -45,9 +45,9 @@ cudaError_t launch_render(const RenderArgs& a, int variant, int grid, cudaStream
 cudaError_t launch_gen_primary(const rt_camera& cam, int w, int h, int q, const rt_pixel_sample* ps,
                                size_t count, size_t offset, rt_sample* out, cudaStream_t s);
 cudaError_t launch_trace(const SceneView& S, const rt_sample* smp, int n, rt_hit* hits,
-                         uint32_t* status, cudaStream_t s);
+                         uint32_t* status, int sms, cudaStream_t s);
 cudaError_t launch_shadow(const SceneView& S, const rt_lights& L, int n, rt_hit* hits,
-                          uint32_t* status, cudaStream_t s);
+                          uint32_t* status, int sms, cudaStream_t s);
 cudaError_t launch_shade(const SceneView& S, const rt_lights& L, const rt_sample* smp,
                          const rt_hit* hits, int n, uint32_t* image, cudaStream_t s);
 cudaError_t launch_gen_secondary(const SceneView& S, const rt_sample* in, int n, const rt_hit* hits,

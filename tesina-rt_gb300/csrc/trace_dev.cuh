@@ -419,22 +419,28 @@ __device__ __forceinline__ HitInfo complete_hit(const SceneView& S, f3 o, f3 d, 
     return hi;
 }
 
-// Shadow ray of shadow_trace_single for one light (shadow-trace-bvh.cl:
-// 375-418); point lights as spot lights without a cone.
-template <bool STAY = false, bool PAIR = false>
-__device__ __forceinline__ bool occluded(const SceneView& S, const BvhHeader& H, const rt_light& L,
-                                         f3 hp, uint32_t* status) {
-    f3 dir;
+// Direction of the shadow ray of shadow_trace_single to a light (shadow-trace-
+// bvh.cl:375-418); point lights as spot lights without a cone.  False: the
+// light does not reach hp, whatever lies in between.
+__device__ __forceinline__ bool shadow_dir(const rt_light& L, f3 hp, f3& dir) {
     if (L.type == RT_DIR_L) {
         dir = neg(mk3(L.dir[0], L.dir[1], L.dir[2]));
     } else if (L.type == RT_SPOT_L) {
         dir = normalize(sub(mk3(L.pos[0], L.pos[1], L.pos[2]), hp));
-        if (dot(neg(dir), mk3(L.dir[0], L.dir[1], L.dir[2])) < L.angle) return true;
+        if (dot(neg(dir), mk3(L.dir[0], L.dir[1], L.dir[2])) < L.angle) return false;
     } else if (L.type == RT_POINT_L) {
         dir = normalize(sub(mk3(L.pos[0], L.pos[1], L.pos[2]), hp));
     } else {
-        return true;
+        return false;
     }
+    return true;
+}
+
+template <bool STAY = false, bool PAIR = false>
+__device__ __forceinline__ bool occluded(const SceneView& S, const BvhHeader& H, const rt_light& L,
+                                         f3 hp, uint32_t* status) {
+    f3 dir;
+    if (!shadow_dir(L, hp, dir)) return true;
     const f3 inv = mk3(1.0f / dir.x, 1.0f / dir.y, 1.0f / dir.z);
     const TRay r = make_tray(hp, dir, inv, 0.01f);
     return any_hit<STAY, PAIR>(S, H, r, 1e37f, status);
