@@ -378,7 +378,9 @@ RT_API int32_t rt_render(rt_ctx* ctx, rt_scene* scene, const rt_camera* cam, int
  * resident blocks launched, and the pixels a warp takes per work fetch. */
 typedef struct rt_render_config {
     int32_t variant;         /* kernel variant, 0 .. rt_render_variants() - 1           */
-    int32_t blocks_per_sm;   /* resident blocks per SM to launch; 0 = occupancy maximum */
+    int32_t blocks_per_sm;   /* resident blocks per SM to launch; 0 = chosen by the frame's
+                              * size, up to the occupancy maximum (with the default variant a
+                              * small frame then takes the kernel with four lanes per pixel) */
     int32_t chunk;           /* pixels per warp work fetch: 32, 64, 128 or 256          */
     int32_t stack_depth;     /* traversal stack entries (fixed: 32, enough for depth <= 31) */
 } rt_render_config;

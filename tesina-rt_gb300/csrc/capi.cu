@@ -1039,16 +1039,31 @@ int32_t rt_fb_copy(rt_ctx* c, const uint32_t* img, uint8_t* rgba, size_t px, rt_
 // ---------------------------------------------------------------------------
 // fused path
 // ---------------------------------------------------------------------------
-static cudaError_t launch_render_cfg(rt_ctx* c, rt::RenderArgs a, const rt_render_config& cfg,
+static cudaError_t launch_render_cfg(rt_ctx* c, rt::RenderArgs a, rt_render_config cfg,
                                      cudaStream_t cs) {
+    const int64_t pixels = (int64_t)a.width * a.height;
+    // The default configuration leaves the kernel open: a frame too small to fill
+    // the SMs goes to the one with four lanes per pixel.  Against the pooled kernel
+    // on 362 x 362 (just above the line): 1k triangles 55 -> 57 us, 10k 217 -> 171,
+    // 200k 286 -> 250, 1.2 M 553 -> 471; on 512 x 512 61 -> 78, 233 -> 253, 355 -> 359,
+    // 701 -> 738.
+    if (cfg.variant == kDefaultVariant && cfg.blocks_per_sm == 0 &&
+        pixels <= (int64_t)rt::kQuadRaysPerSm * c->num_sms)
+        cfg.variant = rt::render_quad_variant();
     int threads = 0, minb = 0;
     const void* fn = nullptr;
     rt::render_variant_info(cfg.variant, &threads, &minb, &fn);
+    if (rt::render_variant_quad(cfg.variant)) {
+        // fewer than eight pixels to a warp as long as that leaves no more than
+        // 32 warps per SM (64 x 64 of 10k triangles: 8 pixels 103 us, 4 with a line
+        // at 16 warps 83, 2 at 32 warps 64)
+        cfg.chunk = 8;
+        while (cfg.chunk > 1 && pixels <= (int64_t)32 * c->num_sms * (cfg.chunk / 2)) cfg.chunk /= 2;
+    }
     int bps = cfg.blocks_per_sm > 0 ? cfg.blocks_per_sm : c->variant_occupancy[cfg.variant];
     if (bps > c->variant_occupancy[cfg.variant]) bps = c->variant_occupancy[cfg.variant];
     // process-wide per kernel: set when it changes
     rt::set_carveout(c, fn, bps, &c->variant_carveout[cfg.variant]);
-    const int64_t pixels = (int64_t)a.width * a.height;
     // Left to us: fewer warps for a small frame.  Its tiles are gone before
     // warps at full residency have pooled enough rays to run dense, so up to
     // about 160 tiles (of 32 pixels) per SM fewer warps with more tiles each are

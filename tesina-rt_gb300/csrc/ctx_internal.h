@@ -10,6 +10,10 @@
 #include "../../include/rt_cuda.h"
 #include "rt_internal.cuh"
 
+// The render variant of the default configuration.  With the residency left
+// open (0 blocks per SM) launch_render_cfg chooses by the size of the frame.
+constexpr int kDefaultVariant = 9;
+
 struct rt_ctx {
     int device = 0;
     int num_sms = 0;
@@ -48,11 +52,10 @@ struct rt_ctx {
     };
     std::map<cudaStream_t, HostRender> host_by_stream;
     float inv1e6 = 1.0f / 1e6f;
-    // until the autotuner or the caller picks one: the pooled kernel with the
-    // most warps (variant 9, k_render_pool<128, 8>; against variant 8, which
-    // holds 7 blocks: 4K of 17.7 M triangles 9.64 -> 9.28 ms, mid-scale frame
-    // 2.51 -> 2.46) at the residency that launch_render_cfg chooses
-    rt_render_config render_cfg = {9, 0, 32, 32};
+    // until the autotuner or the caller picks one (k_render_pool<128, 8>: against
+    // k_render_pool<128, 6>, which holds 7 blocks, 4K of 17.7 M triangles 9.64 ->
+    // 9.28 ms, mid-scale frame 2.51 -> 2.46)
+    rt_render_config render_cfg = {kDefaultVariant, 0, 32, 32};
     int variant_occupancy[rt::kMaxRenderVariants] = {0};   // resident blocks per SM per variant
     int variant_carveout[rt::kMaxRenderVariants];          // shared-memory carveout set (%), -1 unset
     int smem_per_sm = 0;                            // bytes of shared memory an SM offers

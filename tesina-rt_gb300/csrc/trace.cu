@@ -69,6 +69,138 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render(RenderArgs a) {
     }
 }
 
+// The pixel's sum, as it is and as RGBA8.
+__device__ __forceinline__ void write_pixel(const RenderArgs& a, int pix, uint3 sum) {
+    if (a.image_rgb) {
+        uint32_t* q = a.image_rgb + 3 * (size_t)pix;
+        q[0] = sum.x;
+        q[1] = sum.y;
+        q[2] = sum.z;
+    }
+    reinterpret_cast<uchar4*>(a.rgba)[pix] = rgba8_of(sum, a.inv1e6);
+}
+
+// ---------------------------------------------------------------------------
+// k_render_quad: the same rays as k_render, a pixel's path by four lanes
+// (trace_quad.cuh), for frames with too few pixels to fill the SMs: these take as
+// long as the chain of a path's rays.  A warp takes `chunk` (at most eight)
+// neighbouring pixels at a time; its (hit, light) tasks are spread over all
+// eight places, so that lights and places without a path do not lengthen the
+// chain (against one light after the other, 64 x 64 of 1.2 M triangles: 400 ->
+// 114 us).  Render of 64 x 64 / 256 x 256, pooled and this: 1k triangles 48 -> 30 /
+// 55 -> 49 us, 10k 168 -> 64 / 221 -> 152, 200k 211 -> 96 / 275 -> 185, a terrain
+// of 1.2 M 291 -> 114 / 389 -> 300.  Six blocks per SM: with eight, spills, +8 %.
+// ---------------------------------------------------------------------------
+template <int THREADS, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB) k_render_quad(RenderArgs a) {
+    const SceneView S = a.scene;
+    __shared__ BvhHeader sH;
+    __shared__ rt_lights sL;
+    __shared__ QuadStack stacks[THREADS / 4];
+    __shared__ uint8_t tasks[THREADS / 32][8 * RT_MAX_LIGHTS];
+    __shared__ unsigned blocks[THREADS / 32][8];
+    if (threadIdx.x == 0) sH = *S.hdr;
+    for (int i = threadIdx.x; i < (int)(sizeof(rt_lights) / 4); i += blockDim.x)
+        reinterpret_cast<uint32_t*>(&sL)[i] = reinterpret_cast<const uint32_t*>(&a.lights)[i];
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const bool writer = (lane & 3) == 0;   // of the ray's four lanes
+    int2* st = stacks[threadIdx.x / 4].e;
+    uint8_t* list = tasks[threadIdx.x / 32];
+    unsigned* blocked = blocks[threadIdx.x / 32];
+    const int per = a.chunk;   // pixels of a warp
+    const int pixels = a.width * a.height;
+    unsigned n_sec = 0, n_hits = 0, n_prim = 0;
+    for (;;) {
+        int base = 0;
+        if (lane == 0) base = (int)atomicAdd(a.work_counter, (unsigned)per);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (base >= pixels) break;
+        const int gid = base + lane / 4;
+        const bool valid = gid < pixels && lane / 4 < per;
+        bool live = valid;
+        int x, y;
+        pixel_of(warp_tile_order(min(gid, pixels - 1), a.width, a.height), a.width, a.height, 32, x, y);
+        f3 o = mk3(a.cam.pos[0], a.cam.pos[1], a.cam.pos[2]);
+        f3 d = primary_dir(a.cam, x, y, a.width, a.height, 0.0f, 0.0f);
+        float tmin = 0.0f, tmax = 1e36f, contribution = 1.0f;
+        uint3 sum = make_uint3(0u, 0u, 0u);
+        n_prim += valid;
+        for (int bounce = 0;; ++bounce) {
+            const TRay r = make_tray(o, d, mk3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z), tmin);
+            const Hit hit = closest_hit_quad(S, sH, r, tmax, live, st, a.status);
+            live = live && hit.id >= 0;
+            HitInfo hi{};
+            rt_material mat{};
+            if (live) {
+                hi = complete_hit(S, o, d, hit);
+                mat = S.mats[__ldg(&S.map[hit.id])];
+            }
+            uint32_t mask = 0;
+            int nt = 0;
+            for (int l = 0; l < sL.count; ++l) {
+                const bool counts = live && !light_vanishes(sL.light[l], mat, hi.hp, hi.n, d);
+                f3 dir;
+                const bool reaches = counts && shadow_dir(sL.light[l], hi.hp, dir);
+                if (counts && !reaches) mask |= 1u << l;
+                const unsigned m = __ballot_sync(0xffffffffu, reaches && writer);
+                if (reaches && writer)
+                    list[nt + __popc(m & ((1u << lane) - 1u))] = (uint8_t)(lane / 4 | l << 3);
+                nt += __popc(m);
+            }
+            if (lane < 8) blocked[lane] = 0u;
+            __syncwarp();
+            for (int t0 = 0; t0 < nt; t0 += 8) {
+                const bool task = t0 + lane / 4 < nt;
+                const int e = task ? list[t0 + lane / 4] : 0, from = (e & 7) * 4;
+                const f3 hp = mk3(__shfl_sync(0xffffffffu, hi.hp.x, from),
+                                  __shfl_sync(0xffffffffu, hi.hp.y, from),
+                                  __shfl_sync(0xffffffffu, hi.hp.z, from));
+                f3 dir = mk3(0.f, 0.f, 0.f);
+                if (task) shadow_dir(sL.light[e >> 3], hp, dir);
+                const TRay sr = make_tray(hp, dir, mk3(1.0f / dir.x, 1.0f / dir.y, 1.0f / dir.z), 0.01f);
+                if (any_hit_quad(S, sH, sr, 1e37f, task, st, a.status) && writer)
+                    atomicOr(&blocked[e & 7], 1u << (e >> 3));
+            }
+            __syncwarp();
+            mask |= blocked[lane / 4];
+            __syncwarp();
+            if (live) {
+                ++n_hits;
+                const uint3 c = shade_hit(sL, mat, hi.hp, hi.n, d, contribution, mask);
+                sum.x += c.x;
+                sum.y += c.y;
+                sum.z += c.z;
+                live = bounce < a.max_bounces && mat.reflectiveness > 0.0f;
+                if (live) {
+                    f3 nd;
+                    reflect_ray(d, hi.n, nd);
+                    contribution = contribution * mat.reflectiveness * 1.0f;
+                    o = hi.hp;
+                    d = nd;
+                    tmin = 0.0001f;
+                    tmax = 1e37f;
+                    ++n_sec;
+                }
+            }
+            if (!__any_sync(0xffffffffu, live)) break;
+        }
+        if (valid && writer) write_pixel(a, a.width * y + x, sum);
+    }
+    if (a.stats) {
+        n_prim = __reduce_add_sync(0xffffffffu, writer ? n_prim : 0u);
+        n_sec = __reduce_add_sync(0xffffffffu, writer ? n_sec : 0u);
+        n_hits = __reduce_add_sync(0xffffffffu, writer ? n_hits : 0u);
+        if (lane == 0) {
+            atomicAdd((unsigned long long*)&a.stats->primary_rays, (unsigned long long)n_prim);
+            atomicAdd((unsigned long long*)&a.stats->secondary_rays, (unsigned long long)n_sec);
+            atomicAdd((unsigned long long*)&a.stats->shadow_rays,
+                      (unsigned long long)n_hits * (unsigned)sL.count);
+            atomicAdd((unsigned long long*)&a.stats->hits, (unsigned long long)n_hits);
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // k_render_pool: the same rays as k_render, scheduled so that a warp's lanes
 // stay busy.  A warp takes a tile of 32 pixels and traces their primary rays
@@ -103,17 +235,6 @@ struct WarpPool {
     uint8_t task[32 * RT_MAX_LIGHTS];           // shadow tasks that need a ray
 };
 }  // namespace
-
-// The pixel's sum, as it is and as RGBA8.
-__device__ __forceinline__ void write_pixel(const RenderArgs& a, int pix, uint3 sum) {
-    if (a.image_rgb) {
-        uint32_t* q = a.image_rgb + 3 * (size_t)pix;
-        q[0] = sum.x;
-        q[1] = sum.y;
-        q[2] = sum.z;
-    }
-    reinterpret_cast<uchar4*>(a.rgba)[pix] = rgba8_of(sum, a.inv1e6);
-}
 
 template <int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB) k_render_pool(RenderArgs a) {
@@ -839,8 +960,10 @@ static const RenderVariant kVariants[] = {
     {128, 6, k_render<128, 6, true>, false, true},
     {128, 4, k_render_pool_refr<128, 4, 6>, true, true, 6},
     {128, 5, k_render_pool_refr<128, 5, 4>, true, true, 4},
+    {128, 6, k_render_quad<128, 6>, false},
 };
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
+constexpr int kQuadVariant = kNumVariants - 1;
 static_assert(kNumVariants <= kMaxRenderVariants, "per-variant context arrays");
 
 int render_variant_count() { return kNumVariants; }
@@ -855,6 +978,8 @@ int render_variant_info(int v, int* threads, int* min_blocks, const void** fn) {
 
 bool render_variant_pooled(int v) { return v >= 0 && v < kNumVariants && kVariants[v].pooled; }
 
+bool render_variant_quad(int v) { return v == kQuadVariant; }
+
 bool render_variant_sums(int v) { return v >= 0 && v < kNumVariants && kVariants[v].sums(); }
 
 bool render_variant_refracts(int v) { return v >= 0 && v < kNumVariants && kVariants[v].refract; }
@@ -863,6 +988,8 @@ bool render_variant_fits(int v, int max_bounces) {
     if (v < 0 || v >= kNumVariants) return false;
     return kVariants[v].max_bounces == 0 || max_bounces <= kVariants[v].max_bounces;
 }
+
+int render_quad_variant() { return kQuadVariant; }
 
 int render_refract_variant(int max_bounces) {
     // the pooled variant with the smallest pool that holds the frame, else
@@ -900,12 +1027,12 @@ cudaError_t launch_gen_primary(const rt_camera& cam, int w, int h, int q, const 
 }
 
 // Launches with few rays take four lanes per ray (trace_quad.cuh).  Up to 768
-// rays per SM (primary rays of 10k / 200k triangles, trace and shadow: 65k rays
+// (kQuadRaysPerSm) rays per SM (primary rays of 10k / 200k triangles, trace and shadow: 65k rays
 // 140 -> 117 / 185 -> 153 us, 131k 150 -> 141 / 216 -> 192, 262k 181 -> 187 /
 // 262 -> 269); and of these, fewer than eight to a warp as long as that leaves
 // no more than 16 warps per SM (2k to 20k rays, whole pipeline 532 -> 520 us).
 static int quad_rays_per_warp(int n, int sms) {
-    if (n > 768 * sms) return 0;
+    if (n > kQuadRaysPerSm * sms) return 0;
     int per = 8;
     while (per > 1 && n <= 16 * sms * (per / 2)) per /= 2;
     return per;
