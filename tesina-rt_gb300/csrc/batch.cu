@@ -366,9 +366,8 @@ struct WarpPoolB {
     uint32_t rai[BPOOL], racc[3][CARRY ? BPOOL : 1];
     float hn[3][32];
     int hid[32];
-    unsigned hmask[32];
+    unsigned hmask[32];                 // blocked lights; from bit 8 the place; bit 16 inverse_n
     uint16_t hoff[32];
-    uint8_t hslot[CARRY ? 32 : 64];     // the hits' places; glass: then inverse_n
     uint8_t task[32 * RT_MAX_LIGHTS];   // shadow tasks that need a ray
 };
 }  // namespace
@@ -379,6 +378,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
     constexpr bool CARRY = MAXB == 0;
     static_assert(BPOOL <= 256, "places of the pool in 8 bits");
     static_assert(kMaxBatchViews <= 65536, "views in 16 bits");
+    static_assert(RT_MAX_LIGHTS <= 8, "a hit's place above its lights' bits");
     __shared__ WarpPoolB<BPOOL, CARRY> sQ[THREADS / 32];
     const int lane = threadIdx.x & 31;
     WarpPoolB<BPOOL, CARRY>& Q = sQ[threadIdx.x >> 5];
@@ -453,9 +453,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
             Q.ro[0][at] = hi.hp.x; Q.ro[1][at] = hi.hp.y; Q.ro[2][at] = hi.hp.z;
             Q.hn[0][k] = hi.n.x; Q.hn[1][k] = hi.n.y; Q.hn[2][k] = hi.n.z;
             Q.hid[k] = hit.id;
-            Q.hslot[k] = (uint8_t)at;
-            if (!CARRY) Q.hslot[32 + k] = hi.inverse_n;
-            Q.hmask[k] = 0u;
+            Q.hmask[k] = (unsigned)at << 8 | (unsigned)hi.inverse_n << 16;
             if (primary) {
                 Q.rd[0][at] = d.x; Q.rd[1][at] = d.y; Q.rd[2][at] = d.z;
                 Q.rc[at] = 1.0f;
@@ -498,7 +496,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
                         hi2 = mid - 1;
                 }
                 l = t - Q.hoff[lo];
-                const int j = Q.hslot[lo];
+                const int j = Q.hmask[lo] >> 8 & 255;
                 const BatchView& V = A.views[Q.rv[j]];
                 nd = !light_vanishes(V.lights->light[l],
                                      V.scene.mats[__ldg(&V.scene.map[Q.hid[lo]])],
@@ -513,7 +511,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
         __syncwarp();
         for (int i = lane; i < nt; i += 32) {
             const int e = Q.task[i], lo = e & 31, l = e >> 5;
-            const int j = Q.hslot[lo];
+            const int j = Q.hmask[lo] >> 8 & 255;
             const BatchView& V = A.views[Q.rv[j]];
             const BvhHeader H = *V.scene.hdr;
             const f3 p = mk3(Q.ro[0][j], Q.ro[1][j], Q.ro[2][j]);
@@ -528,7 +526,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
         uint32_t nai = 0;
         uint3 sum = make_uint3(0u, 0u, 0u);
         if (lane < nh) {
-            const int k = lane, j = Q.hslot[k];
+            const int k = lane, j = Q.hmask[k] >> 8 & 255;
             nv = Q.rv[j];
             const BatchView& V = A.views[nv];
             const f3 p = mk3(Q.ro[0][j], Q.ro[1][j], Q.ro[2][j]);
@@ -536,7 +534,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
             const f3 dk = mk3(Q.rd[0][j], Q.rd[1][j], Q.rd[2][j]);
             const float ck = Q.rc[j];
             const rt_material mat = V.scene.mats[__ldg(&V.scene.map[Q.hid[k]])];
-            const uint3 col = shade_hit(*V.lights, mat, p, n, dk, ck, Q.hmask[k]);
+            const uint3 col = shade_hit(*V.lights, mat, p, n, dk, ck, Q.hmask[k] & 255u);
             nai = Q.rai[j];
             if (CARRY) {
                 sum = make_uint3(Q.racc[0][j] + col.x, Q.racc[1][j] + col.y, Q.racc[2][j] + col.z);
@@ -551,7 +549,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_batch_pool(BatchRender
             if (bk < V.max_bounces) {
                 float R = 1.0f;
                 if (MAXB > 0 && mat.refractive_index > 0.0f &&
-                    refract_ray(dk, n, Q.hslot[32 + k] != 0, mat.refractive_index, R, td)) {
+                    refract_ray(dk, n, Q.hmask[k] >> 16 != 0, mat.refractive_index, R, td)) {
                     tc = ck * mat.reflectiveness * (1.0f - R);
                     push_t = true;
                 }
@@ -624,13 +622,13 @@ struct BatchRenderVariant {
     bool sums() const { return pooled && refract; }   // adds pixels up in BatchRenderArgs::accum
 };
 // Variant 0 serves the request loop (many short launches, where the unpooled
-// kernel measured faster); rt_batch takes the first pooled one (one large
-// launch, where the pool keeps lanes busy).
+// kernel measured faster: 24 requests 4.5-4.6 ms, pooled 4.6); rt_batch takes
+// the first pooled one (one large launch, where the pool keeps lanes busy).  Its
+// eight blocks against six (72 registers): 64 soups 6.82 -> 6.40 ms, 16 1.75 -> 1.65,
+// 2 0.60 -> 0.57 (fewer for small batches, as small frames have, loses); its pool of
+// 15,872 bytes a block fits them into 132 KB of shared memory.
 static const BatchRenderVariant kBatchVariants[] = {
     {128, 8, k_render_batch<128, 8>, false},
-    {128, 6, k_render_batch_pool<128, 6>, true},
-    {256, 4, k_render_batch<256, 4>, false},
-    {128, 6, k_render_batch<128, 6>, false},
     {128, 8, k_render_batch_pool<128, 8>, true},
     {128, 6, k_render_batch<128, 6, true>, false, true},
     {128, 5, k_render_batch_pool<128, 5, 4>, true, true, 4},
