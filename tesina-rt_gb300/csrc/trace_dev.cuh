@@ -203,14 +203,15 @@ constexpr int32_t NO_NODE = (int32_t)0x80000000;   // below every leaf code
 // search has ended stay for the votes, which keeps the warp together; faster
 // in the stage kernels (784 -> 712 us), the instanced render and the
 // one-path-per-lane kernels (served burst 5.5 -> 4.8 ms), slower in the pooled
-// ones.
+// ones; there the leaves wait until they are half of the lanes (a third against
+// that: instances 1.855 -> 1.849 ms, stage pipeline 517 -> 515 us).
 template <bool STAY>
 __device__ __forceinline__ bool leaf_turn(unsigned group, int32_t next, bool& ended) {
     if (STAY) {
         const unsigned lm = __ballot_sync(group, next < 0 && next != NO_NODE);
         const unsigned nm = __ballot_sync(group, next >= 0);
         ended = (lm | nm) == 0u;
-        return 2 * __popc(lm) >= __popc(nm) && next < 0 && next != NO_NODE;
+        return __popc(lm) >= __popc(nm) && next < 0 && next != NO_NODE;
     }
     ended = next == NO_NODE;
     if (ended) return false;

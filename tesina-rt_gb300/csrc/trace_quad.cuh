@@ -8,6 +8,8 @@
 // The rays visit the same leaves in the same order as in trace_dev.cuh, with
 // the same arithmetic.  Trace and shadow stage of a 10k-triangle soup, without
 // and with: 21k secondary rays 93 + 63 -> 61 + 43 us, 2k 100 + 66 -> 46 + 39.
+// A warp's leaves are tested in the turn that reaches them: to wait for more, as
+// leaf_turn does, loses 1 % of a small frame.
 // (Prefetching the records and triangles of the children hit loses 3 %: it is
 // the instructions' latency, not the memory's.)
 #pragma once
@@ -75,8 +77,7 @@ __device__ __forceinline__ Hit closest_quad(const SceneView& S, int32_t root, co
     bool over = false;
     int32_t next = live ? root : NO_NODE;
     for (;;) {
-        const unsigned nm = __ballot_sync(0xffffffffu, next >= 0);
-        if (nm) {
+        if (__any_sync(0xffffffffu, next >= 0)) {
             const bool on = next >= 0;
             Slot s{};
             if (on) s = load_slot(S.nodes, next, q);
@@ -109,10 +110,7 @@ __device__ __forceinline__ Hit closest_quad(const SceneView& S, int32_t root, co
             __syncwarp();
             quad_pop(on && next == NO_NODE, st, sp, best.t, next);
         }
-        const unsigned lm = __ballot_sync(0xffffffffu, next < 0 && next != NO_NODE);
-        if (lm) {
-            const unsigned again = __ballot_sync(0xffffffffu, next >= 0);
-            if (2 * __popc(lm) < __popc(again)) continue;
+        if (__any_sync(0xffffffffu, next < 0 && next != NO_NODE)) {
             const bool leaf = next < 0 && next != NO_NODE;
             bool on = leaf;
             int32_t i = ~next;
@@ -174,10 +172,7 @@ __device__ __forceinline__ bool any_quad(const SceneView& S, int32_t root, const
             __syncwarp();
             if (on && next == NO_NODE && sp > 0) next = st[--sp].x;
         }
-        const unsigned lm = __ballot_sync(0xffffffffu, next < 0 && next != NO_NODE);
-        if (lm) {
-            const unsigned again = __ballot_sync(0xffffffffu, next >= 0);
-            if (2 * __popc(lm) < __popc(again)) continue;
+        if (__any_sync(0xffffffffu, next < 0 && next != NO_NODE)) {
             const bool leaf = next < 0 && next != NO_NODE;
             bool on = leaf;
             int32_t i = ~next;
