@@ -43,19 +43,11 @@ B_RAY_CLOSEST, B_RAY_SHADOW, B_SHADE = 40, 25, 48
 # kernel on the mid-scale frame (ncu, --clock-control none), by kernel; the
 # line's roofline carries it only when the autotuner installed that kernel.
 RENDER_DRAM_BYTES = {
-    "k_render_pool<128, 6>": (297.9 + 32.7) * 1e6,
-    "k_render_pool<128, 8>": (320.0 + 37.3) * 1e6,
-    "k_render_pool<256, 3>": (286.5 + 28.8) * 1e6,
-    "k_render_pool<256, 4>": (318.8 + 37.1) * 1e6,
+    "k_render_pool<128, 8>": (157.0 + 12.5) * 1e6,
 }
 # the same for the stress workload (17.7 M triangles, 3840x2160, 3 lights,
-# depth 6), the mean over its 8 poses
-STRESS_RENDER_DRAM_BYTES = {
-    "k_render_pool<128, 6>": (2041.6 + 177.7) * 1e6,
-    "k_render_pool<128, 8>": (2149.0 + 209.5) * 1e6,
-    "k_render_pool<256, 3>": (1931.3 + 147.6) * 1e6,
-    "k_render_pool<256, 4>": (2148.2 + 209.5) * 1e6,
-}
+# depth 6): not measured since the records became four-wide
+STRESS_RENDER_DRAM_BYTES = {}
 
 
 def log(*a):
@@ -231,7 +223,8 @@ def cpu_c0_full():
 def traversal_work(s, cam, w, h, sample_rays=65536):
     """Node and triangle records the oracle's traversal reads per primary ray
     and per shadow ray of those rays (interior nodes entered, 64 B each;
-    triangles tested, 48 B), on the first `sample_rays` samples."""
+    triangles tested, 48 B), on the first `sample_rays` samples.  The kernels'
+    four-wide records hold two binary levels in 128 B."""
     pyoracle, orc = _oracle()
     smp = pyoracle.gen_primary(orc, cam, w, h, count=sample_rays)
     tc = s.traversal_counts(smp, threads=os.cpu_count() or 1)
@@ -1032,7 +1025,7 @@ def run_gpu(args):
                 "traffic": RENDER_DRAM_BYTES.get(kname),
                 "peak_kind": peak_kind,
                 "algorithmic_bytes_per_launch": render_bytes,
-                "note": "traversal is latency/L2-bound; algorithmic bytes = 88 B per traced "
+                "note": "traversal is bound by its steps' instructions; algorithmic bytes = 88 B per traced "
                         "ray + 25 B per shadow ray"}
     # the emit's levels: 512 triangles per level-0 block, then 8 blocks per block
     emit_levels = emit_levels_of(n_tris)
@@ -1109,7 +1102,7 @@ def run_gpu(args):
         tb = tv["bytes_per_ray"] * rays_step + tv["bytes_per_shadow_ray"] * shadow_step
         roofline["traversal"] = dict(tv, bytes_per_frame=tb,
                                      gbs=tb / (med_render * 1e-3) / 1e9,
-                                     note="node and triangle records the traversal reads per frame "
+                                     note="node and triangle records of the binary order per frame "
                                           "(oracle-counted on the sample's primary rays and their "
                                           "shadow rays, applied to every traced ray), served "
                                           "mostly from L1 and L2")
