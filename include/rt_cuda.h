@@ -204,8 +204,11 @@ RT_API int32_t rt_device_status(rt_ctx* ctx, uint32_t* bits);
  * whose predecessor tile is never launched, so its decoupled look-back polls
  * an unpublished word until its limit (1,024 polls here) runs out.  The
  * kernel then sets RT_DEV_TIMEOUT, finishes its tile inside its buffers and
- * returns; the call synchronises and maps the status as rt_render_host does:
- * RT_ERR_TIMEOUT when the timeout path worked (RT_OK would mean it did not).
+ * returns.  The rest of an LBVH build runs over what it left, which must take
+ * none of it for an order of the triangles (a build whose sort timed out keeps
+ * their order and holds no tree but a leaf of the first one).  The call
+ * synchronises and maps the status as rt_render_host does: RT_ERR_TIMEOUT when
+ * the timeout path worked (RT_OK or RT_ERR would mean it did not).
  * The status stays set for rt_device_status to read and clear; the context
  * stays usable. */
 RT_API int32_t rt_selftest_wait_timeout(rt_ctx* ctx, rt_stream s);

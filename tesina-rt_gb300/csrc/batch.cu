@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(SORT_THREADS, 4) k_batch_build(BatchBuildArgs 
         const size_t words = (size_t)B.passes * (s_tileoff[sc + 1] - s_tileoff[sc]) * 256;
         for (size_t i = gtid; i < words; i += gthreads) B.lookback[i] = 0;
     }
+    for (uint32_t i = gtid; i < (uint32_t)nsc; i += gthreads) A.scenes[i].hdr->status = 0u;
     if (gtid < 4) A.tile_ctr[gtid] = 0;
     grid.sync();
     stamp(A, 1);
@@ -238,7 +239,8 @@ __global__ void __launch_bounds__(SORT_THREADS, 4) k_batch_build(BatchBuildArgs 
             uint32_t* vout = dst ? B.vals_sorted : B.vals1;
             const uint32_t ntiles_s = s_tileoff[s + 1] - s_tileoff[s];
             onesweep_tile<kBatchItems>(S, lt, kin, vin, kout, vout, B.n, 8 * p, B.hist + 256 * p,
-                          B.lookback + (size_t)p * ntiles_s * 256, A.status);
+                          B.lookback + (size_t)p * ntiles_s * 256, A.status,
+                          &B.hdr->status);
         }
         grid.sync();
         if (p == A.passes - 1) stamp(A, 4);

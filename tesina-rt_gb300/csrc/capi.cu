@@ -468,15 +468,18 @@ int32_t rt_selftest_wait_timeout(rt_ctx* c, rt_stream stream) {
     cudaStream_t cs = stream ? (cudaStream_t)stream : c->stream;
     uint32_t* buf = nullptr;
     CU(cudaMalloc(&buf, sizeof(uint32_t) * rt::wait_probe_words()));
-    const cudaError_t e = rt::wait_probe(buf, c->d_status, cs);
+    bool kept = false;
+    const cudaError_t e = rt::wait_probe(buf, c->num_sms, c->d_status, &kept, cs);
     const cudaError_t e2 = cudaStreamSynchronize(cs);
     cudaFree(buf);
     CU(e);
     CU(e2);
     uint32_t bits = 0;
     CU(cudaMemcpy(&bits, c->d_status, sizeof(bits), cudaMemcpyDeviceToHost));
+    if (!kept) return fail(RT_ERR, "rt_selftest_wait_timeout: the build after the sort used its order");
     if (bits & RT_DEV_TIMEOUT)
-        return fail(RT_ERR_TIMEOUT, "rt_selftest_wait_timeout: device wait timed out");
+        return fail(RT_ERR_TIMEOUT, "rt_selftest_wait_timeout: device wait timed out, the build "
+                    "after it kept the triangles' order");
     return RT_OK;
 }
 

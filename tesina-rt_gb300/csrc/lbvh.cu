@@ -28,6 +28,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <mutex>
+#include <vector>
 
 #include "lbvh.cuh"
 #include "lbvh_dev.cuh"
@@ -73,8 +74,10 @@ static cudaError_t launch_dep(void (*kern)(KArgs...), unsigned grid, unsigned bl
 __global__ void __launch_bounds__(256) k_bounds(const float4* __restrict__ pos,
                                                 const uint32_t* __restrict__ idx, uint32_t n,
                                                 uint32_t* __restrict__ bounds,
-                                                uint4* __restrict__ clear, uint32_t clear_n) {
+                                                uint4* __restrict__ clear, uint32_t clear_n,
+                                                uint32_t* __restrict__ build_status) {
     pdl_enter();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *build_status = 0u;
     // the later kernels' counters are cleared here, beside the gathers
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < clear_n; i += gridDim.x * blockDim.x)
         clear[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -166,13 +169,14 @@ template <int MINB>
 __global__ void __launch_bounds__(SORT_THREADS, MINB) k_onesweep(
     const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint32_t* __restrict__ kout,
     uint32_t* __restrict__ vout, uint32_t n, int shift, const uint32_t* __restrict__ hist,
-    uint32_t* __restrict__ lookback, uint32_t* __restrict__ tile_ctr, uint32_t* __restrict__ status) {
+    uint32_t* __restrict__ lookback, uint32_t* __restrict__ tile_ctr, uint32_t* __restrict__ status,
+    uint32_t* __restrict__ failed) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char sort_smem[];
     auto& S = *reinterpret_cast<SortSmem*>(sort_smem);
     if (threadIdx.x == 0) S.tile = atomicAdd(tile_ctr, 1u);   // tiles in launch order
     __syncthreads();
-    onesweep_tile<>(S, S.tile, kin, vin, kout, vout, n, shift, hist, lookback, status);
+    onesweep_tile<>(S, S.tile, kin, vin, kout, vout, n, shift, hist, lookback, status, failed);
 }
 
 constexpr int kOneWaveMinB = 2;
@@ -189,10 +193,10 @@ constexpr uint32_t kProbeSpinLimit = 1024;
 __global__ void __launch_bounds__(SORT_THREADS, 1) k_onesweep_wait_probe(
     const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint32_t* __restrict__ kout,
     uint32_t* __restrict__ vout, uint32_t n, const uint32_t* __restrict__ hist,
-    uint32_t* __restrict__ lookback, uint32_t* __restrict__ status) {
+    uint32_t* __restrict__ lookback, uint32_t* __restrict__ status, uint32_t* __restrict__ failed) {
     __shared__ SortSmem S;
     onesweep_tile<SORT_ITEMS, kProbeSpinLimit>(S, 1, kin, vin, kout, vout, n, 0, hist, lookback,
-                                               status);
+                                               status, failed);
 }
 
 // The permutation of a tree built on the host, whose leaf marks (1: the next
@@ -201,7 +205,7 @@ __global__ void __launch_bounds__(256) k_permute(uint32_t n, PermuteIO P,
                                                   const uint8_t* __restrict__ more) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         float4 lo, hi;
-        permute_tri(i, P, lo, hi);
+        permute_tri(i, P, true, lo, hi);
         if (more[i]) P.tris[3 * (size_t)i].w = 1.0f;
     }
 }
@@ -341,7 +345,8 @@ cudaError_t lbvh_build(const LbvhArgs& a, cudaStream_t s) {
     const size_t clear = (kMaxBuildPasses * kBuildRadix + 4 + (size_t)passes * tiles * kBuildRadix) / 4;
     const int sms = a.num_sms;
     k_bounds<<<grid_for(n, 256, sms * 8), 256, 0, s>>>(a.pos, a.idx_in, n, bounds,
-                                                       reinterpret_cast<uint4*>(hist), (uint32_t)clear);
+                                                       reinterpret_cast<uint4*>(hist), (uint32_t)clear,
+                                                       &a.hdr->status);
     e = launch_dep(k_morton_hist, grid_for(n, 256, sms * 8), 256, 0, s, true, a.pos, a.idx_in, n,
                    bounds, a.depth, passes, a.keys_unsorted, hist);
     if (e) return e;
@@ -355,7 +360,8 @@ cudaError_t lbvh_build(const LbvhArgs& a, cudaStream_t s) {
         e = launch_dep(onesweep_kernel(tiles, sms), (unsigned)tiles, SORT_THREADS,
                        sizeof(SortSmem), s, true, kin, vin, kbuf[dst], vbuf[dst], n,
                        kBuildBits * p, (const uint32_t*)(hist + kBuildRadix * p),
-                       lookback + (size_t)p * tiles * kBuildRadix, tile_ctr + p, a.status);
+                       lookback + (size_t)p * tiles * kBuildRadix, tile_ctr + p, a.status,
+                       &a.hdr->status);
         if (e) return e;
         kin = kbuf[dst];
         vin = vbuf[dst];
@@ -373,22 +379,75 @@ size_t radix_scratch_words(uint32_t n, int passes) {
 
 int radix_tile_size() { return SORT_TILE; }
 
-size_t wait_probe_words() { return (size_t)2 * SORT_TILE * 4 + 256 + 2 * 256; }
+// The probe's scene of two tiles of triangles: what a build of it takes, and
+// the words of the sort probe before it (keys | vals | hist[256] | lookback[2 * 256]).
+constexpr uint32_t kProbeTris = 2 * SORT_TILE;
+constexpr size_t kProbeSortWords = 2 * (size_t)kProbeTris + 3 * 256;
+static size_t probe_bytes() {
+    const size_t n = kProbeTris, words = kProbeSortWords + 2 * n + 10 * n;
+    return 4 * words + 16 * (3 * (n + 3) + 8 * n + 1) + emit_scratch_bytes(kProbeTris) +
+           sizeof(BvhHeader) + 256;
+}
 
-cudaError_t wait_probe(uint32_t* buf, uint32_t* status, cudaStream_t s) {
-    // buf: keys | vals | kout | vout (2 tiles each) | hist[256] | lookback[2 * 256]
-    const uint32_t n = 2 * SORT_TILE;
-    uint32_t* keys = buf;
-    uint32_t* vals = keys + n;
-    uint32_t* kout = vals + n;
-    uint32_t* vout = kout + n;
-    uint32_t* hist = vout + n;
-    uint32_t* lookback = hist + 256;
+size_t wait_probe_words() { return (probe_bytes() + 3) / 4; }
+
+cudaError_t wait_probe(uint32_t* buf, int num_sms, uint32_t* status, bool* kept, cudaStream_t s) {
+    const uint32_t n = kProbeTris;
     cudaError_t e = cudaMemsetAsync(buf, 0, sizeof(uint32_t) * wait_probe_words(), s);
     if (e) return e;
+    // 16-byte types first; all of it zero: every index is vertex 0, every
+    // material 0
+    LbvhArgs a{};
+    a.n = n;
+    a.depth = 30;
+    a.min_leaf = 1;
+    a.num_sms = num_sms;
+    a.status = status;
+    a.nodes = reinterpret_cast<float4*>(buf);   // 128-byte records
+    a.tris = a.nodes + 8 * (size_t)n;
+    float4* pos = a.tris + 3 * ((size_t)n + 3);
+    a.pos = pos;
+    a.hdr = reinterpret_cast<BvhHeader*>(pos + 1);
+    uint8_t* emit = reinterpret_cast<uint8_t*>(a.hdr + 1);
+    uint32_t* w = reinterpret_cast<uint32_t*>(emit + emit_scratch_bytes(n));
+    auto take = [&](size_t words) {
+        uint32_t* p = w;
+        w += words;
+        return p;
+    };
+    uint32_t* keys = take(n);
+    uint32_t* vals = take(n);
+    uint32_t* hist = take(256);
+    uint32_t* lookback = take(2 * 256);
+    a.keys_sorted = take(n);
+    a.vals_sorted = take(n);
+    uint32_t* idx = take(3 * (size_t)n);
+    uint32_t* map = take(n);
+    uint32_t* orig = take(n);
+    a.idx_in = idx;
+    a.map_in = map;
+    a.orig_in = orig;
+    a.idx_out = take(3 * (size_t)n);
+    a.map_out = take(n);
+    a.orig_out = take(n);
+    // the sorted arrays' memory held something else before
+    if ((e = cudaMemsetAsync(a.keys_sorted, 0xa5, 8 * (size_t)n, s))) return e;
+    std::vector<uint32_t> ids(n);
+    for (uint32_t i = 0; i < n; ++i) ids[i] = i ^ 5u;
+    if ((e = cudaMemcpyAsync(orig, ids.data(), 4 * (size_t)n, cudaMemcpyHostToDevice, s))) return e;
     k_radix_hist<<<1, 256, 0, s>>>(keys, n, 1, hist);
-    k_onesweep_wait_probe<<<1, SORT_THREADS, 0, s>>>(keys, vals, kout, vout, n, hist, lookback,
-                                                     status);
+    k_onesweep_wait_probe<<<1, SORT_THREADS, 0, s>>>(keys, vals, a.keys_sorted, a.vals_sorted, n,
+                                                     hist, lookback, status, &a.hdr->status);
+    const PermuteIO P{a.vals_sorted, a.idx_in,  a.map_in,   a.orig_in, a.pos,
+                      a.idx_out,     a.map_out, a.orig_out, a.tris};
+    if ((e = launch_emit<EMIT_PERMUTE>(a, emit, P, s))) return e;
+    std::vector<uint32_t> got(n);
+    BvhHeader h;
+    if ((e = cudaMemcpyAsync(got.data(), a.orig_out, 4 * (size_t)n, cudaMemcpyDeviceToHost, s)) ||
+        (e = cudaMemcpyAsync(&h, a.hdr, sizeof h, cudaMemcpyDeviceToHost, s)) ||
+        (e = cudaStreamSynchronize(s)))
+        return e;
+    *kept = got == ids && h.status == RT_DEV_TIMEOUT && h.root_ref == 0 && h.root_cnt == 1;
     return cudaGetLastError();
 }
 
@@ -415,7 +474,7 @@ cudaError_t radix_sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t*
         uint32_t* vo = to_out ? vout : vtmp;
         onesweep_kernel(tiles, num_sms)<<<(unsigned)tiles, SORT_THREADS, sizeof(SortSmem), s>>>(
             ki, vi, ko, vo, n, 8 * p, hist + 256 * p, lookback + (size_t)p * tiles * 256,
-            tile_ctr + p, status);
+            tile_ctr + p, status, nullptr);
         ki = ko;
         vi = vo;
     }

@@ -59,10 +59,11 @@ inline uint32_t* sort_vals1(float4* tris, uint32_t n) {
 // pairs; passes alternate between out and tmp so that the last lands in out.
 size_t radix_scratch_words(uint32_t n, int passes);
 // Self-test of the device timeout path: a radix-pass tile whose predecessor
-// never publishes, in a zeroed buffer of wait_probe_words() words; sets
-// RT_DEV_TIMEOUT in *status.
+// never publishes, in a buffer of wait_probe_words() words, sets RT_DEV_TIMEOUT
+// in *status; then the build's emit runs over what that pass left, and *kept
+// tells whether the triangles stayed in order under a root leaf.  Synchronises.
 size_t wait_probe_words();
-cudaError_t wait_probe(uint32_t* buf, uint32_t* status, cudaStream_t s);
+cudaError_t wait_probe(uint32_t* buf, int num_sms, uint32_t* status, bool* kept, cudaStream_t s);
 int radix_tile_size();
 cudaError_t radix_sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t* kout,
                              uint32_t* vout, uint32_t* ktmp, uint32_t* vtmp, uint32_t n,

@@ -214,10 +214,13 @@ using SortSmem = SortSmemT<SORT_ITEMS>;
 // 256 digit counts, `lookback` 256 words per tile: tile 0 publishes the global
 // offset of each digit with its count, so the later tiles' prefixes are
 // scatter offsets as they are.  A look-back that polls an unpublished word
-// more than SPIN_LIMIT times gives up: it sets RT_DEV_TIMEOUT in *status and
-// goes on with the counts it has, so every block ends; its writes stay inside
+// more than SPIN_LIMIT times gives up: it sets RT_DEV_TIMEOUT in *status and, if
+// there is one, in *failed (the scene's BvhHeader::status), and goes on with the
+// counts it has, so every block ends; its writes stay inside
 // [0, n): a partial prefix only lowers the offsets, a key's place in its tile is
-// added, and what would lie at or beyond n is dropped.
+// added, and what would lie at or beyond n is dropped.  What the pass leaves is
+// arbitrary then: some places keep what the memory held before, so neither its
+// keys nor its values may be used as a sorted order (see emit_level).
 //
 // What bounds it: the chain of one tile, about 14 us of load and ranking
 // (6.0-6.6), staging (1.3-1.7), look-back (3.4-4.0: 8 to 11 round trips) and
@@ -234,7 +237,8 @@ __device__ __forceinline__ void onesweep_tile_body(SortSmemT<ITEMS>& S, uint32_t
                                                    uint32_t* __restrict__ vout, uint32_t n,
                                                    int shift, const uint32_t* __restrict__ hist,
                                                    uint32_t* __restrict__ lookback,
-                                                   uint32_t* __restrict__ status) {
+                                                   uint32_t* __restrict__ status,
+                                                   uint32_t* __restrict__ failed) {
     constexpr uint32_t TILE = SORT_THREADS * ITEMS;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     RT_SORT_MARK(0);
@@ -365,6 +369,7 @@ __device__ __forceinline__ void onesweep_tile_body(SortSmemT<ITEMS>& S, uint32_t
             p -= used;
             if (wait && ++spins > SPIN_LIMIT) {
                 atomicOr(status, RT_DEV_TIMEOUT);
+                if (failed) atomicOr(failed, RT_DEV_TIMEOUT);
                 break;
             }
             read_window(p);
@@ -396,13 +401,14 @@ __device__ __forceinline__ void onesweep_tile(SortSmemT<ITEMS>& S, uint32_t tile
                                               uint32_t* __restrict__ vout, uint32_t n, int shift,
                                               const uint32_t* __restrict__ hist,
                                               uint32_t* __restrict__ lookback,
-                                              uint32_t* __restrict__ status) {
+                                              uint32_t* __restrict__ status,
+                                              uint32_t* __restrict__ failed) {
     if ((size_t)(tile + 1) * (SORT_THREADS * ITEMS) <= n)
         onesweep_tile_body<ITEMS, SPIN_LIMIT, true>(S, tile, kin, vin, kout, vout, n, shift, hist,
-                                                    lookback, status);
+                                                    lookback, status, failed);
     else
         onesweep_tile_body<ITEMS, SPIN_LIMIT, false>(S, tile, kin, vin, kout, vout, n, shift, hist,
-                                                     lookback, status);
+                                                     lookback, status, failed);
 }
 
 // rearrange_indices / rearrange_map (bvh-builder.cl:49-72) of sorted slot i,
@@ -437,8 +443,11 @@ __device__ __forceinline__ void tri_record(uint32_t i, const PermuteIO& P, uint3
     lo.w = hi.w = 0.f;
 }
 
-__device__ __forceinline__ void permute_tri(uint32_t i, const PermuteIO& P, float4& lo, float4& hi) {
-    const uint32_t o = ld_dep(&P.vals[i]);
+// `sorted` false: there is no order to take (a wait of the sort gave up), the
+// triangles stay where they are.
+__device__ __forceinline__ void permute_tri(uint32_t i, const PermuteIO& P, bool sorted, float4& lo,
+                                            float4& hi) {
+    const uint32_t o = sorted ? ld_dep(&P.vals[i]) : i;
     const uint32_t a = __ldg(&P.idx_old[3 * (size_t)o]), b = __ldg(&P.idx_old[3 * (size_t)o + 1]),
                    c = __ldg(&P.idx_old[3 * (size_t)o + 2]);
     P.idx_new[3 * (size_t)i] = a;
@@ -945,7 +954,11 @@ __device__ __forceinline__ uint32_t gather_runs(EmitSmem<C, T>& S, const WarpIte
 //
 // Level 0 makes its triangles' records itself and keeps their boxes in
 // registers: it performs the permutation of a build (SRC = EMIT_PERMUTE,
-// permute_tri with `perm`) or a refit (EMIT_REFIT, refit_tri).
+// permute_tri with `perm`) or a refit (EMIT_REFIT, refit_tri).  After a sort
+// whose wait gave up (hdr->status) the values are not a permutation, and unsorted
+// keys would give nodes that are their own descendants: the triangles then keep
+// their order, and the tree is the leaf of triangle 0 alone, so that whatever
+// reads it before the caller has seen RT_DEV_TIMEOUT stays in range and ends.
 enum EmitSource { EMIT_ITEMS, EMIT_PERMUTE, EMIT_REFIT };
 template <int C, int T, EmitSource SRC = EMIT_ITEMS>
 __device__ __forceinline__ void emit_level(EmitSmem<C, T>& S, uint32_t blk, uint32_t n,
@@ -967,6 +980,7 @@ __device__ __forceinline__ void emit_level(EmitSmem<C, T>& S, uint32_t blk, uint
     uint32_t m;
     if constexpr (SRC != EMIT_ITEMS) {
         // level 0: warp w joins triangles b0 + 32w ..
+        const bool failed = ld_dep(&hdr->status) != 0u;
         const uint32_t b0 = blk * (uint32_t)C, i = b0 + t;
         const uint32_t w0 = b0 + 32u * w;
         const uint32_t cnt = w0 < n ? min(32u, n - w0) : 0u;
@@ -981,7 +995,7 @@ __device__ __forceinline__ void emit_level(EmitSmem<C, T>& S, uint32_t blk, uint
         float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
         if (have) {
             if constexpr (SRC == EMIT_PERMUTE)
-                permute_tri(i, perm, lo, hi);
+                permute_tri(i, perm, !failed, lo, hi);
             else
                 refit_tri(i, perm, lo, hi);
         }
@@ -990,11 +1004,11 @@ __device__ __forceinline__ void emit_level(EmitSmem<C, T>& S, uint32_t blk, uint
         it.ref = (int32_t)i;
         it.cnt = 1;
         const uint64_t edge = cnt ? delta_or_max(skeys, (int64_t)w0 + cnt - 1, n) : 0ull;
-        if (n == 1) {
-            if (t == 0) {
+        if (n == 1 || failed) {
+            if (i == 0) {
                 hdr->root_ref = 0;
                 hdr->root_cnt = 1;
-                hdr->n_tris = 1;
+                hdr->n_tris = n;
                 hdr->root_lo = lo;
                 hdr->root_hi = hi;
             }

@@ -32,7 +32,7 @@ struct BvhHeader {
     int32_t root_ref;       // interior node index, or first triangle of a root leaf
     int32_t root_cnt;       // 0: interior root; > 0: the whole tree is one leaf
     uint32_t n_tris;
-    uint32_t status;        // RT_DEV_* bits raised while building
+    uint32_t status;        // RT_DEV_TIMEOUT: a wait of the build's sort gave up (no tree)
     float4 root_lo;
     float4 root_hi;
 };

@@ -46,3 +46,18 @@ def test_timeout_on_a_second_stream(ctx):
         assert ctx.device_status() == 0
     finally:
         ctx.stream_destroy(s)
+
+
+def test_build_after_a_timed_out_sort_takes_no_order_from_it(ctx):
+    """The rest of a build runs over arrays that a given-up pass left partly
+    unwritten: the triangles keep their places and the tree is one leaf."""
+    assert ctx.selftest_wait_timeout() == abi.RT_ERR_TIMEOUT
+    assert b"kept the triangles' order" in ctx.lib.rt_last_error()
+    assert ctx.device_status() == abi.RT_DEV_TIMEOUT
+    sc = scenes.soup(9000, seed=22)
+    g = capi.Scene(ctx, sc)
+    g.build(30, 1)   # the next build clears the mark
+    assert not g.canon()[0]["leaf"]
+    g.refit()
+    assert not g.canon()[0]["leaf"] and ctx.device_status() == 0
+    g.close()
