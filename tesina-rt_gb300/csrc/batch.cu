@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(SORT_THREADS, 4) k_batch_build(BatchBuildArgs 
 // EMIT_T_WIDE, the scenes' levels being wide together.
 static_assert(EMIT_C0 != EMIT_T_WIDE, "k_batch_emit tells level 0 by its block size");
 template <int T>
-__global__ void __launch_bounds__(T, T == EMIT_C0 ? RT_EMIT_MINB0 : 2) k_batch_emit(
+__global__ void __launch_bounds__(T, T == EMIT_C0 ? EMIT_MINB0 : 2) k_batch_emit(
     const BatchScene* __restrict__ scenes, int count, int level, const uint32_t* __restrict__ off,
     uint32_t* __restrict__ status) {
     extern __shared__ __align__(16) unsigned char emit_smem[];

@@ -116,10 +116,6 @@ __device__ __forceinline__ float cull_enter(const float4* cull, int i, f3 o, f3 
     return t0 > t1 ? -1.0f : t0;
 }
 
-#ifndef RT_INST_NEAR
-#define RT_INST_NEAR 1   // visit a group's roots near to far (0: in index order)
-#endif
-
 struct MultiHit {
     Hit h;        // id local to the instance's scene; t in world space
     int root;
@@ -171,7 +167,7 @@ __device__ __forceinline__ MultiHit closest_multi(const InstanceArgs& A, f3 o, f
             while (live) {
                 int jm = __ffs(live) - 1;
                 float em = ent[jm];
-                for (uint32_t r = live & (live - 1); RT_INST_NEAR && r && !seq; r &= r - 1) {
+                for (uint32_t r = live & (live - 1); r && !seq; r &= r - 1) {
                     const int j = __ffs(r) - 1;
                     if (ent[j] < em) {
                         em = ent[j];
@@ -179,10 +175,8 @@ __device__ __forceinline__ MultiHit closest_multi(const InstanceArgs& A, f3 o, f
                     }
                 }
                 live &= ~(1u << jm);
-                if (!seq && best.h.id >= 0 && em * dlen > best.h.t) {
-                    if (RT_INST_NEAR) break;   // the rest of the group enters later still
-                    continue;
-                }
+                if (!seq && best.h.id >= 0 && em * dlen > best.h.t)
+                    break;   // the rest of the group enters later still
                 const int i = g + jm;
                 const Hit h = root_closest(A.roots[i], o, d, tmin, tmax, A.status);
                 if (!seq && h.id >= 0 && isnan(h.t)) {
@@ -287,11 +281,8 @@ __device__ __forceinline__ void write_pixel(const InstanceArgs& A, int pix, uint
 
 // 5 blocks per SM, 102 registers: at 6 the four-wide traversal spills (16 roots
 // at 1920 x 1080: 2.16 -> 2.11 ms; 4 blocks 2.24).
-#ifndef RT_INST_MINB
-#define RT_INST_MINB 5
-#endif
 template <int MAXB>
-__global__ void __launch_bounds__(128, MAXB == 6 ? 5 : RT_INST_MINB) k_render_instances(InstanceArgs A) {
+__global__ void __launch_bounds__(128, 5) k_render_instances(InstanceArgs A) {
     constexpr int IPOOL = MAXB ? 32 * (MAXB + 2) : 64;   // reflections only: < 32 left + 32 new
     constexpr bool CARRY = MAXB == 0;
     static_assert(IPOOL <= 256, "places of the pool in 8 bits");

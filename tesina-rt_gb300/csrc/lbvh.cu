@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(256) k_radix_hist(const uint32_t* __restrict__
 // One radix pass of 8-bit digits; dynamic shared memory of sizeof(SortSmem).
 // MINB tiles resident per SM bound the registers: a pass whose tiles all fit in
 // one wave at 2 per SM runs the MINB = 2 instance (7 % faster per mid-scale
-// build), a longer one RT_SORT_MINB (3, 80 registers: the third tile hides
+// build), a longer one SORT_MINB (3, 80 registers: the third tile hides
 // latency).
 template <int MINB>
 __global__ void __launch_bounds__(SORT_THREADS, MINB) k_onesweep(
@@ -183,7 +183,7 @@ constexpr int kOneWaveMinB = 2;
 // The instance for a pass of `tiles` tiles on `sms` SMs.
 static auto onesweep_kernel(size_t tiles, int sms) {
     return tiles <= (size_t)kOneWaveMinB * (size_t)sms ? k_onesweep<kOneWaveMinB>
-                                                       : k_onesweep<RT_SORT_MINB>;
+                                                       : k_onesweep<SORT_MINB>;
 }
 
 // Self-test of the look-back timeout: one block sorts tile 1 of a pass
@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(T, T == EMIT_T_WIDE ? 2 : 1) k_emit_level(
 // index buffer, material map and upload ids in a build) and joins them with
 // their boxes still in registers, so no leaf AABB goes through memory.
 template <EmitSource SRC>
-__global__ void __launch_bounds__(EMIT_C0, RT_EMIT_MINB0) k_emit_level0(
+__global__ void __launch_bounds__(EMIT_C0, EMIT_MINB0) k_emit_level0(
     uint32_t n, const uint32_t* __restrict__ skeys, PermuteIO P, EmitItem* __restrict__ out,
     uint32_t* __restrict__ out_count, float4* __restrict__ nodes, int min_leaf, uint32_t leave,
     BvhHeader* __restrict__ hdr, uint32_t* __restrict__ status) {
@@ -272,7 +272,7 @@ static cudaError_t setup_kernels() {
     opt_in((const void*)k_emit_level<EMIT_T_WIDE>, sizeof(EmitSmem<EMIT_C1, EMIT_T_WIDE>));
     opt_in((const void*)k_emit_level<EMIT_T_NARROW>, sizeof(EmitSmem<EMIT_C1, EMIT_T_NARROW>));
     opt_in((const void*)k_onesweep<kOneWaveMinB>, sizeof(SortSmem));
-    opt_in((const void*)k_onesweep<RT_SORT_MINB>, sizeof(SortSmem));
+    opt_in((const void*)k_onesweep<SORT_MINB>, sizeof(SortSmem));
     if (e != cudaSuccess) return e;
     if (dev < 64) done |= 1ull << dev;
     return cudaSuccess;

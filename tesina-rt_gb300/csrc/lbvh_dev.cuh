@@ -13,15 +13,10 @@
 
 namespace rt {
 
-#ifndef RT_SORT_MINB
-#define RT_SORT_MINB 3   // radix tiles resident per SM (register budget)
-#endif
+constexpr int SORT_MINB = 3;   // radix tiles resident per SM (register budget)
 constexpr int SORT_THREADS = 256;
 constexpr int SORT_WARPS = SORT_THREADS / 32;
-#ifndef RT_SORT_ITEMS
-#define RT_SORT_ITEMS 16   // keys per thread of a radix tile
-#endif
-constexpr int SORT_ITEMS = RT_SORT_ITEMS;
+constexpr int SORT_ITEMS = 16;   // keys per thread of a radix tile
 constexpr int SORT_TILE = SORT_THREADS * SORT_ITEMS;   // 4096 keys per tile
 constexpr uint32_t LB_AGG = 1u << 30, LB_PREFIX = 2u << 30, LB_MASK = (1u << 30) - 1;
 constexpr uint32_t LB_SPIN_LIMIT = 1u << 22;
@@ -30,10 +25,7 @@ constexpr uint32_t LB_SPIN_LIMIT = 1u << 22;
 // than it saves in round trips: 2 to 6 words measured best (32 words: a
 // build of 17.7 M triangles 7 % slower; a sleep between polls changed
 // nothing).
-#ifndef RT_LB_WINDOW
-#define RT_LB_WINDOW 4
-#endif
-constexpr int LB_WINDOW = RT_LB_WINDOW;
+constexpr int LB_WINDOW = 4;
 
 // float <-> order-preserving uint32 (min/max of the integers == fmin/fmax of
 // the floats for non-NaN values).
@@ -188,11 +180,6 @@ __device__ __forceinline__ uint32_t block_excl_scan_256(uint32_t v, uint32_t* s_
     return before + x - v;
 }
 
-// Phase marks of a radix tile (k = 0..6), for timing harnesses; none by default.
-#ifndef RT_SORT_MARK
-#define RT_SORT_MARK(k)
-#endif
-
 template <int ITEMS>
 struct __align__(16) SortSmemT {
     uint32_t keys[SORT_THREADS * ITEMS];
@@ -241,7 +228,6 @@ __device__ __forceinline__ void onesweep_tile_body(SortSmemT<ITEMS>& S, uint32_t
                                                    uint32_t* __restrict__ failed) {
     constexpr uint32_t TILE = SORT_THREADS * ITEMS;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    RT_SORT_MARK(0);
     const uint32_t base = tile * TILE;                 // n < 2^30
     const uint32_t valid = WHOLE ? TILE : n - base;    // keys of this tile
     const uint32_t mine = (uint32_t)warp * (ITEMS * 32) + lane;   // this thread's first key
@@ -303,7 +289,6 @@ __device__ __forceinline__ void onesweep_tile_body(SortSmemT<ITEMS>& S, uint32_t
     }
     __syncthreads();
 
-    RT_SORT_MARK(1);
     // thread tid's digit: counts of the warps, summed in warp order
     uint32_t cnt = 0;
 #pragma unroll
@@ -346,7 +331,6 @@ __device__ __forceinline__ void onesweep_tile_body(SortSmemT<ITEMS>& S, uint32_t
     // count), so relaxed accesses suffice; the words of LB_WINDOW earlier
     // tiles are read per round trip and summed nearest first, up to the first
     // inclusive prefix or the first tile that has not published.
-    RT_SORT_MARK(2);
     if (tile > 0) {
         uint32_t spins = 0;
         bool open = true;   // no inclusive prefix yet
@@ -376,10 +360,8 @@ __device__ __forceinline__ void onesweep_tile_body(SortSmemT<ITEMS>& S, uint32_t
         }
         st_relaxed(my, LB_PREFIX | (excl + cnt));
     }
-    RT_SORT_MARK(3);
     S.goff[tid] = excl - lstart;
     __syncthreads();
-    RT_SORT_MARK(4);
 #pragma unroll 4
     for (uint32_t i = tid; i < valid; i += SORT_THREADS) {
         const uint32_t key = S.keys[i];
@@ -389,7 +371,6 @@ __device__ __forceinline__ void onesweep_tile_body(SortSmemT<ITEMS>& S, uint32_t
             vout[dst] = S.vals[i];
         }
     }
-    RT_SORT_MARK(5);
 }
 
 // A caller that takes several tiles with one S has a barrier between them.
@@ -510,24 +491,11 @@ __device__ __forceinline__ uint64_t delta(const uint32_t* __restrict__ k, uint32
 // boundaries), so chunks and levels compose.
 // ---------------------------------------------------------------------------
 constexpr int EMIT_FMAX = 128;   // items a block may leave
-#ifndef RT_EMIT_GROUP
-#define RT_EMIT_GROUP 8
-#endif
-constexpr int EMIT_GROUP = RT_EMIT_GROUP;   // blocks of one level gathered by a block of the next
-
-#ifndef RT_EMIT_C0
-#define RT_EMIT_C0 512
-#endif
-#ifndef RT_EMIT_MINB0
-#define RT_EMIT_MINB0 3
-#endif
-#ifndef RT_EMIT_LEAVE0
-#define RT_EMIT_LEAVE0 128u   // runs a level-0 block may leave unjoined
-#endif
-#ifndef RT_EMIT_LEAVE1
-#define RT_EMIT_LEAVE1 64u    // the same above level 0
-#endif
-constexpr int EMIT_C0 = RT_EMIT_C0;                // triangles per level-0 block
+constexpr int EMIT_GROUP = 8;   // blocks of one level gathered by a block of the next
+constexpr uint32_t EMIT_LEAVE0 = 128u;   // runs a level-0 block may leave unjoined
+constexpr uint32_t EMIT_LEAVE1 = 64u;    // the same above level 0
+constexpr int EMIT_C0 = 512;             // triangles per level-0 block
+constexpr int EMIT_MINB0 = 3;            // level-0 blocks resident per SM (40 registers)
 constexpr int EMIT_C1 = EMIT_GROUP * EMIT_FMAX;    // items per block above level 0
 // Threads per block above level 0 (its warps take the items' chunks in
 // rounds): 256 in a level of more blocks than SMs, where two blocks per SM
@@ -547,7 +515,7 @@ __host__ __device__ __forceinline__ uint32_t emit_next_level(uint32_t nb) {
 // Runs a block of a level with `blocks` blocks may leave unjoined (a level of
 // one block is the root's and joins everything).
 __host__ __device__ __forceinline__ uint32_t emit_leave(int level, uint32_t blocks) {
-    return blocks > 1 ? (level == 0 ? RT_EMIT_LEAVE0 : RT_EMIT_LEAVE1) : 32u;
+    return blocks > 1 ? (level == 0 ? EMIT_LEAVE0 : EMIT_LEAVE1) : 32u;
 }
 
 // An item: leaf range, keys at its ends, box, ref / count, and the augmented
