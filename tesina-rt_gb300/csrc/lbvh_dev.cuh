@@ -54,7 +54,12 @@ __device__ __forceinline__ void st_relaxed(uint32_t* p, uint32_t v) {
 // start while their predecessor still runs, so its results are not read-only
 // for the kernel's lifetime, as the non-coherent loads that __ldg and const
 // __restrict__ give require: such a load may be moved above the wait for the
-// predecessor.  A volatile asm stays behind it.
+// predecessor.  A volatile asm stays behind it.  What the build's kernels read of
+// one another goes through these: bounds (morton_params), digit counts (tile 0 of
+// a pass), sorted keys, order, item counts and items, the header's status.  The
+// radix tiles' keys and values are read at places that follow from a counter
+// taken after the wait; vertices, indices, materials and ids are no kernel's of
+// the build.
 __device__ __forceinline__ uint32_t ld_dep(const uint32_t* p) {
     uint32_t v;
     asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
@@ -609,11 +614,16 @@ __device__ __forceinline__ void read_item(const EmitItem* p, WarpItem& w) {
 // Shared scratch of one warp for warp_join, 2048 bytes.  st is a sparse table of one axis of
 // the items' boxes (level t at start i: min / max over items i .. i+2^t-1);
 // the arrays hold the items' ranges, end keys and references.  At the end
-// the first 1536 bytes hand the runs left over to the lanes they start at.
+// `stage`, in the same space, hands the runs left over to the lanes they start at.
 struct __align__(16) WarpScratch {
-    float2 st[5][32];
-    uint32_t il[32], ir[32], ikl[32], ikr[32];
-    int32_t iref[32], icnt[32];
+    union {
+        struct {
+            float2 st[5][32];
+            uint32_t il[32], ir[32], ikl[32], ikr[32];
+            int32_t iref[32], icnt[32];
+        };
+        float4 stage[3][32];
+    };
 };
 
 // Level of a boundary delta: its highest set bit (the radix tree's level),
@@ -682,7 +692,7 @@ __device__ __forceinline__ float2 axis_range(const WarpScratch& W, uint32_t a, u
 template <bool TRIS>
 __device__ __forceinline__ bool warp_join(WarpItem& it, uint32_t cnt, uint64_t edge, uint32_t n,
                                           int min_leaf, float4* __restrict__ nodes,
-                                          float4* __restrict__ tris, WarpScratch& W,
+                                          float4* tris, WarpScratch& W,
                                           BvhHeader* __restrict__ hdr) {
     const uint32_t lane = threadIdx.x & 31u;
     const unsigned FULL = 0xffffffffu;
@@ -846,19 +856,18 @@ __device__ __forceinline__ bool warp_join(WarpItem& it, uint32_t cnt, uint64_t e
     }
     // hand each run left over to the lane of its first item
     const uint32_t keep = __reduce_or_sync(FULL, out ? (1u << A) : 0u);
-    float4* stage = reinterpret_cast<float4*>(&W);
     __syncwarp();   // every read of the scratch is done
     if (out) {
-        stage[A] = q0;
-        stage[32 + A] = q1;
-        stage[64 + A] = q2;
+        W.stage[0][A] = q0;
+        W.stage[1][A] = q1;
+        W.stage[2][A] = q2;
     }
     __syncwarp();
     const bool mine = (keep >> lane) & 1u;
     if (mine) {
-        q0 = stage[lane];
-        q1 = stage[32 + lane];
-        q2 = stage[64 + lane];
+        q0 = W.stage[0][lane];
+        q1 = W.stage[1][lane];
+        q2 = W.stage[2][lane];
         it.l = __float_as_uint(q0.x);
         it.r = __float_as_uint(q0.y);
         it.kl = __float_as_uint(q0.z);
@@ -927,6 +936,9 @@ __device__ __forceinline__ uint32_t gather_runs(EmitSmem<C, T>& S, const WarpIte
 // keys would give nodes that are their own descendants: the triangles then keep
 // their order, and the tree is the leaf of triangle 0 alone, so that whatever
 // reads it before the caller has seen RT_DEV_TIMEOUT stays in range and ends.
+//
+// `tris` is not __restrict__: at level 0 it is `perm.tris`, whose records the
+// marks are written into.
 enum EmitSource { EMIT_ITEMS, EMIT_PERMUTE, EMIT_REFIT };
 template <int C, int T, EmitSource SRC = EMIT_ITEMS>
 __device__ __forceinline__ void emit_level(EmitSmem<C, T>& S, uint32_t blk, uint32_t n,
@@ -936,7 +948,7 @@ __device__ __forceinline__ void emit_level(EmitSmem<C, T>& S, uint32_t blk, uint
                                            uint32_t n_in, EmitItem* __restrict__ out,
                                            uint32_t* __restrict__ out_count,
                                            float4* __restrict__ nodes,
-                                           float4* __restrict__ tris, int min_leaf,
+                                           float4* tris, int min_leaf,
                                            uint32_t leave, BvhHeader* __restrict__ hdr,
                                            uint32_t* __restrict__ status,
                                            const PermuteIO& perm = PermuteIO{}) {
