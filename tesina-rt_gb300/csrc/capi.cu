@@ -1218,7 +1218,8 @@ int32_t rt_autotune_render(rt_ctx* c, rt_scene* s, const rt_camera* cam, int32_t
     a.cam = *cam;
     a.width = w;
     a.height = h;
-    a.max_bounces = max_bounces;
+    // rt_render takes 0 to 64 bounces, which is what the kernels count to
+    a.max_bounces = max_bounces = std::min(std::max(max_bounces, 0), 64);
     a.inv1e6 = c->inv1e6;
     a.rgba = rgba;
     a.image_rgb = nullptr;
