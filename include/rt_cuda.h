@@ -314,8 +314,8 @@ RT_API int32_t rt_bvh_refit_lbvh(rt_ctx* ctx, rt_scene* scene, rt_stream s);
  * scene's triangles in their current order, built on the host's threads and
  * laid out as the LBVH's device tree (the triangles reordered likewise), so
  * that every render call traverses it; returns when it is on the device.
- * RT_ERR_INVALID when an interior node lies deeper than the traversal's
- * 32-entry stack; such a tree cannot be refit (build it again). */
+ * RT_ERR_INVALID when an interior node lies deeper than the 32 levels that
+ * the traversals' stacks are sized for; such a tree cannot be refit (build it again). */
 RT_API int32_t rt_bvh_build_sah(rt_ctx* ctx, rt_scene* scene, rt_stream s);
 /* Canonical pre-order tree (synchronous).  *count receives the node count;
  * pass out == NULL to query it. */
@@ -384,8 +384,9 @@ typedef struct rt_render_config {
     int32_t blocks_per_sm;   /* resident blocks per SM to launch; 0 = chosen by the frame's
                               * size, up to the occupancy maximum (with the default variant a
                               * small frame then takes the kernel with four lanes per pixel) */
-    int32_t chunk;           /* pixels per warp work fetch: 32, 64, 128 or 256          */
-    int32_t stack_depth;     /* traversal stack entries (fixed: 32, enough for depth <= 31) */
+    int32_t chunk;           /* pixels per warp work fetch: 32, 64, 128 or 256 (the kernel
+                              * with four lanes per pixel fetches 1 to 8, by the frame's size) */
+    int32_t stack_depth;     /* 32, the deepest path of a tree; nothing else is taken */
 } rt_render_config;
 
 RT_API int32_t rt_render_variants(int32_t* count);

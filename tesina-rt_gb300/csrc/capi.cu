@@ -812,7 +812,7 @@ int32_t rt_bvh_build_sah(rt_ctx* c, rt_scene* s, rt_stream stream) {
                                  hw ? (int)std::min(hw, 64u) : 1, &t);
     if (rc == -2)
         return fail(RT_ERR_INVALID, "rt_bvh_build_sah: the tree is deeper than the traversal's "
-                    "32-entry stack");
+                    "32 levels");
     if (rc) return fail(RT_ERR_INVALID, "rt_bvh_build_sah: vertex index out of range");
     rt::LbvhArgs a = lbvh_args(c, s);
     CU(cudaMemcpyAsync(s->d_vals_sorted, t.order.data(), 4 * (size_t)s->N, cudaMemcpyHostToDevice,
@@ -1241,6 +1241,8 @@ int32_t rt_autotune_render(rt_ctx* c, rt_scene* s, const rt_camera* cam, int32_t
             for (int bj = 0; bj < bi; ++bj) seen = seen || bps_list[bj] == bps_list[bi];
             if (seen) continue;
             for (int ch : chunks) {
+                // four lanes per pixel: the share of a warp follows from the frame alone
+                if (rt::render_variant_quad(v) && ch != chunks[0]) continue;
                 rt_render_config cfg = {v, bps_list[bi], ch, 32};
                 std::vector<float> ts;
                 for (int t = 0; t < trials + 1; ++t) {   // the first launch warms caches

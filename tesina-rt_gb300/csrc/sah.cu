@@ -83,7 +83,7 @@ struct TNode {
     bool leaf;
 };
 
-constexpr uint32_t kMaxInteriorDepth = 31;   // the traversal's 32-entry stack
+constexpr uint32_t kMaxInteriorDepth = 31;   // 32 levels: the paths that the traversals' stacks are sized for
 
 struct Builder {
     const std::vector<Box>& boxes;

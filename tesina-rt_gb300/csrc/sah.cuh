@@ -21,7 +21,7 @@ struct SahTree {
 // The reference's CPU SAH BVH over N triangles (idx, 3 per triangle, into V
 // float4 positions) in their current order, subtrees built on `threads`
 // host threads.  0 on success, -1 for invalid input, -2 when an interior
-// node would lie deeper than the traversal's 32-entry stack reaches.
+// node would lie deeper than the 32 levels that the traversals' stacks are sized for.
 int sah_build(const float4* pos, uint32_t V, const uint32_t* idx, uint32_t N, int threads,
               SahTree* out);
 

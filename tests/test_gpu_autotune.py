@@ -38,3 +38,17 @@ def test_autotune_depth_is_bounded(ctx, bounces):
     ctx.set_render_config(saved.variant, saved.blocks_per_sm, saved.chunk)
     assert ctx.device_status() == 0
     g.close()
+
+
+def test_autotune_reports_the_chunk_in_use(ctx):
+    """The kernel with four lanes per pixel shares a frame out by its size: the
+    tuner tries it with one chunk and reports that one."""
+    g = capi.Scene(ctx, scenes.soup(3000, seed=8))
+    g.build(30, 1)
+    saved = ctx.render_config()
+    quad = len(ctx.variants()) - 1
+    for w, h in ((16, 16), (40, 24), (64, 64)):
+        cfg, ms = g.autotune(scenes.camera((0, 0, -4), (0, 0, 0), aspect=w / h), w, h, 3, trials=5)
+        assert ms > 0 and (cfg.variant != quad or cfg.chunk == 32)
+    ctx.set_render_config(saved.variant, saved.blocks_per_sm, saved.chunk)
+    g.close()
