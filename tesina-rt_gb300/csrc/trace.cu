@@ -693,12 +693,14 @@ __global__ void __launch_bounds__(128) k_trace(SceneView S, const rt_sample* __r
     if (threadIdx.x == 0) sH = *S.hdr;
     __syncthreads();
     const int lane = threadIdx.x & 31, ray_of = threadIdx.x / (32 / RAYS);   // in the block
-    const int base = blockIdx.x * 4 * per + threadIdx.x / 32 * per, i = base + ray_of % RAYS;
+    const int base = blockIdx.x * 4 * per + threadIdx.x / 32 * per;
     if (base >= n) return;
-    n = min(n, base + per);
+    n = min(per, n - base);   // this warp's rays (n may be the largest int)
+    const int i = ray_of % RAYS;
     float* sm = stage + ray_of * STAGE_PITCH;
     float* warp = sm - ray_of % RAYS * STAGE_PITCH;
-    stage_in<20, RAYS>(warp, smp + base, min(RAYS, n - base));
+    hits += base;
+    stage_in<20, RAYS>(warp, smp + base, n);
     const rt_ray& ray = *reinterpret_cast<const rt_ray*>(sm);
     const f3 o = f3_of(ray.ori), d = f3_of(ray.dir);
     bool hit = false;
@@ -723,7 +725,7 @@ __global__ void __launch_bounds__(128) k_trace(SceneView S, const rt_sample* __r
             hits[i].hit = 0;
         }
     }
-    stage_out<16, RAYS>(warp, hits + base, __ballot_sync(0xffffffffu, hit));
+    stage_out<16, RAYS>(warp, hits, __ballot_sync(0xffffffffu, hit));
 }
 
 template <bool QUAD>
@@ -736,11 +738,13 @@ __global__ void __launch_bounds__(128) k_shadow(SceneView S, rt_lights Ls, int n
     if (threadIdx.x == 0) sH = *S.hdr;
     __syncthreads();
     const int lane = threadIdx.x & 31, ray_of = threadIdx.x / (32 / RAYS);   // in the block
-    const int base = blockIdx.x * 4 * per + threadIdx.x / 32 * per, i = base + ray_of % RAYS;
+    const int base = blockIdx.x * 4 * per + threadIdx.x / 32 * per;
     if (base >= n) return;
-    n = min(n, base + per);
+    n = min(per, n - base);   // this warp's rays (n may be the largest int)
+    const int i = ray_of % RAYS;
     const float* sm = stage + ray_of * STAGE_PITCH;
-    stage_in<16, RAYS>(stage + (ray_of - ray_of % RAYS) * STAGE_PITCH, hits + base, min(RAYS, n - base));
+    hits += base;
+    stage_in<16, RAYS>(stage + (ray_of - ray_of % RAYS) * STAGE_PITCH, hits, n);
     const rt_hit& h = *reinterpret_cast<const rt_hit*>(sm);
     const bool hit = i < n && h.hit;
     const f3 hp = f3_of(h.hit_point);
