@@ -380,10 +380,12 @@ RT_API int32_t rt_render(rt_ctx* ctx, rt_scene* scene, const rt_camera* cam, int
  * the register budget (minimum resident blocks per SM), the number of
  * resident blocks launched, and the pixels a warp takes per work fetch. */
 typedef struct rt_render_config {
-    int32_t variant;         /* kernel variant, 0 .. rt_render_variants() - 1           */
+    int32_t variant;         /* kernel variant, 0 .. rt_render_variants() - 1; the last, the
+                              * default, is not a kernel of its own: a small frame takes the one
+                              * with four lanes per pixel, a larger one the pooled one that
+                              * rt_render_variant_info reports for it */
     int32_t blocks_per_sm;   /* resident blocks per SM to launch; 0 = chosen by the frame's
-                              * size, up to the occupancy maximum (with the default variant a
-                              * small frame then takes the kernel with four lanes per pixel) */
+                              * size, up to the occupancy maximum */
     int32_t chunk;           /* pixels per warp work fetch: 32, 64, 128 or 256 (the kernel
                               * with four lanes per pixel fetches 1 to 8, by the frame's size) */
     int32_t stack_depth;     /* 32, the deepest path of a tree; nothing else is taken */

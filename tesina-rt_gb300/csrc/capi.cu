@@ -1045,18 +1045,17 @@ int32_t rt_fb_copy(rt_ctx* c, const uint32_t* img, uint8_t* rgba, size_t px, rt_
 static cudaError_t launch_render_cfg(rt_ctx* c, rt::RenderArgs a, rt_render_config cfg,
                                      cudaStream_t cs) {
     const int64_t pixels = (int64_t)a.width * a.height;
-    // The default configuration leaves the kernel open: a frame too small to fill
-    // the SMs goes to the one with four lanes per pixel.  Against the pooled kernel
-    // on 362 x 362 (just above the line): 1k triangles 55 -> 57 us, 10k 217 -> 171,
-    // 200k 286 -> 250, 1.2 M 553 -> 471; on 512 x 512 61 -> 78, 233 -> 253, 355 -> 359,
-    // 701 -> 738.
-    if (cfg.variant == kDefaultVariant && cfg.blocks_per_sm == 0 &&
-        pixels <= (int64_t)rt::kQuadRaysPerSm * c->num_sms)
-        cfg.variant = rt::render_quad_variant();
+    // The default leaves the kernel open: a frame too small to fill the SMs goes to
+    // the one with four lanes per pixel.  Against the pooled kernel on 362 x 362
+    // (just above the line): 1k triangles 55 -> 57 us, 10k 217 -> 171, 200k 286 ->
+    // 250, 1.2 M 553 -> 471; on 512 x 512 61 -> 78, 233 -> 253, 355 -> 359, 701 -> 738.
+    if (cfg.variant == rt::kAutoVariant)
+        cfg.variant = pixels <= (int64_t)rt::kQuadRaysPerSm * c->num_sms ? rt::kQuadVariant
+                                                                         : rt::kPoolVariant;
     int threads = 0, minb = 0;
     const void* fn = nullptr;
     rt::render_variant_info(cfg.variant, &threads, &minb, &fn);
-    if (rt::render_variant_quad(cfg.variant)) {
+    if (cfg.variant == rt::kQuadVariant) {
         // fewer than eight pixels to a warp as long as that leaves no more than
         // 32 warps per SM (64 x 64 of 10k triangles: 8 pixels 103 us, 4 with a line
         // at 16 warps 83, 2 at 32 warps 64)
@@ -1230,6 +1229,7 @@ int32_t rt_autotune_render(rt_ctx* c, rt_scene* s, const rt_camera* cam, int32_t
     float bestt = 1e30f;
     const int chunks[] = {32, 64, 128};
     for (int v = 0; v < rt::render_variant_count(); ++v) {
+        if (v == rt::kAutoVariant) continue;   // two of the others
         if (rt::render_variant_refracts(v) != s->refracts) continue;   // the variants that fit the scene
         if (!rt::render_variant_fits(v, max_bounces)) continue;
         // full residency, one and two blocks fewer (more L1 per block:
@@ -1242,7 +1242,7 @@ int32_t rt_autotune_render(rt_ctx* c, rt_scene* s, const rt_camera* cam, int32_t
             if (seen) continue;
             for (int ch : chunks) {
                 // four lanes per pixel: the share of a warp follows from the frame alone
-                if (rt::render_variant_quad(v) && ch != chunks[0]) continue;
+                if (v == rt::kQuadVariant && ch != chunks[0]) continue;
                 rt_render_config cfg = {v, bps_list[bi], ch, 32};
                 std::vector<float> ts;
                 for (int t = 0; t < trials + 1; ++t) {   // the first launch warms caches

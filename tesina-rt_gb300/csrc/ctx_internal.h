@@ -10,10 +10,6 @@
 #include "../../include/rt_cuda.h"
 #include "rt_internal.cuh"
 
-// The render variant of the default configuration.  With the residency left
-// open (0 blocks per SM) launch_render_cfg chooses by the size of the frame.
-constexpr int kDefaultVariant = 9;
-
 struct rt_ctx {
     int device = 0;
     int num_sms = 0;
@@ -52,10 +48,8 @@ struct rt_ctx {
     };
     std::map<cudaStream_t, HostRender> host_by_stream;
     float inv1e6 = 1.0f / 1e6f;
-    // until the autotuner or the caller picks one (k_render_pool<128, 8>: against
-    // k_render_pool<128, 6>, which holds 7 blocks, 4K of 17.7 M triangles 9.64 ->
-    // 9.28 ms, mid-scale frame 2.51 -> 2.46)
-    rt_render_config render_cfg = {kDefaultVariant, 0, 32, 32};
+    // until the autotuner or the caller picks one
+    rt_render_config render_cfg = {rt::kAutoVariant, 0, 32, 32};
     int variant_occupancy[rt::kMaxRenderVariants] = {0};   // resident blocks per SM per variant
     int variant_carveout[rt::kMaxRenderVariants];          // shared-memory carveout set (%), -1 unset
     int smem_per_sm = 0;                            // bytes of shared memory an SM offers

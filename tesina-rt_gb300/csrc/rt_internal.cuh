@@ -60,10 +60,13 @@ struct TriRec {
     float4 v0, e1, e2;
 };
 
-// Views passed to kernels.
 // Render kernel variants a context keeps per-variant state for.
 constexpr int kMaxRenderVariants = 32;
+// The pooled kernel of large frames, the one with four lanes per pixel, and the
+// choice between them by the size of the frame, which is the default.
+constexpr int kPoolVariant = 9, kQuadVariant = 15, kAutoVariant = 16;
 
+// Views passed to kernels.
 struct SceneView {
     const float4* __restrict__ nodes;     // 8 float4 per record
     const float4* __restrict__ tris;      // 3 float4 per triangle

@@ -965,9 +965,14 @@ static const RenderVariant kVariants[] = {
     {128, 4, k_render_pool_refr<128, 4, 6>, true, true, 6},
     {128, 5, k_render_pool_refr<128, 5, 4>, true, true, 4},
     {128, 6, k_render_quad<128, 6>, false},
+    // by the frame's size k_render_quad or this (against k_render_pool<128, 6>,
+    // which holds 7 blocks, 4K of 17.7 M triangles 9.64 -> 9.28 ms, mid-scale
+    // frame 2.51 -> 2.46)
+    {128, 8, k_render_pool<128, 8>, true},
 };
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
-constexpr int kQuadVariant = kNumVariants - 1;
+static_assert(kAutoVariant == kNumVariants - 1 && kQuadVariant == kNumVariants - 2 && kPoolVariant == 9,
+              "the variants' numbers");
 static_assert(kNumVariants <= kMaxRenderVariants, "per-variant context arrays");
 
 int render_variant_count() { return kNumVariants; }
@@ -982,8 +987,6 @@ int render_variant_info(int v, int* threads, int* min_blocks, const void** fn) {
 
 bool render_variant_pooled(int v) { return v >= 0 && v < kNumVariants && kVariants[v].pooled; }
 
-bool render_variant_quad(int v) { return v == kQuadVariant; }
-
 bool render_variant_sums(int v) { return v >= 0 && v < kNumVariants && kVariants[v].sums(); }
 
 bool render_variant_refracts(int v) { return v >= 0 && v < kNumVariants && kVariants[v].refract; }
@@ -992,8 +995,6 @@ bool render_variant_fits(int v, int max_bounces) {
     if (v < 0 || v >= kNumVariants) return false;
     return kVariants[v].max_bounces == 0 || max_bounces <= kVariants[v].max_bounces;
 }
-
-int render_quad_variant() { return kQuadVariant; }
 
 int render_refract_variant(int max_bounces) {
     // the pooled variant with the smallest pool that holds the frame, else

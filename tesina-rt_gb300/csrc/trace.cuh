@@ -32,12 +32,10 @@ int render_variant_info(int v, int* threads, int* min_blocks, const void** fn);
 // way at once).
 bool render_variant_pooled(int v);
 bool render_variant_sums(int v);
-// The variant with four lanes per pixel, k_render_quad: `chunk` is its pixels per
-// warp, one to eight.  Trace launches and frames of up to kQuadRaysPerSm rays or
-// pixels per SM run by four lanes.
+// Trace launches of up to kQuadRaysPerSm rays per SM, and frames of as many pixels
+// where the variant is kAutoVariant, run by four lanes per ray.  k_render_quad's
+// `chunk` is its pixels per warp, one to eight.
 constexpr int kQuadRaysPerSm = 768;
-bool render_variant_quad(int v);
-int render_quad_variant();
 // True for the variants that follow refracted rays; the scenes with
 // refracting materials render with one of them.
 bool render_variant_refracts(int v);
