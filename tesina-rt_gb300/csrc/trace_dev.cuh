@@ -73,7 +73,8 @@ __device__ __forceinline__ void leaf_closest(const SceneView& S, const TRay& r, 
                                              Hit& best) {
     auto test = [&](const TriRec& T, int32_t id, bool valid) {
         float t, u, v;
-        const bool h = mt(T, r.o, r.d, t, u, v) & (t <= best.t) & (t >= r.tmin) & valid;
+        bool h = mt(T, r.o, r.d, t, u, v);   // before t is read: & does not order its operands
+        h = h & (t <= best.t) & (t >= r.tmin) & valid;
         best.id = h ? id : best.id;
         best.t = h ? t : best.t;
         best.u = h ? u : best.u;
@@ -98,19 +99,23 @@ __device__ __forceinline__ void leaf_closest(const SceneView& S, const TRay& r, 
 
 template <bool PAIR>
 __device__ __forceinline__ bool leaf_any(const SceneView& S, const TRay& r, int32_t i, float tmax) {
+    auto test = [&](const TriRec& T) {
+        float t, u, v;
+        const bool h = mt(T, r.o, r.d, t, u, v);
+        return h & (t < tmax) & (t > r.tmin);
+    };
     bool more, hit;
     do {
         const TriRec A = load_tri(S.tris, i);
         more = A.v0.w != 0.0f;
-        float t, u, v;
         if (PAIR) {
             const TriRec B = load_tri(S.tris, i + 1);
-            hit = mt(A, r.o, r.d, t, u, v) & (t < tmax) & (t > r.tmin);
-            hit = hit | (mt(B, r.o, r.d, t, u, v) & (t < tmax) & (t > r.tmin) & more);
+            hit = test(A);
+            hit = hit | (test(B) & more);
             more = more & (B.v0.w != 0.0f);
             i += 2;
         } else {
-            hit = mt(A, r.o, r.d, t, u, v) & (t < tmax) & (t > r.tmin);
+            hit = test(A);
             ++i;
         }
     } while (more & !hit);

@@ -21,7 +21,9 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 # host code as the device code: no fused multiply-add (gcc contracts by default
 # where the machine has FMA, as the Arm hosts do)
 FLAGS = ARCH + ["-O3", "-lineinfo", "--fmad=false", "-std=c++17", "-Xcompiler", "-fPIC",
-                "-Xcompiler", "-fvisibility=hidden", "-Xcompiler", "-ffp-contract=off"]
+                "-Xcompiler", "-fvisibility=hidden", "-Xcompiler", "-ffp-contract=off",
+                # "used before its value is set": in a & b, b may be evaluated first
+                "-diag-error", "549"]
 
 
 def _run(cmd):
