@@ -346,7 +346,8 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_pool(RenderArgs a) {
             },
             [&](int k, int l) {
                 const int j = Q.hslot[k];
-                if (occluded(S, H, sL.light[l], mk3(Q.ro[0][j], Q.ro[1][j], Q.ro[2][j]), a.status))
+                if (occluded<false, false, true>(S, H, sL.light[l],
+                                                 mk3(Q.ro[0][j], Q.ro[1][j], Q.ro[2][j]), a.status))
                     atomicOr(&Q.hmask[k], 1u << l);
             });
         __syncwarp();
@@ -711,7 +712,7 @@ __global__ void __launch_bounds__(128) k_trace(SceneView S, const rt_sample* __r
         if (QUAD)
             h = closest_hit_quad(S, sH, r, tmax, i < n, stacks[QUAD ? ray_of : 0].e, status);
         else
-            h = closest_hit<true, true>(S, sH, r, tmax, status);
+            h = closest_hit<true, true, true>(S, sH, r, tmax, status);
         const bool mine = i < n && (!QUAD || lane % 4 == 0);   // one lane writes
         hit = mine && h.id >= 0;
         if (hit) {
@@ -763,7 +764,7 @@ __global__ void __launch_bounds__(128) k_shadow(SceneView S, rt_lights Ls, int n
     }
     if (!hit) return;
     for (int l = 0; l < Ls.count; ++l)
-        if (occluded<true, true>(S, sH, Ls.light[l], hp, status)) mask |= 1u << l;
+        if (occluded<true, true, true>(S, sH, Ls.light[l], hp, status)) mask |= 1u << l;
     hits[i].shadow_hit = (uint8_t)mask;
 }
 

@@ -24,10 +24,15 @@
 // tests of the two levels, on lower corners that the minima give exactly.  A
 // pushed entry keeps its entry distance A and is dropped if A > tMax when
 // popped (tMax only shrinks, the far distances do not change).  Monotonicity
-// needs slabs without 0 * inf: a ray with an infinite inverse component, an
-// infinite or NaN origin, no usable axis or an infinite tMax (within which an
-// empty slot's box at infinity lies) is "careful": a search of its own takes
-// the two binary levels one at a time.
+// needs slabs without 0 * inf, and an empty slot's box at infinity must be out of
+// reach.  Rays for which that is not sure (careful_ray) have searches of their
+// own.  With an infinite inverse component, a ray parallel to an axis, a box that
+// passes has a parent that passes unless the box is flat in that axis and lies in
+// the ray's plane: the axis' slab is else no bound or empty, the parent's no bound
+// where the box's is, and A comes from the other axes.  Such rays take the same
+// steps until they meet a box of that kind (WIDE); from there on, and rays from
+// infinite or NaN origins and the like always, the two binary levels are taken one
+// at a time (BINARY).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -166,12 +171,54 @@ __device__ __forceinline__ bool slab_slot(const SlabRay& r, float tmax, const Sl
     return A <= B;
 }
 
-// Rays whose slab tests need not be monotone (see the top of the file).
+enum SearchKind { PLAIN, WIDE, BINARY };
+
+// slab_slot for rays parallel to an axis: an empty slot is no hit (tMax may be
+// infinite), and a hit sets `flat` if both slabs of an axis are NaN.  SHADOW:
+// slab_shadow's rule, by which 0 * inf at the lower corner takes the axis out.
+template <bool SHADOW>
+__device__ __forceinline__ bool slab_wide(const SlabRay& r, float tmax, const Slot& s, float& A,
+                                          float& B, bool& flat) {
+    const float2 l = add_mul2(make_float2(s.lox, s.loy), r.no_xy, r.iv_xy);
+    const float2 h = add_mul2(make_float2(s.hix, s.hiy), r.no_xy, r.iv_xy);
+    const float2 z = add_mul2(make_float2(s.loz, s.hiz), r.no_zz, r.iv_zz);
+    const float nx = fminf(l.x, h.x), ny = fminf(l.y, h.y), nz = fminf(z.x, z.y);
+    float fx = fmaxf(l.x, h.x), fy = fmaxf(l.y, h.y), fz = fmaxf(z.x, z.y);
+    float mx = nx, my = ny, mz = nz;
+    if (SHADOW) {
+        mx = l.x == l.x ? mx : l.x;
+        fx = l.x == l.x ? fx : l.x;
+        my = l.y == l.y ? my : l.y;
+        fy = l.y == l.y ? fy : l.y;
+        mz = z.x == z.x ? mz : z.x;
+        fz = z.x == z.x ? fz : z.x;
+    }
+    A = fmaxf(max3f(r.tmin, mx, my), mz);
+    B = fminf(min3f(tmax, fx, fy), fz);
+    const bool hit = (A <= B) & (s.aux != EMPTY_SLOT);
+    flat |= hit & ((nx != nx) | (ny != ny) | (nz != nz));
+    return hit;
+}
+
+// Rays whose slab tests need not be monotone (see the top of the file); those of
+// them for which a flat box is not the only reason; and rays whose bounds may take
+// in an empty slot's box.
+__device__ __forceinline__ bool finite_origin(const TRay& r) {
+    const float INF = __int_as_float(0x7f800000);
+    return fabsf(r.o.x) < INF && fabsf(r.o.y) < INF && fabsf(r.o.z) < INF;
+}
 __device__ __forceinline__ bool careful_ray(const TRay& r) {
     const float INF = __int_as_float(0x7f800000);
     const bool inf = fabsf(r.inv.x) == INF || fabsf(r.inv.y) == INF || fabsf(r.inv.z) == INF;
     const bool axis = r.inv.x == r.inv.x || r.inv.y == r.inv.y || r.inv.z == r.inv.z;
-    return inf || !axis || !(fabsf(r.o.x) < INF && fabsf(r.o.y) < INF && fabsf(r.o.z) < INF);
+    return inf || !axis || !finite_origin(r);
+}
+__device__ __forceinline__ bool binary_ray(const TRay& r) {
+    return !finite_origin(r) || !(r.tmin > -__int_as_float(0x7f800000));
+}
+__device__ __forceinline__ bool unbounded_ray(const TRay& r, float tmax) {
+    const float INF = __int_as_float(0x7f800000);
+    return !(tmax < INF) || !(r.tmin > -INF);
 }
 
 // The two binary children of a record in place of its four grandchildren:
@@ -228,14 +275,15 @@ __device__ __forceinline__ bool leaf_turn(unsigned group, int32_t next, bool& en
 // The steps branch as little as they can: a step is a chain of dependent
 // instructions, and each branch in it costs more than the selects that take
 // its place.  The rejections of mt(), a leaf's hit, an any-hit visit and the
-// pushes' conditions are selects, and `careful` is a template argument, so that
+// pushes' conditions are selects, and the kind is a template argument, so that
 // ordinary rays' code has none of its tests.  Together: mid-scale frame 2.87 ->
 // 2.51 ms, 4K of 17.7 M triangles 11.3 -> 9.7, glass 11.3 -> 9.3, 64 soups 7.8
 // -> 6.8, instances 2.04 -> 1.86, 10k-triangle frame 365 -> 322 us, thumbnail
 // 66 -> 52.  (Pushes that store always and move `sp` by the condition lose 4 %.)
-template <bool STAY, bool PAIR, bool careful>
+// WIDE: `flat` tells that the search was given up at a flat box.
+template <bool STAY, bool PAIR, SearchKind KIND>
 __device__ __forceinline__ Hit closest_search(const SceneView& S, const BvhHeader& H, const TRay& r,
-                                              float tmax, uint32_t* status) {
+                                              float tmax, uint32_t* status, bool& flat) {
     Hit best{-1, tmax, 0.f, 0.f};
     int2 st[STACK];   // code, entry distance
     int sp = 0;
@@ -263,17 +311,20 @@ __device__ __forceinline__ Hit closest_search(const SceneView& S, const BvhHeade
                        fminf(s2.lox, s3.lox), fminf(s2.loy, s3.loy), fminf(s2.loz, s3.loz));
         const bool ll_first = near_first(r.d, s0.lox, s0.loy, s0.loz, s1.lox, s1.loy, s1.loz);
         const bool rl_first = near_first(r.d, s2.lox, s2.loy, s2.loz, s3.lox, s3.loy, s3.loz);
-        if (careful) {
+        if (KIND == BINARY) {
             binary_step(s0, s1);
             binary_step(s2, s3);
         }
         float a0, a1, a2, a3, far;
-        if (!slab_slot(w, best.t, s0, a0, far)) a0 = MISS;
-        if (!slab_slot(w, best.t, s1, a1, far) || careful) a1 = MISS;
-        if (!slab_slot(w, best.t, s2, a2, far)) a2 = MISS;
-        if (!slab_slot(w, best.t, s3, a3, far) || careful) a3 = MISS;
+        auto test = [&](const Slot& s, float& a) {
+            return KIND == WIDE ? slab_wide<false>(w, best.t, s, a, far, flat) : slab_slot(w, best.t, s, a, far);
+        };
+        if (!test(s0, a0)) a0 = MISS;
+        if (!test(s1, a1) || KIND == BINARY) a1 = MISS;
+        if (!test(s2, a2)) a2 = MISS;
+        if (!test(s3, a3) || KIND == BINARY) a3 = MISS;
         int32_t c0 = s0.code, c1 = s1.code, c2 = s2.code, c3 = s3.code;
-        // careful: slot 0 before slot 1 whatever the (meaningless) inner test says
+        // BINARY: slot 0 before slot 1 whatever the (meaningless) inner test says
         swap_if(!ll_first, c0, c1, a0, a1);
         swap_if(!rl_first, c2, c3, a2, a3);
         swap_if(!l_first, c0, c2, a0, a2);
@@ -287,6 +338,7 @@ __device__ __forceinline__ Hit closest_search(const SceneView& S, const BvhHeade
         if (h1 & h0) st[sp++] = make_int2(c1, __float_as_int(a1));
         next = h0 ? c0 : h1 ? c1 : h2 ? c2 : h3 ? c3 : NO_NODE;
         if (next == NO_NODE) pop();
+        if (KIND == WIDE && flat) next = NO_NODE;
     };
     for (;;) {
         if (next >= 0) node(next);
@@ -303,7 +355,15 @@ __device__ __forceinline__ Hit closest_search(const SceneView& S, const BvhHeade
     }
 }
 
-template <bool STAY, bool PAIR>
+// PARALLEL (closest_hit): for the callers' own rays, which may have any bounds and
+// all be parallel to an axis; camera rays and reflections seldom are, and their
+// bounds are given.  PARALLEL (any_hit): the shadow rays of a directional light may be
+// too.  By levels and WIDE, ordinary rays beside them: trace of 4 M rays over 10k
+// triangles 2140 -> 1552 us (1493), shadows of 4 M hits 445 -> 310 (285), 3840 x
+// 2160 of a 20k-triangle field under a light straight above 1298 -> 1088 (1007).  A
+// third search costs other rays 0.6-1.6 % in the glass, instanced, batched and
+// one-path-per-lane kernels: such rays go by levels there.
+template <bool STAY, bool PAIR, bool PARALLEL = false>
 static __device__ Hit closest_hit(const SceneView& S, const BvhHeader& H, const TRay& r, float tmax,
                                   uint32_t* status) {
     Hit best{-1, tmax, 0.f, 0.f};
@@ -315,9 +375,15 @@ static __device__ Hit closest_hit(const SceneView& S, const BvhHeader& H, const 
         leaf_closest(S, r, H.root_ref, H.root_cnt, best);
         return best;
     }
-    if (careful_ray(r) || !(tmax < __int_as_float(0x7f800000)))
-        return closest_search<false, false, true>(S, H, r, tmax, status);
-    return closest_search<STAY, PAIR, false>(S, H, r, tmax, status);
+    bool flat = false;
+    if (careful_ray(r) || (PARALLEL ? unbounded_ray(r, tmax) : !(tmax < __int_as_float(0x7f800000)))) {
+        if (PARALLEL && !binary_ray(r)) {
+            best = closest_search<false, false, WIDE>(S, H, r, tmax, status, flat);
+            if (!flat) return best;
+        }
+        return closest_search<false, false, BINARY>(S, H, r, tmax, status, flat);
+    }
+    return closest_search<STAY, PAIR, PLAIN>(S, H, r, tmax, status, flat);
 }
 
 // Whether anything blocks the ray.  tMax does not shrink, so the order of
@@ -325,9 +391,9 @@ static __device__ Hit closest_hit(const SceneView& S, const BvhHeader& H, const 
 // it enters the one it crosses for longest, the likeliest to hold a blocker.
 // Against the last child first: 64 soups 9.29 -> 8.97 ms, glass 11.9 -> 11.7,
 // 4K of 17.7 M triangles 11.75 -> 11.60 (the nearest child first: 13.9).
-template <bool STAY, bool PAIR, bool careful>
+template <bool STAY, bool PAIR, SearchKind KIND>
 __device__ __forceinline__ bool any_search(const SceneView& S, const BvhHeader& H, const TRay& r,
-                                           float tmax, uint32_t* status) {
+                                           float tmax, uint32_t* status, bool& flat) {
     int32_t st[STACK];
     int sp = 0;
     bool over = false;
@@ -345,7 +411,7 @@ __device__ __forceinline__ bool any_search(const SceneView& S, const BvhHeader& 
         };
         over |= sp > STACK - 3;
         sp = min(sp, STACK - 3);
-        if (careful) {   // the shadow kernel's own NaN rules
+        if (KIND == BINARY) {   // the shadow kernel's own NaN rules
 #pragma unroll 1
             for (int k = 0; k < 4; k += 2) {
                 Slot a = load_slot(S.nodes, cur, k);
@@ -358,7 +424,8 @@ __device__ __forceinline__ bool any_search(const SceneView& S, const BvhHeader& 
             float longest = -1.f;   // of the children met so far: a hit's is >= 0
             auto visit = [&](const Slot& s) {
                 float A, B;
-                const bool hit = slab_slot(w, tmax, s, A, B);
+                const bool hit = KIND == WIDE ? slab_wide<true>(w, tmax, s, A, B, flat)
+                                              : slab_slot(w, tmax, s, A, B);
                 const float len = B - A;
                 const bool first = hit & (len > longest), push = hit & (longest >= 0.f);
                 const int32_t other = first ? next : s.code;
@@ -372,6 +439,7 @@ __device__ __forceinline__ bool any_search(const SceneView& S, const BvhHeader& 
             visit(s3);
         }
         if (next == NO_NODE && sp > 0) next = st[--sp];
+        if (KIND == WIDE && flat) next = NO_NODE;
     };
     for (;;) {
         if (next >= 0) node(next);
@@ -388,15 +456,22 @@ __device__ __forceinline__ bool any_search(const SceneView& S, const BvhHeader& 
     }
 }
 
-template <bool STAY, bool PAIR>
+template <bool STAY, bool PAIR, bool PARALLEL = false>
 static __device__ bool any_hit(const SceneView& S, const BvhHeader& H, const TRay& r, float tmax,
                                uint32_t* status) {
     if (!slab_shadow(r, tmax, H.root_lo.x, H.root_lo.y, H.root_lo.z, H.root_hi.x, H.root_hi.y,
                      H.root_hi.z))
         return false;
     if (H.root_cnt > 0) return leaf_any(S, r, H.root_ref, H.root_cnt, tmax);
-    if (careful_ray(r)) return any_search<false, false, true>(S, H, r, tmax, status);
-    return any_search<STAY, PAIR, false>(S, H, r, tmax, status);
+    bool flat = false;
+    if (careful_ray(r)) {
+        if (PARALLEL && !binary_ray(r)) {
+            const bool found = any_search<false, false, WIDE>(S, H, r, tmax, status, flat);
+            if (!flat) return found;
+        }
+        return any_search<false, false, BINARY>(S, H, r, tmax, status, flat);
+    }
+    return any_search<STAY, PAIR, PLAIN>(S, H, r, tmax, status, flat);
 }
 
 // Hit record of complete_trace_info.
@@ -442,14 +517,14 @@ __device__ __forceinline__ bool shadow_dir(const rt_light& L, f3 hp, f3& dir) {
     return true;
 }
 
-template <bool STAY = false, bool PAIR = false>
+template <bool STAY = false, bool PAIR = false, bool PARALLEL = false>
 __device__ __forceinline__ bool occluded(const SceneView& S, const BvhHeader& H, const rt_light& L,
                                          f3 hp, uint32_t* status) {
     f3 dir;
     if (!shadow_dir(L, hp, dir)) return true;
     const f3 inv = mk3(1.0f / dir.x, 1.0f / dir.y, 1.0f / dir.z);
     const TRay r = make_tray(hp, dir, inv, 0.01f);
-    return any_hit<STAY, PAIR>(S, H, r, 1e37f, status);
+    return any_hit<STAY, PAIR, PARALLEL>(S, H, r, 1e37f, status);
 }
 
 // Light direction (from the light toward the hit) and colour at a hit, as

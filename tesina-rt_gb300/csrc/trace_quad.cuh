@@ -203,11 +203,12 @@ __device__ __forceinline__ Hit closest_hit_quad(const SceneView& S, const BvhHea
     float A;
     live = live && slab(r, tmax, H.root_lo.x, H.root_lo.y, H.root_lo.z, H.root_hi.x, H.root_hi.y,
                         H.root_hi.z, A);
-    const bool careful = careful_ray(r) || !(tmax < __int_as_float(0x7f800000));
+    const bool careful = careful_ray(r) || unbounded_ray(r, tmax);
+    bool flat = false;
     if (live && H.root_cnt > 0)
         leaf_closest(S, r, H.root_ref, H.root_cnt, best);
     else if (live && careful)
-        best = closest_search<false, false, true>(S, H, r, tmax, status);
+        best = closest_search<false, false, BINARY>(S, H, r, tmax, status, flat);
     live = live && H.root_cnt <= 0 && !careful;
     __syncwarp();
     const Hit h = closest_quad(S, H.root_ref, r, tmax, live, st, status);
@@ -220,10 +221,11 @@ __device__ __forceinline__ bool any_hit_quad(const SceneView& S, const BvhHeader
     live = live && slab_shadow(r, tmax, H.root_lo.x, H.root_lo.y, H.root_lo.z, H.root_hi.x,
                                H.root_hi.y, H.root_hi.z);
     const bool careful = careful_ray(r);
+    bool flat = false;
     if (live && H.root_cnt > 0)
         found = leaf_any(S, r, H.root_ref, H.root_cnt, tmax);
     else if (live && careful)
-        found = any_search<false, false, true>(S, H, r, tmax, status);
+        found = any_search<false, false, BINARY>(S, H, r, tmax, status, flat);
     live = live && H.root_cnt <= 0 && !careful;
     __syncwarp();
     const bool f = any_quad(S, H.root_ref, r, tmax, live, st, status);
