@@ -463,7 +463,8 @@ typedef struct rt_server rt_server;
 enum { RT_REQ_RENDER = 0, RT_REQ_UPLOAD = 1 };
 
 typedef struct rt_server_cfg {
-    uint64_t hbm_budget_bytes;   /* resident scenes + framebuffer arena            */
+    uint64_t hbm_budget_bytes;   /* resident scenes + framebuffer arena + the scratch
+                                  * of builds in progress                          */
     uint64_t fb_arena_bytes;     /* device framebuffers of admitted requests        */
     int32_t  max_batch_views;    /* requests per render launch; 1 = plain path     */
     int32_t  max_inflight;       /* render launches on the GPU at once (streams)   */
@@ -491,7 +492,7 @@ typedef struct rt_request_info {
 
 typedef struct rt_server_stats {
     uint64_t completed, rejected, evicted, batches, rays, resident_scenes;
-    uint64_t resident_bytes;
+    uint64_t resident_bytes;     /* charged to hbm_budget_bytes                     */
     double   p50_ms, p99_ms, mean_batch_views, first_submit_ms, last_done_ms;
 } rt_server_stats;
 

@@ -100,6 +100,7 @@ struct ServedScene {
     rt_scene* scene = nullptr;
     rt_lights* d_lights = nullptr;
     uint64_t bytes = 0;
+    uint64_t building = 0;      // of them the build's own, given back when it is done
     int refs = 0;               // in-flight renders
     int pending = 0;            // queued renders not yet launched
     uint64_t last_use = 0;      // submission clock of the latest use
@@ -158,7 +159,8 @@ struct rt_server {
     std::deque<uint64_t> incoming;     // tickets in arrival order
     std::unordered_map<uint64_t, Req> reqs;
     std::map<uint64_t, ServedScene> scenes;
-    uint64_t resident_bytes = 0;
+    uint64_t resident_bytes = 0;       // charged to the budget
+    uint64_t building_bytes = 0;       // of them what builds in progress will give back
     // device resources
     Arena arena;
     uint8_t* d_fb = nullptr;
@@ -188,7 +190,13 @@ uint64_t scene_bytes(const rt_scene_desc* d) {
     const uint64_t V = d->vertex_count, N = d->triangle_count, M = d->material_count;
     return 32 * V + 40 * N + 32 * M       // geometry, both orders
            + N * (8 + 48 + 128)            // sorted keys and order, triangles, nodes
-           + 4096;                         // (a build's scratch goes back to the pool)
+           + 4096;
+}
+
+// What a scene's build takes besides, which goes back to the pool after it: radix
+// and emit scratch, unsorted keys.
+uint64_t build_bytes(const rt_scene_desc* d) {
+    return rt::lbvh_scratch_bytes(d->triangle_count, 4) + 4 * (uint64_t)d->triangle_count;
 }
 
 // Scene memory: a device pool that keeps what is freed for later uploads.
@@ -241,27 +249,45 @@ void evict(rt_server* S, uint64_t id) {
     S->up_cv.notify_all();
 }
 
-// Evicts least-recently-used idle scenes until `need` more bytes fit; evicts
-// nothing when even all idle scenes together would not make enough room.
-bool make_room(rt_server* S, uint64_t need) {
-    if (S->resident_bytes + need <= S->cfg.hbm_budget_bytes) return true;
+// Charges a scene's bytes, `building` of them for the time of its build.
+void charge(rt_server* S, uint64_t bytes, uint64_t building) {
+    S->resident_bytes += bytes;
+    S->building_bytes += building;
+}
+
+// Takes back the charge of a build that is done (its scene stays), or of a scene
+// that was not built.
+void uncharge(rt_server* S, uint64_t bytes, uint64_t building) {
+    S->resident_bytes -= bytes;
+    S->building_bytes -= building;
+    S->cv.notify_all();
+    S->done_cv.notify_all();   // rt_server_add_scene waits for room
+}
+
+// Evicts least-recently-used idle scenes until `need` more bytes fit, those that
+// builds in progress will give back being free; evicts nothing when even all idle
+// scenes together would not make enough room.
+enum Room { NO_ROOM, ROOM_LATER, ROOM };   // ROOM_LATER: once those builds are done
+Room make_room(rt_server* S, uint64_t need) {
+    const uint64_t budget = S->cfg.hbm_budget_bytes;
+    auto held = [&] { return S->resident_bytes - S->building_bytes; };
     uint64_t idle = 0;
     for (auto& kv : S->scenes) {
         const ServedScene& sc = kv.second;
         if (sc.ready && sc.refs == 0 && sc.pending == 0) idle += sc.bytes;
     }
-    if (S->resident_bytes - idle + need > S->cfg.hbm_budget_bytes) return false;
-    while (S->resident_bytes + need > S->cfg.hbm_budget_bytes) {
+    if (held() - idle + need > budget) return NO_ROOM;
+    while (held() + need > budget) {
         ServedScene* victim = nullptr;
         for (auto& kv : S->scenes) {
             ServedScene& sc = kv.second;
             if (!sc.ready || sc.refs > 0 || sc.pending > 0) continue;
             if (!victim || sc.last_use < victim->last_use) victim = &sc;
         }
-        if (!victim) return false;
+        if (!victim) return NO_ROOM;
         evict(S, victim->id);
     }
-    return true;
+    return S->resident_bytes + need <= budget ? ROOM : ROOM_LATER;
 }
 
 int32_t create_scene(rt_server* S, const rt_scene_desc* d, cudaStream_t stream, ServedScene* out) {
@@ -330,6 +356,9 @@ void retire(rt_server* S) {
         if (sc.ready || !sc.built) continue;
         if (cudaEventQuery(sc.built) != cudaSuccess) continue;
         sc.ready = true;
+        sc.bytes -= sc.building;
+        uncharge(S, sc.building, sc.building);
+        sc.building = 0;
         if (sc.upload_ticket) {
             Req& q = S->reqs[sc.upload_ticket];
             q.scene_id = sc.id;
@@ -485,22 +514,24 @@ void admit_uploads(rt_server* S) {
             keep.push_back(tk);
             continue;
         }
-        const uint64_t need = scene_bytes(q.r.upload);
-        if (!make_room(S, need)) {
-            if (S->inflight.empty()) {   // nothing will free memory: reject
+        const uint64_t extra = build_bytes(q.r.upload), need = scene_bytes(q.r.upload) + extra;
+        const Room room = make_room(S, need);
+        if (room != ROOM) {
+            if (room == NO_ROOM && S->inflight.empty()) {   // nothing will free memory: reject
                 S->scenes.erase(q.scene_id);   // its queued renders fail
                 finish(S, q, RT_ERR_REJECTED, now_ms());
                 S->done_cv.notify_all();
             } else {
-                keep.push_back(tk);      // retry when renders release scenes
+                keep.push_back(tk);      // retry when renders or builds release memory
             }
             continue;
         }
         ServedScene& sc = S->scenes[q.scene_id];
         sc.bytes = need;
+        sc.building = extra;
         sc.admitted = true;
         q.start_ms = now_ms();
-        S->resident_bytes += need;
+        charge(S, need, extra);
         UpJob j;
         j.ticket = tk;
         j.scene_id = q.scene_id;
@@ -544,7 +575,7 @@ void upload_loop(rt_server* S) {
                 cudaEventDestroy(made.built);
             }
             if (it != S->scenes.end()) {
-                S->resident_bytes -= it->second.bytes;
+                uncharge(S, it->second.bytes, it->second.building);
                 S->scenes.erase(it);
             }
             finish(S, S->reqs[j.ticket], r ? r : RT_ERR, now_ms());
@@ -696,12 +727,14 @@ int32_t rt_server_destroy(rt_server* S) {
 
 int32_t rt_server_add_scene(rt_server* S, const rt_scene_desc* d, uint64_t* id) {
     if (!S || !d || !id) return fail(RT_ERR_INVALID, "rt_server_add_scene: null argument");
-    const uint64_t need = scene_bytes(d);
+    const uint64_t extra = build_bytes(d), need = scene_bytes(d) + extra;
     std::unique_lock<std::mutex> lk(S->mu);
-    if (!make_room(S, need))
+    Room room;
+    while ((room = make_room(S, need)) == ROOM_LATER) S->done_cv.wait(lk);
+    if (room == NO_ROOM)
         return fail(RT_ERR_REJECTED, "rt_server_add_scene: %llu bytes exceed the budget",
                     (unsigned long long)need);
-    S->resident_bytes += need;   // reserved while the scene is built unlocked
+    charge(S, need, extra);   // reserved while the scene is built unlocked
     lk.unlock();
     ServedScene sc;
     int32_t r = create_scene(S, d, S->build_stream, &sc);
@@ -713,13 +746,14 @@ int32_t rt_server_add_scene(rt_server* S, const rt_scene_desc* d, uint64_t* id) 
     }
     lk.lock();
     if (r) {
-        S->resident_bytes -= need;
+        uncharge(S, need, extra);
         return r;
     }
+    uncharge(S, extra, extra);
     sc.id = S->next_scene++;
     sc.ready = true;
     sc.admitted = true;
-    sc.bytes = need;
+    sc.bytes = need - extra;
     sc.last_use = S->use_clock++;
     S->scenes[sc.id] = sc;
     *id = sc.id;
