@@ -15,18 +15,15 @@ from test_gpu_wide import _grid_scene, _samples
 pytestmark = pytest.mark.gpu
 
 
-def compare_both_sides(ctx, orc, sc, smp, min_leaf=1, scene=None):
+def compare_both_sides(ctx, orc, sc, smp, min_leaf=1):
     """The samples as they are (four lanes per ray) and repeated past 768 per SM (one
     lane per ray); the oracle traces them once.  Returns the number of hits."""
     n = smp.shape[0]
     line = 768 * torch.cuda.get_device_properties(0).multi_processor_count
     assert n <= line
-    if scene is None:
-        g, o = capi.Scene(ctx, sc), orc.new_scene(sc)
-        g.build(30, min_leaf)
-        o.build(30, min_leaf, 0)
-    else:
-        g, o = scene
+    g, o = capi.Scene(ctx, sc), orc.new_scene(sc)
+    g.build(30, min_leaf)
+    o.build(30, min_leaf, 0)
     ref = o.trace(smp)
     o.shadow(smp, ref)
     hit = ref["hit"] == 1
