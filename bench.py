@@ -43,11 +43,19 @@ B_RAY_CLOSEST, B_RAY_SHADOW, B_SHADE = 40, 25, 48
 # kernel on the mid-scale frame (ncu, --clock-control none), by kernel; the
 # line's roofline carries it only when the autotuner installed that kernel.
 RENDER_DRAM_BYTES = {
-    "k_render_pool<128, 8>": (157.0 + 12.5) * 1e6,
+    "k_render_pool<128, 6>": (153.3 + 8.5) * 1e6,
+    "k_render_pool<128, 8>": (157.4 + 9.9) * 1e6,
+    "k_render_pool<256, 3>": (147.8 + 7.3) * 1e6,
+    "k_render_pool<256, 4>": (157.4 + 9.9) * 1e6,
 }
 # the same for the stress workload (17.7 M triangles, 3840x2160, 3 lights,
-# depth 6): not measured since the records became four-wide
-STRESS_RENDER_DRAM_BYTES = {}
+# depth 6), mean over its poses
+STRESS_RENDER_DRAM_BYTES = {
+    "k_render_pool<128, 6>": (874.1 + 58.7) * 1e6,
+    "k_render_pool<128, 8>": (900.0 + 65.9) * 1e6,
+    "k_render_pool<256, 3>": (846.5 + 52.1) * 1e6,
+    "k_render_pool<256, 4>": (900.4 + 66.2) * 1e6,
+}
 
 
 def log(*a):
