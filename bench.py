@@ -654,8 +654,8 @@ def measure_instances(ctx, torch, frames=5):
 def measure_sah(ctx, torch, frames=5):
     """LBVH against the reference's CPU SAH BVH (rt_bvh_build_sah) on a
     1M-triangle soup (the small workload's kind of scene; the mid-scale
-    terrain's SAH tree is 36 levels deep, beyond the traversal's 32-entry
-    stack, and is refused): the SAH build's wall time (device to host copy,
+    terrain's SAH tree is 36 levels deep, more than the traversals take,
+    and is refused): the SAH build's wall time (device to host copy,
     the host build on all cores, the tree back on the device) and the same
     1920x1080 depth-4 frame rendered over either tree."""
     from rtgb import capi, scenes

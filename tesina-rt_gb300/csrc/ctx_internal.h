@@ -115,8 +115,9 @@ void scene_release_build(rt_scene* s);
 SceneView scene_view(const rt_scene* s);
 // Asks for just the shared memory that `blocks_per_sm` blocks of kernel fn take,
 // so that the rest of an SM's 256 KB is L1 for nodes, triangles and traversal
-// stacks; *current is the hint in force (-1: none).  Six blocks of the pooled
-// kernel fit the 100 KB size instead of 132 KB: 1.5-2 % on whole frames.
+// stacks; *current is the hint in force (-1: none).  One size more, when six blocks of
+// the pooled kernel took 132 KB instead of 100, cost 1.5-2 % of a frame; the default's
+// eight blocks take 132 KB.
 void set_carveout(const rt_ctx* c, const void* fn, int blocks_per_sm, int* current);
 // The persistent-kernel work counter for launches on stream s (nullptr if it
 // cannot be allocated).

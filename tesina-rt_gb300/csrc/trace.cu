@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_quad(RenderArgs a) {
 // 32 rays at a time whichever pixels they come from.  A pixel has one ray on
 // the way at a time, so its fixed-point sum travels with the ray, and the lane
 // that ends the path writes the pixel: no accumulation buffer to clear, add to
-// and convert afterwards (thumbnail 74 -> 66 us, 1920 x 1080 frames 0.5-1.5 %).
+// and convert afterwards (11 % of a thumbnail, 0.5-1.5 % of 1920 x 1080 frames).
 // Every ray is
 // traversed and shaded exactly as in render_pixel, so the image is
 // bit-identical to k_render's.
@@ -614,8 +614,7 @@ __global__ void __launch_bounds__(THREADS, MINB) k_render_pool_refr(RenderArgs a
 // into 32 sectors; the records of a warp go through shared memory instead, in
 // accesses of 32 neighbouring words.  Words, because the callers' arrays need
 // no more than a word's alignment.  A pitch of 20 words lets eight lanes' 16-byte
-// parts meet each bank once.  k_gen_primary, 1000 x 701: 60 -> 14 us; the whole
-// pipeline of 10k triangles 629 -> 610.
+// parts meet each bank once.  k_gen_primary, 1000 x 701: 60 -> 14 us.
 constexpr int STAGE_PITCH = 20;
 
 // The first `cnt` (at most 32) records at g to the warp's stage.

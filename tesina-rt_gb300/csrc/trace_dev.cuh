@@ -71,8 +71,8 @@ __device__ __forceinline__ bool leaf_any(const SceneView& S, const TRay& r, int3
 // leaves (at most three triangles with the usual minimum) wait for memory
 // once; the second may lie one past the scene's last record, which is
 // allocated.  Worth its registers where the kernel has them to spare: the
-// stage kernels (1000 x 701 of 10k triangles, whole pipeline 712 -> 672 us) and
-// the glass pool (12.1 -> 11.9 ms); the instanced render loses 8 % to spills.
+// stage kernels (6 % of a 1000 x 701 pipeline of 10k triangles) and the glass
+// pool (2 %); the instanced render loses 8 % to spills.
 template <bool PAIR>
 __device__ __forceinline__ void leaf_closest(const SceneView& S, const TRay& r, int32_t i,
                                              Hit& best) {
@@ -239,24 +239,21 @@ constexpr int STACK = 48;
 constexpr int32_t NO_NODE = (int32_t)0x80000000;   // below every leaf code
 
 // What bounds it: each step waits for one record (L1 / L2 latency) and the
-// lanes of a warp take different numbers of steps.  Two binary levels per
-// step against one (64 B pair records, four 128-bit loads): mid-scale frame
-// from host buffers 5.05 -> 3.10 ms, 3840 x 2160 of 17.7 M triangles 18.4-20.2
-// -> 10.3 ms, the mid-scale field under glass 25.5 -> 13.0 ms, 64 soups built
-// and rendered 17.8 -> 10.1 ms.
+// lanes of a warp take different numbers of steps; the mid-scale frame issues in
+// 65 % of the cycles with 15 of 32 lanes.  Frames over binary records, one level and
+// 64 B per step, took 1.6 to 2 times as long.
 //
 // Leaves, met directly or popped, are tested in one place, by the lanes that
 // have one together: a lane that reaches a leaf waits until the lanes with a
 // leaf are a third of those still searching (leaf_turn).  At once, a leaf step
-// had 5.2-6.8 lanes where a node step had 17-18; against that rule: 4K of 17.7
-// M triangles 12.7 -> 11.8 ms, glass 13.3 -> 12.1, 64 soups 10.1 -> 9.3, stage
-// pipeline 870 -> 712 us, thumbnail 71 -> 74 us (a fixed 4 to 16 lanes gains
-// less; setting a leaf aside and walking on loses 2-5 %).  STAY: lanes whose
-// search has ended stay for the votes, which keeps the warp together; faster
-// in the stage kernels (784 -> 712 us), the instanced render and the
-// one-path-per-lane kernels (served burst 5.5 -> 4.8 ms), slower in the pooled
-// ones; there the leaves wait until they are half of the lanes (a third against
-// that: instances 1.855 -> 1.849 ms, stage pipeline 517 -> 515 us).
+// had 5.2-6.8 lanes where a node step had 17-18: 7-9 % of large frames, 18 % of
+// the stage pipeline (a fixed 4 to 16 lanes gains less; setting a leaf aside and
+// walking on loses 2-5 %; small frames lose 4 % and run by four lanes).  STAY: lanes
+// whose search has ended stay for the votes, which keeps the warp together; 9 %
+// faster in the stage kernels, 13 % in the one-path-per-lane kernels, faster too in
+// the instanced render, slower in the pooled ones; there the leaves wait until they
+// are half of the lanes (a third: instances 1.855 -> 1.849 ms, stage pipeline 517 ->
+// 515 us).
 template <bool STAY>
 __device__ __forceinline__ bool leaf_turn(unsigned group, int32_t next, bool& ended) {
     if (STAY) {
@@ -276,10 +273,8 @@ __device__ __forceinline__ bool leaf_turn(unsigned group, int32_t next, bool& en
 // instructions, and each branch in it costs more than the selects that take
 // its place.  The rejections of mt(), a leaf's hit, an any-hit visit and the
 // pushes' conditions are selects, and the kind is a template argument, so that
-// ordinary rays' code has none of its tests.  Together: mid-scale frame 2.87 ->
-// 2.51 ms, 4K of 17.7 M triangles 11.3 -> 9.7, glass 11.3 -> 9.3, 64 soups 7.8
-// -> 6.8, instances 2.04 -> 1.86, 10k-triangle frame 365 -> 322 us, thumbnail
-// 66 -> 52.  (Pushes that store always and move `sp` by the condition lose 4 %.)
+// ordinary rays' code has none of its tests: together 9-21 % of a frame.  (Pushes
+// that store always and move `sp` by the condition lose 4 %.)
 // WIDE: `flat` tells that the search was given up at a flat box.
 template <bool STAY, bool PAIR, SearchKind KIND>
 __device__ __forceinline__ Hit closest_search(const SceneView& S, const BvhHeader& H, const TRay& r,
@@ -388,9 +383,8 @@ static __device__ Hit closest_hit(const SceneView& S, const BvhHeader& H, const 
 
 // Whether anything blocks the ray.  tMax does not shrink, so the order of
 // the visits does not matter to the answer; of the children that the ray meets
-// it enters the one it crosses for longest, the likeliest to hold a blocker.
-// Against the last child first: 64 soups 9.29 -> 8.97 ms, glass 11.9 -> 11.7,
-// 4K of 17.7 M triangles 11.75 -> 11.60 (the nearest child first: 13.9).
+// it enters the one it crosses for longest, the likeliest to hold a blocker: 1-3 %
+// of a frame against the last child first, 20 % against the nearest first.
 template <bool STAY, bool PAIR, SearchKind KIND>
 __device__ __forceinline__ bool any_search(const SceneView& S, const BvhHeader& H, const TRay& r,
                                            float tmax, uint32_t* status, bool& flat) {
