@@ -10,6 +10,7 @@ import pytest
 import torch
 
 from rtgb import abi, capi, scenes
+from test_gpu_trace import _render_both
 from test_gpu_wide import _grid_scene, _samples
 
 pytestmark = pytest.mark.gpu
@@ -119,6 +120,20 @@ def test_bounds_and_origins_at_infinity(ctx, orc):
     smp["inv_dir"][neg, :3] = np.float32(1) / smp["dir"][neg, :3]
     smp["tmin"][neg] = -inf
     assert compare_both_sides(ctx, orc, _blocks(DIRS[2]), smp) > 1000
+
+
+@pytest.mark.parametrize("light_dir", DIRS)
+@pytest.mark.parametrize("w,h", [(150, 97), (401, 397)])
+def test_frames_under_parallel_lights(ctx, orc, light_dir, w, h):
+    """The fused renders, on both sides of the line: every pixel of a field of
+    blocks with mirrors, lit along an axis or in a plane of two."""
+    sc = _blocks(light_dir)
+    sc.mats["reflectiveness"] = 0.4
+    cam = scenes.camera((7.0, 26.0, -9.0), (7.0, 3.0, 7.0), aspect=w / h)
+    img, _, st, rimg, rst, _, _ = _render_both(ctx, orc, sc, cam, w, h, 3)
+    assert np.array_equal(img, rimg)
+    assert (st[0], st[1], st[2], st[3]) == (rst.primary_rays, rst.secondary_rays, rst.shadow_rays, rst.hits)
+    assert rst.hits > 0 and ctx.device_status() == 0
 
 
 @pytest.mark.parametrize("what", ["trace", "shadow"])
